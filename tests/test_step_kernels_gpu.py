@@ -1,0 +1,34 @@
+"""Kernels chosen by size: each at the edges of its range against float64."""
+import pytest
+import torch
+
+from rvllm_b200.kernels import get_library
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    return get_library("cuda:0")
+
+
+def rel_err(a, ref):
+    return float((a.double().cpu() - ref).abs().max() / ref.abs().max().clamp(min=1e-30))
+
+
+@pytest.mark.parametrize("N,Kd", [(17, 32), (130, 512), (300, 516), (64, 1028), (129, 2052), (40, 30), (5000, 96), (16, 4100)])
+def test_gemm_f32_rows_do_not_depend_on_the_batch(K, N, Kd):
+    """Few rows take the streaming kernel (in six sizes), more the tiles with K over 1, 2 or 4 CTAs: one order of summation, so
+    the same bits; K with short last segments, fewer segments than 16, and rows that are not whole 16-byte words."""
+    torch.manual_seed(N + Kd)
+    x = torch.randn(300, Kd, device="cuda")
+    w = torch.randn(N, Kd, device="cuda")
+    b, r = torch.randn(N, device="cuda"), torch.randn(300, N, device="cuda")
+    ref = x.double().cpu() @ w.double().cpu().t() + b.double().cpu() + r.double().cpu()
+    whole = K.linear(x, w, b, r)
+    # a segment is a chain of at most K / 16 + 32 roundings of 2^-24 each, on sums of about sqrt(K): far below 3e-6 of the largest value
+    assert rel_err(whole, ref) < 3e-6
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 128, 129):
+        assert torch.equal(K.linear(x[:M].contiguous(), w, b, r[:M].contiguous()), whole[:M]), M
+    shifted = torch.empty(5 * Kd + 1, device="cuda")[1:].view(5, Kd).copy_(x[:5])        # not on a 16-byte boundary
+    assert torch.equal(K.linear(shifted, w, b, r[:5].contiguous()), whole[:5])
