@@ -146,6 +146,25 @@ __device__ __forceinline__ float rv_load_param(const void* p, int dtype, int i) 
                                  : __bfloat162float(((const __nv_bfloat16*)p)[i]);
 }
 
+// Four neighbours of a row in either type as float; i a multiple of 4, the pointer aligned to four elements.
+__device__ __forceinline__ float4 rv_load4(const void* p, int dtype, size_t i) {
+    if (dtype == RV_DTYPE_F32) return *reinterpret_cast<const float4*>((const float*)p + i);
+    const uint2 u = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)p + i);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void rv_store4(void* p, int dtype, size_t i, float4 v) {
+    if (dtype == RV_DTYPE_F32) {
+        *reinterpret_cast<float4*>((float*)p + i) = v;
+    } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        uint2 u;
+        u.x = *reinterpret_cast<const uint32_t*>(&lo); u.y = *reinterpret_cast<const uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>((__nv_bfloat16*)p + i) = u;
+    }
+}
+
 __device__ __forceinline__ float rv_warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

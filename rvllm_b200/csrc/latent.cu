@@ -28,37 +28,49 @@ __device__ __forceinline__ void lt_store(void* p, int dtype, size_t i, float v) 
     else ((__nv_bfloat16*)p)[i] = __float2bfloat16_rn(v);
 }
 
-// queries of one token: per head dq plain elements, then dr rotated ones (dr - half items: a pair or a single element)
+// queries of one token: per head dq plain elements (in words of four where `vec`), then dr rotated ones (dr - half items: a pair
+// or a single element).  `first` and `step`: this thread's items.
 __device__ __forceinline__ void lt_queries(const void* __restrict__ proj, int in_dtype, size_t row, int t, const float* cs, const float* sn,
                                            int half, int halves, void* __restrict__ q_plain, void* __restrict__ q_row, int out_dtype,
-                                           int nh, int dq, int dr, int R) {
-    const int per_head = dq + dr - half, D = R + dr;
-    for (int item = threadIdx.x; item < nh * per_head; item += blockDim.x) {
-        const int h = item / per_head, i = item - h * per_head;
-        const size_t src = row + (size_t)h * (dq + dr);
-        if (i < dq) {
-            lt_store(q_plain, out_dtype, ((size_t)t * nh + h) * dq + i, lt_load(proj, in_dtype, src + i));
-            continue;
-        }
-        const int k = i - dq;
-        const size_t dst = ((size_t)t * nh + h) * D + R;
+                                           int nh, int dq, int dr, int R, int vec, int first, int step) {
+    const int D = R + dr, width = vec ? 4 : 1, words = dq / width, turned = dr - half;
+    for (int item = first; item < nh * words; item += step) {
+        const int h = item / words, i = (item - h * words) * width;
+        const size_t src = row + (size_t)h * (dq + dr) + i, dst = ((size_t)t * nh + h) * dq + i;
+        if (vec) rv_store4(q_plain, out_dtype, dst, rv_load4(proj, in_dtype, src));
+        else lt_store(q_plain, out_dtype, dst, lt_load(proj, in_dtype, src));
+    }
+    for (int item = first; item < nh * turned; item += step) {
+        const int h = item / turned, k = item - h * turned;
+        const size_t src = row + (size_t)h * (dq + dr) + dq, dst = ((size_t)t * nh + h) * D + R;
         if (k < half) {
             const int ia = halves ? k : 2 * k, ib = halves ? k + half : 2 * k + 1;
-            const float a = lt_load(proj, in_dtype, src + dq + ia), b = lt_load(proj, in_dtype, src + dq + ib);
+            const float a = lt_load(proj, in_dtype, src + ia), b = lt_load(proj, in_dtype, src + ib);
             const float c = cs[k], s = sn[k];
             lt_store(q_row, out_dtype, dst + ia, a * c - b * s);
             lt_store(q_row, out_dtype, dst + ib, b * c + a * s);
         } else {
             const int j = k + half;
-            lt_store(q_row, out_dtype, dst + j, lt_load(proj, in_dtype, src + dq + j));
+            lt_store(q_row, out_dtype, dst + j, lt_load(proj, in_dtype, src + j));
         }
     }
+}
+static inline int lt_vec(const void* proj, int in_dtype, size_t row_elements, const void* q_plain, int out_dtype, int dq, int dr) {
+    const uintptr_t im = in_dtype == RV_DTYPE_F32 ? 15 : 7, om = out_dtype == RV_DTYPE_F32 ? 15 : 7;
+    return dq % 4 == 0 && dr % 4 == 0 && row_elements % 4 == 0 && !(reinterpret_cast<uintptr_t>(proj) & im) && !(reinterpret_cast<uintptr_t>(q_plain) & om);
+}
+// Blocks that share a token's queries: a step of few tokens is bound by the chain of one block (eight tokens of 32 heads: 10.8 us
+// with one, 3.4 with these), one of many fills the SMs anyway.
+static inline int lt_query_blocks(int n_tokens, int nh, int dq) {
+    if (n_tokens >= 4 * rv_sm_count()) return 1;
+    const int want = (nh * dq / 4 + 255) / 256;
+    return want < 1 ? 1 : (want > 16 ? 16 : want);
 }
 
 __global__ void __launch_bounds__(256)
 latent_queries_kernel(const void* __restrict__ q, int in_dtype, const int* __restrict__ positions, const float* __restrict__ cos_t,
                       const float* __restrict__ sin_t, int rot, int table_rows, int halves, void* __restrict__ q_plain,
-                      void* __restrict__ q_row, int out_dtype, int nh, int dq, int dr, int R) {
+                      void* __restrict__ q_row, int out_dtype, int nh, int dq, int dr, int R, int vec) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     const int t = blockIdx.x, half = rot >> 1;
@@ -67,16 +79,17 @@ latent_queries_kernel(const void* __restrict__ q, int in_dtype, const int* __res
     if (pos >= table_rows) pos = table_rows - 1;      // the host refuses such positions; never read outside
     const float* cs = cos_t ? cos_t + (size_t)pos * half : nullptr;
     const float* sn = sin_t ? sin_t + (size_t)pos * half : nullptr;
-    lt_queries(q, in_dtype, (size_t)t * nh * (dq + dr), t, cs, sn, half, halves, q_plain, q_row, out_dtype, nh, dq, dr, R);
+    lt_queries(q, in_dtype, (size_t)t * nh * (dq + dr), t, cs, sn, half, halves, q_plain, q_row, out_dtype, nh, dq, dr, R, vec,
+               blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
 }
 
-// One block per token.
+// grid (tokens, 1 + blocks of the queries): block 0 of a token forms the latent row and the gate, the others its queries.
 __global__ void __launch_bounds__(256)
 latent_prepare_kernel(const void* __restrict__ proj, int in_dtype, int row_stride, const void* __restrict__ c_gamma, int gamma_dtype,
                       const int* __restrict__ positions, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                       int rot, int table_rows, const int* __restrict__ slot_mapping, void* __restrict__ cache,
                       void* __restrict__ q_plain, void* __restrict__ q_row, int out_dtype, float* __restrict__ gate_out,
-                      int nh, int dq, int dr, int R, float eps, int write_kv, int halves) {
+                      int nh, int dq, int dr, int R, float eps, int write_kv, int halves, int vec) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     __shared__ float scratch[33];
@@ -84,16 +97,21 @@ latent_prepare_kernel(const void* __restrict__ proj, int in_dtype, int row_strid
     const size_t row = (size_t)t * row_stride;
     const int qw = nh * (dq + dr), D = R + dr;
     const size_t c0 = row + qw;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < R; i += blockDim.x) { const float v = lt_load(proj, in_dtype, c0 + i); ss = fmaf(v, v, ss); }
-    ss = rv_block_sum(ss, scratch);
-    const float rc = 1.0f / sqrtf(ss / (float)R + eps);
     int pos = positions[t];
     if (pos < 0) pos = 0;
     if (pos >= table_rows) pos = table_rows - 1;      // the host refuses such positions; never read outside
     const int half = rot >> 1;
     const float* cs = cos_t ? cos_t + (size_t)pos * half : nullptr;
     const float* sn = sin_t ? sin_t + (size_t)pos * half : nullptr;
+    if (blockIdx.y > 0) {
+        lt_queries(proj, in_dtype, row, t, cs, sn, half, halves, q_plain, q_row, out_dtype, nh, dq, dr, R, vec,
+                   (blockIdx.y - 1) * blockDim.x + threadIdx.x, (gridDim.y - 1) * blockDim.x);
+        return;
+    }
+    float ss = 0.f;
+    for (int i = threadIdx.x; i < R; i += blockDim.x) { const float v = lt_load(proj, in_dtype, c0 + i); ss = fmaf(v, v, ss); }
+    ss = rv_block_sum(ss, scratch);
+    const float rc = 1.0f / sqrtf(ss / (float)R + eps);
     const int slot = write_kv ? slot_mapping[t] : -1;
     if (slot >= 0) {
         const size_t d0 = (size_t)slot * D;                      // one plane, one kv head: a slot is a row
@@ -113,7 +131,6 @@ latent_prepare_kernel(const void* __restrict__ proj, int in_dtype, int row_strid
             }
         }
     }
-    lt_queries(proj, in_dtype, row, t, cs, sn, half, halves, q_plain, q_row, out_dtype, nh, dq, dr, R);
     if (gate_out)
         for (int h = threadIdx.x; h < nh; h += blockDim.x) {
             const float g = lt_load(proj, in_dtype, row + qw + D + h);
@@ -131,9 +148,9 @@ RV_EXPORT int rv_latent_prepare(const void* proj, int in_dtype, int row_stride, 
     if ((in_dtype | gamma_dtype | out_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (n_tokens == 0) return RV_OK;
     if (!cos_t || !sin_t) rot = 0;
-    RV_LAUNCH_ST = rv_launch(latent_prepare_kernel, dim3(n_tokens), dim3(256), 0, stream, proj, in_dtype, row_stride, c_gamma,
+    RV_LAUNCH_ST = rv_launch(latent_prepare_kernel, dim3(n_tokens, 1 + lt_query_blocks(n_tokens, nh, dq)), dim3(256), 0, stream, proj, in_dtype, row_stride, c_gamma,
                              gamma_dtype, positions, cos_t, sin_t, rot, table_rows, slot_mapping, cache, q_plain, q_row, out_dtype,
-                             gate_out, nh, dq, dr, R, eps, write_kv, halves);
+                             gate_out, nh, dq, dr, R, eps, write_kv, halves, lt_vec(proj, in_dtype, (size_t)row_stride, q_plain, out_dtype, dq, dr));
     return rv_launch_status();
 }
 
@@ -376,8 +393,9 @@ RV_EXPORT int rv_latent_queries(const void* q, int in_dtype, const int* position
                                  (const float*)q, positions, cos_t, sin_t, rot, table_rows, q_plain, q_row, out_dtype, nh, dq, dr, R, total);
         return rv_launch_status();
     }
-    RV_LAUNCH_ST = rv_launch(latent_queries_kernel, dim3(n_tokens), dim3(256), 0, stream, q, in_dtype, positions, cos_t, sin_t, rot,
-                             table_rows, halves, q_plain, q_row, out_dtype, nh, dq, dr, R);
+    RV_LAUNCH_ST = rv_launch(latent_queries_kernel, dim3(n_tokens, lt_query_blocks(n_tokens, nh, dq)), dim3(256), 0, stream, q, in_dtype, positions,
+                             cos_t, sin_t, rot, table_rows, halves, q_plain, q_row, out_dtype, nh, dq, dr, R,
+                             lt_vec(q, in_dtype, (size_t)nh * (dq + dr), q_plain, out_dtype, dq, dr));
     return rv_launch_status();
 }
 

@@ -98,12 +98,75 @@ stream_add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const
         so_store(rounded, rounded_dtype, base + i, x[base + i] * r * rv_load_param(gamma, gamma_dtype, i));
 }
 
+// The same with the row in registers, four columns a thread and access: x and y are read once, gamma before
+// griddepcontrol.wait (four rows of 4,096 columns in a decode step: 13.2 -> 2.3 us).
+template <int NV>
+__global__ void __launch_bounds__(512)
+stream_add_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const void* __restrict__ gamma, int gamma_dtype,
+                           void* __restrict__ rounded, int rounded_dtype, int cols, float eps) {
+    rv_pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const size_t base = (size_t)blockIdx.x * cols;
+    const int quads = cols >> 2;
+    float4 v[NV], g[NV], b[NV];
+    if (gamma) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i < quads) g[j] = rv_load4(gamma, gamma_dtype, 4 * (size_t)i);
+        }
+    }
+    rv_pdl_wait();
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j] = b[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < quads) {
+            v[j] = reinterpret_cast<const float4*>(x + base)[i];
+            if (y) b[j] = reinterpret_cast<const float4*>(y + base)[i];
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i >= quads) continue;
+        if (y) {
+            v[j].x += b[j].x; v[j].y += b[j].y; v[j].z += b[j].z; v[j].w += b[j].w;
+            reinterpret_cast<float4*>(x + base)[i] = v[j];
+        }
+        ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        if (rounded && !gamma) rv_store4(rounded, rounded_dtype, base + 4 * (size_t)i, v[j]);
+    }
+    if (!rounded || !gamma) return;
+    ss = rv_block_sum(ss, scratch);
+    const float r = 1.0f / sqrtf(ss / (float)cols + eps);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < quads)
+            rv_store4(rounded, rounded_dtype, base + 4 * (size_t)i,
+                      make_float4(v[j].x * r * g[j].x, v[j].y * r * g[j].y, v[j].z * r * g[j].z, v[j].w * r * g[j].w));
+    }
+}
+
+static inline bool so_aligned(const void* p, int dtype) { return (reinterpret_cast<uintptr_t>(p) & (dtype == RV_DTYPE_F32 ? 15 : 7)) == 0; }
+
 RV_EXPORT int rv_stream_add_norm(float* x, const float* y, const void* gamma, int gamma_dtype, void* rounded, int rounded_dtype,
                                  int rows, int cols, float eps, cudaStream_t stream) {
     if (rows < 0 || cols <= 0) return RV_ERR_BAD_SIZE;
     if ((gamma_dtype | rounded_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (rows == 0 || (!y && !rounded)) return RV_OK;
-    RV_LAUNCH_ST = rv_launch(stream_add_norm_kernel, dim3(rows), dim3(cols >= 1024 ? 256 : 128), 0, stream, x, y, gamma, gamma_dtype,
+    auto kernel = stream_add_norm_kernel;
+    int threads = cols >= 1024 ? 256 : 128;
+    if (cols % 4 == 0 && cols <= 512 * 4 * 8 && so_aligned(x, RV_DTYPE_F32) && so_aligned(y, RV_DTYPE_F32) &&
+        so_aligned(gamma, gamma_dtype) && so_aligned(rounded, rounded_dtype)) {
+        threads = cols > 1024 ? 512 : (cols > 512 ? 256 : 128);
+        const int nv = (cols / 4 + threads - 1) / threads;
+        kernel = nv <= 1 ? stream_add_norm_vec_kernel<1> : (nv <= 2 ? stream_add_norm_vec_kernel<2>
+                                                         : (nv <= 4 ? stream_add_norm_vec_kernel<4> : stream_add_norm_vec_kernel<8>));
+    }
+    RV_LAUNCH_ST = rv_launch(kernel, dim3(rows), dim3(threads), 0, stream, x, y, gamma, gamma_dtype,
                              rounded, rounded_dtype, cols, eps);
     return rv_launch_status();
 }
@@ -161,10 +224,30 @@ __global__ void scaled_sum_kernel(const float* a, float sa, const float* __restr
         out[i] = a ? fmaf(sa, a[i], sb * b[i]) : sb * b[i];
 }
 
+__global__ void scaled_sum_vec_kernel(const float4* a, float sa, const float4* __restrict__ b, float sb, float4* out, size_t quads) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (size_t)gridDim.x * blockDim.x) {
+        const float4 q = b[i];
+        float4 r = make_float4(sb * q.x, sb * q.y, sb * q.z, sb * q.w);
+        if (a) {
+            const float4 p = a[i];
+            r = make_float4(fmaf(sa, p.x, r.x), fmaf(sa, p.y, r.y), fmaf(sa, p.z, r.z), fmaf(sa, p.w, r.w));
+        }
+        out[i] = r;
+    }
+}
+
 RV_EXPORT int rv_scaled_sum(const float* a, float sa, const float* b, float sb, float* out, long long total, cudaStream_t stream) {
     if (total < 0) return RV_ERR_BAD_SIZE;
     if (total == 0) return RV_OK;
     const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (total % 4 == 0 && so_aligned(a, RV_DTYPE_F32) && so_aligned(b, RV_DTYPE_F32) && so_aligned(out, RV_DTYPE_F32)) {
+        const long long quads = total / 4;
+        const int vec_blocks = (int)((quads + 255) / 256 < 148 * 8 ? (quads + 255) / 256 : 148 * 8);
+        RV_LAUNCH_ST = rv_launch(scaled_sum_vec_kernel, dim3(vec_blocks), dim3(256), 0, stream, (const float4*)a, sa, (const float4*)b, sb, (float4*)out, (size_t)quads);
+        return rv_launch_status();
+    }
     RV_LAUNCH_ST = rv_launch(scaled_sum_kernel, dim3(blocks), dim3(256), 0, stream, a, sa, b, sb, out, (size_t)total);
     return rv_launch_status();
 }
@@ -181,6 +264,26 @@ __global__ void act_mul_clamp_kernel(const void* __restrict__ gate_up, int in_dt
     }
 }
 
+// inter % 4 == 0 and aligned pointers: four columns a thread, 32-bit indices (2,048 rows of 14,336: 91 -> 48 us)
+__global__ void __launch_bounds__(256)
+act_mul_clamp_vec_kernel(const void* __restrict__ gate_up, int in_dtype, void* __restrict__ out, int out_dtype,
+                         int inter, float limit, float alpha) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    const size_t row = blockIdx.y;
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4; c < inter; c += gridDim.x * blockDim.x * 4) {
+        const float4 gv = rv_load4(gate_up, in_dtype, row * 2 * inter + c), uv = rv_load4(gate_up, in_dtype, row * 2 * inter + inter + c);
+        const float gs[4] = {gv.x, gv.y, gv.z, gv.w}, us[4] = {uv.x, uv.y, uv.z, uv.w};
+        float r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float g = fminf(gs[j], limit), u = fminf(fmaxf(us[j], -limit), limit);
+            r[j] = g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
+        }
+        rv_store4(out, out_dtype, row * inter + c, make_float4(r[0], r[1], r[2], r[3]));
+    }
+}
+
 RV_EXPORT int rv_act_mul_clamp(const void* gate_up, int in_dtype, void* out, int out_dtype, int rows, int inter, float limit,
                                float alpha, cudaStream_t stream) {
     if (rows < 0 || inter <= 0 || !(limit > 0.f)) return RV_ERR_BAD_SIZE;
@@ -188,6 +291,11 @@ RV_EXPORT int rv_act_mul_clamp(const void* gate_up, int in_dtype, void* out, int
     if (rows == 0) return RV_OK;
     const size_t total = (size_t)rows * inter;
     const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (inter % 4 == 0 && rows <= 65535 && so_aligned(gate_up, in_dtype) && so_aligned(out, out_dtype)) {
+        RV_LAUNCH_ST = rv_launch(act_mul_clamp_vec_kernel, dim3((inter / 4 + 255) / 256, rows), dim3(256), 0, stream, gate_up, in_dtype, out, out_dtype,
+                                 inter, limit, alpha);
+        return rv_launch_status();
+    }
     RV_LAUNCH_ST = rv_launch(act_mul_clamp_kernel, dim3(blocks), dim3(256), 0, stream, gate_up, in_dtype, out, out_dtype, inter, total,
                              limit, alpha);
     return rv_launch_status();
@@ -237,6 +345,22 @@ __global__ void dynamic_tanh_kernel(const void* __restrict__ x, int x_dtype, con
         const int c = (int)(i % cols);
         so_store(out, out_dtype, i, fmaf(tanhf(a * so_load(x, x_dtype, i)), w[c], b[c]));
     }
+}
+
+// cols % 4 == 0 and aligned pointers: four columns a thread; alpha, w and b are read before griddepcontrol.wait.
+__global__ void dynamic_tanh_vec_kernel(const void* __restrict__ x, int x_dtype, const float* __restrict__ alpha, const float* __restrict__ w,
+                                        const float* __restrict__ b, void* __restrict__ out, int out_dtype, int cols) {
+    rv_pdl_launch_dependents();
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const size_t at = (size_t)blockIdx.y * cols + c;
+    float a = 0.f;
+    float4 wv = make_float4(0.f, 0.f, 0.f, 0.f), bv = wv;
+    if (c < cols) { a = alpha[0]; wv = *reinterpret_cast<const float4*>(w + c); bv = *reinterpret_cast<const float4*>(b + c); }
+    rv_pdl_wait();
+    if (c >= cols) return;
+    const float4 v = rv_load4(x, x_dtype, at);
+    rv_store4(out, out_dtype, at, make_float4(fmaf(tanhf(a * v.x), wv.x, bv.x), fmaf(tanhf(a * v.y), wv.y, bv.y),
+                                              fmaf(tanhf(a * v.z), wv.z, bv.z), fmaf(tanhf(a * v.w), wv.w, bv.w)));
 }
 
 // x and y float [rows, cols]; `next` (alpha2, w2, b2) optional.  vec: cols % 4 == 0 and 16-byte aligned float pointers.
@@ -293,6 +417,10 @@ RV_EXPORT int rv_dynamic_tanh(const void* x, int x_dtype, const float* alpha, co
     if ((x_dtype | out_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (rows == 0) return RV_OK;
     const size_t total = (size_t)rows * cols;
+    if (cols % 4 == 0 && rows <= 65535 && so_aligned(x, x_dtype) && so_aligned(w, RV_DTYPE_F32) && so_aligned(b, RV_DTYPE_F32) && so_aligned(out, out_dtype)) {
+        RV_LAUNCH_ST = rv_launch(dynamic_tanh_vec_kernel, dim3((cols / 4 + 255) / 256, rows), dim3(256), 0, stream, x, x_dtype, alpha, w, b, out, out_dtype, cols);
+        return rv_launch_status();
+    }
     RV_LAUNCH_ST = rv_launch(dynamic_tanh_kernel, dim3(so_blocks(total)), dim3(256), 0, stream, x, x_dtype, alpha, w, b, out, out_dtype,
                              cols, total);
     return rv_launch_status();

@@ -72,6 +72,57 @@ kv_prepare_kernel(const void* __restrict__ proj, int p_dtype, int p_stride, cons
     }
 }
 
+// The same in words of four elements, the q, key and value parts of a row side by side in blocks of their own (grid.y: blocks of
+// 1,024 columns of q, then the keys, then the values): a decode step's few rows are bound by the chain of one block (four
+// rows of 32 + 8 heads of 128: 13.2 -> 2.7 us).
+template <typename TC>
+__global__ void __launch_bounds__(256)
+kv_prepare_vec_kernel(const void* __restrict__ proj, int p_dtype, int p_stride, const int* __restrict__ slot_mapping,
+                      TC* __restrict__ cache, void* __restrict__ q_out, int q_dtype, int nh, int nkv, int hd, int vd, int page_size,
+                      float eps, int norm_v, int q_blocks) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    constexpr int cdt = sizeof(TC) == 4 ? RV_DTYPE_F32 : RV_DTYPE_BF16;
+    const int t = blockIdx.x;
+    const size_t row = (size_t)t * p_stride;
+    const int qw = nh * hd, kw = nkv * hd;
+    if ((int)blockIdx.y < q_blocks) {
+        const int i = ((int)blockIdx.y * 256 + threadIdx.x) * 4;
+        if (i < qw) rv_store4(q_out, q_dtype, (size_t)t * qw + i, rv_load4(proj, p_dtype, row + i));
+        return;
+    }
+    const int slot = slot_mapping[t];
+    if (slot < 0) return;
+    const size_t page_elems = (size_t)nkv * page_size * (hd + vd);
+    TC* page = cache + (size_t)(slot / page_size) * page_elems;
+    const int off = slot % page_size;
+    if ((int)blockIdx.y == q_blocks) {
+        for (int i = threadIdx.x * 4; i < kw; i += 1024) {
+            const int g = i / hd, e = i - g * hd;
+            rv_store4(page, cdt, ((size_t)g * page_size + off) * hd + e, rv_load4(proj, p_dtype, row + qw + i));
+        }
+        return;
+    }
+    TC* vpage = page + (size_t)nkv * page_size * hd;
+    const int lane = threadIdx.x & 31;
+    for (int g = threadIdx.x >> 5; g < nkv; g += 8) {
+        const size_t vb = row + qw + kw + (size_t)g * vd;
+        float r = 1.0f;
+        if (norm_v) {
+            float ss = 0.f;
+            for (int e = lane * 4; e < vd; e += 128) {
+                const float4 v = rv_load4(proj, p_dtype, vb + e);
+                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            }
+            r = 1.0f / sqrtf(rv_warp_sum(ss) / (float)vd + eps);
+        }
+        for (int e = lane * 4; e < vd; e += 128) {
+            const float4 v = rv_load4(proj, p_dtype, vb + e);
+            rv_store4(vpage, cdt, ((size_t)g * page_size + off) * vd + e, make_float4(v.x * r, v.y * r, v.z * r, v.w * r));
+        }
+    }
+}
+
 RV_EXPORT int rv_kv_prepare(const void* proj, int p_dtype, int p_stride, const int* slot_mapping, void* cache, int cache_dtype,
                             void* q_out, int q_dtype, int n_tokens, int nh, int nkv, int hd, int vd, int page_size, float eps,
                             int norm_v, int write_kv, cudaStream_t stream) {
@@ -79,6 +130,19 @@ RV_EXPORT int rv_kv_prepare(const void* proj, int p_dtype, int p_stride, const i
         return RV_ERR_BAD_SIZE;
     if ((p_dtype | q_dtype | cache_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (n_tokens == 0) return RV_OK;
+    const uintptr_t pm = p_dtype == RV_DTYPE_F32 ? 15 : 7, qm = q_dtype == RV_DTYPE_F32 ? 15 : 7, cm = cache_dtype == RV_DTYPE_F32 ? 15 : 7;
+    const int q_blocks = (nh * hd + 1023) / 1024;
+    if (hd % 4 == 0 && vd % 4 == 0 && p_stride % 4 == 0 && q_blocks < 60000 && !(reinterpret_cast<uintptr_t>(proj) & pm) &&
+        !(reinterpret_cast<uintptr_t>(q_out) & qm) && !(reinterpret_cast<uintptr_t>(cache) & cm)) {
+        const dim3 grid(n_tokens, q_blocks + (write_kv ? 2 : 0));
+        if (cache_dtype == RV_DTYPE_F32)
+            RV_LAUNCH_ST = rv_launch(kv_prepare_vec_kernel<float>, grid, dim3(256), 0, stream, proj, p_dtype, p_stride, slot_mapping,
+                                     (float*)cache, q_out, q_dtype, nh, nkv, hd, vd, page_size, eps, norm_v, q_blocks);
+        else
+            RV_LAUNCH_ST = rv_launch(kv_prepare_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, proj, p_dtype, p_stride, slot_mapping,
+                                     (__nv_bfloat16*)cache, q_out, q_dtype, nh, nkv, hd, vd, page_size, eps, norm_v, q_blocks);
+        return rv_launch_status();
+    }
     if (cache_dtype == RV_DTYPE_F32)
         RV_LAUNCH_ST = rv_launch(kv_prepare_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, proj, p_dtype, p_stride, slot_mapping,
                                  (float*)cache, q_out, q_dtype, nh, nkv, hd, vd, page_size, eps, norm_v, write_kv);

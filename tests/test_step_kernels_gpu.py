@@ -32,3 +32,24 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch(K, N, Kd):
         assert torch.equal(K.linear(x[:M].contiguous(), w, b, r[:M].contiguous()), whole[:M]), M
     shifted = torch.empty(5 * Kd + 1, device="cuda")[1:].view(5, Kd).copy_(x[:5])        # not on a 16-byte boundary
     assert torch.equal(K.linear(shifted, w, b, r[:5].contiguous()), whole[:5])
+
+
+@pytest.mark.parametrize("rows,cols,y_dtype", [(3, 4, torch.float32), (2, 1028, torch.bfloat16), (5, 4096, torch.float32), (2, 16384, torch.float32),
+                                               (2, 16388, torch.bfloat16), (3, 130, torch.float32)])
+def test_stream_norms_in_words_of_four(K, rows, cols, y_dtype):
+    """Rows in registers (whole words of four, up to 16,384 columns) and rows read again: the same sums and norms."""
+    torch.manual_seed(cols)
+    y = torch.randn(rows, cols, device="cuda").to(y_dtype)
+    x = torch.randn(rows, cols, device="cuda")
+    g, g2 = torch.randn(cols, device="cuda"), torch.randn(cols, device="cuda").bfloat16()
+    rms = lambda v, w, e: v / (v.square().mean(-1, keepdim=True) + e).sqrt() * w.double().cpu()      # noqa: E731
+    new = x.double().cpu() + rms(y.double().cpu(), g, 1e-5)
+    got, nxt = K.residual_rmsnorm(y, g, 1e-5, x.clone(), torch.float32, next_norm=(g2, 1e-6))
+    # float sums of `cols` squares in a tree: a few 2^-24 times log2(cols)
+    assert rel_err(got, new) < 2e-6 and rel_err(nxt, rms(new, g2, 1e-6)) < 4e-6
+    got, same = K.residual_rmsnorm(y, g, 1e-5, None, torch.bfloat16)
+    assert rel_err(got, rms(y.double().cpu(), g, 1e-5)) < 2e-6 and torch.equal(same, got.bfloat16())
+    if y_dtype == torch.float32:
+        got, nxt = K.stream_add_norm(x.clone(), y, (g, 1e-5), torch.float32)
+        want = x.double().cpu() + y.double().cpu()
+        assert rel_err(got, want) < 2e-7 and rel_err(nxt, rms(want, g, 1e-5)) < 4e-6
