@@ -17,7 +17,7 @@
 //
 // Measured against one 64 x 64 tile kernel for every M (4 x 4 outputs a thread), which this replaced: 3 rows of 3584 x 18944
 // 2,120 -> 72 us (3.8 TB/s), of 37888 x 3584 836 -> 105 us (5.2 TB/s), of 152064 x 3584 3,235 -> 349 us (6.2 TB/s); 433 rows of
-// 37888 x 3584 5,381 -> 3,560 us (33 TFLOP/s); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
+// 37888 x 3584 5,381 -> 3,392 us (35 TFLOP/s); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
 //
 // Shapes of the layer's five products: v3/crates/rvllm-runtime/src/layer_exec.rs:240-266,
 // 433-444, 478-488, 511-522 of the reference (which calls cuBLASLt there); bias as a row
@@ -165,18 +165,20 @@ __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-// blockIdx.x = column tile * splits + part (the parts of a tile form a cluster), blockIdx.y = row tile.  Part p of S walks
-// the segments of groups p * 4 / S .. (p + 1) * 4 / S - 1.
+// blockIdx.x = tile * splits + part (the parts of a tile form a cluster), tile = column tile * row tiles + row tile: the CTAs
+// that share rows of W run side by side (column tiles first, W came from memory once per row tile, and the way of
+// a tile from there was longer than the work on one).  Part p of S walks the segments of groups p * 4 / S .. (p + 1) * 4 / S - 1.
 template <bool VEC>
 __global__ void __launch_bounds__(256, 1)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias,
                      int bias_dtype, const float* __restrict__ residual, float* __restrict__ out,
-                     int M, int N, int K, int splits) {
-    extern __shared__ __align__(16) float smem[];           // two stages of xs | ws [TK][TPITCH]; later a part's sums [128][TPITCH]
+                     int M, int N, int K, int splits, int row_tiles) {
+    extern __shared__ __align__(128) float smem[];           // two stages of xs | ws [TK][TPITCH]; later a part's sums [128][TPITCH]
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int part = blockIdx.x % splits, m0 = blockIdx.y * TB, n0 = (blockIdx.x / splits) * TB;
+    const int part = blockIdx.x % splits, tile = blockIdx.x / splits;
+    const int m0 = (tile % row_tiles) * TB, n0 = (tile / row_tiles) * TB;
     // a warp covers 32 x 64 outputs (4 x 8 lanes of 8 x 8, as two halves of 4 each way)
     const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;
     const int am = wm + (lane >> 3) * 4, bn = wn + (lane & 7) * 4;       // and +16 rows, +32 columns
@@ -376,22 +378,22 @@ RV_EXPORT int rv_gemm_f32(const float* x, const float* w, const void* bias, int 
         return rv_launch_status();
     }
     const long long rows = (M + TB - 1) / TB, cols = (N + TB - 1) / TB;
-    if (rows > 65535 || cols > 0x7fffffffll / 4) return RV_ERR_BAD_SIZE;
+    if (rows * cols > 0x7fffffffll / 4) return RV_ERR_BAD_SIZE;
     // K over a cluster of CTAs while all parts stay within the SMs (one CTA each)
     const int sms = rv_sm_count();
     const int splits = rows * cols * 4 <= sms ? 4 : (rows * cols * 2 <= sms ? 2 : 1);
     const int smem = (4 * TK * TPITCH + 2 * 64 * 256) * 4;   // stages, two parked groups (>= a part's sums)
     static_assert(4 * TK * TPITCH + 2 * 64 * 256 >= TB * TPITCH, "a part's sums fit");
     static RvPerDevice conf_v, conf_s;
-    const dim3 grid((unsigned)(cols * splits), (unsigned)rows);
+    const dim3 grid((unsigned)(rows * cols * splits));
     if (vec) {
         if (int st = rv_configure_smem(conf_v, gemm_f32_tile_kernel<true>, smem)) return st;
-        RV_LAUNCH_ST = splits == 1 ? rv_launch(gemm_f32_tile_kernel<true>, grid, dim3(256), smem, stream, x, w, bias, bias_dtype, residual, out, M, N, K, splits)
-                                   : rv_launch_cluster(gemm_f32_tile_kernel<true>, grid, dim3(256), smem, stream, splits, x, w, bias, bias_dtype, residual, out, M, N, K, splits);
+        RV_LAUNCH_ST = splits == 1 ? rv_launch(gemm_f32_tile_kernel<true>, grid, dim3(256), smem, stream, x, w, bias, bias_dtype, residual, out, M, N, K, splits, (int)rows)
+                                   : rv_launch_cluster(gemm_f32_tile_kernel<true>, grid, dim3(256), smem, stream, splits, x, w, bias, bias_dtype, residual, out, M, N, K, splits, (int)rows);
     } else {
         if (int st = rv_configure_smem(conf_s, gemm_f32_tile_kernel<false>, smem)) return st;
-        RV_LAUNCH_ST = splits == 1 ? rv_launch(gemm_f32_tile_kernel<false>, grid, dim3(256), smem, stream, x, w, bias, bias_dtype, residual, out, M, N, K, splits)
-                                   : rv_launch_cluster(gemm_f32_tile_kernel<false>, grid, dim3(256), smem, stream, splits, x, w, bias, bias_dtype, residual, out, M, N, K, splits);
+        RV_LAUNCH_ST = splits == 1 ? rv_launch(gemm_f32_tile_kernel<false>, grid, dim3(256), smem, stream, x, w, bias, bias_dtype, residual, out, M, N, K, splits, (int)rows)
+                                   : rv_launch_cluster(gemm_f32_tile_kernel<false>, grid, dim3(256), smem, stream, splits, x, w, bias, bias_dtype, residual, out, M, N, K, splits, (int)rows);
     }
     return rv_launch_status();
 }
