@@ -218,6 +218,301 @@ static int moe_launch(const void* x, const int* chosen, const float* weights, co
     return rv_launch_status();
 }
 
+// ------------------------------------------------------------------ few bfloat16 tokens on the tensor cores
+// A step of few tokens is bound by reading the matrices of the experts that any of them chose.  The kernels above read them
+// once per (token, slot) pair; these read each once: the pairs of an expert are the columns of an mma.sync (m16n8k16, float
+// accumulators; the rate needed is one per 23 clocks and SM), sixteen rows of the matrix its rows.  The order of k inside a
+// product is free, so a lane takes 8 neighbouring k of its row and of its pair as one 16-byte load each (k = 32 c + 8 (lane & 3))
+// and these four words are the operands of two products: nothing passes through shared memory on the way in.
+//   moe_mma_gate_up   a CTA per (expert, 16 features): eight warps share k (gated: four on the gate rows, four on the up rows),
+//                     their sums meet in shared memory
+//   moe_mma_down      a CTA per 16 columns of the result: its warps share the (expert, quarter of k) items, and the sums of a
+//                     token's slots are added in the slots' order
+// 32 experts (4096 x 2048, gated), 4 of them for each of 8 / 64 tokens, both products: 290 / 1,411 us with the kernels above, 179 /
+// 291 us (5.6 TB/s) with these.  The cuts of k depend on the sizes alone, so a row's result does not depend on the rest of
+// the batch.
+__device__ __forceinline__ void moe_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Weights are read once: they leave the first-level cache to the vectors.
+__device__ __forceinline__ uint4 moe_ld_weight(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// acc[n]: 16 matrix rows (this lane's rows wlo, whi) against NT blocks of 8 vectors (this lane's x[n]), over the 32-wide blocks
+// c0 .. c1 - 1 of k, U of them in flight (4 with one CTA more per SM: 10 % slower).  The pointers stand at 8 (lane & 3)
+// elements of their row.
+template <int NT>
+__device__ __forceinline__ void moe_mma_span(const uint4* wlo, const uint4* whi, const uint4* const (&x)[NT], int c0, int c1, float (&acc)[NT][4]) {
+    constexpr int U = NT > 2 ? 4 : 8;
+    int c = c0;
+    for (; c + U <= c1; c += U) {
+        uint4 lo[U], hi[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) { lo[u] = moe_ld_weight(wlo + (c + u) * 4); hi[u] = moe_ld_weight(whi + (c + u) * 4); }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const uint4 b = x[n][(c + u) * 4];
+                moe_mma(acc[n], lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
+                moe_mma(acc[n], lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+            }
+    }
+    for (; c < c1; ++c) {
+        const uint4 lo = moe_ld_weight(wlo + c * 4), hi = moe_ld_weight(whi + c * 4);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const uint4 b = x[n][c * 4];
+            moe_mma(acc[n], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+            moe_mma(acc[n], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+        }
+    }
+}
+
+#define MM_WARPS 8
+#define MM_PASS 32              // pairs of one expert that one pass over its rows serves
+
+// NT blocks of 8 pairs from list[p0] on: the products of this warp's rows (gated experts: the first half of the warps takes the
+// gate rows, the second the up rows) and part of k, left in red[warp][row][pair].
+template <bool GATED, int NT>
+__device__ __forceinline__ void moe_gate_up_pass(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* w0,
+                                                 const int* list, int count, int p0, int f0, int top, int ff, int width, float* red) {
+    constexpr int PARTS = GATED ? MM_WARPS / 2 : MM_WARPS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3, part = warp % PARTS;
+    const __nv_bfloat16* w = w0 + (warp >= PARTS ? (size_t)ff * width : 0);
+    const uint4* wlo = reinterpret_cast<const uint4*>(w + (size_t)min(ff - 1, f0 + g) * width) + q;
+    const uint4* whi = reinterpret_cast<const uint4*>(w + (size_t)min(ff - 1, f0 + g + 8) * width) + q;
+    const uint4* xr[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)                            // (a column beyond the list repeats its last pair and is not stored)
+        xr[n] = reinterpret_cast<const uint4*>(x + (size_t)(list[min(count - 1, p0 + n * 8 + g)] / top) * width) + q;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+    const int blocks = width / 32;
+    moe_mma_span<NT>(wlo, whi, xr, part * blocks / PARTS, (part + 1) * blocks / PARTS, acc);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) red[(warp * 16 + g + 8 * (j >> 1)) * MM_PASS + n * 8 + 2 * q + (j & 1)] = acc[n][j];
+}
+
+// grid (at most min(pairs, experts) experts in use, feature blocks); shared memory: presence bits, the expert's pairs, the sums
+template <bool GATED>
+__global__ void __launch_bounds__(MM_WARPS * 32, 2)
+moe_mma_gate_up_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ chosen, const __nv_bfloat16* __restrict__ gate_up,
+                       __nv_bfloat16* __restrict__ act, int pairs, int top, int experts, int ff, int width) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    extern __shared__ __align__(16) float mm_smem[];
+    constexpr int MT = GATED ? 2 : 1, PARTS = MM_WARPS / MT;
+    float* red = mm_smem;                                   // [warps][16][MM_PASS]
+    int* bits = reinterpret_cast<int*>(red + MM_WARPS * 16 * MM_PASS);
+    int* list = bits + (experts + 31) / 32;
+    __shared__ int expert_s, count_s;
+    const int words = (experts + 31) / 32, tid = threadIdx.x;
+    if (tid == 0) { expert_s = -1; count_s = 0; }
+    for (int i = tid; i < words; i += blockDim.x) bits[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < pairs; i += blockDim.x) {
+        const int e = chosen[i];
+        if (e >= 0 && e < experts) atomicOr(&bits[e >> 5], 1 << (e & 31));
+    }
+    __syncthreads();
+    if (tid < 32) {                                         // the blockIdx.x-th expert in use
+        int before = 0;
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const unsigned b = w0 + tid < words ? (unsigned)bits[w0 + tid] : 0u;
+            int n = __popc(b), at = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, at, o); if (tid >= o) at += v; }
+            const int first = before + at - n;
+            if ((int)blockIdx.x >= first && (int)blockIdx.x < first + n) expert_s = (w0 + tid) * 32 + __fns(b, 0, blockIdx.x - first + 1);
+            before += __shfl_sync(0xffffffffu, at, 31);
+        }
+    }
+    __syncthreads();
+    const int e = expert_s;
+    if (e < 0) return;
+    for (int i = tid; i < pairs; i += blockDim.x)
+        if (chosen[i] == e) list[atomicAdd(&count_s, 1)] = i;
+    __syncthreads();
+    const int count = count_s, f0 = blockIdx.y * 16;
+    const __nv_bfloat16* w = gate_up + (size_t)e * MT * ff * width;
+    for (int p0 = 0; p0 < count; p0 += MM_PASS) {
+        const int left = min(MM_PASS, count - p0);
+        if (left <= 8) moe_gate_up_pass<GATED, 1>(x, w, list, count, p0, f0, top, ff, width, red);
+        else if (left <= 16) moe_gate_up_pass<GATED, 2>(x, w, list, count, p0, f0, top, ff, width, red);
+        else moe_gate_up_pass<GATED, 4>(x, w, list, count, p0, f0, top, ff, width, red);
+        __syncthreads();
+        for (int i = tid; i < left * 16; i += blockDim.x) {
+            const int row = i & 15, p = i >> 4, f = f0 + row;
+            float s[MT];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                s[m] = 0.f;
+#pragma unroll
+                for (int w = 0; w < PARTS; ++w) s[m] += red[((m * PARTS + w) * 16 + row) * MM_PASS + p];
+            }
+            float v;
+            if constexpr (GATED) v = s[0] / (1.0f + expf(-s[0])) * s[MT - 1];
+            else { v = fmaxf(s[0], 0.f); v *= v; }
+            if (f < ff) act[(size_t)list[p0 + p] * ff + f] = __float2bfloat16_rn(v);
+        }
+        __syncthreads();
+    }
+}
+
+#define MM_QUARTERS 4
+
+template <int NT>
+__device__ __forceinline__ void moe_down_pass(const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* wd, const int* list, int count,
+                                              int p0, int n0, int quarter, int ff, int width, float* part, int pairs) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const uint4* wlo = reinterpret_cast<const uint4*>(wd + (size_t)min(width - 1, n0 + g) * ff) + q;
+    const uint4* whi = reinterpret_cast<const uint4*>(wd + (size_t)min(width - 1, n0 + g + 8) * ff) + q;
+    const uint4* xr[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) xr[n] = reinterpret_cast<const uint4*>(act + (size_t)list[min(count - 1, p0 + n * 8 + g)] * ff) + q;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+    const int blocks = ff / 32;
+    moe_mma_span<NT>(wlo, whi, xr, quarter * blocks / MM_QUARTERS, (quarter + 1) * blocks / MM_QUARTERS, acc);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int p = p0 + n * 8 + 2 * q + (j & 1);
+            if (p < count) part[((size_t)quarter * pairs + list[p]) * 16 + g + 8 * (j >> 1)] = acc[n][j];
+        }
+}
+
+// grid: blocks of 16 columns; shared memory: partial sums [quarters][pairs][16], counts and offsets per expert, experts in use, sorted pairs
+template <typename TO>
+__global__ void __launch_bounds__(MM_WARPS * 32, 2)
+moe_mma_down_kernel(const __nv_bfloat16* __restrict__ act, const int* __restrict__ chosen, const __nv_bfloat16* __restrict__ down,
+                    const float* add, TO* out, int tokens, int top, int experts, int ff, int width, float weight,
+                    const float* __restrict__ weights, const float* __restrict__ add_scale, const __nv_bfloat16* __restrict__ identity_x) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    extern __shared__ __align__(16) float mm_smem[];
+    const int pairs = tokens * top, tid = threadIdx.x, n0 = blockIdx.x * 16;
+    float* part = mm_smem;
+    int* counts = reinterpret_cast<int*>(part + (size_t)MM_QUARTERS * pairs * 16);
+    int* offsets = counts + experts;
+    int* used = offsets + experts;                          // at most min(pairs, experts)
+    int* list = used + min(pairs, experts);
+    __shared__ int used_s;
+    for (int i = tid; i < experts; i += blockDim.x) counts[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < pairs; i += blockDim.x) {
+        const int e = chosen[i];
+        if (e >= 0 && e < experts) atomicAdd(&counts[e], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int rows = 0, n_used = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int n = e0 + tid < experts ? counts[e0 + tid] : 0;
+            int at = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, at, o); if (tid >= o) at += v; }
+            const unsigned has = __ballot_sync(0xffffffffu, n > 0);
+            if (n > 0) used[n_used + __popc(has & ((1u << tid) - 1u))] = e0 + tid;
+            if (e0 + tid < experts) offsets[e0 + tid] = rows + at - n;
+            rows += __shfl_sync(0xffffffffu, at, 31);
+            n_used += __popc(has);
+        }
+        if (tid == 0) used_s = n_used;
+    }
+    __syncthreads();
+    for (int i = tid; i < pairs; i += blockDim.x) {
+        const int e = chosen[i];
+        if (e >= 0 && e < experts) list[atomicAdd(&offsets[e], 1)] = i;      // (afterwards offsets[e] is the end of e's pairs)
+    }
+    __syncthreads();
+    const int items = used_s * MM_QUARTERS;
+    for (int item = tid >> 5; item < items; item += MM_WARPS) {
+        const int e = used[item / MM_QUARTERS], quarter = item % MM_QUARTERS, count = counts[e];
+        const int* mine = list + offsets[e] - count;
+        const __nv_bfloat16* wd = down + (size_t)e * width * ff;
+        for (int p0 = 0; p0 < count; p0 += MM_PASS) {
+            const int left = min(MM_PASS, count - p0);
+            if (left <= 8) moe_down_pass<1>(act, wd, mine, count, p0, n0, quarter, ff, width, part, pairs);
+            else if (left <= 16) moe_down_pass<2>(act, wd, mine, count, p0, n0, quarter, ff, width, part, pairs);
+            else moe_down_pass<4>(act, wd, mine, count, p0, n0, quarter, ff, width, part, pairs);
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < tokens * 16; i += blockDim.x) {
+        const int t = i >> 4, n = n0 + (i & 15);
+        if (n >= width) continue;
+        float sum = 0.f;
+        for (int k = 0; k < top; ++k) {                     // the slots in their order: one sum per element
+            const int pair = t * top + k, e = chosen[pair];
+            const float wk = weights ? weights[pair] : 1.f;
+            if (e >= experts && identity_x) sum = fmaf(wk, __bfloat162float(identity_x[(size_t)t * width + n]), sum);
+            if (e < 0 || e >= experts) continue;
+            const float* p = part + (size_t)pair * 16 + (i & 15);
+            const size_t step = (size_t)pairs * 16;
+            sum = fmaf(wk, (p[0] + p[step]) + (p[2 * step] + p[3 * step]), sum);
+        }
+        float v = sum * weight;
+        if (add) v += add_scale ? add_scale[t] * add[(size_t)t * width + n] : add[(size_t)t * width + n];
+        out[(size_t)t * width + n] = rv_from_float<TO>(v);
+    }
+}
+
+// Whether the kernels above serve the sizes: rows of whole 32-wide blocks, and sums and lists that fit shared memory.
+static size_t moe_mma_gate_up_smem(int pairs, int experts) {
+    return (size_t)MM_WARPS * 16 * MM_PASS * 4 + (size_t)((experts + 31) / 32 + pairs) * 4;
+}
+static size_t moe_mma_down_smem(int pairs, int experts) {
+    return (size_t)MM_QUARTERS * pairs * 16 * 4 + (size_t)(2 * experts + (pairs < experts ? pairs : experts) + pairs) * 4;
+}
+#define MM_SMEM_MAX (160 * 1024)
+
+static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float* weights, const __nv_bfloat16* gate_up,
+                          const __nv_bfloat16* down, __nv_bfloat16* act, const float* add, const float* add_scale, void* out, int out_f32,
+                          int tokens, int top, int experts, int ff, int width, float weight, int gated, int identity, cudaStream_t stream) {
+    static RvPerDevice once[4];
+    const int pairs = tokens * top;
+    const dim3 grid(pairs < experts ? pairs : experts, (ff + 15) / 16);
+    const size_t smem_a = moe_mma_gate_up_smem(pairs, experts), smem_b = moe_mma_down_smem(pairs, experts);
+    int st;
+    if (gated) {
+        if ((st = rv_configure_smem(once[0], moe_mma_gate_up_kernel<true>, MM_SMEM_MAX)) != RV_OK) return st;
+        st = rv_launch(moe_mma_gate_up_kernel<true>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
+    } else {
+        if ((st = rv_configure_smem(once[1], moe_mma_gate_up_kernel<false>, MM_SMEM_MAX)) != RV_OK) return st;
+        st = rv_launch(moe_mma_gate_up_kernel<false>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
+    }
+    if (st != RV_OK) return st;
+    const dim3 grid_b((width + 15) / 16);
+    const __nv_bfloat16* own = identity ? x : nullptr;
+    if (out_f32) {
+        if ((st = rv_configure_smem(once[2], moe_mma_down_kernel<float>, MM_SMEM_MAX)) != RV_OK) return st;
+        st = rv_launch(moe_mma_down_kernel<float>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act, chosen, down, add, (float*)out, tokens, top,
+                       experts, ff, width, weight, weights, add_scale, own);
+    } else {
+        if ((st = rv_configure_smem(once[3], moe_mma_down_kernel<__nv_bfloat16>, MM_SMEM_MAX)) != RV_OK) return st;
+        st = rv_launch(moe_mma_down_kernel<__nv_bfloat16>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act, chosen, down, add, (__nv_bfloat16*)out,
+                       tokens, top, experts, ff, width, weight, weights, add_scale, own);
+    }
+    RV_LAUNCH_ST = st;
+    return rv_launch_status();
+}
+
 // x [tokens, width], act [tokens * top, ff] (scratch of the weights' type), add float [tokens, width] or null, add_scale float
 // [tokens] or null (1),
 // weights float [tokens, top] or null, out [tokens, width] float (out_f32) or of the weights' type.  gated: 1 the experts'
@@ -231,6 +526,11 @@ RV_EXPORT int rv_moe_experts_ex(const void* x, const int* chosen, const float* w
     if (dtype == RV_DTYPE_F32)
         return moe_launch<float>(x, chosen, weights, gate_up, down, act, add, add_scale, out, 1, tokens, top, experts, ff, width, weight, gated, identity, 0,
                                  stream);
+    if (dtype == RV_DTYPE_BF16 && width % 32 == 0 && ff % 32 == 0 && (long long)tokens * top <= 4096 && experts <= 4096 && (ff + 15) / 16 <= 65535 &&
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(act)) & 15) == 0 &&
+        moe_mma_gate_up_smem(tokens * top, experts) <= MM_SMEM_MAX && moe_mma_down_smem(tokens * top, experts) <= MM_SMEM_MAX)
+        return moe_mma_launch((const __nv_bfloat16*)x, chosen, weights, (const __nv_bfloat16*)gate_up, (const __nv_bfloat16*)down, (__nv_bfloat16*)act,
+                              add, add_scale, out, out_f32, tokens, top, experts, ff, width, weight, gated, identity, stream);
     if (dtype == RV_DTYPE_BF16)
         return moe_launch<__nv_bfloat16>(x, chosen, weights, gate_up, down, act, add, add_scale, out, out_f32, tokens, top, experts, ff, width,
                                          weight, gated, identity, 4, stream);

@@ -53,3 +53,31 @@ def test_stream_norms_in_words_of_four(K, rows, cols, y_dtype):
         got, nxt = K.stream_add_norm(x.clone(), y, (g, 1e-5), torch.float32)
         want = x.double().cpu() + y.double().cpu()
         assert rel_err(got, want) < 2e-7 and rel_err(nxt, rms(want, g, 1e-5)) < 4e-6
+
+
+@pytest.mark.parametrize("T,E,top,ff,width,gated,identity", [(1, 8, 2, 32, 64, True, False), (7, 5, 3, 96, 160, False, True), (33, 40, 4, 160, 96, True, False),
+                                                             (100, 3, 2, 64, 96, True, False), (9, 70, 4, 1408, 2048, False, False)])
+def test_moe_of_few_tokens_on_the_tensor_cores(K, T, E, top, ff, width, gated, identity):
+    """Every expert's pairs as the columns of one product: lists of one to many pairs (several passes), numbers that name
+    nobody (-1) or the token itself, rows of 16 that end inside the matrix; and a token's bits do not depend on the others."""
+    torch.manual_seed(T * E)
+    gu = (torch.randn(E, (2 if gated else 1) * ff, width, device="cuda") * 0.1).bfloat16()
+    dn = (torch.randn(E, width, ff, device="cuda") * 0.1).bfloat16()
+    x = torch.randn(T, width, device="cuda").bfloat16()
+    ch = torch.randint(-1, E + (2 if identity else 0), (T, top), device="cuda", dtype=torch.int32)
+    w, add, scale = torch.rand(T, top, device="cuda"), torch.randn(T, width, device="cuda"), torch.rand(T, device="cuda")
+    run = lambda n: K.moe_experts(x[:n].contiguous(), ch[:n].contiguous(), gu, dn, 0.5, add=add[:n].contiguous(), out_dtype=torch.float32,      # noqa: E731
+                                  weights=w[:n].contiguous(), activation="silu" if gated else "relu2", add_scale=scale[:n].contiguous(), identity=identity)
+    out, ref = run(T), (scale[:, None] * add).double().cpu()
+    for t in range(T):
+        for k in range(top):
+            e = int(ch[t, k])
+            if e >= E:
+                ref[t] += 0.5 * float(w[t, k]) * x[t].double().cpu()
+            if not 0 <= e < E:
+                continue
+            h = gu[e].double().cpu() @ x[t].double().cpu()
+            a = torch.nn.functional.silu(h[:ff]) * h[ff:] if gated else torch.relu(h) ** 2
+            ref[t] += 0.5 * float(w[t, k]) * (dn[e].double().cpu() @ a)
+    assert rel_err(out, ref) < 4e-3                          # the activations are rounded to bfloat16 (2^-9) before the second product
+    assert torch.equal(run(1), out[:1])
