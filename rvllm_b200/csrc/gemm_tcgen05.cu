@@ -72,6 +72,7 @@ static_assert(BN == 256 || BN == 128, "tiles of 256 or 128 columns");
 #define EPI_GATED 2
 #define EPI_GATED_GELU 4    // (launcher only) EPI_GATED with the tanh form of GELU in place of SiLU
 #define EPI_ROPE 3          // the q/k/v product: bias, rotation of q and k, k and v into the paged cache
+#define EPI_GATED_CLAMP 5   // (launcher only) EPI_GATED with act 3
 #define EPI_PLAIN_RELU2 6   // (launcher only) EPI_PLAIN whose results pass relu(v)^2 before they are stored
 
 struct GemmParams {
@@ -87,7 +88,7 @@ struct GemmParams {
     // its shared memory (where its stages were) and adds them in the order of the parts.  Not for EPI_GATED.
     int splits;
     // EPI_ROPE: W rows are [q heads | k heads | v heads] of hd (64, 128 or 256) features
-    const void* bias;                // [N] or nullptr
+    const void* bias;                // [N] or nullptr (also of the plain, residual and gated epilogues: added to the float sums)
     int bias_dtype;
     __nv_bfloat16* q_out;            // [M, nh * hd]
     __nv_bfloat16* kv_cache;         // [pages, 2, nkv, page_size, hd]
@@ -96,7 +97,8 @@ struct GemmParams {
     const float* cos_t;              // [table_rows, hd / 2] or nullptr (no rotation)
     const float* sin_t;
     int nh, nkv, hd, page_size, table_rows;
-    int act;                       // EPI_GATED: 0 SiLU, 1 the tanh form of GELU; EPI_PLAIN: 0 none, 2 the square of relu
+    int act;                       // EPI_GATED: 0 SiLU, 1 the tanh form of GELU, 3 the clamped form (limit, alpha); EPI_PLAIN: 0 none, 2 the square of relu
+    float limit, alpha;
     // Grouped product (plain and gated epilogues): W holds `groups` matrices of N rows one below the other, and work
     // unit t (m_tiles of them) multiplies rows of x with matrix tile_group[t]; a negative entry marks a unit that nobody
     // uses, which every role of the kernel skips.  The rows of x are sorted by group and every group's rows padded to
@@ -138,6 +140,46 @@ __device__ __forceinline__ float plain_act(float v, int act) {
 }
 __device__ __forceinline__ float gate_act(float g, int act) {
     return act == 1 ? g / (1.0f + expf(-1.5957691216057308f * (g + 0.044715f * g * g * g))) : silu_f(g);
+}
+// a gated result: act(gate) up, or (act 3) g sigmoid(alpha g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit)
+__device__ __forceinline__ float gated_value(const GemmParams& p, float g, float u) {
+    if (p.act == 3) {
+        g = fminf(g, p.limit);
+        u = fminf(fmaxf(u, -p.limit), p.limit);
+        return g / (1.0f + expf(-p.alpha * g)) * (u + 1.0f);
+    }
+    return gate_act(g, p.act) * u;
+}
+// r[e] += bias[n + e] for the columns below `limit`, as float; the addresses are the same for the whole warp
+__device__ __forceinline__ void add_bias(const GemmParams& p, uint32_t (&r)[32], int n, int limit) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p.bias) + (size_t)n * (p.bias_dtype == RV_DTYPE_F32 ? 4 : 2);
+    if (n + 32 <= limit && (at & 15) == 0) {
+        if (p.bias_dtype == RV_DTYPE_F32) {
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const float4 b = __ldg(reinterpret_cast<const float4*>(at) + v);
+                r[4 * v] = __float_as_uint(__uint_as_float(r[4 * v]) + b.x);
+                r[4 * v + 1] = __float_as_uint(__uint_as_float(r[4 * v + 1]) + b.y);
+                r[4 * v + 2] = __float_as_uint(__uint_as_float(r[4 * v + 2]) + b.z);
+                r[4 * v + 3] = __float_as_uint(__uint_as_float(r[4 * v + 3]) + b.w);
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const uint4 b = __ldg(reinterpret_cast<const uint4*>(at) + v);
+                const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    r[8 * v + 2 * j] = __float_as_uint(__uint_as_float(r[8 * v + 2 * j]) + __uint_as_float(w[j] << 16));
+                    r[8 * v + 2 * j + 1] = __float_as_uint(__uint_as_float(r[8 * v + 2 * j + 1]) + __uint_as_float(w[j] & 0xffff0000u));
+                }
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 32; ++e)
+        if (n + e < limit) r[e] = __float_as_uint(__uint_as_float(r[e]) + rv_load_param(p.bias, p.bias_dtype, n + e));
 }
 // a cluster of CTAs that share a tile's K (the build on single CTAs)
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }     // the four epilogue warps
@@ -518,6 +560,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tmem_ld_wait();
                     if (m < p.M) {
                         const int n = n_out0 + c;
+                        if (p.bias) {
+                            add_bias(p, g, n, half_n);
+                            add_bias(p, u, half_n + n, p.N);
+                        }
                         if (!p.out_f32 && n + 32 <= half_n && (half_n & 7) == 0) {
                             __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)m * half_n + n;
 #pragma unroll
@@ -527,8 +573,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) {
                                     const int e = v * 8 + 2 * j;
-                                    oh[j] = __floats2bfloat162_rn(gate_act(__uint_as_float(g[e]), p.act) * __uint_as_float(u[e]),
-                                                                  gate_act(__uint_as_float(g[e + 1]), p.act) * __uint_as_float(u[e + 1]));
+                                    oh[j] = __floats2bfloat162_rn(gated_value(p, __uint_as_float(g[e]), __uint_as_float(u[e])),
+                                                                  gated_value(p, __uint_as_float(g[e + 1]), __uint_as_float(u[e + 1])));
                                 }
                                 *reinterpret_cast<uint4*>(dst + v * 8) = o;
                             }
@@ -536,7 +582,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                             for (int e = 0; e < 32; ++e) {
                                 if (n + e >= half_n) continue;
-                                const float val = gate_act(__uint_as_float(g[e]), p.act) * __uint_as_float(u[e]);
+                                const float val = gated_value(p, __uint_as_float(g[e]), __uint_as_float(u[e]));
                                 if (p.out_f32) ((float*)p.out)[(size_t)m * half_n + n + e] = val;
                                 else ((__nv_bfloat16*)p.out)[(size_t)m * half_n + n + e] = __float2bfloat16_rn(val);
                             }
@@ -574,6 +620,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     load_acc(c, r);
                     if (m < p.M) {
                         const int n = n0 + c;
+                        if (p.bias) add_bias(p, r, n, p.N);
                         const bool vec = n + 32 <= p.N && (p.N & 7) == 0 && wide_ok;
                         if (vec && !p.out_f32) {
                             __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)m * ldc + coff + n;
@@ -667,7 +714,8 @@ static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const
 // 1 if this library was built for pairs of CTAs
 RV_EXPORT int rv_gemm_tcgen05_is_pair() { return RV_PAIR; }
 
-// epilogue: 0 plain, 1 + residual (bf16 [M, N]), 2 gated (W rows [gate | up], out has N/2 columns), 4 gated with GELU (tanh form).
+// epilogue: 0 plain, 1 + residual (bf16 [M, N]), 2 gated (W rows [gate | up], out has N/2 columns), 4 gated with GELU (tanh form),
+// 5 gated with the clamped form (limit, alpha; see gated_value).  bias: float or bfloat16 [N] or null, added to the sums in float.
 // status: optional device int that receives a non-zero code if a wait inside the kernel gave up.
 // splits (both entry points): 1, or 2 / 4 on the build for single CTAs: the CTAs of a tile share its K as a cluster
 // (see GemmParams); not with the gated epilogue, and with the rotary one only while a CTA's columns hold whole heads.
@@ -679,11 +727,13 @@ static int check_splits(int splits, int K, int epilogue, int hd) {
     return RV_OK;
 }
 
-RV_EXPORT int rv_gemm_tcgen05_bf16(const void* x, const void* w, const void* residual, void* out, int out_f32,
-                                   int M, int N, int K, int epilogue, int* status, int max_ctas, int splits,
+RV_EXPORT int rv_gemm_tcgen05_bf16(const void* x, const void* w, const void* bias, int bias_dtype, const void* residual, void* out, int out_f32,
+                                   int M, int N, int K, int epilogue, float limit, float alpha, int* status, int max_ctas, int splits,
                                    cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0) return RV_ERR_BAD_SIZE;
-    const int act = epilogue == EPI_GATED_GELU ? 1 : 0;            // the gated epilogue with the other activation
+    if (bias_dtype & ~1) return RV_ERR_BAD_DTYPE;
+    const int act = epilogue == EPI_GATED_GELU ? 1 : (epilogue == EPI_GATED_CLAMP ? 3 : 0);      // the gated epilogue with another activation
+    if (act == 3 && !(limit > 0.f)) return RV_ERR_BAD_SIZE;
     if (act) epilogue = EPI_GATED;
     if (int e = check_splits(splits, K, epilogue, 0)) return e;
     if (K % 8) return RV_ERR_UNSUPPORTED;                          // rows must start on 16-byte boundaries
@@ -701,7 +751,8 @@ RV_EXPORT int rv_gemm_tcgen05_bf16(const void* x, const void* w, const void* res
     GemmParams p = {};
     p.out = out; p.residual = epilogue == EPI_RESIDUAL ? (const __nv_bfloat16*)residual : nullptr;
     p.status = status; p.M = M; p.N = N; p.K = K; p.out_f32 = out_f32; p.epilogue = epilogue;
-    p.splits = splits; p.act = act;
+    p.splits = splits; p.act = act; p.limit = limit; p.alpha = alpha;
+    p.bias = bias; p.bias_dtype = bias_dtype;
     p.m_tiles = (M + TILE_ROWS - 1) / TILE_ROWS;
     // gated: a tile is 128 gate rows and the 128 up rows of the same output columns; gate rows past
     // N/2 read up rows, whose products the epilogue never stores

@@ -1,6 +1,6 @@
 // bfloat16 linear layer for few rows (decode) on the fifth-generation tensor cores:
 //     out[M, N] = x[M, K] . W[N, K]^T (+ bias[N]) (+ residual[M, N]),       M <= 128,
-// or GATED with W rows [gate (N/2) | up (N/2)]:  out[M, N/2] = silu(x Wg^T) * (x Wu^T).
+// or GATED with W rows [gate (N/2) | up (N/2)]:  out[M, N/2] = silu(x Wg^T + bg) * (x Wu^T + bu) and its other forms.
 //
 // The product is computed transposed: the WEIGHTS are the 128-row A operand of tcgen05.mma and
 // the batch is its N dimension (16 to 128 columns of tensor memory), so a CTA streams a tile of
@@ -58,7 +58,8 @@ struct DecodeGemmParams {
     int* counters;           // [tiles], zero between launches
     int* status;
     int M, N, K;
-    int out_f32, gated;            // gated: 0 no, 1 SiLU-gated, 2 gated with the tanh form of GELU
+    int out_f32, gated;            // gated: 0 no, 1 SiLU-gated, 2 gated with the tanh form of GELU, 3 the clamped form (limit, alpha)
+    float limit, alpha;
     int splits, n_tiles;
     int cluster;             // 1: the CTAs of a tile are a thread-block cluster and add their partials in the
                              // cluster's shared memory (M <= 64, 2 <= splits <= 8); scratch and counters unused
@@ -134,6 +135,12 @@ __device__ __forceinline__ float4 load_part(const float* src) {
 __device__ __forceinline__ float silu_gate(float g, float u, bool exact, bool gelu = false) {
     const float a = gelu ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
     return exact ? g / (1.0f + expf(-a)) * u : __fdividef(g, 1.0f + __expf(-a)) * u;
+}
+// g sigmoid(alpha g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit)
+__device__ __forceinline__ float clamped_gate(float g, float u, float limit, float alpha) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
 }
 
 template <int MB, bool IN_SMEM>
@@ -651,6 +658,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     // features 0..63 are gate rows, 64..127 the up rows of the same output columns
                     const int fo = et & 63;
                     const int n = tile * (TILE_F / 2) + fo;
+                    const float bg = p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, n) : 0.f;
+                    const float bu = p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, half_n + n) : 0.f;
                     // eight rows of an output column per pass: eight independent chains per thread
                     for (int m0 = (et >> 6) * 8; m0 < p.M && n < half_n; m0 += 16) {
                         const float4 ga = *reinterpret_cast<const float4*>(fin + fo * FS + m0);
@@ -661,7 +670,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const float u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
                         float v[8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = silu_gate(g[j], u[j], p.out_f32 != 0, p.gated == 2);
+                        for (int j = 0; j < 8; ++j)
+                            v[j] = p.gated == 3 ? clamped_gate(g[j] + bg, u[j] + bu, p.limit, p.alpha) : silu_gate(g[j] + bg, u[j] + bu, p.out_f32 != 0, p.gated == 2);
                         if (p.out_f32) {
                             float* o = (float*)p.out + (size_t)m0 * half_n + n;
 #pragma unroll
@@ -854,15 +864,16 @@ static int run_decode(const void* x, const void* w, DecodeGemmParams p, cudaStre
 
 RV_EXPORT int rv_gemm_tcgen05_decode_bf16(const void* x, const void* w, const void* bias, int bias_dtype,
                                           const void* residual, void* out, int out_f32, int M, int N, int K,
-                                          int gated, int splits, int cluster, float* scratch, int* counters, int* status,
-                                          const void* norm_gamma, int norm_gamma_dtype, float norm_eps,
+                                          int gated, float limit, float alpha, int splits, int cluster, float* scratch, int* counters,
+                                          int* status, const void* norm_gamma, int norm_gamma_dtype, float norm_eps,
                                           cudaStream_t stream) {
-    if (gated && ((N & 1) || bias || residual)) return RV_ERR_BAD_SIZE;
+    if (gated && ((N & 1) || residual)) return RV_ERR_BAD_SIZE;
+    if (gated < 0 || gated > 3 || (gated == 3 && !(limit > 0.f))) return RV_ERR_BAD_SIZE;
     if (residual && out_f32) return RV_ERR_BAD_SIZE;
     DecodeGemmParams p = {};
     p.out = out; p.residual = (const __nv_bfloat16*)residual; p.bias = bias; p.bias_dtype = bias_dtype;
     p.scratch = scratch; p.counters = counters; p.status = status;
-    p.M = M; p.N = N; p.K = K; p.out_f32 = out_f32; p.gated = gated; p.splits = splits; p.cluster = cluster;
+    p.M = M; p.N = N; p.K = K; p.out_f32 = out_f32; p.gated = gated; p.limit = limit; p.alpha = alpha; p.splits = splits; p.cluster = cluster;
     p.norm_gamma = norm_gamma; p.norm_gamma_dtype = norm_gamma_dtype; p.norm_eps = norm_eps;
     return run_decode(x, w, p, stream);
 }

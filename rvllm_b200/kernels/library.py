@@ -569,9 +569,9 @@ class CudaKernels:
         if self._use_decode_gemm(M, weight.shape[0], K, False) and out_dtype in (torch.bfloat16, torch.float32) \
                 and (residual is None or (residual.dtype == torch.bfloat16 and out_dtype == torch.bfloat16)):
             return self.linear_decode(x, weight, bias, residual, out_dtype)
-        if self._tcgen05_fills(M, weight.shape[0]) and K % 8 == 0 and bias is None and out_dtype in (torch.bfloat16, torch.float32) \
+        if self._tcgen05_fills(M, weight.shape[0]) and K % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32) \
                 and (residual is None or (residual.dtype == torch.bfloat16 and out_dtype == torch.bfloat16)):
-            return self.linear_tcgen05(x, weight, residual, out_dtype)
+            return self.linear_tcgen05(x, weight, residual, out_dtype, bias=bias)
         if out_dtype == torch.float32:
             out = torch.mm(x, weight.t(), out_dtype=torch.float32)
             if bias is not None:
@@ -632,9 +632,10 @@ class CudaKernels:
         return self._lib("gemm_tcgen05.cu", defines)
 
     def linear_tcgen05(self, x, weight, residual=None, out_dtype=None, gated=False, status=None, max_ctas=0, pair=None,
-                       splits=None, activation="silu"):
-        """The tcgen05 / TMEM / TMA GEMM for bfloat16 (any M; K a multiple of 8).  gated: weight rows
-        are [gate | up] and the result is silu(x gate^T) * (x up^T).  `status`: optional int32 device
+                       splits=None, activation="silu", bias=None, limit=0.0, alpha=0.0):
+        """The tcgen05 / TMEM / TMA GEMM for bfloat16 (any M; K a multiple of 8), with a bias (float32 or bfloat16,
+        added to the float sums).  gated: weight rows are [gate | up] and the result is silu(x gate^T) * (x up^T)
+        ("gelu_tanh", "swiglu_clamp" with `limit` and `alpha`: the forms of `act_mul`).  `status`: optional int32 device
         tensor that receives a non-zero code if a bounded wait inside the kernel gave up.  `pair`:
         the build on pairs of CTAs (cta_group::2) or on single CTAs; default: by the number of rows."""
         _need(x, "x", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
@@ -644,7 +645,11 @@ class CudaKernels:
         out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
         if residual is not None:
             _need(residual, "residual", torch.bfloat16, 2)
-        epilogue = (4 if activation == "gelu_tanh" else 2) if gated else (1 if residual is not None else 0)
+        if bias is not None:
+            _need(bias, "bias", dims=1)
+            if bias.shape[0] != N:
+                raise KernelError(f"linear: bias has {bias.shape[0]} entries for {N} features")
+        epilogue = {"silu": 2, "gelu_tanh": 4, "swiglu_clamp": 5}[activation] if gated else (1 if residual is not None else 0)
         if splits is None:
             splits = self._prefill_splits(M, N, K, gated) if (max_ctas == 0 and pair is None) else 1
         if splits > 1:
@@ -652,8 +657,8 @@ class CudaKernels:
         else:
             lib = self._prefill_gemm_lib(M, pair, N, gated)
         st = lib.rv_gemm_tcgen05_bf16(
-            _ptr(x), _ptr(weight), _ptr(residual), _ptr(out), c_int(1 if out_dtype == torch.float32 else 0),
-            c_int(M), c_int(N), c_int(K), c_int(epilogue), _ptr(status if status is not None else self._status), c_int(max_ctas),
+            _ptr(x), _ptr(weight), _ptr(bias), c_int(self._dt(bias, "bias") if bias is not None else 0), _ptr(residual), _ptr(out),
+            c_int(1 if out_dtype == torch.float32 else 0), c_int(M), c_int(N), c_int(K), c_int(epilogue), c_float(limit), c_float(alpha), _ptr(status if status is not None else self._status), c_int(max_ctas),
             c_int(splits), self._stream())
         _check("gemm_tcgen05", st)
         return out
@@ -716,7 +721,7 @@ class CudaKernels:
         return splits, bool(cluster)
 
     def linear_decode(self, x, weight, bias=None, residual=None, out_dtype=None, gated=False, splits=None, status=None,
-                      norm=None, cluster=None, activation="silu"):
+                      norm=None, cluster=None, activation="silu", limit=0.0, alpha=0.0):
         """The weight-streaming tcgen05 GEMM for few rows of bfloat16 activations (beyond 128 rows:
         in blocks of 128, K split inside a cluster or not at all).
         norm = (gamma, eps): RMSNorm applied to x inside the kernel (at most 16 rows)."""
@@ -745,7 +750,7 @@ class CudaKernels:
         st = lib.rv_gemm_tcgen05_decode_bf16(
             _ptr(x), _ptr(weight), _ptr(bias), c_int(self._dt(bias, "bias") if bias is not None else 0), _ptr(residual),
             _ptr(out), c_int(1 if out_dtype == torch.float32 else 0), c_int(M), c_int(N), c_int(K),
-            c_int((2 if activation == "gelu_tanh" else 1) if gated else 0), c_int(splits), c_int(1 if cluster else 0), _ptr(scratch),
+            c_int({"silu": 1, "gelu_tanh": 2, "swiglu_clamp": 3}[activation] if gated else 0), c_float(limit), c_float(alpha), c_int(splits), c_int(1 if cluster else 0), _ptr(scratch),
             _ptr(self._decode_counters if splits > 1 else None),
             _ptr(status if status is not None else self._status), *self._norm_args(norm, K), self._stream())
         _check("gemm_tcgen05_decode", st)
@@ -881,6 +886,21 @@ class CudaKernels:
             return self.silu_mul(self.linear(x, weight))
         # the product leaves its kernel in float; the activation kernel rounds once
         return self.act_mul(self.linear(x, weight, out_dtype=torch.float32), activation, x.dtype)
+
+    def gate_up_clamp(self, x, weight, bias, limit: float, alpha: float) -> torch.Tensor:
+        """g sigmoid(alpha g) (u + 1) with g = min(x Wg^T + bg, limit), u = clamp(x Wu^T + bu, -limit, limit) for weight rows
+        [Wg | Wu], in x's type.  Where one of the bfloat16 GEMMs serves the product it is its epilogue: the product in float32,
+        rows of 4 N bytes, never goes through memory (2,048 tokens, N = 28,672: passes of 470 MB for the bias and of
+        290 MB for the activation, 230 us of a layer)."""
+        M, K = x.shape
+        N = weight.shape[0]
+        if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and N % 2 == 0 and K % 8 == 0 and limit > 0:
+            options = dict(bias=bias, gated=True, activation="swiglu_clamp", limit=limit, alpha=alpha)
+            if self._use_decode_gemm(M, N, K, True):
+                return self.linear_decode(x, weight, **options)
+            if self._tcgen05_fills(M, N, True):
+                return self.linear_tcgen05(x, weight, **options)
+        return self.act_mul(self.linear(x, weight, bias, None, torch.float32), "swiglu_clamp", x.dtype, limit=limit, alpha=alpha)
 
     # ------------------------------------------------------------------ output-norm layers, gated attention, state-space mixer
     def residual_rmsnorm(self, y, gamma, eps: float, residual: Optional[torch.Tensor], rounded_dtype=None,

@@ -44,8 +44,8 @@ FEED_FORWARDS.register("gated_mlp", GatedMLP)
 
 class ClampedGluMLP(Part):
     """down( g sigmoid(alpha g) (u + 1) ) with g = min(gate(x), limit) and u = clamp(up(x), -limit, limit); every
-    product has a bias.  gate and up are one stacked product [gate | up] that leaves its kernel in float32; the
-    activation kernel rounds once."""
+    product has a bias.  gate and up are one stacked product [gate | up]; bias and activation act on its float32 sums, in the
+    product's epilogue or in a kernel of their own, and the result is rounded once."""
 
     def __init__(self, hidden_size: int, intermediate_size: int, limit: float, alpha: float = 1.702,
                  names=("gate", "up", "down"), suffix: str = "", bias_suffix: str = ".b"):
@@ -65,8 +65,12 @@ class ClampedGluMLP(Part):
         self.down.bind(get)
 
     def __call__(self, x, ctx, residual=None, out_dtype=None):
-        gu = self.gate_up(x, ctx, out_dtype=torch.float32)
-        h = ctx.kernels.act_mul(gu, "swiglu_clamp", x.dtype, limit=self.limit, alpha=self.alpha)
+        fused = getattr(ctx.kernels, "gate_up_clamp", None)
+        if fused is not None:
+            h = fused(x, self.gate_up.weight, self.gate_up.bias, self.limit, self.alpha)
+        else:
+            gu = self.gate_up(x, ctx, out_dtype=torch.float32)
+            h = ctx.kernels.act_mul(gu, "swiglu_clamp", x.dtype, limit=self.limit, alpha=self.alpha)
         return self.down(h, ctx, residual=residual, out_dtype=out_dtype)
 
 

@@ -81,3 +81,20 @@ def test_moe_of_few_tokens_on_the_tensor_cores(K, T, E, top, ff, width, gated, i
             ref[t] += 0.5 * float(w[t, k]) * (dn[e].double().cpu() @ a)
     assert rel_err(out, ref) < 4e-3                          # the activations are rounded to bfloat16 (2^-9) before the second product
     assert torch.equal(run(1), out[:1])
+
+
+@pytest.mark.parametrize("M,N,Kd", [(130, 264, 72), (300, 96, 128), (512, 512, 4096), (5, 200, 136), (64, 1024, 264), (200, 130, 72)])
+@pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16])
+def test_bias_and_clamped_gate_in_the_products_epilogues(K, M, N, Kd, bias_dtype):
+    """Plain, residual and clamp-gated products with a bias: both GEMMs, one CTA, pairs and K split over a cluster."""
+    torch.manual_seed(M + N)
+    x, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") * 0.1).bfloat16()
+    b, r = torch.randn(N, device="cuda").to(bias_dtype), torch.randn(M, N, device="cuda").bfloat16()
+    ref = x.double().cpu() @ w.double().cpu().t() + b.double().cpu()
+    assert rel_err(K.linear(x, w, b, None, torch.float32), ref) < 2e-5      # float sums of exact products
+    if N % 8 == 0:
+        assert rel_err(K.linear(x, w, b, r), ref + r.double().cpu()) < 5e-3      # one rounding to bfloat16
+    half = N // 2
+    gate, up = ref[:, :half].clamp(max=2.0), ref[:, half:].clamp(-2.0, 2.0)
+    want = gate * torch.sigmoid(1.7 * gate) * (up + 1)
+    assert rel_err(K.gate_up_clamp(x, w, b, 2.0, 1.7), want) < 5e-3
