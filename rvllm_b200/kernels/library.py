@@ -1028,6 +1028,7 @@ class CudaKernels:
         COUNTERS['launches'] += 1 if taps > 1 else 0
         return out
 
+    SCAN_CHUNK_MIN_TOKENS = 32         # tokens of a portion from which the recurrence goes chunk by chunk (32 tokens: 50 us against 85)
     SCAN_SEGMENT_TOKENS = 256          # a sequence that brings more than twice as many tokens to a step is scanned in segments
     SCAN_SEGMENT_SCRATCH = 1 << 30     # ... of this many tokens side by side, while the segments' states fit these bytes of scratch
     SCAN_SEGMENT_ALWAYS = False        # ... and only where the one-pass walk would have fewer CTAs than the device has SMs (measured:
@@ -1036,13 +1037,15 @@ class CudaKernels:
 
     def ssm_scan(self, xbc, proj, dt_col0: int, dt_bias, a_log, d_skip, cu_seqlens, state_slots, state, heads: int,
                  head_dim: int, state_size: int, groups: int, columns: int = 0, max_q_len: Optional[int] = None,
-                 segment_tokens: Optional[int] = None) -> torch.Tensor:
+                 segment_tokens: Optional[int] = None, chunked: Optional[bool] = None) -> torch.Tensor:
         """The selective-state recurrence over the step's tokens, continued from and leaving behind each request's
         S in `state` (float [slots, floats], [heads][N][P] at offset 0).  xbc rows: [x | B | C]; raw dt is read
         from columns dt_col0 .. of `proj`.  Returns y float32 [T, heads * head_dim].  `columns`: columns of the
         state per thread (1 or 2); 0 lets the launcher choose by the size of the grid.  `max_q_len`: the most tokens any
         sequence brings (known on the host); long portions are then cut into segments of `segment_tokens` (default
-        `SCAN_SEGMENT_TOKENS`) that are scanned side by side and joined by two small kernels."""
+        `SCAN_SEGMENT_TOKENS`) that are scanned side by side and joined by two small kernels.  Portions of
+        `SCAN_CHUNK_MIN_TOKENS` bfloat16 tokens and more take the chunked form on the tensor cores (ssm_chunk.cu) where it serves
+        the sizes; `chunked` asks for or against it."""
         _need(xbc, "xbc", dims=2); _need(proj, "proj", dims=2); _need(state, "state", torch.float32, 2)
         for name, p in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
             _need(p, name, dt_bias.dtype, 1)
@@ -1051,6 +1054,17 @@ class CudaKernels:
         if state.shape[1] < heads * state_size * head_dim:
             raise KernelError("ssm_scan: the state rows are too short")
         y = torch.empty((xbc.shape[0], heads * head_dim), dtype=torch.float32, device=xbc.device)
+        if chunked is None:
+            chunked = columns == 0 and segment_tokens is None and max_q_len is not None and max_q_len >= self.SCAN_CHUNK_MIN_TOKENS
+        if chunked and xbc.dtype == torch.bfloat16 and state_size in (64, 128) and head_dim % 16 == 0 and xbc.shape[1] % 8 == 0 \
+                and xbc.data_ptr() % 16 == 0:
+            st = self._lib("ssm_chunk.cu").rv_ssm_chunk(
+                _ptr(xbc), c_int(xbc.shape[1]), _ptr(proj), c_int(self._dt(proj, "proj")), c_int(proj.shape[1]), c_int(dt_col0),
+                _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), c_int(self._dt(dt_bias, "dt_bias")), _ptr(cu_seqlens), _ptr(state_slots),
+                _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(y), c_int(state_slots.shape[0]), c_int(heads), c_int(head_dim),
+                c_int(state_size), c_int(groups), self._stream())
+            _check("ssm_chunk", st)
+            return y
         seg = self.SCAN_SEGMENT_TOKENS if segment_tokens is None else segment_tokens
         n_seqs, max_segs, seg_state, seg_decay, dcum = state_slots.shape[0], 1, None, None, None
         few_ctas = self.SCAN_SEGMENT_ALWAYS or segment_tokens is not None or -(-head_dim // 32) * heads * n_seqs < self.num_sms

@@ -98,3 +98,37 @@ def test_bias_and_clamped_gate_in_the_products_epilogues(K, M, N, Kd, bias_dtype
     gate, up = ref[:, :half].clamp(max=2.0), ref[:, half:].clamp(-2.0, 2.0)
     want = gate * torch.sigmoid(1.7 * gate) * (up + 1)
     assert rel_err(K.gate_up_clamp(x, w, b, 2.0, 1.7), want) < 5e-3
+
+
+@pytest.mark.parametrize("heads,P,N,groups,lens", [(4, 64, 128, 2, (33, 1, 64, 65)), (6, 48, 64, 3, (130, 2)), (2, 80, 128, 1, (40,)), (2, 16, 64, 1, (200,))])
+def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
+    """The chunked form against the recurrence in float64: portions that end inside a chunk, single tokens, a padding row, column
+    blocks that are not full, a state to continue from, decays from weak to total."""
+    torch.manual_seed(P)
+    T, C = sum(lens), heads * P + 2 * groups * N
+    xbc = torch.randn(T, C, device="cuda").bfloat16()
+    proj = torch.randn(T, heads + 3, device="cuda") * 2
+    bias, a_log, D = torch.randn(heads, device="cuda") - 2, torch.linspace(-2, 3, heads, device="cuda"), torch.randn(heads, device="cuda")
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    slots = list(range(len(lens)))
+    if len(lens) > 2:
+        slots[1] = -1
+    state = torch.randn(len(lens), heads * N * P + 8, device="cuda")
+    S = state[:, :heads * N * P].double().cpu().view(-1, heads, N, P).clone()
+    xd = xbc.double().cpu()
+    x, B, Cm = xd[:, :heads * P].view(T, heads, P), xd[:, heads * P:heads * P + groups * N].view(T, groups, N), xd[:, heads * P + groups * N:].view(T, groups, N)
+    dt = torch.nn.functional.softplus((proj[:, 3:] + bias).double().cpu())
+    a = torch.exp(-torch.exp(a_log.double().cpu()) * dt)
+    want, rep = torch.zeros(T, heads, P, dtype=torch.float64), heads // groups
+    for s, slot in enumerate(slots):
+        for t in range(cu[s], cu[s + 1]):
+            if slot >= 0:
+                S[s] = a[t][:, None, None] * S[s] + (dt[t][:, None] * B[t].repeat_interleave(rep, 0))[:, :, None] * x[t][:, None, :]
+                want[t] = torch.einsum("hn,hnp->hp", Cm[t].repeat_interleave(rep, 0), S[s]) + D.double().cpu()[:, None] * x[t]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    got = K.ssm_scan(xbc, proj, 3, bias, a_log, D, i32(cu), i32(slots), state, heads, P, N, groups, max_q_len=max(lens), chunked=True)
+    # three bfloat16 terms hold a float: the error is that of float sums over N and 64 products
+    assert rel_err(got, want.view(T, -1)) < 2e-6
+    assert rel_err(state[:, :heads * N * P], S.view(len(lens), -1)) < 2e-6
