@@ -1025,7 +1025,7 @@ class CudaKernels:
             ctypes.c_longlong(state.shape[1]), ctypes.c_longlong(conv_off), _ptr(out), c_int(_DT[out_dtype]), c_int(T),
             c_int(state_slots.shape[0]), c_int(channels), c_int(taps), self._stream())
         _check("causal_conv_silu", st)
-        COUNTERS['launches'] += 1 if taps > 1 else 0
+        COUNTERS['launches'] += 1 if taps > 4 or (taps > 1 and T > 2 * state_slots.shape[0]) else 0
         return out
 
     SCAN_CHUNK_MIN_TOKENS = 32         # tokens of a portion from which the recurrence goes chunk by chunk (32 tokens: 50 us against 85)
@@ -1245,7 +1245,7 @@ class CudaKernels:
             _ptr(u), c_int(self._dt(u, "u")), _ptr(dt_raw), _ptr(dt_bias), _ptr(a), _ptr(bc), c_int(bc.shape[1]), c_int(b_col0),
             c_int(c_col0), _ptr(d_skip), _ptr(z), c_int(self._dt(z, "z")), c_int(z.shape[1]), c_int(z_col0), _ptr(cu_seqlens),
             _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out), c_int(_DT[out_dtype]),
-            c_int(state_slots.shape[0]), c_int(inner), c_int(N), self._stream())
+            c_int(T), c_int(state_slots.shape[0]), c_int(inner), c_int(N), self._stream())
         _check("selective_scan", st)
         return out
 

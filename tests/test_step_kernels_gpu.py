@@ -132,3 +132,49 @@ def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
     # three bfloat16 terms hold a float: the error is that of float sums over N and 64 products
     assert rel_err(got, want.view(T, -1)) < 2e-6
     assert rel_err(state[:, :heads * N * P], S.view(len(lens), -1)) < 2e-6
+
+
+@pytest.mark.parametrize("inner,N,lens", [(70, 16, (1, 5, 16, 17, 35)), (33, 32, (18, 2)), (32, 16, (64,))])
+def test_selective_scan_in_two_roles(K, inner, N, lens):
+    torch.manual_seed(inner)
+    T = sum(lens)
+    u, z = torch.randn(T, inner, device="cuda"), torch.randn(T, inner + 4, device="cuda")
+    raw, bias, A = torch.randn(T, inner, device="cuda"), torch.randn(inner, device="cuda"), -torch.rand(inner, N, device="cuda") * 4
+    bc, D = torch.randn(T, 2 * N + 3, device="cuda"), torch.randn(inner, device="cuda")
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    state = torch.randn(len(lens), inner * N + 4, device="cuda")
+    S = state[:, :inner * N].double().cpu().view(-1, inner, N).clone()
+    dt, b64, u64 = torch.nn.functional.softplus((raw + bias).double().cpu()), bc.double().cpu(), u.double().cpu()
+    want = torch.empty(T, inner, dtype=torch.float64)
+    for s in range(len(lens)):
+        for t in range(cu[s], cu[s + 1]):
+            S[s] = torch.exp(dt[t][:, None] * A.double().cpu()) * S[s] + (dt[t] * u64[t])[:, None] * b64[t, 3:3 + N]
+            want[t] = (S[s] * b64[t, 3 + N:]).sum(1) + D.double().cpu() * u64[t]
+    want *= torch.nn.functional.silu(z[:, 4:].double().cpu())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    got = K.selective_scan(u, raw, bias, A.contiguous(), bc, 3, 3 + N, D, z, 4, i32(cu), i32(list(range(len(lens)))), state, torch.float32)
+    assert rel_err(got, want) < 2e-6 and rel_err(state[:, :inner * N], S.view(len(lens), -1)) < 2e-6
+
+
+@pytest.mark.parametrize("taps,lens", [(4, (1, 1, 1)), (3, (2, 1)), (1, (1,)), (2, (1, 1)), (4, (2,))])
+def test_convolution_of_single_tokens_in_one_launch(K, taps, lens):
+    """One launch for the outputs and the state: the same as a long portion cut into these steps."""
+    torch.manual_seed(taps)
+    T, C = sum(lens), 131
+    proj, w, b = torch.randn(T, C + 5, device="cuda"), torch.randn(C, taps, device="cuda"), torch.randn(C, device="cuda")
+    state = torch.randn(len(lens) + 1, (taps - 1) * C + 7, device="cuda")
+    hist = state[:, 7:].double().cpu().view(len(lens) + 1, taps - 1, C).clone()
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    seq = [s for s, n in enumerate(lens) for _ in range(n)]
+    got = K.causal_conv_silu(proj, 5, C, w, b, i32(seq), i32(cu), i32(list(range(1, len(lens) + 1))), state, 7, torch.float32)
+    for s, n in enumerate(lens):
+        row = torch.cat([hist[s + 1], proj[cu[s]:cu[s + 1], 5:].double().cpu()])
+        for t in range(n):
+            v = b.double().cpu() + (row[t:t + taps] * w.double().cpu().t()).sum(0)
+            assert rel_err(got[cu[s] + t], torch.nn.functional.silu(v)) < 2e-6
+        assert taps == 1 or rel_err(state[s + 1, 7:], row[n:].reshape(-1)) < 1e-7
