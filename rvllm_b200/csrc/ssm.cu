@@ -1196,12 +1196,302 @@ delta_rule_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, c
     }
 }
 
+// The same for keys of 33 to 128 elements and values in multiples of four columns.  What bound the kernel above is shared
+// memory: every warp reads the whole of q and k for the eight columns it holds, 16 wide reads a lane and token.  Here a lane
+// holds 8 entries of FOUR columns: PARTS lanes (8 or 16) share four neighbouring columns, a token costs a lane four wide reads,
+// and the four sums of S^T k are met by a reduction that also deals them out, one column to every PARTS / 4 lanes, which
+// then form that column's u.  S^T q is formed of the state before the token, beside S^T k, and the result is
+// g S^T q + (k . q) u: the chain from token to token is one sum over the lanes, not two.  Four warps walk, four others
+// bring the next chunk, turn q and k into unit vectors and stage them (double buffers, one barrier a chunk).  2,048 tokens of
+// 32 / 16 heads of 128 x 128: 1,051 / 923 us before, 694 / 536 us; portions of 1,024 twice: 569 / 524 and 378 / 350 us.  (The
+// kernel above with more lanes a column - 16 or 8 entries each - is slower: 1,078 and 1,109 us.)
+template <int PARTS>
+struct DeltaStage {
+    static constexpr int ROW = PARTS * 12;                 // 8 entries a lane, 12 floats apart: a lane's reads fall on banks of their own
+    static constexpr int COLS = 4 * (32 / PARTS) * 4;      // columns of a block
+    float q[DR_CHUNK][ROW], k[DR_CHUNK][ROW];
+    float v[DR_CHUNK][COLS];
+    float g[DR_CHUNK], beta[DR_CHUNK], kq[DR_CHUNK];
+};
+
+// four sums over PARTS neighbouring lanes; returns the one of column part / (PARTS / 4)
+template <int PARTS>
+__device__ __forceinline__ float delta_sum4(const float (&v)[4], int part) {
+    const bool hi = part & (PARTS / 2), mid = part & (PARTS / 4);
+    const float k0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], PARTS / 2);
+    const float k1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], PARTS / 2);
+    float r = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, PARTS / 4);
+#pragma unroll
+    for (int o = PARTS / 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
+template <int PARTS>
+__global__ void __launch_bounds__(256)
+delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
+                       int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
+                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    using Stage = DeltaStage<PARTS>;
+    extern __shared__ __align__(16) unsigned char dw_raw[];
+    Stage* stages = reinterpret_cast<Stage*>(dw_raw);      // [2]
+    const int seq = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * Stage::COLS;
+    const int slot = state_slots[seq];
+    if (slot < 0) return;
+    const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    const int chunks = (n_tok + DR_CHUNK - 1) / DR_CHUNK;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 4) {                                        // ---- the walk
+        constexpr int Q = PARTS / 4;                       // lanes of a column after the reduction
+        const int part = lane % PARTS, group = lane / PARTS;
+        const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;      // (vd is a multiple of 4: a group's columns are all there or none)
+        const bool live = col < vd;
+        const int n0 = part * 8, mine = part / Q;          // this lane's column after the reduction
+        float S[8][4];
+        float* srow = state + (size_t)slot * state_stride + (size_t)h * d * vd + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && n0 + i < d) v = *reinterpret_cast<const float4*>(srow + (size_t)(n0 + i) * vd);
+            S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
+        }
+        __syncthreads();                                   // the first chunk is staged
+        for (int c = 0; c < chunks; ++c) {
+            const Stage& st = stages[c & 1];
+            const int t0 = c * DR_CHUNK, nt = min(DR_CHUNK, n_tok - t0);
+            // (threads beyond the last column walk along: the shuffles need every lane)
+            auto step = [&](int tt) {
+                float kr[8], qr[8];
+                *reinterpret_cast<float4*>(kr) = *reinterpret_cast<const float4*>(&st.k[tt][part * 12]);
+                *reinterpret_cast<float4*>(kr + 4) = *reinterpret_cast<const float4*>(&st.k[tt][part * 12 + 4]);
+                *reinterpret_cast<float4*>(qr) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12]);
+                *reinterpret_cast<float4*>(qr + 4) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12 + 4]);
+                const float g = st.g[tt], vv = st.v[tt][cb + mine];
+                float ak[4], aq[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { ak[j] = S[0][j] * kr[0]; aq[j] = S[0][j] * qr[0]; }
+#pragma unroll
+                for (int i = 1; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { ak[j] = fmaf(S[i][j], kr[i], ak[j]); aq[j] = fmaf(S[i][j], qr[i], aq[j]); }
+                const float acc = delta_sum4<PARTS>(ak, part);
+                const float u = st.beta[tt] * (vv - g * acc);
+                float uj[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) uj[j] = __shfl_sync(0xffffffffu, u, group * PARTS + j * Q);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) S[i][j] = fmaf(g, S[i][j], kr[i] * uj[j]);
+                const float ov = delta_sum4<PARTS>(aq, part);
+                if (part % Q == 0 && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
+            };
+            if (nt == DR_CHUNK) {                          // a whole chunk: neighbouring tokens may run into one another
+#pragma unroll 4
+                for (int tt = 0; tt < DR_CHUNK; ++tt) step(tt);
+            } else {
+                for (int tt = 0; tt < nt; ++tt) step(tt);
+            }
+            __syncthreads();                               // this chunk is walked, the next one staged
+        }
+        if (live) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (n0 + i < d) *reinterpret_cast<float4*>(srow + (size_t)(n0 + i) * vd) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+        }
+        return;
+    }
+    // ---- staging: a warp per token for q and k, the block's columns of v, a thread per token for g and beta
+    const int tid = threadIdx.x - 128, sw = warp - 4;
+    const int kh = h / (heads / qk_heads), qk = qk_heads * d;
+    const float q_scale = rsqrtf((float)d);
+    const float decay_rate = expf(a_log[h]), a_bias = dt_bias[h];
+    constexpr int E = PARTS / 4;                           // elements of q (and k) per lane: 8 PARTS / 32
+    constexpr int PV = DR_CHUNK * Stage::COLS / 128;
+    uint32_t pq[DR_CHUNK / 4][E], pk[DR_CHUNK / 4][E], pv[PV];      // raw bits: converted when their chunk's turn comes
+    float pb = 0.f, pa = 0.f;
+    auto load_chunk = [&](int c) {
+        const int t0 = c * DR_CHUNK, nt = min(DR_CHUNK, n_tok - t0);
+#pragma unroll
+        for (int x = 0; x < DR_CHUNK / 4; ++x) {
+            const int tt = sw + 4 * x;
+            const size_t row = (size_t)(start + t0 + tt) * qkv_stride + (size_t)kh * d;
+#pragma unroll
+            for (int y = 0; y < E; ++y) {
+                const int e = lane + 32 * y;
+                pq[x][y] = 0; pk[x][y] = 0;
+                if (tt < nt && e < d) {
+                    pq[x][y] = rv_load_raw(qkv, qkv_dtype, row + e);
+                    pk[x][y] = rv_load_raw(qkv, qkv_dtype, row + qk + e);
+                }
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < PV; ++y) {
+            const int i = tid + 128 * y, tt = i / Stage::COLS, cc = col0 + i % Stage::COLS;
+            pv[y] = 0;
+            if (tt < nt && cc < vd) pv[y] = rv_load_raw(qkv, qkv_dtype, (size_t)(start + t0 + tt) * qkv_stride + 2 * qk + (size_t)h * vd + cc);
+        }
+        if (tid < nt) {
+            const size_t row = (size_t)(start + t0 + tid) * proj_stride;
+            pb = proj[row + b_col0 + h];
+            pa = proj[row + a_col0 + h];
+        }
+    };
+    auto stage = [&](int c) {
+        Stage& st = stages[c & 1];
+        float sq[DR_CHUNK / 4], sk[DR_CHUNK / 4], sx[DR_CHUNK / 4];
+#pragma unroll
+        for (int x = 0; x < DR_CHUNK / 4; ++x) {           // (beyond the sequence: zeros)
+            sq[x] = sk[x] = sx[x] = 0.f;
+#pragma unroll
+            for (int y = 0; y < E; ++y) {
+                const float fq = rv_raw_value(pq[x][y], qkv_dtype), fk = rv_raw_value(pk[x][y], qkv_dtype);
+                sq[x] = fmaf(fq, fq, sq[x]); sk[x] = fmaf(fk, fk, sk[x]); sx[x] = fmaf(fk, fq, sx[x]);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int x = 0; x < DR_CHUNK / 4; ++x) {
+                sq[x] += __shfl_xor_sync(0xffffffffu, sq[x], o);
+                sk[x] += __shfl_xor_sync(0xffffffffu, sk[x], o);
+                sx[x] += __shfl_xor_sync(0xffffffffu, sx[x], o);
+            }
+#pragma unroll
+        for (int x = 0; x < DR_CHUNK / 4; ++x) {
+            const int tt = sw + 4 * x;
+            const float rq = q_scale / sqrtf(sq[x] + unit_eps), rk = 1.0f / sqrtf(sk[x] + unit_eps);
+            if (lane == 0) st.kq[tt] = sx[x] * rq * rk;
+#pragma unroll
+            for (int y = 0; y < E; ++y) {
+                const int e = lane + 32 * y, at = (e >> 3) * 12 + (e & 7);
+                st.q[tt][at] = rv_raw_value(pq[x][y], qkv_dtype) * rq;
+                st.k[tt][at] = rv_raw_value(pk[x][y], qkv_dtype) * rk;
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < PV; ++y) st.v[(tid + 128 * y) / Stage::COLS][(tid + 128 * y) % Stage::COLS] = rv_raw_value(pv[y], qkv_dtype);
+        if (tid < DR_CHUNK) {
+            const float a = pa + a_bias;
+            const float sp = a > 20.f ? a : log1pf(expf(a));
+            st.beta[tid] = 1.0f / (1.0f + expf(-pb));
+            st.g[tid] = expf(-decay_rate * sp);
+        }
+    };
+    if (chunks > 0) { load_chunk(0); stage(0); }
+    if (chunks > 1) load_chunk(1);
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {                     // while chunk c is walked: c + 1 in, c + 2 on its way
+        if (c + 1 < chunks) {
+            stage(c + 1);
+            if (c + 2 < chunks) load_chunk(c + 2);
+        }
+        __syncthreads();
+    }
+}
+
+// Steps of few tokens a sequence: a block per (128 columns of a head, sequence), a thread on four neighbouring columns of 16 rows,
+// all its rows in flight together.  Bound by the state's way from memory and back: 64 sequences of 32 heads of 128 x 128
+// (268 MB) 130 us with the walk's set-up around one token, 57 us; 4 sequences 13.8 and 9.9 us of a decode step.
+__global__ void __launch_bounds__(256)
+delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
+                       int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
+                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    __shared__ __align__(16) float sq[128], sk[128], su[128];
+    __shared__ __align__(16) float pk[8][128], pq[8][128];
+    __shared__ float sums[3][4];
+    const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int slot = state_slots[seq];
+    if (slot < 0) return;
+    const int start = cu_seqlens[seq], end = cu_seqlens[seq + 1];
+    const int cl = lane * 4, col = blockIdx.x * 128 + cl, n0 = warp * 16;
+    const bool live = col < vd;
+    const int kh = h / (heads / qk_heads), qk = qk_heads * d;
+    float* srow = state + (size_t)slot * state_stride + (size_t)h * d * vd + col;
+    float4 S[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) S[i] = live && n0 + i < d ? *reinterpret_cast<const float4*>(srow + (size_t)(n0 + i) * vd) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = start; t < end; ++t) {
+        const size_t row = (size_t)t * qkv_stride;
+        float fq = 0.f, fk = 0.f;
+        if (tid < 128) {
+            if (tid < d) {
+                fq = rv_load_any(qkv, qkv_dtype, row + (size_t)kh * d + tid);
+                fk = rv_load_any(qkv, qkv_dtype, row + qk + (size_t)kh * d + tid);
+            }
+            const float q2 = rv_warp_sum(fq * fq), k2 = rv_warp_sum(fk * fk), kq = rv_warp_sum(fk * fq);
+            if (lane == 0) { sums[0][warp] = q2; sums[1][warp] = k2; sums[2][warp] = kq; }
+        }
+        __syncthreads();
+        const float rq = rsqrtf((float)d) / sqrtf(sums[0][0] + sums[0][1] + sums[0][2] + sums[0][3] + unit_eps);
+        const float rk = 1.0f / sqrtf(sums[1][0] + sums[1][1] + sums[1][2] + sums[1][3] + unit_eps);
+        if (tid < 128) { sq[tid] = fq * rq; sk[tid] = fk * rk; su[tid] = 0.f; }
+        const float a = proj[(size_t)t * proj_stride + a_col0 + h] + dt_bias[h];
+        const float sp = a > 20.f ? a : log1pf(expf(a));
+        const float g = expf(-expf(a_log[h]) * sp);
+        __syncthreads();
+        float4 ak = make_float4(0.f, 0.f, 0.f, 0.f), aq = ak;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float k = sk[n0 + i], q = sq[n0 + i];
+            ak.x = fmaf(S[i].x, k, ak.x); ak.y = fmaf(S[i].y, k, ak.y); ak.z = fmaf(S[i].z, k, ak.z); ak.w = fmaf(S[i].w, k, ak.w);
+            aq.x = fmaf(S[i].x, q, aq.x); aq.y = fmaf(S[i].y, q, aq.y); aq.z = fmaf(S[i].z, q, aq.z); aq.w = fmaf(S[i].w, q, aq.w);
+        }
+        *reinterpret_cast<float4*>(&pk[warp][cl]) = ak;
+        *reinterpret_cast<float4*>(&pq[warp][cl]) = aq;
+        __syncthreads();
+        if (tid < 128 && blockIdx.x * 128 + tid < vd) {
+            const int c = blockIdx.x * 128 + tid;
+            float kv = 0.f, qv = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) { kv += pk[w][tid]; qv += pq[w][tid]; }
+            const float beta = 1.0f / (1.0f + expf(-proj[(size_t)t * proj_stride + b_col0 + h]));
+            const float u = beta * (rv_load_any(qkv, qkv_dtype, row + 2 * qk + (size_t)h * vd + c) - g * kv);
+            const float kq = (sums[2][0] + sums[2][1] + sums[2][2] + sums[2][3]) * rq * rk;
+            su[tid] = u;
+            out[((size_t)t * heads + h) * vd + c] = fmaf(g, qv, kq * u);
+        }
+        __syncthreads();
+        const float4 u = *reinterpret_cast<const float4*>(&su[cl]);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float k = sk[n0 + i];
+            S[i].x = fmaf(g, S[i].x, k * u.x); S[i].y = fmaf(g, S[i].y, k * u.y);
+            S[i].z = fmaf(g, S[i].z, k * u.z); S[i].w = fmaf(g, S[i].w, k * u.w);
+        }
+        __syncthreads();                                   // sums, sk and su are written again for the next token
+    }
+    if (live && end > start) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (n0 + i < d) *reinterpret_cast<float4*>(srow + (size_t)(n0 + i) * vd) = S[i];
+    }
+}
+
+template <int PARTS>
+static int launch_delta_walk(cudaStream_t stream, int n_seqs, int heads, int vd, const void* qkv, int qkv_dtype, int qkv_stride, const float* proj,
+                             int proj_stride, int b_col0, int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens,
+                             const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps) {
+    constexpr int smem = 2 * (int)sizeof(DeltaStage<PARTS>), cols = DeltaStage<PARTS>::COLS;
+    static RvPerDevice once;
+    if (int st = rv_configure_smem(once, delta_rule_walk_kernel<PARTS>, smem)) return st;
+    return rv_launch(delta_rule_walk_kernel<PARTS>, dim3((vd + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, qkv, qkv_dtype,
+                     qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, state_stride, out, heads,
+                     qk_heads, d, vd, unit_eps);
+}
+
 // qkv rows: [q: qk_heads x d | k: qk_heads x d | v: heads x vd] (after the convolution); the logits of beta and of the
-// decay are float columns b_col0 .. and a_col0 .. of `proj`; out: float [tokens, heads x vd].
+// decay are float columns b_col0 .. and a_col0 .. of `proj`; out: float [n_tokens, heads x vd].
 RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, const float* proj, int proj_stride, int b_col0,
                             int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens, const int* state_slots,
                             float* state, long long state_stride, float* out, int n_seqs, int heads, int qk_heads, int d, int vd,
-                            float unit_eps, cudaStream_t stream) {
+                            float unit_eps, int n_tokens, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || qk_heads <= 0 || heads % qk_heads || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 ||
         heads > 65535)
         return RV_ERR_BAD_SIZE;
@@ -1210,6 +1500,20 @@ RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, cons
         return RV_ERR_BAD_SIZE;
     if (qkv_dtype & ~1) return RV_ERR_BAD_DTYPE;
     if (n_seqs == 0) return RV_OK;
+    const bool words = vd % 4 == 0 && state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;      // whole words of four columns
+    if (words && d <= 128 && n_tokens <= 2LL * n_seqs) {
+        RV_LAUNCH_ST = rv_launch(delta_rule_step_kernel, dim3((vd + 127) / 128, heads, n_seqs), dim3(256), 0, stream, qkv, qkv_dtype, qkv_stride, proj,
+                                 proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, (size_t)state_stride, out, heads,
+                                 qk_heads, d, vd, unit_eps);
+        return rv_launch_status();
+    }
+    if (words && d > 32 && d <= 128) {
+        RV_LAUNCH_ST = d > 64 ? launch_delta_walk<16>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
+                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps)
+                              : launch_delta_walk<8>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
+                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps);
+        return rv_launch_status();
+    }
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128
     int parts = 1;
     while (parts * ns < d) parts <<= 1;                // a power of two of at most 32 lanes of one warp

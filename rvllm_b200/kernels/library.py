@@ -1265,7 +1265,7 @@ class CudaKernels:
             _ptr(qkv), c_int(self._dt(qkv, "qkv")), c_int(qkv.shape[1]), _ptr(proj), c_int(proj.shape[1]), c_int(b_col0), c_int(a_col0),
             _ptr(a_log), _ptr(dt_bias), _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out),
             c_int(state_slots.shape[0]), c_int(heads), c_int(qk_heads), c_int(head_dim), c_int(value_dim), c_float(unit_eps),
-            self._stream())
+            c_int(T), self._stream())
         _check("delta_rule", st)
         return out
 

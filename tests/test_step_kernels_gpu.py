@@ -178,3 +178,35 @@ def test_convolution_of_single_tokens_in_one_launch(K, taps, lens):
             v = b.double().cpu() + (row[t:t + taps] * w.double().cpu().t()).sum(0)
             assert rel_err(got[cu[s] + t], torch.nn.functional.silu(v)) < 2e-6
         assert taps == 1 or rel_err(state[s + 1, 7:], row[n:].reshape(-1)) < 1e-7
+
+
+@pytest.mark.parametrize("d,vd,heads,qk,lens", [(128, 128, 4, 2, (1, 15, 16, 17, 70)), (100, 36, 2, 1, (33,)), (64, 68, 2, 2, (20, 1)), (40, 4, 2, 1, (18,)),
+                                                (128, 128, 4, 2, (1, 1, 1)), (100, 132, 2, 1, (2,)), (24, 8, 2, 2, (1, 2, 1))])
+def test_delta_rule_of_portions_and_of_single_tokens(K, d, vd, heads, qk, lens):
+    torch.manual_seed(d + vd)
+    T = sum(lens)
+    qkv, proj = torch.randn(T, 2 * qk * d + heads * vd, device="cuda"), torch.randn(T, 2 * heads + 1, device="cuda")
+    a_log, bias = torch.randn(heads, device="cuda"), torch.randn(heads, device="cuda")
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    state = torch.randn(len(lens), heads * d * vd + 4, device="cuda")
+    S = state[:, :heads * d * vd].double().cpu().view(-1, heads, d, vd).clone()
+    f = qkv.double().cpu()
+    rep = heads // qk
+    q, k = (f[:, i * qk * d:(i + 1) * qk * d].view(T, qk, d).repeat_interleave(rep, 1) for i in (0, 1))
+    v = f[:, 2 * qk * d:].view(T, heads, vd)
+    q, k = q / (q.square().sum(-1, keepdim=True) + 1e-6).sqrt() * d ** -0.5, k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    beta = torch.sigmoid(proj[:, 1:1 + heads].double().cpu())
+    g = torch.exp(-torch.exp(a_log.double().cpu()) * torch.nn.functional.softplus((proj[:, 1 + heads:] + bias).double().cpu()))
+    want = torch.empty(T, heads, vd, dtype=torch.float64)
+    for s in range(len(lens)):
+        for t in range(cu[s], cu[s + 1]):
+            S[s] = g[t][:, None, None] * S[s]
+            un = beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S[s], k[t]))
+            S[s] = S[s] + k[t][:, :, None] * un[:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", S[s], q[t])
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
+    got = K.delta_rule(qkv, proj, 1, 1 + heads, a_log, bias, i32(cu), i32(list(range(len(lens)))), state, heads, qk, d, vd, 1e-6)
+    # float sums of d products along a chain of at most 70 tokens
+    assert rel_err(got, want.view(T, -1)) < 3e-6 and rel_err(state[:, :heads * d * vd], S.view(len(lens), -1)) < 3e-6
