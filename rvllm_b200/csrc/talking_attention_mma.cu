@@ -17,7 +17,7 @@
 #include <mma.h>
 
 #define TA_BN 32
-#define TA_MAX_WARPS 8
+#define TA_MAX_WARPS 16
 
 __device__ __forceinline__ void tm_ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
@@ -81,8 +81,8 @@ __device__ __forceinline__ void tm_fetch(__nv_bfloat16* dst, const TmArgs& a, co
     }
 }
 
-template <int HD, int VD>
-__global__ void __launch_bounds__(TA_MAX_WARPS * 32)
+template <int HD, int VD, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 talking_attention_mma_kernel(const TmArgs a) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
@@ -334,43 +334,55 @@ talking_attention_mma_kernel(const TmArgs a) {
     }
 }
 
-static RvPerDevice g_tm_once[2];
+static RvPerDevice g_tm_once[4];
 
 // 1 if the sizes fit this build (the caller falls back to the plain kernel otherwise).
 RV_EXPORT int rv_talking_attention_mma_fits(int nh, int nkv, int hd, int vd) {
     if (nh <= 0 || nkv <= 0 || nh % nkv) return 0;
     const int rep = nh / nkv;
-    if (rep > 16 || (16 % rep) || nkv > TA_MAX_WARPS) return 0;
+    if (rep > 16 || (16 % rep) || nkv > 8) return 0;
     if (hd % 16 || vd % 16 || hd > 128 || vd > 128 || hd < 16 || vd < 16) return 0;
     return 1;
 }
 
 RV_EXPORT int rv_talking_attention_mma(const void* q, const void* cache, const int* block_tables, const int* cu_seqlens, const int* ctx_lens,
                                        void* out, int n_seqs, int max_q_len, int nh, int nkv, int hd, int vd, int page_size, int max_blocks,
-                                       float scale, const float* r1, const float* r2, const float* talk, int chunk, cudaStream_t stream) {
+                                       float scale, const float* r1, const float* r2, const float* talk, int chunk, int max_warps, cudaStream_t stream) {
     if (!rv_talking_attention_mma_fits(nh, nkv, hd, vd)) return RV_ERR_UNSUPPORTED;
     if (n_seqs < 0 || max_q_len < 0 || page_size <= 0 || max_blocks <= 0 || n_seqs > 65535) return RV_ERR_BAD_SIZE;
+    if (max_warps != 0 && max_warps != 8 && max_warps != 16) return RV_ERR_BAD_SIZE;
     if ((r1 == nullptr) != (r2 == nullptr)) return RV_ERR_BAD_SIZE;
     if (((uintptr_t)cache | (uintptr_t)q | (uintptr_t)out) % 16) return RV_ERR_ALIGNMENT;
     if (n_seqs == 0 || max_q_len == 0) return RV_OK;
     const int rep = nh / nkv, TOK = 16 / rep;
-    int tg = TA_MAX_WARPS / nkv;
-    while (tg > 1 && (tg - 1) * TOK >= max_q_len) --tg;             // no token groups beyond the longest portion
-    const int CT = tg * TOK, warps = tg * nkv, nh4 = (nh + 3) & ~3;
-    const size_t smem = 2 * ((size_t)nkv * TA_BN * (hd + 8) + (size_t)nkv * TA_BN * (vd + 8) + (size_t)warps * 16 * (TA_BN + 8)) +
-                        4 * ((size_t)nh * CT * TA_BN + (size_t)nh * nh4);
+    // Sixteen warps are one CTA per SM of twice the tokens behind the same tiles; eight are more CTAs, which even out better.
+    // Sixteen where they still leave one and a half CTAs per SM: 2,048 tokens of 32 heads on 8: 976 us against 1,315; of 16
+    // heads on 4 they leave 128 CTAs: 704 against 491.  (max_warps 0: this rule; 8 or 16.)
+    const int nh4 = (nh + 3) & ~3;
+    int tg = 1;
+    size_t smem = 0;
+    for (int limit = max_warps ? max_warps : TA_MAX_WARPS;; limit = 8) {
+        tg = limit / nkv;
+        while (tg > 1 && (tg - 1) * TOK >= max_q_len) --tg;         // no token groups beyond the longest portion
+        const int ct = tg * TOK, w = tg * nkv;
+        smem = 2 * ((size_t)nkv * TA_BN * (hd + 8) + (size_t)nkv * TA_BN * (vd + 8) + (size_t)w * 16 * (TA_BN + 8)) +
+               4 * ((size_t)nh * ct * TA_BN + (size_t)nh * nh4);
+        const bool filled = max_warps != 0 || 2LL * ((max_q_len + ct - 1) / ct) * n_seqs >= 3LL * rv_sm_count();
+        if (limit == 8 || (filled && smem <= 220 * 1024)) break;
+    }
     if (smem > 220 * 1024) return RV_ERR_UNSUPPORTED;
+    const int CT = tg * TOK, warps = tg * nkv;
     TmArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, block_tables, cu_seqlens, ctx_lens, (__nv_bfloat16*)out, r1, r2, talk,
              nh, nkv, hd, vd, page_size, max_blocks, chunk, tg, scale};
     const dim3 grid((max_q_len + CT - 1) / CT, n_seqs);
-    if (hd <= 64 && vd <= 64) {
-        const int st = rv_configure_smem(g_tm_once[0], talking_attention_mma_kernel<64, 64>, 220 * 1024);
-        if (st != RV_OK) return st;
-        RV_LAUNCH_ST = rv_launch(talking_attention_mma_kernel<64, 64>, grid, dim3(warps * 32), smem, stream, a);
-    } else {
-        const int st = rv_configure_smem(g_tm_once[1], talking_attention_mma_kernel<128, 128>, 220 * 1024);
-        if (st != RV_OK) return st;
-        RV_LAUNCH_ST = rv_launch(talking_attention_mma_kernel<128, 128>, grid, dim3(warps * 32), smem, stream, a);
-    }
+#define TA_LAUNCH(I, HD, VD, W)                                                                                             \
+    do {                                                                                                                        \
+        const int st = rv_configure_smem(g_tm_once[I], talking_attention_mma_kernel<HD, VD, W>, 220 * 1024);                    \
+        if (st != RV_OK) return st;                                                                                             \
+        RV_LAUNCH_ST = rv_launch(talking_attention_mma_kernel<HD, VD, W>, grid, dim3(warps * 32), smem, stream, a);             \
+    } while (0)
+    if (hd <= 64 && vd <= 64) { if (warps > 8) TA_LAUNCH(0, 64, 64, 16); else TA_LAUNCH(1, 64, 64, 8); }
+    else { if (warps > 8) TA_LAUNCH(2, 128, 128, 16); else TA_LAUNCH(3, 128, 128, 8); }
+#undef TA_LAUNCH
     return rv_launch_status();
 }

@@ -78,9 +78,11 @@ class CudaKernels:
     NARROW_TILES = True                # ... with tiles of 128 columns where those of 256 would occupy at most half of the SMs
     PAIR_GEMM = True                   # the tcgen05 GEMM runs on pairs of CTAs (cta_group::2) where the rows fill its 256-row tiles
     TALKING_MMA = True                 # attention with mixed head weights: bfloat16 prompt portions go to the tensor-core kernel when it fits
+    TALKING_WARPS = 0                  # ... whose CTAs have up to 8 or 16 warps (0: by the number of CTAs)
     TALKING_SPLIT = True               # attention with mixed head weights: few tokens behind many keys go to the split-key kernels
     TALKING_SPLIT_MAX_TOKENS = 64      # ... up to this many tokens in the step
-    TALKING_SPLIT_SPAN = 64            # ... in ranges of a multiple of this many keys
+    TALKING_SPLIT_MIN_KEYS = 64        # ... behind more than this many keys
+    TALKING_SPLIT_SPAN = 32            # ... in ranges of a multiple of this many keys (four tokens at 1,500 keys: 64 takes 41 us a layer, 32 takes 32)
     TALKING_SPLIT_MAX_SCRATCH = 512 << 20   # ... while the scores of the step fit this many bytes of scratch
     TCGEN05_ATTENTION = True           # prompt portions go to the tcgen05 attention kernel when it fits
     TCGEN05_ATTENTION_MIN_TOKENS = 16  # ... from this many tokens in the longest portion of the step
@@ -1323,7 +1325,7 @@ class CudaKernels:
         out = torch.empty((T, num_heads * value_dim), dtype=q.dtype, device=q.device)
         visible = min(meta.max_ctx_len, chunk) if chunk else meta.max_ctx_len
         if self.TALKING_SPLIT and 0 < T and (T <= self.TALKING_SPLIT_MAX_TOKENS or meta.max_q_len == 1) \
-                and visible > self.TALKING_SPLIT_SPAN and num_heads * head_dim * 4 <= 48 * 1024 \
+                and visible > self.TALKING_SPLIT_MIN_KEYS and num_heads * head_dim * 4 <= 48 * 1024 \
                 and T * num_heads * (visible + 64) * 4 <= self.TALKING_SPLIT_MAX_SCRATCH:
             # few tokens behind many keys (or single tokens only): the keys of a token are cut over CTAs, into as many
             # ranges as give the GPU about two CTAs an SM (at most 64), each a multiple of TALKING_SPLIT_SPAN keys
@@ -1348,7 +1350,8 @@ class CudaKernels:
                 st = lib.rv_talking_attention_mma(
                     _ptr(q), _ptr(cache_layer), _ptr(meta.block_tables), _ptr(meta.cu_seqlens), _ptr(meta.ctx_lens), _ptr(out),
                     c_int(meta.num_seqs), c_int(meta.max_q_len), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim),
-                    c_int(ps), c_int(meta.max_blocks), c_float(scale), _ptr(r1), _ptr(r2), _ptr(talk), c_int(chunk or 0), self._stream())
+                    c_int(ps), c_int(meta.max_blocks), c_float(scale), _ptr(r1), _ptr(r2), _ptr(talk), c_int(chunk or 0),
+                    c_int(self.TALKING_WARPS), self._stream())
                 if st != -4:            # (-4: the tiles of these sizes do not fit the shared memory; the plain kernel takes them)
                     _check("talking_attention_mma", st)
                     return out

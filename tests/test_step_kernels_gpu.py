@@ -210,3 +210,23 @@ def test_delta_rule_of_portions_and_of_single_tokens(K, d, vd, heads, qk, lens):
     got = K.delta_rule(qkv, proj, 1, 1 + heads, a_log, bias, i32(cu), i32(list(range(len(lens)))), state, heads, qk, d, vd, 1e-6)
     # float sums of d products along a chain of at most 70 tokens
     assert rel_err(got, want.view(T, -1)) < 3e-6 and rel_err(state[:, :heads * d * vd], S.view(len(lens), -1)) < 3e-6
+
+
+def test_talking_attention_on_eight_and_sixteen_warps(K):
+    """The same tiles for twice the tokens a CTA: the same bits."""
+    from rvllm_b200.kernels.library import AttentionMeta
+    torch.manual_seed(3)
+    nh, nkv, hd, ps, T = 8, 4, 64, 16, 75
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    cache = torch.randn(5, nkv * ps * 2 * hd, device="cuda").bfloat16()
+    meta = AttentionMeta(block_tables=i32([[3, 1, 0, 4, 2]]), cu_seqlens=i32([0, T]), ctx_lens=i32([T]), token_seq=i32([0] * T), slot_mapping=i32([0] * T),
+                         num_seqs=1, max_q_len=T, max_ctx_len=T, page_size=ps)
+    q = torch.randn(T, nh * hd, device="cuda").bfloat16()
+    r, talk = torch.rand(nh, device="cuda"), torch.randn(nh, nh, device="cuda")
+    out = []
+    try:
+        for K.TALKING_WARPS in (8, 16):
+            out.append(K.talking_attention(q, cache, meta, None, nh, nkv, hd, hd, hd ** -0.5, r, r, talk, None))
+    finally:
+        del K.TALKING_WARPS
+    assert torch.equal(*out)
