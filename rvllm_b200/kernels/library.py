@@ -619,17 +619,28 @@ class CudaKernels:
         return 1
 
     def _prefill_gemm_lib(self, M: int, pair=None, N: int = 0, gated: bool = False, head_dim: int = 0):
-        """The tcgen05 GEMM library for M rows: built for pairs of CTAs (tiles of 256 rows) unless the
-        last tile's second half would be empty, or for one CTA per tile (tiles of 128 rows); with
-        tiles of 128 columns instead of 256 where the wide ones would leave half of the workers without
-        a tile (N given: a few hundred rows of a product with few weight rows)."""
+        """The tcgen05 GEMM library for M rows and N weight rows: built for pairs of CTAs (tiles of 256 rows) or for one CTA per
+        tile (tiles of 128 rows), whichever takes less by the rounds of its persistent workers; with tiles of 128 columns
+        instead of 256 where the wide ones leave half of the workers without a tile (N given: a few hundred rows of a
+        product with few weight rows).
+
+        A round of the pairs takes 0.88 of a round of single CTAs (both SMs' tiles share the weights; 0.96 with the gated epilogue):
+        3584 x 18944 at 1,304 rows, two rounds each: 207 against 227 us; gated 37888 x 3584, 12 rounds against 11: 316 against
+        286 us.  Half of the workers means half: tiles of 128 columns beyond that start a second round (4096 x 14336 at
+        520 rows: 160 tiles on 148 SMs took 173 us, 48 pairs of wide tiles take 99)."""
         if pair is None:
             pair = self.PAIR_GEMM and (M % 256 == 0 or M % 256 > 128)
+            if self.PAIR_GEMM and N:
+                columns = -(-(N // 2) // 128) if gated else -(-N // 256)
+                tiles = -(-M // 128) * columns
+                if not pair and 2 * tiles > self.num_sms:       # (else: one round of narrow tiles on single CTAs)
+                    single, double = -(-tiles // self.num_sms), -(-(-(-M // 256) * columns) // (self.num_sms // 2))
+                    pair = double * (96 if gated else 88) <= single * 100
         defines = ("-DRV_PAIR=1",) if pair else ()
         if N and self.NARROW_TILES and head_dim <= 128:        # (a head's rotation pairs lie in one tile)
             rows, workers = (256, self.num_sms // 2) if pair else (128, self.num_sms)
             tiles = -(-M // rows) * (-(-(N // 2) // 128) if gated else -(-N // 256))
-            if 2 * tiles <= workers + workers // 8:
+            if 2 * tiles <= workers:
                 defines = defines + ("-DBN=128",)
         return self._lib("gemm_tcgen05.cu", defines)
 
