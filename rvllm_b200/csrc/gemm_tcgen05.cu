@@ -142,8 +142,9 @@ __device__ __forceinline__ float gate_act(float g, int act) {
     return act == 1 ? g / (1.0f + expf(-1.5957691216057308f * (g + 0.044715f * g * g * g))) : silu_f(g);
 }
 // a gated result: act(gate) up, or (act 3) g sigmoid(alpha g) (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit)
+template <bool EXTRAS>
 __device__ __forceinline__ float gated_value(const GemmParams& p, float g, float u) {
-    if (p.act == 3) {
+    if (EXTRAS && p.act == 3) {
         g = fminf(g, p.limit);
         u = fminf(fmaxf(u, -p.limit), p.limit);
         return g / (1.0f + expf(-p.alpha * g)) * (u + 1.0f);
@@ -296,6 +297,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
     else tcgen05_commit(bar);
 }
 
+// EXTRAS: a bias outside the rotary epilogue, or the clamped gate.  Built apart: the tests for them in the other epilogues cost 1 to
+// 2 % of a prompt's products.
+template <bool EXTRAS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const GemmParams p) {
@@ -560,7 +564,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tmem_ld_wait();
                     if (m < p.M) {
                         const int n = n_out0 + c;
-                        if (p.bias) {
+                        if (EXTRAS && p.bias) {
                             add_bias(p, g, n, half_n);
                             add_bias(p, u, half_n + n, p.N);
                         }
@@ -573,8 +577,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) {
                                     const int e = v * 8 + 2 * j;
-                                    oh[j] = __floats2bfloat162_rn(gated_value(p, __uint_as_float(g[e]), __uint_as_float(u[e])),
-                                                                  gated_value(p, __uint_as_float(g[e + 1]), __uint_as_float(u[e + 1])));
+                                    oh[j] = __floats2bfloat162_rn(gated_value<EXTRAS>(p, __uint_as_float(g[e]), __uint_as_float(u[e])),
+                                                                  gated_value<EXTRAS>(p, __uint_as_float(g[e + 1]), __uint_as_float(u[e + 1])));
                                 }
                                 *reinterpret_cast<uint4*>(dst + v * 8) = o;
                             }
@@ -582,7 +586,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                             for (int e = 0; e < 32; ++e) {
                                 if (n + e >= half_n) continue;
-                                const float val = gated_value(p, __uint_as_float(g[e]), __uint_as_float(u[e]));
+                                const float val = gated_value<EXTRAS>(p, __uint_as_float(g[e]), __uint_as_float(u[e]));
                                 if (p.out_f32) ((float*)p.out)[(size_t)m * half_n + n + e] = val;
                                 else ((__nv_bfloat16*)p.out)[(size_t)m * half_n + n + e] = __float2bfloat16_rn(val);
                             }
@@ -620,7 +624,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     load_acc(c, r);
                     if (m < p.M) {
                         const int n = n0 + c;
-                        if (p.bias) add_bias(p, r, n, p.N);
+                        if (EXTRAS && p.bias) add_bias(p, r, n, p.N);
                         const bool vec = n + 32 <= p.N && (p.N & 7) == 0 && wide_ok;
                         if (vec && !p.out_f32) {
                             __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)m * ldc + coff + n;
@@ -684,18 +688,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
 // ---------------------------------------------------------------- host side
 // One CTA per tile and SM, or (RV_PAIR) one cluster of two CTAs per tile and pair of SMs.
-static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int max_ctas, cudaStream_t stream) {
+template <bool EXTRAS>
+static int launch_gemm_as(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int max_ctas, cudaStream_t stream) {
     const int smem = STAGES * STAGE_BYTES + 1024;
     // (the largest a launch may ask for: the pieces of an exchange between four CTAs)
     const int most_pieces = 2 * 3 * BM * (BN / 4 + 4) * 4 + 1024;
     static RvPerDevice configured;
-    if (int e = rv_configure_smem(configured, gemm_tcgen05_kernel, most_pieces > smem ? most_pieces : smem)) return e;
+    if (int e = rv_configure_smem(configured, gemm_tcgen05_kernel<EXTRAS>, most_pieces > smem ? most_pieces : smem)) return e;
     int workers = p.m_tiles * p.n_tiles;
 #if !RV_PAIR
     if (p.splits > 1) {      // one cluster of `splits` CTAs per tile; the pieces of the exchange lie where the stages were
         const int pieces = 2 * (p.splits - 1) * BM * (BN / p.splits + 4) * 4 + 1024;
         const int split_smem = pieces > smem ? pieces : smem;
-        RV_LAUNCH_ST = rv_launch_cluster(gemm_tcgen05_kernel, dim3(workers * p.splits), dim3(NUM_THREADS), split_smem, stream,
+        RV_LAUNCH_ST = rv_launch_cluster(gemm_tcgen05_kernel<EXTRAS>, dim3(workers * p.splits), dim3(NUM_THREADS), split_smem, stream,
                                          (unsigned)p.splits, map_a, map_b, p);
         return rv_launch_status();
     }
@@ -704,11 +709,16 @@ static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const
     if (workers > limit) workers = limit;
     if (workers < 1) workers = 1;
 #if RV_PAIR
-    RV_LAUNCH_ST = rv_launch_cluster(gemm_tcgen05_kernel, dim3(2 * workers), dim3(NUM_THREADS), smem, stream, 2u, map_a, map_b, p);
+    RV_LAUNCH_ST = rv_launch_cluster(gemm_tcgen05_kernel<EXTRAS>, dim3(2 * workers), dim3(NUM_THREADS), smem, stream, 2u, map_a, map_b, p);
 #else
-    RV_LAUNCH_ST = rv_launch(gemm_tcgen05_kernel, dim3(workers), dim3(NUM_THREADS), smem, stream, map_a, map_b, p);
+    RV_LAUNCH_ST = rv_launch(gemm_tcgen05_kernel<EXTRAS>, dim3(workers), dim3(NUM_THREADS), smem, stream, map_a, map_b, p);
 #endif
     return rv_launch_status();
+}
+
+static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int max_ctas, cudaStream_t stream) {
+    const bool extras = p.epilogue != EPI_ROPE && (p.bias || p.act == 3);
+    return extras ? launch_gemm_as<true>(map_a, map_b, p, max_ctas, stream) : launch_gemm_as<false>(map_a, map_b, p, max_ctas, stream);
 }
 
 // 1 if this library was built for pairs of CTAs

@@ -267,7 +267,8 @@ __device__ __forceinline__ void finish_from_parts(const DecodeGemmParams& p, int
     }
 }
 
-template <int MB>
+// EXTRAS: the gated epilogue with a bias or the clamped form (built apart: their tests cost the others about 1 %)
+template <int MB, bool EXTRAS>
 __global__ void __launch_bounds__(NUM_THREADS, (MB <= 16 || MB == 64) ? 3 : 2)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                    const DecodeGemmParams p_in) {
@@ -658,8 +659,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     // features 0..63 are gate rows, 64..127 the up rows of the same output columns
                     const int fo = et & 63;
                     const int n = tile * (TILE_F / 2) + fo;
-                    const float bg = p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, n) : 0.f;
-                    const float bu = p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, half_n + n) : 0.f;
+                    const float bg = EXTRAS && p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, n) : 0.f;
+                    const float bu = EXTRAS && p.bias && n < half_n ? rv_load_param(p.bias, p.bias_dtype, half_n + n) : 0.f;
                     // eight rows of an output column per pass: eight independent chains per thread
                     for (int m0 = (et >> 6) * 8; m0 < p.M && n < half_n; m0 += 16) {
                         const float4 ga = *reinterpret_cast<const float4*>(fin + fo * FS + m0);
@@ -670,8 +671,12 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const float u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
                         float v[8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            v[j] = p.gated == 3 ? clamped_gate(g[j] + bg, u[j] + bu, p.limit, p.alpha) : silu_gate(g[j] + bg, u[j] + bu, p.out_f32 != 0, p.gated == 2);
+                        for (int j = 0; j < 8; ++j) {
+                            if constexpr (EXTRAS)
+                                v[j] = p.gated == 3 ? clamped_gate(g[j] + bg, u[j] + bu, p.limit, p.alpha)
+                                                    : silu_gate(g[j] + bg, u[j] + bu, p.out_f32 != 0, p.gated == 2);
+                            else v[j] = silu_gate(g[j], u[j], p.out_f32 != 0, p.gated == 2);
+                        }
                         if (p.out_f32) {
                             float* o = (float*)p.out + (size_t)m0 * half_n + n;
 #pragma unroll
@@ -785,14 +790,14 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (p.cluster && warp < 2) cluster_wait();
 }
 
-template <int MB>
+template <int MB, bool EXTRAS>
 static int launch_decode(const CUtensorMap& mw, const CUtensorMap& mx, const DecodeGemmParams& p, cudaStream_t stream) {
     constexpr int STAGES = STAGES_FOR(MB);
     const int stage = A_BYTES + MB * BK * 2;
     const int fin = TILE_F * (MB + 4) * 4;
     int smem = (STAGES * stage > fin ? STAGES * stage : fin) + 1024;
     static RvPerDevice configured;
-    if (int e = rv_configure_smem(configured, gemm_decode_kernel<MB>, smem + MAX_NORM_K * 4 + (64 + 8) * TILE_F * 4)) return e;
+    if (int e = rv_configure_smem(configured, gemm_decode_kernel<MB, EXTRAS>, smem + MAX_NORM_K * 4 + (64 + 8) * TILE_F * 4)) return e;
     if (p.norm_gamma || p.cluster) {
         const int num_kb = (p.K + BK - 1) / BK;
         smem = STAGES * stage + 1024;
@@ -802,10 +807,10 @@ static int launch_decode(const CUtensorMap& mw, const CUtensorMap& mx, const Dec
     }
     const int row_blocks = MB == 128 ? (p.M + MB - 1) / MB : 1;
     if (p.cluster)
-        RV_LAUNCH_ST = rv_launch_cluster(gemm_decode_kernel<MB>, dim3(p.n_tiles * p.splits, row_blocks), dim3(NUM_THREADS), smem, stream,
+        RV_LAUNCH_ST = rv_launch_cluster(gemm_decode_kernel<MB, EXTRAS>, dim3(p.n_tiles * p.splits, row_blocks), dim3(NUM_THREADS), smem, stream,
                                          (unsigned)p.splits, mw, mx, p);
     else
-        RV_LAUNCH_ST = rv_launch(gemm_decode_kernel<MB>, dim3(p.n_tiles * p.splits, row_blocks), dim3(NUM_THREADS), smem, stream, mw, mx, p);
+        RV_LAUNCH_ST = rv_launch(gemm_decode_kernel<MB, EXTRAS>, dim3(p.n_tiles * p.splits, row_blocks), dim3(NUM_THREADS), smem, stream, mw, mx, p);
     return rv_launch_status();
 }
 
@@ -854,11 +859,19 @@ static int run_decode(const void* x, const void* w, DecodeGemmParams p, cudaStre
     st = rv_make_bf16_map(&mx, x, p.M, p.K, mb);
     if (st != RV_OK) return st;
     p.n_tiles = rv_gemm_decode_tiles(p.N, p.gated);
+    if (p.gated && (p.bias || p.gated == 3)) {
+        switch (mb) {
+            case 16: return launch_decode<16, true>(mw, mx, p, stream);
+            case 32: return launch_decode<32, true>(mw, mx, p, stream);
+            case 64: return launch_decode<64, true>(mw, mx, p, stream);
+            default: return launch_decode<128, true>(mw, mx, p, stream);
+        }
+    }
     switch (mb) {
-        case 16: return launch_decode<16>(mw, mx, p, stream);
-        case 32: return launch_decode<32>(mw, mx, p, stream);
-        case 64: return launch_decode<64>(mw, mx, p, stream);
-        default: return launch_decode<128>(mw, mx, p, stream);
+        case 16: return launch_decode<16, false>(mw, mx, p, stream);
+        case 32: return launch_decode<32, false>(mw, mx, p, stream);
+        case 64: return launch_decode<64, false>(mw, mx, p, stream);
+        default: return launch_decode<128, false>(mw, mx, p, stream);
     }
 }
 

@@ -22,6 +22,7 @@ from ..errors import KernelError
 from . import build
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
+_GATED_PREFILL, _GATED_DECODE = {"silu": 2, "gelu_tanh": 4, "swiglu_clamp": 5}, {"silu": 1, "gelu_tanh": 2, "swiglu_clamp": 3}
 COUNTERS = {'launches': 0}   # kernels of this project launched so far (library GEMMs are not counted)
 _STATUS = {-1: "a size is out of range", -2: "unsupported dtype", -3: "misaligned pointer or stride",
            -4: "size not supported by this kernel"}
@@ -662,7 +663,7 @@ class CudaKernels:
             _need(bias, "bias", dims=1)
             if bias.shape[0] != N:
                 raise KernelError(f"linear: bias has {bias.shape[0]} entries for {N} features")
-        epilogue = {"silu": 2, "gelu_tanh": 4, "swiglu_clamp": 5}[activation] if gated else (1 if residual is not None else 0)
+        epilogue = _GATED_PREFILL[activation] if gated else (1 if residual is not None else 0)
         if splits is None:
             splits = self._prefill_splits(M, N, K, gated) if (max_ctas == 0 and pair is None) else 1
         if splits > 1:
@@ -671,8 +672,8 @@ class CudaKernels:
             lib = self._prefill_gemm_lib(M, pair, N, gated)
         st = lib.rv_gemm_tcgen05_bf16(
             _ptr(x), _ptr(weight), _ptr(bias), c_int(self._dt(bias, "bias") if bias is not None else 0), _ptr(residual), _ptr(out),
-            c_int(1 if out_dtype == torch.float32 else 0), c_int(M), c_int(N), c_int(K), c_int(epilogue), c_float(limit), c_float(alpha), _ptr(status if status is not None else self._status), c_int(max_ctas),
-            c_int(splits), self._stream())
+            c_int(1 if out_dtype == torch.float32 else 0), c_int(M), c_int(N), c_int(K), c_int(epilogue), c_float(limit), c_float(alpha),
+            _ptr(status if status is not None else self._status), c_int(max_ctas), c_int(splits), self._stream())
         _check("gemm_tcgen05", st)
         return out
 
@@ -763,7 +764,7 @@ class CudaKernels:
         st = lib.rv_gemm_tcgen05_decode_bf16(
             _ptr(x), _ptr(weight), _ptr(bias), c_int(self._dt(bias, "bias") if bias is not None else 0), _ptr(residual),
             _ptr(out), c_int(1 if out_dtype == torch.float32 else 0), c_int(M), c_int(N), c_int(K),
-            c_int({"silu": 1, "gelu_tanh": 2, "swiglu_clamp": 3}[activation] if gated else 0), c_float(limit), c_float(alpha), c_int(splits), c_int(1 if cluster else 0), _ptr(scratch),
+            c_int(_GATED_DECODE[activation] if gated else 0), c_float(limit), c_float(alpha), c_int(splits), c_int(1 if cluster else 0), _ptr(scratch),
             _ptr(self._decode_counters if splits > 1 else None),
             _ptr(status if status is not None else self._status), *self._norm_args(norm, K), self._stream())
         _check("gemm_tcgen05_decode", st)
