@@ -171,6 +171,18 @@ __device__ __forceinline__ float rv_warp_sum(float v) {
     return v;
 }
 
+// Four sums over PARTS (8, 16 or 32) neighbouring lanes, dealt out: a lane gets sum number part / (PARTS / 4).
+template <int PARTS>
+__device__ __forceinline__ float rv_sum4_dealt(const float (&v)[4], int part) {
+    const bool hi = part & (PARTS / 2), mid = part & (PARTS / 4);
+    const float k0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], PARTS / 2);
+    const float k1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], PARTS / 2);
+    float r = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, PARTS / 4);
+#pragma unroll
+    for (int o = PARTS / 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
 __device__ __forceinline__ float rv_warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

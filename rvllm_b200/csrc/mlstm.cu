@@ -202,17 +202,208 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     // all of them, stores the sequence's last m)
 }
 
+// The same for keys of 33 to 128 elements and portions of tokens, in two roles and with another cut of the columns.  What bound the
+// kernel above is shared memory: every warp reads the whole of q and k for the eight columns it holds.  Here a lane holds 8
+// entries of FOUR neighbouring columns, which PARTS lanes (8 or 16) share: a token costs it four wide reads of q and k, and the
+// four sums of S^T q are met by a reduction that deals them out.  Four warps walk, four others bring the next chunk, form
+// its gates and stage it (double buffers, one barrier a chunk); a warp walks the running maximum through a chunk with the gates
+// in its lanes.  The numbers and their order along the tokens are those of the kernel above.
+// 2,048 tokens of 8 heads, 128 x 256: 628 -> 401 us; of 16 heads 755 -> 514; four sequences of 500, 8 heads 198 -> 143.
+template <int PARTS>
+struct MlstmStage {
+    static constexpr int ROW = PARTS * 12;                 // 8 entries a lane, 12 floats apart: a lane's reads fall on banks of their own
+    static constexpr int COLS = 4 * (32 / PARTS) * 4;      // columns of a block
+    float q[ML_CHUNK][ROW], k[ML_CHUNK][ROW];
+    float v[ML_CHUNK][COLS];
+    float a[ML_CHUNK], b[ML_CHUNK];
+};
+
+template <int PARTS>
+__global__ void __launch_bounds__(256)
+mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_col0, const float* __restrict__ i_bias,
+                  const float* __restrict__ f_bias, const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots,
+                  float* __restrict__ state, size_t state_stride, float* __restrict__ raw, float* __restrict__ top, int heads, int d,
+                  int vd, float cap) {
+    rv_pdl_launch_dependents();
+    rv_pdl_wait();
+    using Stage = MlstmStage<PARTS>;
+    extern __shared__ __align__(16) unsigned char mw_raw[];
+    Stage* stages = reinterpret_cast<Stage*>(mw_raw);      // [2]
+    const int seq = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * Stage::COLS;
+    const int slot = state_slots[seq];
+    if (slot < 0) return;
+    const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    const int chunks = (n_tok + ML_CHUNK - 1) / ML_CHUNK;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int width = vd + 1;                              // columns of a head's state: the values and the constant 1
+    if (warp < 4) {                                        // ---- the walk
+        constexpr int Q = PARTS / 4;                       // lanes of a column after the reduction
+        const int part = lane % PARTS, group = lane / PARTS;
+        const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;
+        const int n0 = part * 8, mine = part / Q;          // this lane's column after the reduction
+        float S[8][4];
+        float* srow = state + (size_t)slot * state_stride + (size_t)h * d * width + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) S[i][j] = (col + j < width && n0 + i < d) ? srow[(size_t)(n0 + i) * width + j] : 0.f;
+        __syncthreads();                                   // the first chunk is staged
+        for (int c = 0; c < chunks; ++c) {
+            const Stage& st = stages[c & 1];
+            const int t0 = c * ML_CHUNK, nt = min(ML_CHUNK, n_tok - t0);
+            // (threads beyond the last column walk along: the shuffles need every lane)
+            auto step = [&](int tt) {
+                float kr[8], qr[8];
+                *reinterpret_cast<float4*>(kr) = *reinterpret_cast<const float4*>(&st.k[tt][part * 12]);
+                *reinterpret_cast<float4*>(kr + 4) = *reinterpret_cast<const float4*>(&st.k[tt][part * 12 + 4]);
+                *reinterpret_cast<float4*>(qr) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12]);
+                *reinterpret_cast<float4*>(qr + 4) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12 + 4]);
+                const float4 v = *reinterpret_cast<const float4*>(&st.v[tt][cb]);
+                const float a = st.a[tt], b = st.b[tt];
+                const float bu[4] = {b * v.x, b * v.y, b * v.z, b * v.w};
+                float aq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        S[i][j] = fmaf(a, S[i][j], kr[i] * bu[j]);
+                        aq[j] = fmaf(S[i][j], qr[i], aq[j]);
+                    }
+                const float ov = rv_sum4_dealt<PARTS>(aq, part);
+                if (part % Q == 0 && col + mine < width) raw[((size_t)(start + t0 + tt) * heads + h) * width + col + mine] = ov;
+            };
+            if (nt == ML_CHUNK) {
+#pragma unroll 4
+                for (int tt = 0; tt < ML_CHUNK; ++tt) step(tt);
+            } else {
+                for (int tt = 0; tt < nt; ++tt) step(tt);
+            }
+            __syncthreads();                               // this chunk is walked, the next one staged
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (col + j < width && n0 + i < d) srow[(size_t)(n0 + i) * width + j] = S[i][j];
+        return;
+    }
+    // ---- staging: a warp per token for q and k, the block's columns of v; the first of these warps forms the gates
+    const int tid = threadIdx.x - 128, sw = warp - 4, qk = heads * d;
+    const float q_scale = rsqrtf((float)d);
+    float m = state[(size_t)slot * state_stride + (size_t)heads * d * width + h];
+    const float bi = i_bias[h], bf = f_bias[h], inv_cap = 1.0f / cap;
+    constexpr int E = PARTS / 4;                           // elements of q (and k) per lane: 8 PARTS / 32
+    constexpr int PV = ML_CHUNK * Stage::COLS / 128;
+    float pq[ML_CHUNK / 4][E], pk[ML_CHUNK / 4][E], pv[PV], pgi = 0.f, pgf = 0.f;
+    auto load_chunk = [&](int c) {
+        const int t0 = c * ML_CHUNK, nt = min(ML_CHUNK, n_tok - t0);
+#pragma unroll
+        for (int x = 0; x < ML_CHUNK / 4; ++x) {
+            const int tt = sw + 4 * x;
+            const size_t row = (size_t)(start + t0 + tt) * stride + (size_t)h * d;
+#pragma unroll
+            for (int y = 0; y < E; ++y) {
+                const int e = lane + 32 * y;
+                pq[x][y] = 0.f; pk[x][y] = 0.f;
+                if (tt < nt && e < d) {
+                    pq[x][y] = proj[row + e];
+                    pk[x][y] = proj[row + qk + e];
+                }
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < PV; ++y) {
+            const int i = tid + 128 * y, tt = i / Stage::COLS, cc = col0 + i % Stage::COLS;
+            pv[y] = 0.f;
+            if (tt < nt && cc <= vd) pv[y] = cc < vd ? proj[(size_t)(start + t0 + tt) * stride + 2 * qk + (size_t)h * vd + cc] : 1.f;
+        }
+        if (tid < nt) {
+            const size_t row = (size_t)(start + t0 + tid) * stride;
+            pgi = proj[row + i_col0 + h];
+            pgf = proj[row + f_col0 + h];
+        }
+    };
+    auto stage = [&](int c) {
+        Stage& st = stages[c & 1];
+        const int t0 = c * ML_CHUNK, nt = min(ML_CHUNK, n_tok - t0);
+        if (sw == 0) {
+            const float gi = cap * tanhf((pgi + bi) * inv_cap);
+            const float x = cap * tanhf((pgf + bf) * inv_cap);
+            const float gf = x < 0.f ? x - log1pf(expf(x)) : -log1pf(expf(-x));          // log sigmoid
+            float m_old = 0.f, m_new = 0.f;
+#pragma unroll
+            for (int t = 0; t < ML_CHUNK; ++t) {
+                const float f = __shfl_sync(0xffffffffu, gf, t), i = __shfl_sync(0xffffffffu, gi, t);
+                if (t < nt) {
+                    const float next = fmaxf(f + m, i);
+                    if (lane == t) { m_old = m; m_new = next; }
+                    m = next;
+                }
+            }
+            if (lane < nt) {
+                st.a[lane] = expf(gf + m_old - m_new);
+                st.b[lane] = expf(gi - m_new);
+                if (blockIdx.x == 0) top[(size_t)(start + t0 + lane) * heads + h] = m_new;
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < ML_CHUNK / 4; ++x) {
+            const int tt = sw + 4 * x;
+#pragma unroll
+            for (int y = 0; y < E; ++y) {
+                const int e = lane + 32 * y, at = (e >> 3) * 12 + (e & 7);
+                st.q[tt][at] = pq[x][y] * q_scale;
+                st.k[tt][at] = pk[x][y];
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < PV; ++y) st.v[(tid + 128 * y) / Stage::COLS][(tid + 128 * y) % Stage::COLS] = pv[y];
+    };
+    if (chunks > 0) { load_chunk(0); stage(0); }
+    if (chunks > 1) load_chunk(1);
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {                     // while chunk c is walked: c + 1 in, c + 2 on its way
+        if (c + 1 < chunks) {
+            stage(c + 1);
+            if (c + 2 < chunks) load_chunk(c + 2);
+        }
+        __syncthreads();
+    }
+    // (m is read by every column block of the head and so must not be written here: the output kernel, which runs after
+    // all of them, stores the sequence's last m)
+}
+
+template <int PARTS>
+static int launch_mlstm_walk(cudaStream_t stream, int n_seqs, const float* proj, int stride, int i_col0, int f_col0, const float* i_bias,
+                             const float* f_bias, const int* cu_seqlens, const int* state_slots, float* state, size_t state_stride, float* raw,
+                             float* top, int heads, int d, int vd, float cap) {
+    constexpr int smem = 2 * (int)sizeof(MlstmStage<PARTS>), cols = MlstmStage<PARTS>::COLS;
+    static RvPerDevice once;
+    if (int st = rv_configure_smem(once, mlstm_walk_kernel<PARTS>, smem)) return st;
+    return rv_launch(mlstm_walk_kernel<PARTS>, dim3((vd + 1 + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, proj, stride, i_col0,
+                     f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, state_stride, raw, top, heads, d, vd, cap);
+}
+
 // proj rows: [q: heads x d | k: heads x d | v: heads x vd | ...]; the raw gate columns at i_col0 .. and f_col0 ..;
-// raw: float [tokens, heads x (vd + 1)], top: float [tokens, heads].
+// raw: float [n_tokens, heads x (vd + 1)], top: float [n_tokens, heads].
 RV_EXPORT int rv_mlstm_scan(const float* proj, int stride, int i_col0, int f_col0, const float* i_bias, const float* f_bias,
                             const int* cu_seqlens, const int* state_slots, float* state, long long state_stride, float* raw, float* top,
-                            int n_seqs, int heads, int d, int vd, float cap, cudaStream_t stream) {
+                            int n_tokens, int n_seqs, int heads, int d, int vd, float cap, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 || heads > 65535 || !(cap > 0.f))
         return RV_ERR_BAD_SIZE;
     if (stride < 2 * heads * d + heads * vd || i_col0 < 0 || f_col0 < 0 || i_col0 + heads > stride || f_col0 + heads > stride ||
         state_stride < (long long)heads * d * (vd + 1) + heads)
         return RV_ERR_BAD_SIZE;
     if (n_seqs == 0) return RV_OK;
+    // From two chunks a sequence on: 40 tokens take 36.6 us (39.3 in one role), but 17 take 84.7 (81.5; 16 sequences, 16 heads) and 6
+    // take 57.1 (49.1): the second role has nothing to run ahead of.
+    if (d > 32 && d <= 128 && n_tokens >= 2LL * ML_CHUNK * n_seqs) {
+        RV_LAUNCH_ST = d > 64 ? launch_mlstm_walk<16>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
+                                                      (size_t)state_stride, raw, top, heads, d, vd, cap)
+                              : launch_mlstm_walk<8>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
+                                                     (size_t)state_stride, raw, top, heads, d, vd, cap);
+        return rv_launch_status();
+    }
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128
     int parts = 1;
     while (parts * ns < d) parts <<= 1;                // a power of two of at most 32 lanes of one warp

@@ -1214,18 +1214,6 @@ struct DeltaStage {
     float g[DR_CHUNK], beta[DR_CHUNK], kq[DR_CHUNK];
 };
 
-// four sums over PARTS neighbouring lanes; returns the one of column part / (PARTS / 4)
-template <int PARTS>
-__device__ __forceinline__ float delta_sum4(const float (&v)[4], int part) {
-    const bool hi = part & (PARTS / 2), mid = part & (PARTS / 4);
-    const float k0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], PARTS / 2);
-    const float k1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], PARTS / 2);
-    float r = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, PARTS / 4);
-#pragma unroll
-    for (int o = PARTS / 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    return r;
-}
-
 template <int PARTS>
 __global__ void __launch_bounds__(256)
 delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
@@ -1276,7 +1264,7 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
                 for (int i = 1; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) { ak[j] = fmaf(S[i][j], kr[i], ak[j]); aq[j] = fmaf(S[i][j], qr[i], aq[j]); }
-                const float acc = delta_sum4<PARTS>(ak, part);
+                const float acc = rv_sum4_dealt<PARTS>(ak, part);
                 const float u = st.beta[tt] * (vv - g * acc);
                 float uj[4];
 #pragma unroll
@@ -1285,7 +1273,7 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) S[i][j] = fmaf(g, S[i][j], kr[i] * uj[j]);
-                const float ov = delta_sum4<PARTS>(aq, part);
+                const float ov = rv_sum4_dealt<PARTS>(aq, part);
                 if (part % Q == 0 && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
             };
             if (nt == DR_CHUNK) {                          // a whole chunk: neighbouring tokens may run into one another

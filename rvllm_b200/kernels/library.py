@@ -2006,7 +2006,7 @@ class CudaKernels:
         top = torch.empty((T, heads), dtype=torch.float32, device=proj.device)
         st = self._lib("mlstm.cu").rv_mlstm_scan(
             _ptr(proj), c_int(proj.shape[1]), c_int(i_col0), c_int(f_col0), _ptr(i_bias), _ptr(f_bias), _ptr(cu_seqlens), _ptr(state_slots),
-            _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(raw), _ptr(top), c_int(cu_seqlens.shape[0] - 1), c_int(heads),
+            _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(raw), _ptr(top), c_int(T), c_int(cu_seqlens.shape[0] - 1), c_int(heads),
             c_int(head_dim), c_int(value_dim), c_float(cap), self._stream())
         _check("mlstm_scan", st)
         return raw, top

@@ -230,3 +230,32 @@ def test_talking_attention_on_eight_and_sixteen_warps(K):
     finally:
         del K.TALKING_WARPS
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("d,vd,heads,lens", [(128, 256, 2, (5, 15, 16, 50, 80)), (100, 30, 2, (33,)), (64, 63, 1, (48, 17)), (40, 5, 2, (47,))])
+def test_mlstm_of_portions_in_two_roles(K, d, vd, heads, lens):
+    torch.manual_seed(d + vd)
+    T, W = sum(lens), vd + 1
+    proj = torch.randn(T, heads * (2 * d + vd + 2), device="cuda")
+    ib, fb, cap, g0 = torch.randn(heads, device="cuda"), torch.randn(heads, device="cuda") + 2, 15.0, heads * (2 * d + vd)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    state = torch.randn(len(lens), heads * d * W + heads, device="cuda")
+    S = state[:, :heads * d * W].double().cpu().view(-1, heads, d, W).clone()
+    m = state[:, heads * d * W:].double().cpu().clone()
+    f = proj.double().cpu()
+    q, k = f[:, :heads * d].view(T, heads, d) * d ** -0.5, f[:, heads * d:2 * heads * d].view(T, heads, d)
+    v = torch.cat([f[:, 2 * heads * d:g0].view(T, heads, vd), torch.ones(T, heads, 1, dtype=torch.float64)], 2)
+    gi = cap * torch.tanh((f[:, g0:g0 + heads] + ib.double().cpu()) / cap)
+    gf = torch.nn.functional.logsigmoid(cap * torch.tanh((f[:, g0 + heads:] + fb.double().cpu()) / cap))
+    raw, top = torch.empty(T, heads, W, dtype=torch.float64), torch.empty(T, heads, dtype=torch.float64)
+    for s in range(len(lens)):
+        for t in range(cu[s], cu[s + 1]):
+            new = torch.maximum(gf[t] + m[s], gi[t])
+            S[s] = torch.exp(gf[t] + m[s] - new)[:, None, None] * S[s] + torch.exp(gi[t] - new)[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+            m[s], top[t], raw[t] = new, new, torch.einsum("hdv,hd->hv", S[s], q[t])
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
+    got, got_top = K.mlstm_scan(proj, g0, g0 + heads, ib, fb, i32(cu), i32(list(range(len(lens)))), state, heads, d, vd, cap)
+    # float sums of d products; the gates' logarithms and exponentials to a few last places
+    assert rel_err(got, raw.view(T, -1)) < 3e-6 and rel_err(got_top, top) < 1e-6 and rel_err(state[:, :heads * d * W], S.view(len(lens), -1)) < 3e-6
