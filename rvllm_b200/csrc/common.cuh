@@ -35,18 +35,29 @@ __device__ __forceinline__ void rv_pdl_launch_dependents() { asm volatile("gridd
 __device__ __forceinline__ void rv_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-static inline int rv_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                            Args&&... args) {
+static inline int rv_launch_if(int early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_rv_pdl ? 1 : 0;
+    cfg.numAttrs = early ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
     if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return RV_OK;
+}
+
+template <typename... KArgs, typename... Args>
+static inline int rv_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    return rv_launch_if(g_rv_pdl, kernel, grid, block, smem, stream, args...);
+}
+
+// Without the attribute, whatever the switch says: for a kernel that must find its SMs empty.
+template <typename... KArgs, typename... Args>
+static inline int rv_launch_alone(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    return rv_launch_if(0, kernel, grid, block, smem, stream, args...);
 }
 
 // The same with the grid's CTAs grouped into clusters of `cluster_x` along x (distributed shared memory).

@@ -489,13 +489,16 @@ static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float
     const int pairs = tokens * top;
     const dim3 grid(pairs < experts ? pairs : experts, (ff + 15) / 16);
     const size_t smem_a = moe_mma_gate_up_smem(pairs, experts), smem_b = moe_mma_down_smem(pairs, experts);
+    // The first kernel waits for its predecessors at the launch: its loads go through L1, and CTAs that came in early, beside a product
+    // whose stages fill the SM's shared memory, kept the SM in that division, with no room for what they ask for (8 tokens
+    // of 4 experts, 2048 x 4096, behind the shared expert's products: 312 us for both kernels, 171 us launched so).
     int st;
     if (gated) {
         if ((st = rv_configure_smem(once[0], moe_mma_gate_up_kernel<true>, MM_SMEM_MAX)) != RV_OK) return st;
-        st = rv_launch(moe_mma_gate_up_kernel<true>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
+        st = rv_launch_alone(moe_mma_gate_up_kernel<true>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
     } else {
         if ((st = rv_configure_smem(once[1], moe_mma_gate_up_kernel<false>, MM_SMEM_MAX)) != RV_OK) return st;
-        st = rv_launch(moe_mma_gate_up_kernel<false>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
+        st = rv_launch_alone(moe_mma_gate_up_kernel<false>, grid, dim3(MM_WARPS * 32), smem_a, stream, x, chosen, gate_up, act, pairs, top, experts, ff, width);
     }
     if (st != RV_OK) return st;
     const dim3 grid_b((width + 15) / 16);
