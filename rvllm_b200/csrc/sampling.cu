@@ -13,9 +13,8 @@
 //   u * (kept mass), with u = Philox4x32-10(key = seed, counter = index of the output token).
 // The uniform depends on (seed, output index) only, never on the batch a row is sampled in.
 //
-// Rows with a top-k take two passes over the row (maximum + counts per bin of the top 12 bits of the
-// ordered bit pattern, then the candidates from the k-th token's bin upwards and the whole mass), rows
-// with a top-p alone three (arg-max, counts and fixed-point masses per bin, candidates); the at most
+// Rows with a top-k or a top-p take two passes over the row (maximum + counts per bin of the top 12 bits of
+// the ordered bit pattern, then the tokens from a bin upwards and the whole mass); the at most
 // 2,048 candidates are sorted and cut exactly in the first CTA's shared memory.  Rows whose candidates
 // do not fit (a flat distribution under top-p alone, a k beyond 2,048) take the general search: eight
 // passes of four bits over the row.  All sums that decide anything are integers or are added in a fixed
@@ -147,9 +146,17 @@ __device__ __forceinline__ void slice_scan(const float* row, int lo_s, int hi_s,
     hi = min(hi_s, lo + C);
     float local = 0.f;
     last_kept = -1;
-    for (int i = lo; i < hi; ++i) {
-        const float v = row[i];
+    auto take = [&](float v, int i) {
         if (order_key(v) >= tau && !(v != v)) { local += expf((v - m) * inv_t); last_kept = i; }
+    };
+    if (((lo | hi) & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+#pragma unroll 4
+        for (int i = lo; i < hi; i += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(row + i);
+            take(q.x, i); take(q.y, i + 1); take(q.z, i + 2); take(q.w, i + 3);
+        }
+    } else {
+        for (int i = lo; i < hi; ++i) take(row[i], i);
     }
     float incl = local;
 #pragma unroll
@@ -183,19 +190,16 @@ __device__ __forceinline__ void slice_scan(const float* row, int lo_s, int hi_s,
 }
 
 // ---------------------------------------------------------------------------------------------
-// The short way to the top-k / top-p threshold: three passes over the row instead of eleven.
+// The short way to the top-k / top-p threshold: two passes over the row instead of eleven.
 //
-// Pass 1 (arg-max) has given the row's maximum m.  Pass 2 builds ONE histogram of the row over the top
-// 12 bits of the ordered bit pattern (sign, exponent, three bits of mantissa: 4,096 bins): tokens per bin
-// and their mass exp((v - m) / T) as a 40-bit fixed-point integer, added with integer atomics in shared
-// memory - so the sums do not depend on the order of the additions, on the number of CTAs that share the
-// row or on the run.  The CTAs of a row add their bins into the first CTA's histogram through distributed
-// shared memory.  From the top bin downwards the first CTA finds the bin in which the k-th token lies and
-// the bin in which the cumulated mass reaches top_p x (the whole mass); the threshold lies in the higher
-// of the two, and every token from that bin upwards is a candidate.  If there are at most FAST_CANDIDATES
-// of them (a peaked distribution, or a small k), pass 3 gathers them - ordered bit pattern and index, in
-// any order - into the first CTA's shared memory, where they are sorted (bitonic, by value then index:
-// a total order, so the result is the same whatever order they arrived in), cut exactly by count and by
+// A histogram counts the row's tokens over the top 12 bits of the ordered bit pattern (sign, exponent, three bits of
+// mantissa: 4,096 bins); the CTAs of a row add their bins into the first CTA's histogram through distributed shared
+// memory.  The threshold lies in the bin of the k-th token, or in the one in which the cumulated mass exp((v - m) / T)
+// reaches top_p x (the whole mass); masses are 40-bit fixed-point integers, so their sums do not depend on the order of the
+// additions, on the number of CTAs that share the row or on the run.  Every token from the threshold's bin upwards is a
+// candidate.  If there are at most FAST_CANDIDATES of them (a peaked distribution, or a small k), they are gathered
+// - ordered bit pattern and index, in any order - in the first CTA's shared memory, where they are sorted (bitonic, by
+// value then index: a total order, so the result is the same whatever order they arrived in), cut exactly by count and by
 // cumulated mass, sorted back into vocabulary order and drawn from.  Otherwise (a flat distribution under
 // top-p alone, a huge k) the kernel goes on with the general search below.
 #define FAST_BINS 4096
@@ -267,10 +271,9 @@ struct FastShared {
 };
 
 // The first CTA's end of the short way: sort the gathered candidates, cut by count and by mass, draw.
-__device__ void short_way_finish(unsigned long long* cand, float* cmass, float m, float inv_t, int k, float pp, bool use_k, bool use_p,
-                                 unsigned long long seed, long long draw, int* out_token, float* s_scan, FastShared* fs) {
+__device__ void short_way_finish(unsigned long long* cand, float* cmass, int n, float m, float inv_t, int k, float pp, bool use_k,
+                                 bool use_p, unsigned long long seed, long long draw, int* out_token, float* s_scan, FastShared* fs) {
     const int tid = threadIdx.x;
-    const int n = (int)min(fs->n_cand, (unsigned int)FAST_CANDIDATES);
     int n_pad = 2;
     while (n_pad < n) n_pad <<= 1;
     for (int i = n + tid; i < n_pad; i += SAMPLE_THREADS) cand[i] = 0ull;       // sorts behind every candidate
@@ -328,130 +331,46 @@ __device__ void short_way_finish(unsigned long long* cand, float* cmass, float m
     }
 }
 
-// Returns true if the row has been sampled (out[r] written by the first CTA); false: go on with the general search.
-__device__ bool sample_short_way(const float* __restrict__ row, int V, float m, float inv_t, int k, float pp, bool use_k, bool use_p,
-                                 unsigned long long seed, long long draw, int* out_token, unsigned char* s_dyn, float* s_scan,
-                                 FastShared* fs) {
-    const int CL = gridDim.x, rank = (int)sc_rank(), tid = threadIdx.x;
-    unsigned int* h_cnt = reinterpret_cast<unsigned int*>(s_dyn);                                   // [FAST_BINS]
-    unsigned long long* h_mass = reinterpret_cast<unsigned long long*>(s_dyn + FAST_BINS * 4);      // [FAST_BINS]
-    unsigned long long* cand = h_mass + FAST_BINS;                                                  // [FAST_CANDIDATES]
-    float* cmass = reinterpret_cast<float*>(cand + FAST_CANDIDATES);                                // [FAST_CANDIDATES]
-    for (int b = tid; b < FAST_BINS; b += SAMPLE_THREADS) { h_cnt[b] = 0u; h_mass[b] = 0ull; }
-    if (tid == 0) { fs->n_cand = 0u; fs->go = 0; fs->bin = 0; fs->kept = 0; fs->pick = -1; fs->z_q = 0ull; }
-    __syncthreads();
-    // this CTA's share of the row
-    const int per = (((V + CL - 1) / CL) + 3) & ~3;
-    const int lo = min(V, rank * per), hi = min(V, lo + per);
-    for (int i = lo + tid; i < hi; i += SAMPLE_THREADS) {
-        const float v = row[i];
-        if (v != v) continue;
-        const uint32_t bin = order_key(v) >> 20;
-        atomicAdd(&h_cnt[bin], 1u);
-        atomicAdd(&h_mass[bin], __float2ull_rz(expf((v - m) * inv_t) * FAST_SCALE));
-    }
-    sc_sync();                                            // every CTA's histogram is complete (and the first CTA's is no longer being zeroed)
-    if (rank != 0) {
-        for (int b = tid; b < FAST_BINS; b += SAMPLE_THREADS)
-            if (h_cnt[b]) { sc_red_add(sc_map(&h_cnt[b], 0), h_cnt[b]); sc_red_add(sc_map(&h_mass[b], 0), h_mass[b]); }
-    }
-    sc_sync();
-    if (rank == 0) {
-        // cumulated counts and masses from the top bin down: thread t owns the bins 4095 - 4t ... 4092 - 4t
-        const int lane = tid & 31, warp = tid >> 5;
-        unsigned int c_own = 0u;
-        unsigned long long m_own = 0ull;
+// f(value, index) for every token of [lo, hi) that is a thread's: four 16-byte words in flight where the share is made of such words
+// (one word at a time left the memory idle between a pass's steps), else token by token; indices rise within a thread.
+template <typename F>
+__device__ __forceinline__ void sample_walk(const float* __restrict__ row, int lo, int hi, const F& f) {
+    if (((lo | hi) & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+        const float4* r4 = reinterpret_cast<const float4*>(row);
+        const int end = hi >> 2;
+        for (int i0 = (lo >> 2) + threadIdx.x; i0 < end; i0 += 4 * SAMPLE_THREADS) {
+            float4 q[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { c_own += h_cnt[FAST_BINS - 1 - 4 * tid - j]; m_own += h_mass[FAST_BINS - 1 - 4 * tid - j]; }
-        unsigned int c_inc = c_own;
-        unsigned long long m_inc = m_own;
+            for (int j = 0; j < 4; ++j)
+                if (i0 + j * SAMPLE_THREADS < end) q[j] = r4[i0 + j * SAMPLE_THREADS];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned int cv = __shfl_up_sync(0xffffffffu, c_inc, o);
-            const unsigned long long mv = __shfl_up_sync(0xffffffffu, m_inc, o);
-            if (lane >= o) { c_inc += cv; m_inc += mv; }
-        }
-        __shared__ unsigned int w_cnt[32];
-        __shared__ unsigned long long w_mass[32];
-        __shared__ int s_bk, s_bp;
-        if (lane == 31) { w_cnt[warp] = c_inc; w_mass[warp] = m_inc; }
-        if (tid == 0) { s_bk = -1; s_bp = -1; }
-        __syncthreads();
-        unsigned int c_before = 0u, c_total = 0u;
-        unsigned long long m_before = 0ull, m_total = 0ull;
-        for (int w = 0; w < 32; ++w) {
-            if (w < warp) { c_before += w_cnt[w]; m_before += w_mass[w]; }
-            c_total += w_cnt[w]; m_total += w_mass[w];
-        }
-        c_before += c_inc - c_own;
-        m_before += m_inc - m_own;
-        // the bin of the k-th token and the bin in which the mass reaches the target: exactly one thread finds each
-        const unsigned long long target = use_p ? (unsigned long long)((double)pp * (double)m_total) : 0ull;
-        unsigned int c_run = c_before;
-        unsigned long long m_run = m_before;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int b = FAST_BINS - 1 - 4 * tid - j;
-            const unsigned int c = h_cnt[b];
-            const unsigned long long mm = h_mass[b];
-            if (use_k && c_run < (unsigned int)k && c_run + c >= (unsigned int)k) s_bk = b;
-            if (use_p && target > 0ull && m_run < target && m_run + mm >= target) s_bp = b;
-            c_run += c; m_run += mm;
-        }
-        __syncthreads();
-        // (fewer than k tokens, or a mass that rounding keeps below the target: that filter keeps everything)
-        const bool k_on = use_k && s_bk >= 0, p_on = use_p && s_bp >= 0;
-        const int bin = max(k_on ? s_bk : 0, p_on ? s_bp : 0);
-        // tokens from `bin` upwards: one more pass over the cumulated counts
-        __shared__ unsigned int s_n;
-        if (tid == 0) s_n = 0u;
-        __syncthreads();
-        {
-            unsigned int mine = 0u;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { const int b = FAST_BINS - 1 - 4 * tid - j; if (b >= bin) mine += h_cnt[b]; }
-            if (mine) atomicAdd(&s_n, mine);
-        }
-        __syncthreads();
-        const bool go = (k_on || p_on) && s_n > 0u && s_n <= FAST_CANDIDATES && c_total > 0u;
-        if (tid < CL) { sc_store(sc_map(&fs->go, tid), go ? 1 : 0); sc_store(sc_map(&fs->bin, tid), bin); }
-        if (tid == 0) fs->z_q = m_total;
-    }
-    sc_sync();
-    if (!fs->go) return false;
-    // ---- pass 3: the candidates go to the first CTA, (ordered bits, complemented index) in one word
-    {
-        const uint32_t bin = (uint32_t)fs->bin;
-        const uint32_t cnt_addr = sc_map(&fs->n_cand, 0), cand_addr = sc_map(cand, 0);
-        for (int i = lo + tid; i < hi; i += SAMPLE_THREADS) {
-            const float v = row[i];
-            if (v != v) continue;
-            const uint32_t key = order_key(v);
-            if ((key >> 20) >= bin) {
-                const unsigned int pos = sc_atom_add(cnt_addr, 1u);
-                if (pos < FAST_CANDIDATES) sc_store(cand_addr + pos * 8u, ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i));
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * SAMPLE_THREADS;
+                if (i >= end) break;
+                f(q[j].x, 4 * i); f(q[j].y, 4 * i + 1); f(q[j].z, 4 * i + 2); f(q[j].w, 4 * i + 3);
             }
         }
+        return;
     }
-    sc_sync();
-    if (rank != 0) return true;                           // the first CTA finishes the row; nobody's shared memory is touched from outside any more
-    short_way_finish(cand, cmass, m, inv_t, k, pp, use_k, use_p, seed, draw, out_token, s_scan, fs);
-    return true;
+    for (int i = lo + threadIdx.x; i < hi; i += SAMPLE_THREADS) f(row[i], i);
 }
 
-// The short way for rows with a top-k: TWO passes over the row.  Pass A finds the row's maximum (larger value, then
-// lower index - the same whatever the order) and counts the tokens per bin; no exponential, no mass: the bin of the
-// k-th token follows from the counts alone.  Pass B gathers the tokens from that bin upwards and adds up the row's
-// whole mass as 40-bit fixed-point integers in registers (needed only for a top-p cut, which then lies among the
-// candidates or below them all).  `m_out` / `best_out` carry the maximum on to the general search if there are too
-// many candidates (a k beyond FAST_CANDIDATES, a huge tie).
-__device__ bool sample_short_way_k(const float* __restrict__ row, int V, float inv_t, int k, float pp, bool use_p,
-                                   unsigned long long seed, long long draw, int* out_token, unsigned char* s_dyn, float* s_scan,
-                                   float* s_val, int* s_idx, FastShared* fs, float& m_out, int& best_out) {
+// The short way: TWO passes over the row.  Pass A finds the row's maximum (larger value, then lower index - the same whatever
+// the order) and counts the tokens per bin; no exponential, no mass.  With a top-k the bin of the k-th token follows from the
+// counts alone; with a top-p alone, pass B takes the tokens of as many bins from the top as hold at most FAST_CANDIDATES.
+// Pass B gathers the tokens from that bin upwards and adds up the row's whole mass as 40-bit fixed-point integers in registers.
+// A top-p cut behind a top-k lies among the candidates or below them all; a top-p cut alone is then found among the bins of the
+// candidates, by their masses: where these do not reach it, the tokens down to it are more than FAST_CANDIDATES.  (The masses
+// of all tokens, added per bin by 64-bit atomics in shared memory, took three passes: 64 rows of 128,256 tokens 134 us, now 42;
+// one of 152,064 52, now 25; behind a top-k 40 and 34.)  `m_out` / `best_out` carry the maximum on to the general search where the candidates are too many.
+__device__ bool sample_short_way(const float* __restrict__ row, int V, float inv_t, int k, float pp, bool use_k, bool use_p,
+                                 unsigned long long seed, long long draw, int* out_token, unsigned char* s_dyn, float* s_scan,
+                                 float* s_val, int* s_idx, FastShared* fs, float& m_out, int& best_out) {
     const int CL = gridDim.x, rank = (int)sc_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned int* h_cnt = reinterpret_cast<unsigned int*>(s_dyn);                                   // [FAST_BINS]
-    unsigned long long* h_mass = reinterpret_cast<unsigned long long*>(s_dyn + FAST_BINS * 4);      // (unused here; keeps the layout)
-    unsigned long long* cand = h_mass + FAST_BINS;                                                  // [FAST_CANDIDATES]
+    unsigned int* h_low = h_cnt + FAST_BINS;               // [FAST_BINS], [FAST_BINS]: the candidates' masses, low 20 bits and the others, added
+    unsigned int* h_high = h_low + FAST_BINS;              // apart (2,048 times 2^20 fit 32 bits: adds of 64 bits in shared memory are loops)
+    unsigned long long* cand = reinterpret_cast<unsigned long long*>(h_high + FAST_BINS);           // [FAST_CANDIDATES]
     float* cmass = reinterpret_cast<float*>(cand + FAST_CANDIDATES);                                // [FAST_CANDIDATES]
     __shared__ float x_val[8];
     __shared__ int x_idx[8];
@@ -463,12 +382,11 @@ __device__ bool sample_short_way_k(const float* __restrict__ row, int V, float i
     // ---- pass A: maximum and counts
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = lo + tid; i < hi; i += SAMPLE_THREADS) {
-        const float v = row[i];
-        if (v != v) continue;
+    sample_walk(row, lo, hi, [&](float v, int i) {
+        if (v != v) return;
         if (v > bv) { bv = v; bi = i; }                   // indices rise within a thread: a strict comparison keeps the lowest
         atomicAdd(&h_cnt[order_key(v) >> 20], 1u);
-    }
+    });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -513,7 +431,7 @@ __device__ bool sample_short_way_k(const float* __restrict__ row, int V, float i
         __shared__ int s_bk;
         __shared__ unsigned int s_n;
         if (lane == 31) w_cnt[warp] = c_inc;
-        if (tid == 0) { s_bk = -1; s_n = 0u; }
+        if (tid == 0) { s_bk = use_k ? -1 : FAST_BINS; s_n = 0u; }
         __syncthreads();
         unsigned int c_run = c_inc - c_own;
         for (int w = 0; w < warp; ++w) c_run += w_cnt[w];
@@ -521,11 +439,40 @@ __device__ bool sample_short_way_k(const float* __restrict__ row, int V, float i
         for (int j = 0; j < 4; ++j) {
             const int b = FAST_BINS - 1 - 4 * tid - j;
             const unsigned int c = h_cnt[b];
-            if (c_run < (unsigned int)k && c_run + c >= (unsigned int)k) { s_bk = b; s_n = c_run + c; }
+            if (use_k) {
+                if (c_run < (unsigned int)k && c_run + c >= (unsigned int)k) { s_bk = b; s_n = c_run + c; }
+            } else if (c_run + c <= FAST_CANDIDATES) {      // (all bins from the top down to the lowest of these)
+                atomicMin(&s_bk, b);
+                atomicMax(&s_n, c_run + c);
+            }
             c_run += c;
         }
         __syncthreads();
-        const bool go = s_bk >= 0 && s_n <= FAST_CANDIDATES;         // (fewer than k tokens in the row: the general search)
+        // (fewer than k tokens in the row, or more than FAST_CANDIDATES in its first bins: the general search)
+        bool go = use_k ? s_bk >= 0 && s_n <= FAST_CANDIDATES : s_n > 0u;
+        if (!use_k && go) {
+            // a flat row: the counts and the edges of the bins bound the candidates' mass from above and the whole mass
+            // from below; where these cannot meet, pass B would be for nothing (empty bins and edges that are no numbers add nothing)
+            float most = 0.f, least = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int b = FAST_BINS - 1 - 4 * tid - j;
+                if (!h_cnt[b]) continue;
+                const float c = (float)h_cnt[b], low = key_value((uint32_t)b << 20), high = key_value(((uint32_t)b << 20) | 0xfffffu);
+                if (low == low) least += c * expf((low - m) * inv_t);
+                if (b >= s_bk) most += c * (high == high ? expf((fminf(high, m) - m) * inv_t) : 1.f);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                most += __shfl_xor_sync(0xffffffffu, most, o);
+                least += __shfl_xor_sync(0xffffffffu, least, o);
+            }
+            if (lane == 0) { s_val[warp] = most; s_scan[warp] = least; }
+            __syncthreads();
+            most = least = 0.f;
+            for (int w = 0; w < SAMPLE_THREADS / 32; ++w) { most += s_val[w]; least += s_scan[w]; }
+            go = !(most * 1.001f < pp * least);            // (a thousandth: far above what the sums' rounding can do)
+        }
         if (tid < CL) { sc_store(sc_map(&fs->go, tid), go ? 1 : 0); sc_store(sc_map(&fs->bin, tid), s_bk); }
     }
     sc_sync();
@@ -535,16 +482,18 @@ __device__ bool sample_short_way_k(const float* __restrict__ row, int V, float i
         const uint32_t bin = (uint32_t)fs->bin;
         const uint32_t cnt_addr = sc_map(&fs->n_cand, 0), cand_addr = sc_map(cand, 0);
         unsigned long long z = 0ull;
-        for (int i = lo + tid; i < hi; i += SAMPLE_THREADS) {
-            const float v = row[i];
-            if (v != v) continue;
+        sample_walk(row, lo, hi, [&](float v, int i) {
+            if (v != v) return;
             const uint32_t key = order_key(v);
             if (use_p) z += __float2ull_rz(expf((v - m) * inv_t) * FAST_SCALE);
             if ((key >> 20) >= bin) {
-                const unsigned int pos = sc_atom_add(cnt_addr, 1u);
+                const unsigned int now = __activemask(), first = __ffs(now) - 1;       // one add for the lanes that are here together
+                unsigned int pos = 0u;
+                if (lane == (int)first) pos = sc_atom_add(cnt_addr, __popc(now));
+                pos = __shfl_sync(now, pos, first) + __popc(now & ((1u << lane) - 1u));
                 if (pos < FAST_CANDIDATES) sc_store(cand_addr + pos * 8u, ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i));
             }
-        }
+        });
         if (use_p) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
@@ -552,8 +501,70 @@ __device__ bool sample_short_way_k(const float* __restrict__ row, int V, float i
         }
     }
     sc_sync();
-    if (rank != 0) return true;
-    short_way_finish(cand, cmass, m, inv_t, k, pp, true, use_p, seed, draw, out_token, s_scan, fs);
+    int n = 0;
+    if (rank == 0) n = (int)min(fs->n_cand, (unsigned int)FAST_CANDIDATES);
+    if (!use_k) {
+        // ---- the bin in which the candidates' masses, from the top down, reach top_p x the whole mass
+        if (rank == 0) {
+            __shared__ unsigned long long w_mass[32];
+            __shared__ int s_bp, s_kept;
+            for (int b = tid; b < FAST_BINS; b += SAMPLE_THREADS) h_low[b] = h_high[b] = 0u;
+            if (tid == 0) { s_bp = -1; s_kept = 0; }
+            __syncthreads();
+            for (int i = tid; i < n; i += SAMPLE_THREADS) {
+                const uint32_t key = (uint32_t)(cand[i] >> 32);
+                const unsigned long long q = __float2ull_rz(expf((key_value(key) - m) * inv_t) * FAST_SCALE);
+                atomicAdd(&h_low[key >> 20], (uint32_t)q & 0xfffffu);
+                atomicAdd(&h_high[key >> 20], (uint32_t)(q >> 20));
+            }
+            __syncthreads();
+            auto mass_of = [&](int b) { return ((unsigned long long)h_high[b] << 20) + h_low[b]; };
+            unsigned long long m_own = 0ull;               // thread t owns the bins 4095 - 4t ... 4092 - 4t
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m_own += mass_of(FAST_BINS - 1 - 4 * tid - j);
+            unsigned long long m_inc = m_own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long mv = __shfl_up_sync(0xffffffffu, m_inc, o);
+                if (lane >= o) m_inc += mv;
+            }
+            if (lane == 31) w_mass[warp] = m_inc;
+            __syncthreads();
+            unsigned long long m_run = m_inc - m_own;
+            for (int w = 0; w < warp; ++w) m_run += w_mass[w];
+            const unsigned long long target = (unsigned long long)((double)pp * (double)fs->z_q);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {                  // exactly one thread finds it
+                const int b = FAST_BINS - 1 - 4 * tid - j;
+                const unsigned long long mm = mass_of(b);
+                if (target > 0ull && m_run < target && m_run + mm >= target) s_bp = b;
+                m_run += mm;
+            }
+            __syncthreads();
+            // (a row whose maximum is +inf has masses that are no numbers: its infinities are the candidates)
+            if (tid == 0 && m == INFINITY) s_bp = fs->z_q ? (int)(order_key(INFINITY) >> 20) : -1;
+            __syncthreads();
+            // candidates below that bin are none: the others close ranks (what is sorted is what a cut can keep)
+            static_assert(FAST_CANDIDATES <= 2 * SAMPLE_THREADS, "a thread holds two candidates");
+            unsigned long long own[2] = {tid < n ? cand[tid] : 0ull, tid + SAMPLE_THREADS < n ? cand[tid + SAMPLE_THREADS] : 0ull};
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (tid + j * SAMPLE_THREADS < n && (int)(own[j] >> 52) >= s_bp) {
+                    const unsigned int now = __activemask(), first = __ffs(now) - 1;
+                    int pos = 0;
+                    if (lane == (int)first) pos = atomicAdd(&s_kept, __popc(now));
+                    cand[__shfl_sync(now, pos, first) + __popc(now & ((1u << lane) - 1u))] = own[j];
+                }
+            __syncthreads();
+            n = s_kept;
+            if (tid < CL) sc_store(sc_map(&fs->go, tid), s_bp >= 0 ? 1 : 0);
+        }
+        sc_sync();
+        if (!fs->go) return false;                         // (not reached, or rounding keeps the mass below the target)
+    }
+    if (rank != 0) return true;                           // the first CTA finishes the row; nobody's shared memory is touched from outside any more
+    short_way_finish(cand, cmass, n, m, inv_t, k, pp, use_k, use_p, seed, draw, out_token, s_scan, fs);
     return true;
 }
 
@@ -592,9 +603,9 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     float m = -INFINITY;
     int best = 0x7fffffff;
     bool have_max = false;
-    if (T > 0.f && uk_row && g_sample_short_way) {
-        // top-k rows: maximum, counts and candidates in two passes; too many candidates: the maximum is kept, the search below goes on
-        if (sample_short_way_k(row, V, 1.0f / T, k_row, p_row, up_row, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan,
+    if (T > 0.f && (uk_row || up_row) && g_sample_short_way) {
+        // maximum, counts and candidates in two passes; too many candidates: the maximum is kept, the search below goes on
+        if (sample_short_way(row, V, 1.0f / T, k_row, p_row, uk_row, up_row, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan,
                                s_val, s_idx, &fast_shared, m, best))
             return;
         have_max = true;
@@ -623,18 +634,9 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     }
     const float inv_t = 1.0f / T;
 
-    // ---- top-k / top-p: the short way (one histogram, then the few candidates) where it serves the row
-    {
-        const int k_ = k_row;
-        const float p_ = p_row;
-        const bool uk = uk_row, up = up_row;
-        if (!uk && up && g_sample_short_way) {
-            if (sample_short_way(row, V, m, inv_t, k_, p_, uk, up, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan, &fast_shared))
-                return;
-        }
-    }
-
-    // ---- mass of everything
+    // ---- mass of everything, where a top-p is measured by it
+    float total = 0.f;
+    if (up_row) {
     for (int sl = first; sl < first + per; ++sl) {
         const int lo_s = min(V, sl * S), hi_s = min(V, lo_s + S);
         float part = 0.f;
@@ -643,9 +645,9 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         if (tid < CL) sc_store(sc_map(&xch[turn].val[sl], tid), part);
     }
     sc_sync();
-    float total = 0.f;
     for (int sl = 0; sl < SAMPLE_SLICES; ++sl) total += xch[turn].val[sl];
     turn ^= 1;
+    }
 
     // ---- threshold key: keep tokens whose order key is >= tau.  tau is the largest key c with
     // count(key >= c) >= k (top-k), or with mass(key >= c) >= top_p * total (top-p); it is found four

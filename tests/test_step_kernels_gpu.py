@@ -259,3 +259,30 @@ def test_mlstm_of_portions_in_two_roles(K, d, vd, heads, lens):
     got, got_top = K.mlstm_scan(proj, g0, g0 + heads, ib, fb, i32(cu), i32(list(range(len(lens)))), state, heads, d, vd, cap)
     # float sums of d products; the gates' logarithms and exponentials to a few last places
     assert rel_err(got, raw.view(T, -1)) < 3e-6 and rel_err(got_top, top) < 1e-6 and rel_err(state[:, :heads * d * W], S.view(len(lens), -1)) < 3e-6
+
+
+@pytest.mark.parametrize("vocab,ctas", [(1000, 1), (2048, 2), (2049, 1), (40001, 4), (128256, 8)])
+def test_top_p_rows_by_their_candidates(K, vocab, ctas):
+    """Top-p alone: rows whose candidates reach the mass, fall short of it (flat: told by the bins' edges, or only by the candidates'
+    masses), number just the limit, or hold infinities, draw what the general search over the whole row draws."""
+    from ctypes import c_int
+    torch.manual_seed(vocab)
+    spread = [0.0, 0.01, 0.5, 1.0, 2.0, 4.0, 8.0, 100.0] * 3
+    x = torch.randn(len(spread), vocab) * torch.tensor(spread)[:, None]
+    x[3, ::2] = float("-inf")
+    x[4, 7] = float("nan")
+    x[5, vocab - 2] = float("inf")
+    args = (x.cuda(), torch.full((24,), 0.9).cuda(), None, torch.tensor([0.9, 0.999, 1e-5] * 8).cuda(), torch.arange(24).cuda(), torch.arange(24).cuda() * 3)
+    lib = K._lib("sampling.cu")
+    try:
+        lib.rv_sample_set_cluster(c_int(ctas))
+        assert lib.rv_sample_set_short_way(c_int(0)) == 0
+        general = K.sample(*args).tolist()
+        assert lib.rv_sample_set_short_way(c_int(1)) == 0
+        short = K.sample(*args).tolist()
+    finally:
+        lib.rv_sample_set_cluster(c_int(0)), lib.rv_sample_set_short_way(c_int(1))
+    assert short[5] == vocab - 2
+    # masses are added in different orders: a draw within rounding (2^-24 log2(vocab)) of a step may differ, one row in thousands
+    rows = [r for r in range(24) if r != 5]
+    assert sum(short[r] != general[r] for r in rows) <= 1
