@@ -8,6 +8,7 @@ from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..errors import SamplingError
@@ -40,12 +41,17 @@ class Sampler:
                                 f"{len(draw_index)} draw indices")
         if all(p.is_greedy for p in params):
             return self.kernels.sample(logits)
-        dev = logits.device
-        host = torch.tensor([[p.temperature, p.top_p] for p in params], dtype=torch.float32)
-        ints = torch.tensor([[p.top_k] for p in params], dtype=torch.int32)
-        longs = torch.tensor([list(seeds), list(draw_index)], dtype=torch.int64)
-        host, ints, longs = host.to(dev, non_blocking=True), ints.to(dev, non_blocking=True), longs.to(dev, non_blocking=True)
-        use_k = any(p.top_k > 0 for p in params)
-        use_p = any(p.top_p < 1.0 for p in params)
-        return self.kernels.sample(logits, host[:, 0].contiguous(), ints[:, 0].contiguous() if use_k else None,
-                                   host[:, 1].contiguous() if use_p else None, longs[0], longs[1])
+        # one buffer and one copy: seeds and draw indices (64 bits), then temperatures, top-p and top-k (32 bits); the
+        # parameters' tensors are views of it on the device
+        host = np.empty((7 * R,), dtype=np.int32)
+        wide, real = host[:4 * R].view(np.int64), host[4 * R:6 * R].view(np.float32)
+        wide[:R] = seeds
+        wide[R:] = draw_index
+        top_ps, top_ks = [p.top_p for p in params], [p.top_k for p in params]
+        real[:R] = [p.temperature for p in params]
+        real[R:] = top_ps
+        host[6 * R:] = top_ks
+        flat = torch.from_numpy(host).to(logits.device, non_blocking=True)
+        wide, real = flat[:4 * R].view(torch.int64), flat[4 * R:6 * R].view(torch.float32)
+        return self.kernels.sample(logits, real[:R], flat[6 * R:] if max(top_ks) > 0 else None,
+                                   real[R:] if min(top_ps) < 1.0 else None, wide[:R], wide[R:])
