@@ -17,7 +17,7 @@
 //
 // Measured against one 64 x 64 tile kernel for every M (4 x 4 outputs a thread), which this replaced: 3 rows of 3584 x 18944
 // 2,120 -> 72 us (3.8 TB/s), of 37888 x 3584 836 -> 105 us (5.2 TB/s), of 152064 x 3584 3,235 -> 349 us (6.2 TB/s); 433 rows of
-// 37888 x 3584 5,381 -> 3,392 us (35 TFLOP/s); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
+// 37888 x 3584 5,381 -> 2,835 us (41.5 TFLOP/s); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
 //
 // Shapes of the layer's five products: v3/crates/rvllm-runtime/src/layer_exec.rs:240-266,
 // 433-444, 478-488, 511-522 of the reference (which calls cuBLASLt there); bias as a row
@@ -36,6 +36,12 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool val
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     const int bytes = valid ? 16 : 0;                       // 0: the destination is filled with zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_4(void* dst, const void* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(d), "l"(src), "r"(bytes) : "memory");
 }
 
 // MB: rows of x (padded); stages are per half warp: [16 rows of W | MB rows of x] x 128 bytes,
@@ -173,47 +179,57 @@ __global__ void __launch_bounds__(256, 1)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, const void* __restrict__ bias,
                      int bias_dtype, const float* __restrict__ residual, float* __restrict__ out,
                      int M, int N, int K, int splits, int row_tiles) {
-    extern __shared__ __align__(128) float smem[];           // two stages of xs | ws [TK][TPITCH]; later a part's sums [128][TPITCH]
+    extern __shared__ __align__(128) float smem[];           // two stages of xs | ws [TK][TPITCH], two parked groups, two stages of words
+                                                            // on their way from memory; later a part's sums [128][TPITCH]
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int part = blockIdx.x % splits, tile = blockIdx.x / splits;
     const int m0 = (tile % row_tiles) * TB, n0 = (tile / row_tiles) * TB;
-    // a warp covers 32 x 64 outputs (4 x 8 lanes of 8 x 8, as two halves of 4 each way)
-    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;
+    // a warp covers 32 x 64 outputs (4 x 8 lanes of 8 x 8, as two halves of 4 each way); the two warps of a scheduler lie 64 rows
+    // apart, so a last row tile of up to 64 rows takes half the time
+    const int wm = (warp >> 2) * 64 + (warp & 1) * 32, wn = ((warp >> 1) & 1) * 64;
+    const bool active = m0 + wm < M;
     const int am = wm + (lane >> 3) * 4, bn = wn + (lane & 7) * 4;       // and +16 rows, +32 columns
     const int seg = segment_length(K), per = MAX_SEGMENTS / splits;
     const int k_first = part * per * seg, k_last = min(K, k_first + per * seg);
 
     // two lanes bring 8 consecutive k of a row: whole 32-byte sectors in, conflict-free columns out
     const int ld_row = (warp >> 1) * 16 + (lane >> 1) , ld_k = (warp & 1) * 8 + (lane & 1) * 4;      // rows +0, +64
-    float4 xa[2], wa[2];
-    auto fetch = [&](int k0) {
-        const int k = k0 + ld_k;
+    // the words wait in shared memory, each in its thread's own places ([stage][4][256 threads] x 16 bytes), until the thread puts
+    // them down by column: in registers the compiler moved the loads to where they are used, and a fifth of the time
+    // was spent waiting for them
+    float4* mail = reinterpret_cast<float4*>(smem + 4 * TK * TPITCH + 2 * 64 * 256);
+    auto fetch = [&](int t) {
+        const int k = k_first + t * TK + ld_k;
+        float4* to = mail + (t & 1) * 4 * 256 + tid;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int m = m0 + ld_row + h * 64, n = n0 + ld_row + h * 64;
-            xa[h] = wa[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* px = x + (size_t)m * K + k;
+            const float* pw = w + (size_t)n * K + k;
             if (VEC) {
-                if (m < M && k < k_last) xa[h] = *reinterpret_cast<const float4*>(x + (size_t)m * K + k);
-                if (n < N && k < k_last) wa[h] = __ldg(reinterpret_cast<const float4*>(w + (size_t)n * K + k));
+                const bool okx = m < M && k < k_last, okw = n < N && k < k_last;
+                cp_async_16(to + h * 256, okx ? px : x, okx);
+                cp_async_16(to + (2 + h) * 256, okw ? pw : w, okw);
             } else {
-                float* a = &xa[h].x;
-                float* b = &wa[h].x;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if (m < M && k + j < k_last) a[j] = x[(size_t)m * K + k + j];
-                    if (n < N && k + j < k_last) b[j] = w[(size_t)n * K + k + j];
+                    const bool okx = m < M && k + j < k_last, okw = n < N && k + j < k_last;
+                    cp_async_4(reinterpret_cast<float*>(to + h * 256) + j, okx ? px + j : x, okx);
+                    cp_async_4(reinterpret_cast<float*>(to + (2 + h) * 256) + j, okw ? pw + j : w, okw);
                 }
             }
         }
     };
-    auto store = [&](int buf) {
-        float* xs = smem + buf * 2 * TK * TPITCH;
+    auto store = [&](int t) {
+        float* xs = smem + (t & 1) * 2 * TK * TPITCH;
         float* ws = xs + TK * TPITCH;
+        const float4* from = mail + (t & 1) * 4 * 256 + tid;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const float a[4] = {xa[h].x, xa[h].y, xa[h].z, xa[h].w}, b[4] = {wa[h].x, wa[h].y, wa[h].z, wa[h].w};
+            const float4 xa = from[h * 256], wa = from[(2 + h) * 256];
+            const float a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {wa.x, wa.y, wa.z, wa.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 xs[(ld_k + j) * TPITCH + ld_row + h * 64] = a[j];
@@ -231,7 +247,11 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
         for (int j = 0; j < 4; ++j) { acc[i][j] = 0ull; total[i][2 * j] = total[i][2 * j + 1] = 0.f; }
     const int n_tiles = k_first < k_last ? (k_last - k_first + TK - 1) / TK : 0;
     const int seg_tiles = seg / TK;
-    if (n_tiles) { fetch(k_first); store(0); }
+    if (n_tiles) fetch(0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (n_tiles > 1) fetch(1);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
+    if (n_tiles) store(0);
     __syncthreads();
     int in_seg = 0, seg_i = 0;
     // the sums of a tile: groups of four segments; the first group's sum waits in shared memory behind the stages while the
@@ -239,9 +259,11 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
     float* park = smem + 4 * TK * TPITCH;                   // [2][64 values][256 threads]
     for (int t = 0; t < n_tiles; ++t) {
         const int buf = t & 1;
-        if (t + 1 < n_tiles) fetch(k_first + (t + 1) * TK);
+        if (t + 2 < n_tiles) fetch(t + 2);                  // (its places were read, by this thread, before the last barrier)
+        asm volatile("cp.async.commit_group;" ::: "memory");
         const float* xs = smem + buf * 2 * TK * TPITCH;
         const float* ws = xs + TK * TPITCH;
+        if (active)
 #pragma unroll
         for (int k = 0; k < TK; ++k) {
             const float4 a0 = *reinterpret_cast<const float4*>(xs + k * TPITCH + am);
@@ -298,7 +320,8 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
                 }
             }
         }
-        if (t + 1 < n_tiles) store(buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        if (t + 1 < n_tiles) store(t + 1);
         __syncthreads();
     }
 
@@ -379,10 +402,15 @@ RV_EXPORT int rv_gemm_f32(const float* x, const float* w, const void* bias, int 
     }
     const long long rows = (M + TB - 1) / TB, cols = (N + TB - 1) / TB;
     if (rows * cols > 0x7fffffffll / 4) return RV_ERR_BAD_SIZE;
-    // K over a cluster of CTAs while all parts stay within the SMs (one CTA each)
+    // K over a cluster of 1, 2 or 4 CTAs (one per SM): the fewest rounds of work, counted in a whole tile's time (a last row tile of
+    // up to 64 rows is half of one), and of ones within a twentieth the fewest parts.  433 rows of 3584 x 18944, 112 tiles: one round of
+    // 1,913 us whole, 1,734 in parts of four; 300 of 4095 x 1023 146 and 119.
     const int sms = rv_sm_count();
-    const int splits = rows * cols * 4 <= sms ? 4 : (rows * cols * 2 <= sms ? 2 : 1);
-    const int smem = (4 * TK * TPITCH + 2 * 64 * 256) * 4;   // stages, two parked groups (>= a part's sums)
+    const long long halves = cols * (2 * rows - (M - (rows - 1) * TB <= TB / 2 ? 1 : 0));
+    int splits = 1;
+    for (int s = 2; s <= 4; s *= 2)
+        if ((halves * s + 2 * sms - 1) / (2 * sms) * splits * 20 < (halves * splits + 2 * sms - 1) / (2 * sms) * s * 19) splits = s;
+    const int smem = (4 * TK * TPITCH + 2 * 64 * 256) * 4 + 2 * 4 * 256 * 16;       // stages, two parked groups (>= a part's sums), words on their way
     static_assert(4 * TK * TPITCH + 2 * 64 * 256 >= TB * TPITCH, "a part's sums fit");
     static RvPerDevice conf_v, conf_s;
     const dim3 grid((unsigned)(rows * cols * splits));
