@@ -56,9 +56,16 @@ struct TmArgs {
 };
 
 // rows [row0, row0 + TA_BN) of one kind (keys: width hd at offset 0 of a page; values: width vd behind the keys) of all
-// key/value heads into `dst` [nkv][TA_BN][width + 8]
-__device__ __forceinline__ void tm_fetch(__nv_bfloat16* dst, const TmArgs& a, const int* table, int j0, int j_end, int width, size_t kind_off,
-                                         int tid, int nthreads) {
+// key/value heads into `dst` [nkv][TA_BN][width + 8]; `place` is that of the thread's first row (tm_look)
+struct TmPlace { int page, slot; };
+// The page of the thread's row of the tile at j0 and its place there.  Asked for a tile ahead: with the lookup in the fetch, a
+// fifth of the warps' time went to waiting for the table (2,048 tokens of 16 heads on 4: 491 -> 467 us, a portion of 100 37 -> 33).
+__device__ __forceinline__ TmPlace tm_look(const TmArgs& a, const int* table, int j0, int j_end, int tid) {
+    const int j = min(j0 + ((tid >> 1) % TA_BN), j_end), pg = j / a.page_size;
+    return {__ldg(table + pg), j - pg * a.page_size};
+}
+__device__ __forceinline__ void tm_fetch(__nv_bfloat16* dst, const TmArgs& a, const int* table, TmPlace place, int j0, int j_end, int width,
+                                         size_t kind_off, int tid, int nthreads) {
     // two lanes per row (a pair copies one 32-byte sector per step): the row's place in the cache is worked out once
     const int chunks = width / 8, ld = width + 8;
     const int rows = a.nkv * TA_BN;
@@ -70,8 +77,8 @@ __device__ __forceinline__ void tm_fetch(__nv_bfloat16* dst, const TmArgs& a, co
         const bool real = j <= j_end;
         const __nv_bfloat16* src = a.cache;
         if (real) {
-            const int pg = j / a.page_size;
-            src += (size_t)table[pg] * page_elems + kind_off + ((size_t)g * a.page_size + (j - pg * a.page_size)) * width + l2 * 8;
+            const TmPlace p = jj == ((tid >> 1) % TA_BN) ? place : tm_look(a, table, j0, j_end, 2 * jj);     // (rows of odd numbers of warps)
+            src += (size_t)p.page * page_elems + kind_off + ((size_t)g * a.page_size + p.slot) * width + l2 * 8;
         }
         const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + ((size_t)g * TA_BN + jj) * ld + l2 * 8);
         const int n = real ? 16 : 0, step = real ? 16 : 0;
@@ -189,15 +196,17 @@ talking_attention_mma_kernel(const TmArgs a) {
     // (the value tile's place is free in this walk: where it is large enough the key tiles alternate between the two, and
     // the next tile is on its way while this one is used)
     const bool two = vd >= hd;
-    tm_fetch(sK, a, table, lo_min, pos_last, hd, 0, tid, nthreads);
+    tm_fetch(sK, a, table, tm_look(a, table, lo_min, pos_last, tid), lo_min, pos_last, hd, 0, tid, nthreads);
     tm_commit();
+    TmPlace next = tm_look(a, table, lo_min + TA_BN, pos_last, tid);
     int turn = 0;
     for (int j0 = lo_min; j0 <= pos_last; j0 += TA_BN, turn ^= 1) {
         const bool more = j0 + TA_BN <= pos_last;
         __nv_bfloat16* cur = (two && turn) ? sV : sK;
         if (two) {
-            if (more) tm_fetch(turn ? sK : sV, a, table, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
+            if (more) tm_fetch(turn ? sK : sV, a, table, next, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
             tm_commit();
+            next = tm_look(a, table, j0 + 2 * TA_BN, pos_last, tid);
             tm_wait<1>();
         } else {
             tm_wait<0>();
@@ -207,8 +216,9 @@ talking_attention_mma_kernel(const TmArgs a) {
         scores(s, j0, cur + my_k_off);
         __syncthreads();
         if (!two) {
-            if (more) tm_fetch(sK, a, table, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
+            if (more) tm_fetch(sK, a, table, next, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
             tm_commit();
+            next = tm_look(a, table, j0 + 2 * TA_BN, pos_last, tid);
         }
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
@@ -242,10 +252,12 @@ talking_attention_mma_kernel(const TmArgs a) {
     for (int nt = 0; nt < VD / 8; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
     tm_wait<0>();
     __syncthreads();
-    tm_fetch(sK, a, table, lo_min, pos_last, hd, 0, tid, nthreads);
+    next = tm_look(a, table, lo_min, pos_last, tid);
+    tm_fetch(sK, a, table, next, lo_min, pos_last, hd, 0, tid, nthreads);
     tm_commit();
-    tm_fetch(sV, a, table, lo_min, pos_last, vd, v_off, tid, nthreads);
+    tm_fetch(sV, a, table, next, lo_min, pos_last, vd, v_off, tid, nthreads);
     tm_commit();
+    next = tm_look(a, table, lo_min + TA_BN, pos_last, tid);
     const int mix_items = CT * (TA_BN / 4) * (nh4 / 4);
     for (int j0 = lo_min; j0 <= pos_last; j0 += TA_BN) {
         const bool more = j0 + TA_BN <= pos_last;
@@ -268,7 +280,7 @@ talking_attention_mma_kernel(const TmArgs a) {
             }
         }
         __syncthreads();                                // all scores are out: the key tile is free
-        if (more) tm_fetch(sK, a, table, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
+        if (more) tm_fetch(sK, a, table, next, j0 + TA_BN, pos_last, hd, 0, tid, nthreads);
         tm_commit();
         if (a.talk) {
             for (int it = tid; it < mix_items; it += nthreads) {
@@ -320,8 +332,9 @@ talking_attention_mma_kernel(const TmArgs a) {
             }
         }
         __syncthreads();                                // the value tile and the weights are free
-        if (more) tm_fetch(sV, a, table, j0 + TA_BN, pos_last, vd, v_off, tid, nthreads);
+        if (more) tm_fetch(sV, a, table, next, j0 + TA_BN, pos_last, vd, v_off, tid, nthreads);
         tm_commit();
+        next = tm_look(a, table, j0 + 2 * TA_BN, pos_last, tid);
     }
     tm_wait<0>();
 #pragma unroll
@@ -356,8 +369,8 @@ RV_EXPORT int rv_talking_attention_mma(const void* q, const void* cache, const i
     if (n_seqs == 0 || max_q_len == 0) return RV_OK;
     const int rep = nh / nkv, TOK = 16 / rep;
     // Sixteen warps are one CTA per SM of twice the tokens behind the same tiles; eight are more CTAs, which even out better.
-    // Sixteen where they still leave one and a half CTAs per SM: 2,048 tokens of 32 heads on 8: 976 us against 1,315; of 16
-    // heads on 4 they leave 128 CTAs: 704 against 491.  (max_warps 0: this rule; 8 or 16.)
+    // Sixteen where they still leave one and a half CTAs per SM: 2,048 tokens of 32 heads on 8: 966 us against 1,230; of 16
+    // heads on 4 they leave 128 CTAs: 701 against 467.  (max_warps 0: this rule; 8 or 16.)
     const int nh4 = (nh + 3) & ~3;
     int tg = 1;
     size_t smem = 0;
