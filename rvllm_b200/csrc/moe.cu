@@ -224,7 +224,7 @@ static int moe_launch(const void* x, const int* chosen, const float* weights, co
 // accumulators; the rate needed is one per 23 clocks and SM), sixteen rows of the matrix its rows.  The order of k inside a
 // product is free, so a lane takes 8 neighbouring k of its row and of its pair as one 16-byte load each (k = 32 c + 8 (lane & 3))
 // and these four words are the operands of two products: nothing passes through shared memory on the way in.
-//   moe_mma_gate_up   a CTA per (expert, 16 features): eight warps share k (gated: four on the gate rows, four on the up rows),
+//   moe_mma_gate_up   a CTA per (expert, 16 features, or 2 x 16): eight warps share k (gated: four on the gate rows, four on the up rows),
 //                     their sums meet in shared memory
 //   moe_mma_down      a CTA per 16 columns of the result: its warps share the (expert, quarter of k) items, and the sums of a
 //                     token's slots are added in the slots' order
@@ -344,8 +344,9 @@ moe_mma_gate_up_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
     for (int i = tid; i < pairs; i += blockDim.x)
         if (chosen[i] == e) list[atomicAdd(&count_s, 1)] = i;
     __syncthreads();
-    const int count = count_s, f0 = blockIdx.y * 16;
+    const int count = count_s;
     const __nv_bfloat16* w = gate_up + (size_t)e * MT * ff * width;
+    for (int f0 = blockIdx.y * 16; f0 < ff; f0 += gridDim.y * 16)
     for (int p0 = 0; p0 < count; p0 += MM_PASS) {
         const int left = min(MM_PASS, count - p0);
         if (left <= 8) moe_gate_up_pass<GATED, 1>(x, w, list, count, p0, f0, top, ff, width, red);
@@ -487,7 +488,11 @@ static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float
                           int tokens, int top, int experts, int ff, int width, float weight, int gated, int identity, cudaStream_t stream) {
     static RvPerDevice once[4];
     const int pairs = tokens * top;
-    const dim3 grid(pairs < experts ? pairs : experts, (ff + 15) / 16);
+    // Two feature blocks a CTA where one each would be more than the SMs hold at a time (two CTAs): finding the expert and its pairs
+    // costs less (16 pairs on 13 experts of 2048 x 4096, both kernels: 80.1 -> 77.2 us; four blocks 81.6).  2 pairs on 88
+    // blocks: 15.1 us so, 16.5 with two.
+    const int used = pairs < experts ? pairs : experts, blocks = (ff + 15) / 16;
+    const dim3 grid(used, (long long)used * blocks > 2LL * rv_sm_count() ? (blocks + 1) / 2 : blocks);
     const size_t smem_a = moe_mma_gate_up_smem(pairs, experts), smem_b = moe_mma_down_smem(pairs, experts);
     // The first kernel waits for its predecessors at the launch: its loads go through L1, and CTAs that came in early, beside a product
     // whose stages fill the SM's shared memory, kept the SM in that division, with no room for what they ask for (8 tokens
