@@ -9,8 +9,12 @@
 // scores, the weighted x) go in as three bfloat16 terms each (24 bits: v = hi + mid + lo), so nothing is rounded below
 // float.  The running sums c are formed in double and kept as two floats, so a difference of two of them is as exact as
 // a sum of the few terms between.  Against float64 the state is as close as the walk's (1.2e-7), y 0.9e-7 against 0.5e-7: both
-// below a float's own last place, and the same figures for the layer's bfloat16 result.  (A value that is infinite or
-// NaN reaches the tokens of its sequence from its block of 16 on.)
+// below a float's own last place, and the same figures for the layer's bfloat16 result.
+//
+// A product multiplies the masked zeros of a block of scores with the x of later tokens, infinities do not split into terms, and
+// a running sum that a single step size dominates does not tell the others' decays any more.  So a chunk with numbers that
+// are not finite, or with a sum of decays beyond 10^5, is walked token by token, as ssm.cu does (the columns of a warp where it
+// is an x or the state, else the whole block): what is not finite stays with its token and those after it.
 //
 // Grid (blocks of 64 columns p, heads, sequences), four warps, one per 16 columns: S^T of them (16 x N) lives in the
 // accumulators' layout in registers, which is also the layout of an A operand, so y needs no pass of S through shared
@@ -170,7 +174,13 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                 ch_mma(G[2 * s + 1], a, b[2], b[3]);
             }
         }
-        __syncthreads();                                   // the sums of the decays are written
+        float odd_g = 0.f;                                 // B_t . C_t is not finite where B_t or C_t is not
+#pragma unroll
+        for (int s = 0; s < CH / 8; ++s)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) odd_g = fmaf(G[s][j], 0.f, odd_g);
+        // (and the sums of the decays are written)
+        bool odd = __syncthreads_or(odd_g != odd_g || !(sm.part[0] + sm.part[1] > -1e5));
 #pragma unroll
         for (int s = 0; s < CH / 8; ++s) {
             if (s > 2 * warp + 1) break;
@@ -192,6 +202,27 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                 *reinterpret_cast<uint32_t*>(&sm.m[2][t][s0]) = w2;
             }
         }
+        // ---- whether this warp's columns hold only finite numbers (zero times anything else is NaN)
+        const uint32_t odd_x = [&] {
+            uint32_t zeros = 0u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                  // rows lane and lane + 32, eight columns a word
+                const uint4 v = *reinterpret_cast<const uint4*>(&sm.x[buf][lane + 32 * (i >> 1)][warp * 16 + 8 * (i & 1)]);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    __nv_bfloat162 z = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]), __nv_bfloat162(0.f, 0.f), *reinterpret_cast<const __nv_bfloat162*>(&zeros));
+                    zeros = *reinterpret_cast<const uint32_t*>(&z);
+                }
+            }
+            return zeros & 0x7fff7fffu;
+        }();
+        float odd_s = 0.f;
+#pragma unroll
+        for (int n = 0; n < N / 8; ++n)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) odd_s = fmaf(S[n][j], 0.f, odd_s);
+        odd = odd || __any_sync(0xffffffffu, odd_x != 0u || odd_s != odd_s);
         // ---- what the state before the chunk gives: Y^T = S^T C^T, then each token's decay.  The leading terms' products are summed
         // in Y, those of the others, 2^-8 of them and less, in Z.  (Eight independent sums stand between two products of one,
         // about the unit's latency.)
@@ -200,6 +231,7 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
         for (int t = 0; t < CH / 8; ++t)
 #pragma unroll
             for (int j = 0; j < 4; ++j) Y[t][j] = Z[t][j] = 0.f;
+        if (!odd) {
 #pragma unroll
         for (int k = 0; k < N / 16; ++k) {
             uint32_t a0[4], a1[4], a2[4], b[CH / 16][4];
@@ -227,7 +259,31 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
         for (int n = 0; n < N / 8; ++n)
 #pragma unroll
             for (int j = 0; j < 4; ++j) S[n][j] *= last;
+        }
         __syncthreads();                                   // the scores are written
+        if (odd) {
+            for (int t = 0; t < min(CH, n_tok - t0); ++t) {
+                const float step = sm.dt[t], keep = expf(A * step);
+                const float x0 = __bfloat162float(sm.x[buf][t][warp * 16 + g]), x1 = __bfloat162float(sm.x[buf][t][warp * 16 + g + 8]);
+                const float u0 = step * x0, u1 = step * x1;
+                float y0 = 0.f, y1 = 0.f;
+#pragma unroll
+                for (int n = 0; n < N / 8; ++n) {
+                    const uint32_t b = *reinterpret_cast<const uint32_t*>(ch_word<N>(sm.b[buf], t, n) + 2 * q);
+                    const uint32_t c2 = *reinterpret_cast<const uint32_t*>(ch_word<N>(sm.c[buf], t, n) + 2 * q);
+                    S[n][0] = fmaf(keep, S[n][0], ch_low(b) * u0); S[n][1] = fmaf(keep, S[n][1], ch_high(b) * u0);
+                    S[n][2] = fmaf(keep, S[n][2], ch_low(b) * u1); S[n][3] = fmaf(keep, S[n][3], ch_high(b) * u1);
+                    y0 = fmaf(S[n][1], ch_high(c2), fmaf(S[n][0], ch_low(c2), y0));
+                    y1 = fmaf(S[n][3], ch_high(c2), fmaf(S[n][2], ch_low(c2), y1));
+                }
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) { y0 += __shfl_xor_sync(0xffffffffu, y0, o); y1 += __shfl_xor_sync(0xffffffffu, y1, o); }
+                float* row = y + (size_t)(start + t0 + t) * inner + h * P;
+                if (q == 0 && pr < P) row[pr] = fmaf(Dh, x0, y0);
+                if (q == 0 && pr + 8 < P) row[pr + 8] = fmaf(Dh, x1, y1);
+            }
+            continue;
+        }
         // ---- the chunk's own tokens: Y^T += x^T M^T; and the state: S^T += (weight x)^T B
 #pragma unroll
         for (int k = 0; k < CH / 16; ++k) {

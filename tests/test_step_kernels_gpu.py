@@ -134,6 +134,54 @@ def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
     assert rel_err(state[:, :heads * N * P], S.view(len(lens), -1)) < 2e-6
 
 
+@pytest.mark.parametrize("N,value,where", [(128, float("inf"), 5), (64, float("nan"), 77), (128, float("-inf"), 64), (64, float("inf"), 129)])
+@pytest.mark.parametrize("place", ["x", "B", "C", "dt"])
+def test_ssm_scan_in_chunks_is_causal(K, N, value, where, place):
+    """A number that is not finite reaches its own token and those after it, an x or a state its own column alone, as in the
+    walk; the tokens before it, in its block of 16 and its chunk, and the other columns are what they are without it."""
+    torch.manual_seed(N + where)
+    heads, P, T = 2, 64, 130
+    xbc = torch.randn(T, heads * P + 2 * N, device="cuda").bfloat16()
+    proj, bias = torch.randn(T, heads, device="cuda"), torch.randn(heads, device="cuda") - 2
+    a_log, D = torch.linspace(-1, 2, heads, device="cuda"), torch.randn(heads, device="cuda")
+    state = torch.randn(1, heads * N * P, device="cuda")
+    cu, slots = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    runs = []
+    for odd in (True, False):
+        target, column = (proj, 0) if place == "dt" else (xbc, {"x": 3, "B": heads * P + 9, "C": heads * P + N + 9}[place])
+        target[where, column] = value if odd else 0.5
+        state.view(heads, N, P)[1, 7, 40] = value if odd and place == "x" else 0.5
+        for chunked in (True, False):
+            s = state.clone()
+            y = K.ssm_scan(xbc, proj, 0, bias, a_log, D, cu, slots, s, heads, P, N, 1, max_q_len=T, chunked=chunked)
+            runs.append((y.view(T, heads, P), s.view(heads, N, P)))
+    for got, walk in zip(runs[0], runs[1]):
+        assert all(torch.equal(kind(got), kind(walk)) for kind in (torch.isnan, torch.isposinf, torch.isneginf))
+    (y, s), _, (plain_y, plain_s), _ = runs
+    assert rel_err(y[:where, 0], plain_y[:where, 0].double().cpu()) < 2e-6
+    if place == "x":
+        assert not y[where, 0, 3].isfinite()
+        other = [p for p in range(P) if p != 3]
+        assert rel_err(y[:, 0][:, other], plain_y[:, 0][:, other].double().cpu()) < 2e-6
+        assert rel_err(s[0][:, other], plain_s[0][:, other].double().cpu()) < 2e-6
+
+
+def test_ssm_scan_in_chunks_beside_a_step_size_that_dwarfs_the_others(K):
+    """A sum of decays that one step of 10^17 dominates still tells the decays of the tokens after it."""
+    torch.manual_seed(1)
+    heads, P, N, T = 1, 16, 64, 64
+    xbc, proj = torch.randn(T, heads * P + 2 * N, device="cuda").bfloat16(), torch.randn(T, heads, device="cuda")
+    proj[20] = 1e17
+    xbc[20, :P] = 0                                          # (what it brings is then nothing)
+    zero, cu, slots = torch.zeros(heads, device="cuda"), torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    runs = []
+    for chunked in (True, False):
+        state = torch.ones(1, heads * N * P, device="cuda")
+        runs.append((K.ssm_scan(xbc, proj, 0, zero, zero, zero, cu, slots, state, heads, P, N, 1, max_q_len=T, chunked=chunked), state))
+    for got, walk in zip(*runs):
+        assert rel_err(got, walk.double().cpu()) < 2e-6
+
+
 @pytest.mark.parametrize("inner,N,lens", [(70, 16, (1, 5, 16, 17, 35)), (33, 32, (18, 2)), (32, 16, (64,))])
 def test_selective_scan_in_two_roles(K, inner, N, lens):
     torch.manual_seed(inner)
