@@ -3,13 +3,15 @@
 //     y_t   = e^(c_t) S^T C_t + sum_{s <= t} (C_t . B_s) e^(c_t - c_s) dt_s x_s + D_h x_t
 //     S_new = e^(c_L) S + sum_s (e^(c_L - c_s) dt_s) B_s x_s^T
 // which is four products per chunk of 64 tokens instead of 64 dependent updates of the whole state: 2,048 tokens of 128 heads
-// of 64 x 128 take 278 us in place of 1,010, portions of 1,228 and 820 tokens 194 in place of 707.
+// of 64 x 128 take 330 us in place of 1,040, portions of 1,228 and 820 tokens 227 in place of 713.
 //
 // x, B and C are bfloat16 as they come, so products among them are exact; the float factors (the state, the weighted
 // scores, the weighted x) go in as three bfloat16 terms each (24 bits: v = hi + mid + lo), so nothing is rounded below
 // float.  The running sums c are formed in double and kept as two floats, so a difference of two of them is as exact as
-// a sum of the few terms between.  Against float64 the state is as close as the walk's (1.2e-7), y 0.9e-7 against 0.5e-7: both
-// below a float's own last place, and the same figures for the layer's bfloat16 result.
+// a sum of the few terms between; an exponential makes up for its argument's rounding.  The tensor cores cut sums off where float
+// rounds them: products of leading terms start from zero and are added in float.  Against float64 (2-norms, decays of dt 0.001
+// to 0.1, rates 1 to 16): y 0.9e-7, state 0.8e-7 to 1.3e-7; the walk 1.4e-7 to 7e-7 and 1.4e-7 to 2e-6.  With one accumulator for
+// all terms and plain exponentials they were 1.8e-7 to 4.6e-7 and up to 8.6e-7, above the walk's for some heads, in 296 us.
 //
 // A product multiplies the masked zeros of a block of scores with the x of later tokens, infinities do not split into terms, and
 // a running sum that a single step size dominates does not tell the others' decays any more.  So a chunk with numbers that
@@ -28,6 +30,23 @@
 __device__ __forceinline__ void ch_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// The same from zero: the tensor cores cut their sums off, they do not round them, so the products of leading terms are kept from
+// running through one accumulator and added in float.
+__device__ __forceinline__ void ch_mma_new(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void ch_mma_add(float (&sum)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    float c[4];
+    ch_mma_new(c, a, b0, b1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[j] += c[j];
+}
+// e^v of a double as a float, to float's last place: the argument's own rounding is made up for
+__device__ __forceinline__ float ch_exp(double v) {
+    const float hi = (float)v, e = expf(hi);
+    return fmaf(e, (float)(v - (double)hi), e);
 }
 __device__ __forceinline__ void ch_ldsm(uint32_t (&r)[4], const void* p) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
@@ -153,9 +172,9 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
             sm.dt[tid] = dt;
             sm.cum[tid] = hi;
             sm.cum_lo[tid] = (float)(c - (double)hi);
-            sm.decay[tid] = expf(hi);
-            sm.weight[tid] = expf((float)(total - c)) * dt;
-            if (tid == 0) sm.last = expf((float)total);
+            sm.decay[tid] = ch_exp(c);
+            sm.weight[tid] = ch_exp(total - c) * dt;
+            if (tid == 0) sm.last = ch_exp(total);
         }
         // ---- scores of this warp's 16 tokens: C_t . B_s for s up to the warp's last token
         float G[CH / 8][4];
@@ -170,8 +189,8 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                 if (s > warp) break;
                 uint32_t b[4];
                 ch_ldsm(b, ch_word<N>(sm.b[buf], s * 16 + (mi >> 1) * 8 + mr, 2 * k + (mi & 1)));
-                ch_mma(G[2 * s], a, b[0], b[1]);
-                ch_mma(G[2 * s + 1], a, b[2], b[3]);
+                ch_mma_add(G[2 * s], a, b[0], b[1]);
+                ch_mma_add(G[2 * s + 1], a, b[2], b[3]);
             }
         }
         float odd_g = 0.f;                                 // B_t . C_t is not finite where B_t or C_t is not
@@ -192,7 +211,11 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                 for (int j = 0; j < 2; ++j) {
                     const int ss = s0 + j;
                     v[j] = 0.f;
-                    if (ss <= t) v[j] = G[s][2 * r + j] * expf((sm.cum[t] - sm.cum[ss]) + (sm.cum_lo[t] - sm.cum_lo[ss])) * sm.dt[ss];
+                    if (ss <= t) {                          // (|c_t| >= |c_s|: what the subtractions round off is known exactly)
+                        const float d = sm.cum[t] - sm.cum[ss], lo = ((sm.cum[t] - d) - sm.cum[ss]) + (sm.cum_lo[t] - sm.cum_lo[ss]);
+                        const float arg = d + lo, e = expf(arg);
+                        v[j] = G[s][2 * r + j] * fmaf(e, lo - (arg - d), e) * sm.dt[ss];
+                    }
                     if (ss == t) v[j] += Dh;
                 }
                 uint32_t w0, w1, w2;
@@ -244,7 +267,7 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
 #pragma unroll
             for (int t = 0; t < CH / 16; ++t) { ch_mma(Z[2 * t], a2, b[t][0], b[t][1]); ch_mma(Z[2 * t + 1], a2, b[t][2], b[t][3]); }
 #pragma unroll
-            for (int t = 0; t < CH / 16; ++t) { ch_mma(Y[2 * t], a0, b[t][0], b[t][1]); ch_mma(Y[2 * t + 1], a0, b[t][2], b[t][3]); }
+            for (int t = 0; t < CH / 16; ++t) { ch_mma_add(Y[2 * t], a0, b[t][0], b[t][1]); ch_mma_add(Y[2 * t + 1], a0, b[t][2], b[t][3]); }
 #pragma unroll
             for (int t = 0; t < CH / 16; ++t) { ch_mma(Z[2 * t], a1, b[t][0], b[t][1]); ch_mma(Z[2 * t + 1], a1, b[t][2], b[t][3]); }
         }
@@ -254,11 +277,6 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
             Y[t][0] *= d0; Y[t][1] *= d1; Y[t][2] *= d0; Y[t][3] *= d1;
             Z[t][0] *= d0; Z[t][1] *= d1; Z[t][2] *= d0; Z[t][3] *= d1;
         }
-        const float last = sm.last;
-#pragma unroll
-        for (int n = 0; n < N / 8; ++n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) S[n][j] *= last;
         }
         __syncthreads();                                   // the scores are written
         if (odd) {
@@ -284,7 +302,7 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
             }
             continue;
         }
-        // ---- the chunk's own tokens: Y^T += x^T M^T; and the state: S^T += (weight x)^T B
+        // ---- the chunk's own tokens: Y^T += x^T M^T
 #pragma unroll
         for (int k = 0; k < CH / 16; ++k) {
             uint32_t xa[4];
@@ -296,28 +314,9 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                     if (k > t) continue;                   // tokens before the block see nothing of it
                     uint32_t b[4];
                     ch_ldsm(b, &sm.m[term][t * 16 + (mi >> 1) * 8 + mr][k * 16 + (mi & 1) * 8]);
-                    ch_mma(term ? Z[2 * t] : Y[2 * t], xa, b[0], b[1]);
-                    ch_mma(term ? Z[2 * t + 1] : Y[2 * t + 1], xa, b[2], b[3]);
+                    if (term) { ch_mma(Z[2 * t], xa, b[0], b[1]); ch_mma(Z[2 * t + 1], xa, b[2], b[3]); }
+                    else { ch_mma_add(Y[2 * t], xa, b[0], b[1]); ch_mma_add(Y[2 * t + 1], xa, b[2], b[3]); }
                 }
-            const float w0 = sm.weight[k * 16 + 2 * q], w1 = sm.weight[k * 16 + 2 * q + 1];
-            const float w2 = sm.weight[k * 16 + 8 + 2 * q], w3 = sm.weight[k * 16 + 8 + 2 * q + 1];
-            uint32_t a0[4], a1[4], a2[4];
-            ch_split(ch_low(xa[0]) * w0, ch_high(xa[0]) * w1, a0[0], a1[0], a2[0]);
-            ch_split(ch_low(xa[1]) * w0, ch_high(xa[1]) * w1, a0[1], a1[1], a2[1]);
-            ch_split(ch_low(xa[2]) * w2, ch_high(xa[2]) * w3, a0[2], a1[2], a2[2]);
-            ch_split(ch_low(xa[3]) * w2, ch_high(xa[3]) * w3, a0[3], a1[3], a2[3]);
-#pragma unroll
-            for (int n0 = 0; n0 < N / 16; n0 += 4) {
-                uint32_t b[4][4];
-#pragma unroll
-                for (int n = 0; n < 4; ++n) ch_ldsm_t(b[n], ch_word<N>(sm.b[buf], k * 16 + (mi & 1) * 8 + mr, 2 * (n0 + n) + (mi >> 1)));
-#pragma unroll
-                for (int n = 0; n < 4; ++n) { ch_mma(S[2 * (n0 + n)], a2, b[n][0], b[n][1]); ch_mma(S[2 * (n0 + n) + 1], a2, b[n][2], b[n][3]); }
-#pragma unroll
-                for (int n = 0; n < 4; ++n) { ch_mma(S[2 * (n0 + n)], a1, b[n][0], b[n][1]); ch_mma(S[2 * (n0 + n) + 1], a1, b[n][2], b[n][3]); }
-#pragma unroll
-                for (int n = 0; n < 4; ++n) { ch_mma(S[2 * (n0 + n)], a0, b[n][0], b[n][1]); ch_mma(S[2 * (n0 + n) + 1], a0, b[n][2], b[n][3]); }
-            }
         }
 #pragma unroll
         for (int t = 0; t < CH / 8; ++t)
@@ -326,6 +325,39 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
                 const int p = pr + 8 * (j >> 1), tt = t0 + t * 8 + 2 * q + (j & 1);
                 if (p < P && tt < n_tok) y[(size_t)(start + tt) * inner + h * P + p] = Y[t][j] + Z[t][j];
             }
+        // ---- the state: S^T = e^(c_L) S^T + (weight x)^T B, 64 of its rows n at a time (sums of the leading terms and of the others)
+        const float last = sm.last;
+#pragma unroll
+        for (int n0 = 0; n0 < N / 16; n0 += 4) {
+            float U[8][4], V[8][4];
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) U[n][j] = V[n][j] = 0.f;
+#pragma unroll
+            for (int k = 0; k < CH / 16; ++k) {
+                uint32_t xa[4], a0[4], a1[4], a2[4], b[4][4];
+                ch_ldsm_t(xa, &sm.x[buf][k * 16 + (mi >> 1) * 8 + mr][warp * 16 + (mi & 1) * 8]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) ch_ldsm_t(b[n], ch_word<N>(sm.b[buf], k * 16 + (mi & 1) * 8 + mr, 2 * (n0 + n) + (mi >> 1)));
+                const float w0 = sm.weight[k * 16 + 2 * q], w1 = sm.weight[k * 16 + 2 * q + 1];
+                const float w2 = sm.weight[k * 16 + 8 + 2 * q], w3 = sm.weight[k * 16 + 8 + 2 * q + 1];
+                ch_split(ch_low(xa[0]) * w0, ch_high(xa[0]) * w1, a0[0], a1[0], a2[0]);
+                ch_split(ch_low(xa[1]) * w0, ch_high(xa[1]) * w1, a0[1], a1[1], a2[1]);
+                ch_split(ch_low(xa[2]) * w2, ch_high(xa[2]) * w3, a0[2], a1[2], a2[2]);
+                ch_split(ch_low(xa[3]) * w2, ch_high(xa[3]) * w3, a0[3], a1[3], a2[3]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) { ch_mma(V[2 * n], a2, b[n][0], b[n][1]); ch_mma(V[2 * n + 1], a2, b[n][2], b[n][3]); }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) { ch_mma_add(U[2 * n], a0, b[n][0], b[n][1]); ch_mma_add(U[2 * n + 1], a0, b[n][2], b[n][3]); }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) { ch_mma(V[2 * n], a1, b[n][0], b[n][1]); ch_mma(V[2 * n + 1], a1, b[n][2], b[n][3]); }
+            }
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) S[2 * n0 + n][j] = fmaf(last, S[2 * n0 + n][j], U[n][j] + V[n][j]);
+        }
     }
 #pragma unroll
     for (int n = 0; n < N / 8; ++n)
