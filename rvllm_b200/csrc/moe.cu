@@ -243,6 +243,12 @@ __device__ __forceinline__ uint4 moe_ld_weight(const uint4* p) {
     return v;
 }
 
+// The same with c = 0.
+__device__ __forceinline__ void moe_mma_new(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // acc[n]: 16 matrix rows (this lane's rows wlo, whi) against NT blocks of 8 vectors (this lane's x[n]), over the 32-wide blocks
 // c0 .. c1 - 1 of k, U of them in flight (4 with one CTA more per SM: 10 % slower).  The pointers stand at 8 (lane & 3)
 // elements of their row.
@@ -255,12 +261,19 @@ __device__ __forceinline__ void moe_mma_span(const uint4* wlo, const uint4* whi,
 #pragma unroll
         for (int u = 0; u < U; ++u) { lo[u] = moe_ld_weight(wlo + (c + u) * 4); hi[u] = moe_ld_weight(whi + (c + u) * 4); }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
+        for (int u0 = 0; u0 < U; u0 += 4)                   // sums of 128 k from zero, then added in float: the tensor cores cut off what
+#pragma unroll                                              // float rounds, so no sum runs through all of k there
             for (int n = 0; n < NT; ++n) {
-                const uint4 b = x[n][(c + u) * 4];
-                moe_mma(acc[n], lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
-                moe_mma(acc[n], lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+                float part[4];
+#pragma unroll
+                for (int u = u0; u < u0 + 4; ++u) {
+                    const uint4 b = x[n][(c + u) * 4];
+                    if (u == u0) moe_mma_new(part, lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
+                    else moe_mma(part, lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
+                    moe_mma(part, lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[n][j] += part[j];
             }
     }
     for (; c < c1; ++c) {
@@ -358,9 +371,10 @@ moe_mma_gate_up_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
             float s[MT];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                s[m] = 0.f;
+                double sum = 0.0;                           // (the parts meet with one rounding)
 #pragma unroll
-                for (int w = 0; w < PARTS; ++w) s[m] += red[((m * PARTS + w) * 16 + row) * MM_PASS + p];
+                for (int w = 0; w < PARTS; ++w) sum += (double)red[((m * PARTS + w) * 16 + row) * MM_PASS + p];
+                s[m] = (float)sum;
             }
             float v;
             if constexpr (GATED) v = s[0] / (1.0f + expf(-s[0])) * s[MT - 1];
@@ -458,19 +472,19 @@ moe_mma_down_kernel(const __nv_bfloat16* __restrict__ act, const int* __restrict
     for (int i = tid; i < tokens * 16; i += blockDim.x) {
         const int t = i >> 4, n = n0 + (i & 15);
         if (n >= width) continue;
-        float sum = 0.f;
-        for (int k = 0; k < top; ++k) {                     // the slots in their order: one sum per element
+        double sum = 0.0;                                   // quarters, slots and `add` meet with one rounding: the parts' cut sums are a little
+        for (int k = 0; k < top; ++k) {                     // further from 64 bits than float chains, and these roundings were as large
             const int pair = t * top + k, e = chosen[pair];
-            const float wk = weights ? weights[pair] : 1.f;
-            if (e >= experts && identity_x) sum = fmaf(wk, __bfloat162float(identity_x[(size_t)t * width + n]), sum);
+            const double wk = weights ? (double)weights[pair] : 1.0;
+            if (e >= experts && identity_x) sum = fma(wk, (double)__bfloat162float(identity_x[(size_t)t * width + n]), sum);
             if (e < 0 || e >= experts) continue;
             const float* p = part + (size_t)pair * 16 + (i & 15);
             const size_t step = (size_t)pairs * 16;
-            sum = fmaf(wk, (p[0] + p[step]) + (p[2 * step] + p[3 * step]), sum);
+            sum = fma(wk, ((double)p[0] + (double)p[step]) + ((double)p[2 * step] + (double)p[3 * step]), sum);
         }
-        float v = sum * weight;
-        if (add) v += add_scale ? add_scale[t] * add[(size_t)t * width + n] : add[(size_t)t * width + n];
-        out[(size_t)t * width + n] = rv_from_float<TO>(v);
+        double v = sum * (double)weight;
+        if (add) v += (add_scale ? (double)add_scale[t] : 1.0) * (double)add[(size_t)t * width + n];
+        out[(size_t)t * width + n] = rv_from_float<TO>((float)v);
     }
 }
 

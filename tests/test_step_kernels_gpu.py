@@ -83,6 +83,26 @@ def test_moe_of_few_tokens_on_the_tensor_cores(K, T, E, top, ff, width, gated, i
     assert torch.equal(run(1), out[:1])
 
 
+@pytest.mark.parametrize("T,E,top,ff,width", [(8, 8, 2, 4096, 1024), (33, 16, 4, 1408, 2048), (20, 16, 4, 256, 1024)])
+def test_moe_sums_of_whole_activations(K, T, E, top, ff, width):
+    """Activations that are whole numbers of at most 256 (squares of sums of few ones and twos) are the same in bfloat16, so
+    what is left is the error of the float sums over ff and the slots."""
+    torch.manual_seed(T)
+    gu = (torch.randint(-2, 3, (E, ff, width), device="cuda") * (torch.rand(E, ff, width, device="cuda") < 4.0 / width)).bfloat16()
+    x, dn = torch.randint(0, 2, (T, width), device="cuda").bfloat16(), (torch.randn(E, width, ff, device="cuda") * 0.02).bfloat16()
+    ch = torch.stack([torch.randperm(E, device="cuda")[:top] for _ in range(T)]).to(torch.int32)
+    w = torch.rand(T, top, device="cuda")
+    out = K.moe_experts(x, ch, gu, dn, 1.0, out_dtype=torch.float32, weights=w, activation="relu2")
+    ref = torch.zeros(T, width, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        h = torch.relu(x.double() @ gu[e].double().t()) ** 2
+        assert h.max() <= 256
+        ref += (h @ dn[e].double().t()) * (w.double() * (ch == e)).sum(1, keepdim=True)
+    # 2-norms: a float's own rounding is up to 2^-24 / sqrt(3) = 3.4e-8; the sums of 128 k add less than that again
+    # (float chains, one pair at a time: 4.2e-8 to 5.8e-8; one accumulator of the tensor cores through all of k: up to 7.5e-8)
+    assert float((out.double() - ref).norm() / ref.norm()) < 5e-8
+
+
 @pytest.mark.parametrize("M,N,Kd", [(130, 264, 72), (300, 96, 128), (512, 512, 4096), (5, 200, 136), (64, 1024, 264), (200, 130, 72)])
 @pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16])
 def test_bias_and_clamped_gate_in_the_products_epilogues(K, M, N, Kd, bias_dtype):
