@@ -1022,14 +1022,22 @@ class CudaKernels:
         _check("qk_norm_rope_cache_write", st)
         return q, gate
 
+    @staticmethod
+    def _longest(T: int, n_seqs: int, max_q_len: Optional[int]) -> int:
+        """The tokens of a step's longest portion, as far as the host knows: of a step of no more tokens than sequences one
+        each, else perhaps all.  It picks among kernels that give the same bits."""
+        return max_q_len if max_q_len is not None else (1 if T <= n_seqs else T)
+
     def causal_conv_silu(self, proj, col0: int, channels: int, weight, bias, token_seq, cu_seqlens, state_slots, state,
-                         conv_off: int, out_dtype) -> torch.Tensor:
+                         conv_off: int, out_dtype, max_q_len: Optional[int] = None) -> torch.Tensor:
         """silu(causal convolution per channel) of columns col0 .. col0 + channels of `proj`, continued from and
-        leaving behind each request's last taps - 1 inputs in `state` (float [slots, floats], at `conv_off`)."""
+        leaving behind each request's last taps - 1 inputs in `state` (float [slots, floats], at `conv_off`).
+        `max_q_len`: the most tokens that any sequence brings (see `_longest`); the bits do not depend on it."""
         _need(proj, "proj", dims=2); _need(weight, "weight", dims=2); _need(state, "state", torch.float32, 2)
         if weight.shape[0] != channels or (bias is not None and (bias.shape != (channels,) or bias.dtype != weight.dtype)):
             raise KernelError("causal_conv_silu: taps and bias do not fit the channels")
         T, taps = proj.shape[0], weight.shape[1]
+        longest = self._longest(T, state_slots.shape[0], max_q_len)
         if conv_off + (taps - 1) * channels > state.shape[1]:
             raise KernelError("causal_conv_silu: the state rows are too short for the convolution's inputs")
         out = torch.empty((T, channels), dtype=out_dtype, device=proj.device)
@@ -1037,9 +1045,9 @@ class CudaKernels:
             _ptr(proj), c_int(self._dt(proj, "proj")), c_int(proj.shape[1]), c_int(col0), _ptr(weight), _ptr(bias),
             c_int(self._dt(weight, "weight")), _ptr(token_seq), _ptr(cu_seqlens), _ptr(state_slots), _ptr(state),
             ctypes.c_longlong(state.shape[1]), ctypes.c_longlong(conv_off), _ptr(out), c_int(_DT[out_dtype]), c_int(T),
-            c_int(state_slots.shape[0]), c_int(channels), c_int(taps), self._stream())
+            c_int(state_slots.shape[0]), c_int(channels), c_int(taps), c_int(longest), self._stream())
         _check("causal_conv_silu", st)
-        COUNTERS['launches'] += 1 if taps > 4 or (taps > 1 and T > 2 * state_slots.shape[0]) else 0
+        COUNTERS['launches'] += 1 if taps > 4 or (taps > 1 and longest > 2) else 0
         return out
 
     SCAN_CHUNK_MIN_TOKENS = 32         # tokens of a portion from which the recurrence goes chunk by chunk (32 tokens: 50 us against 85)

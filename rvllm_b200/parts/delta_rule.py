@@ -63,7 +63,7 @@ class GatedDeltaRule(Part):
         k = ctx.kernels
         proj = self.proj(x, ctx, out_dtype=torch.float32)
         qkv = k.causal_conv_silu(proj, 0, self.channels, self.conv_w, None, ctx.token_seq, ctx.cu_seqlens, ctx.state_slots,
-                                 cache.state, self.state_floats, x.dtype)
+                                 cache.state, self.state_floats, x.dtype, max_q_len=max(ctx.q_lens))
         gate_col = self.channels
         o = k.delta_rule(qkv, proj, gate_col + self.v_dim, gate_col + self.v_dim + self.heads, self.a_log, self.dt_bias,
                          ctx.cu_seqlens, ctx.state_slots, cache.state, self.heads, self.qk_heads, self.head_dim, self.value_dim,

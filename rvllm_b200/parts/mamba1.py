@@ -59,7 +59,7 @@ class Mamba1Mixer(Part):
         k = ctx.kernels
         proj = self.in_proj(x, ctx, out_dtype=torch.float32)                       # [u | z]
         u = k.causal_conv_silu(proj, 0, self.inner, self.conv_w, self.conv_b, ctx.token_seq, ctx.cu_seqlens,
-                               ctx.state_slots, cache.state, self.ssm_floats, x.dtype)
+                               ctx.state_slots, cache.state, self.ssm_floats, x.dtype, max_q_len=max(ctx.q_lens))
         dbc = self.x_proj(u, ctx, out_dtype=torch.float32)                         # [d | B | C]
         d = k.column_slice(dbc, 0, self.dt_rank, x.dtype)
         dt_raw = self.dt_proj(d, ctx, out_dtype=torch.float32)

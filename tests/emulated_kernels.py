@@ -401,7 +401,7 @@ class EmulatedKernels:
         gate = torch.sigmoid(x[:, qw + kw:]) if with_gate else None
         return qo, gate
 
-    def causal_conv_silu(self, proj, col0, channels, weight, bias, token_seq, cu_seqlens, state_slots, state, conv_off, out_dtype):
+    def causal_conv_silu(self, proj, col0, channels, weight, bias, token_seq, cu_seqlens, state_slots, state, conv_off, out_dtype, max_q_len=None):
         taps = weight.shape[1]
         u = proj[:, col0:col0 + channels].float()
         out = torch.zeros_like(u)

@@ -245,13 +245,43 @@ def test_convolution_of_single_tokens_in_one_launch(K, taps, lens):
         cu.append(cu[-1] + n)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
     seq = [s for s, n in enumerate(lens) for _ in range(n)]
-    got = K.causal_conv_silu(proj, 5, C, w, b, i32(seq), i32(cu), i32(list(range(1, len(lens) + 1))), state, 7, torch.float32)
+    got = K.causal_conv_silu(proj, 5, C, w, b, i32(seq), i32(cu), i32(list(range(1, len(lens) + 1))), state, 7, torch.float32,
+                             max_q_len=max(lens))
     for s, n in enumerate(lens):
         row = torch.cat([hist[s + 1], proj[cu[s]:cu[s + 1], 5:].double().cpu()])
         for t in range(n):
             v = b.double().cpu() + (row[t:t + taps] * w.double().cpu().t()).sum(0)
             assert rel_err(got[cu[s] + t], torch.nn.functional.silu(v)) < 2e-6
         assert taps == 1 or rel_err(state[s + 1, 7:], row[n:].reshape(-1)) < 1e-7
+
+
+@pytest.mark.parametrize("taps,lens,in_dtype", [(4, (1, 2, 1, 2), torch.float32), (3, (2, 1), torch.bfloat16), (4, (1,) * 9 + (21,), torch.float32), (2, (2,), torch.bfloat16)])
+def test_convolution_bits_do_not_depend_on_the_step(K, taps, lens, in_dtype):
+    """A request's outputs and state are the same bits whatever runs beside it, and whichever of the two forms a step takes; a
+    padding row (slot -1) starts from zeros and leaves no state."""
+    torch.manual_seed(taps + len(lens))
+    T, C = sum(lens), 131
+    proj, w, b = torch.randn(T, C + 5, device="cuda").to(in_dtype), torch.randn(C, taps, device="cuda"), torch.randn(C, device="cuda")
+    before = torch.randn(len(lens), (taps - 1) * C, device="cuda")
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    slots = list(range(len(lens)))
+    if len(lens) > 2:
+        slots[1] = -1
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+
+    def run(rows, which, longest):
+        state = before.clone()
+        n = [lens[s] for s in which]
+        out = K.causal_conv_silu(proj[rows].contiguous(), 5, C, w, b, i32([i for i, k in enumerate(n) for _ in range(k)]),
+                                 i32([0] + torch.tensor(n).cumsum(0).tolist()), i32([slots[s] for s in which]), state, 0, torch.float32, max_q_len=longest)
+        return out, state
+    whole, state = run(slice(0, T), range(len(lens)), max(lens))
+    forms = [run(slice(0, T), range(len(lens)), longest) for longest in (2, 3, None)]
+    assert all(torch.equal(whole, o) and torch.equal(state, s) for o, s in forms)
+    for s in range(len(lens)):
+        alone, own = run(slice(cu[s], cu[s + 1]), [s], lens[s])
+        assert torch.equal(alone, whole[cu[s]:cu[s + 1]])
+        assert torch.equal(own[s], state[s]) and (slots[s] >= 0 or torch.equal(state[s], before[s]))
 
 
 @pytest.mark.parametrize("d,vd,heads,qk,lens", [(128, 128, 4, 2, (1, 15, 16, 17, 70)), (100, 36, 2, 1, (33,)), (64, 68, 2, 2, (20, 1)), (40, 4, 2, 1, (18,)),
