@@ -182,15 +182,16 @@ __device__ __forceinline__ float rv_warp_sum(float v) {
     return v;
 }
 
-// Four sums over PARTS (8, 16 or 32) neighbouring lanes, dealt out: a lane gets sum number part / (PARTS / 4).
+// Four sums over PARTS (8, 16 or 32) neighbouring lanes, dealt out: a lane gets sum number part & 3.  Neighbours are added first,
+// then neighbouring pairs, and so on up.
 template <int PARTS>
 __device__ __forceinline__ float rv_sum4_dealt(const float (&v)[4], int part) {
-    const bool hi = part & (PARTS / 2), mid = part & (PARTS / 4);
-    const float k0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], PARTS / 2);
-    const float k1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], PARTS / 2);
-    float r = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, PARTS / 4);
+    const bool odd = part & 1, high = part & 2;
+    const float k0 = (odd ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 1);      // sum number 0 or 1
+    const float k1 = (odd ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, odd ? v[2] : v[3], 1);      // 2 or 3
+    float r = (high ? k1 : k0) + __shfl_xor_sync(0xffffffffu, high ? k0 : k1, 2);
 #pragma unroll
-    for (int o = PARTS / 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    for (int o = 4; o < PARTS; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
     return r;
 }
 

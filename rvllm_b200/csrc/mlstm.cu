@@ -237,10 +237,9 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int width = vd + 1;                              // columns of a head's state: the values and the constant 1
     if (warp < 4) {                                        // ---- the walk
-        constexpr int Q = PARTS / 4;                       // lanes of a column after the reduction
         const int part = lane % PARTS, group = lane / PARTS;
         const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;
-        const int n0 = part * 8, mine = part / Q;          // this lane's column after the reduction
+        const int n0 = part * 8, mine = part & 3;          // this lane's column after the reduction
         float S[8][4];
         float* srow = state + (size_t)slot * state_stride + (size_t)h * d * width + col;
 #pragma unroll
@@ -270,7 +269,7 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
                         aq[j] = fmaf(S[i][j], qr[i], aq[j]);
                     }
                 const float ov = rv_sum4_dealt<PARTS>(aq, part);
-                if (part % Q == 0 && col + mine < width) raw[((size_t)(start + t0 + tt) * heads + h) * width + col + mine] = ov;
+                if (part < 4 && col + mine < width) raw[((size_t)(start + t0 + tt) * heads + h) * width + col + mine] = ov;
             };
             if (nt == ML_CHUNK) {
 #pragma unroll 4

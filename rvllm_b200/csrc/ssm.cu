@@ -1220,7 +1220,7 @@ __global__ void __launch_bounds__(256)
 delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
                        int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps) {
+                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     using Stage = DeltaStage<PARTS>;
@@ -1230,14 +1230,14 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok < least) return;                             // (the other kernel's)
     const int chunks = (n_tok + DR_CHUNK - 1) / DR_CHUNK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < 4) {                                        // ---- the walk
-        constexpr int Q = PARTS / 4;                       // lanes of a column after the reduction
         const int part = lane % PARTS, group = lane / PARTS;
         const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;      // (vd is a multiple of 4: a group's columns are all there or none)
         const bool live = col < vd;
-        const int n0 = part * 8, mine = part / Q;          // this lane's column after the reduction
+        const int n0 = part * 8, mine = part & 3;          // this lane's column after the reduction
         float S[8][4];
         float* srow = state + (size_t)slot * state_stride + (size_t)h * d * vd + col;
 #pragma unroll
@@ -1266,16 +1266,16 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
 #pragma unroll
                     for (int j = 0; j < 4; ++j) { ak[j] = fmaf(S[i][j], kr[i], ak[j]); aq[j] = fmaf(S[i][j], qr[i], aq[j]); }
                 const float acc = rv_sum4_dealt<PARTS>(ak, part);
-                const float u = st.beta[tt] * (vv - g * acc);
+                const float u = st.beta[tt] * fmaf(-g, acc, vv);
                 float uj[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) uj[j] = __shfl_sync(0xffffffffu, u, group * PARTS + j * Q);
+                for (int j = 0; j < 4; ++j) uj[j] = __shfl_sync(0xffffffffu, u, group * PARTS + j);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) S[i][j] = fmaf(g, S[i][j], kr[i] * uj[j]);
                 const float ov = rv_sum4_dealt<PARTS>(aq, part);
-                if (part % Q == 0 && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
+                if (part < 4 && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
             };
             if (nt == DR_CHUNK) {                          // a whole chunk: neighbouring tokens may run into one another
 #pragma unroll 4
@@ -1295,7 +1295,7 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     // ---- staging: a warp per token for q and k, the block's columns of v, a thread per token for g and beta
     const int tid = threadIdx.x - 128, sw = warp - 4;
     const int kh = h / (heads / qk_heads), qk = qk_heads * d;
-    const float q_scale = rsqrtf((float)d);
+    const float q_scale = 1.0f / sqrtf((float)d);
     const float decay_rate = expf(a_log[h]), a_bias = dt_bias[h];
     constexpr int E = PARTS / 4;                           // elements of q (and k) per lane: 8 PARTS / 32
     constexpr int PV = DR_CHUNK * Stage::COLS / 128;
@@ -1382,23 +1382,27 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     }
 }
 
-// Steps of few tokens a sequence: a block per (128 columns of a head, sequence), a thread on four neighbouring columns of 16 rows,
+// Sequences of one to four tokens: a block per (128 columns of a head, sequence), a thread on four neighbouring columns of 16 rows,
 // all its rows in flight together.  Bound by the state's way from memory and back: 64 sequences of 32 heads of 128 x 128
-// (268 MB) 130 us with the walk's set-up around one token, 57 us; 4 sequences 13.8 and 9.9 us of a decode step.
-__global__ void __launch_bounds__(256)
+// (268 MB) 148 us in the walk, 58 here; of three tokens 169 and 98, of eight 224 and 199.  CTAS a SM: one (178 registers) where the
+// grid is no larger than the SMs, two else; 4 sequences 12.5 us in the walk, 6.1 and 7.4 here, 64 of them 83 and 58.
+// The sums are those of the walk, entry by entry in the same order (8 neighbouring rows in a chain, then neighbours, then
+// neighbouring pairs ...), so a request's bits do not depend on which of the two a step takes.
+template <int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
 delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
                        int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps) {
+                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps, int most) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     __shared__ __align__(16) float sq[128], sk[128], su[128];
     __shared__ __align__(16) float pk[8][128], pq[8][128];
-    __shared__ float sums[3][4];
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], end = cu_seqlens[seq + 1];
+    if (end - start > most) return;                        // (the other kernel's)
     const int cl = lane * 4, col = blockIdx.x * 128 + cl, n0 = warp * 16;
     const bool live = col < vd;
     const int kh = h / (heads / qk_heads), qk = qk_heads * d;
@@ -1408,53 +1412,58 @@ delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     for (int i = 0; i < 16; ++i) S[i] = live && n0 + i < d ? *reinterpret_cast<const float4*>(srow + (size_t)(n0 + i) * vd) : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int t = start; t < end; ++t) {
         const size_t row = (size_t)t * qkv_stride;
-        float fq = 0.f, fk = 0.f;
         if (tid < 128) {
-            if (tid < d) {
-                fq = rv_load_any(qkv, qkv_dtype, row + (size_t)kh * d + tid);
-                fk = rv_load_any(qkv, qkv_dtype, row + qk + (size_t)kh * d + tid);
-            }
-            const float q2 = rv_warp_sum(fq * fq), k2 = rv_warp_sum(fk * fk), kq = rv_warp_sum(fk * fq);
-            if (lane == 0) { sums[0][warp] = q2; sums[1][warp] = k2; sums[2][warp] = kq; }
+            sq[tid] = tid < d ? rv_load_any(qkv, qkv_dtype, row + (size_t)kh * d + tid) : 0.f;
+            sk[tid] = tid < d ? rv_load_any(qkv, qkv_dtype, row + qk + (size_t)kh * d + tid) : 0.f;
+            su[tid] = 0.f;
         }
-        __syncthreads();
-        const float rq = rsqrtf((float)d) / sqrtf(sums[0][0] + sums[0][1] + sums[0][2] + sums[0][3] + unit_eps);
-        const float rk = 1.0f / sqrtf(sums[1][0] + sums[1][1] + sums[1][2] + sums[1][3] + unit_eps);
-        if (tid < 128) { sq[tid] = fq * rq; sk[tid] = fk * rk; su[tid] = 0.f; }
         const float a = proj[(size_t)t * proj_stride + a_col0 + h] + dt_bias[h];
         const float sp = a > 20.f ? a : log1pf(expf(a));
         const float g = expf(-expf(a_log[h]) * sp);
         __syncthreads();
-        float4 ak = make_float4(0.f, 0.f, 0.f, 0.f), aq = ak;
+        float q2 = 0.f, k2 = 0.f, x2 = 0.f;                // (every warp forms them for itself)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const float fq = sq[lane + 32 * y], fk = sk[lane + 32 * y];
+            q2 = fmaf(fq, fq, q2); k2 = fmaf(fk, fk, k2); x2 = fmaf(fk, fq, x2);
+        }
+        q2 = rv_warp_sum(q2); k2 = rv_warp_sum(k2); x2 = rv_warp_sum(x2);
+        const float rq = 1.0f / sqrtf((float)d) / sqrtf(q2 + unit_eps), rk = 1.0f / sqrtf(k2 + unit_eps);
+        float4 ak[2], aq[2];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float k = sk[n0 + i], q = sq[n0 + i];
-            ak.x = fmaf(S[i].x, k, ak.x); ak.y = fmaf(S[i].y, k, ak.y); ak.z = fmaf(S[i].z, k, ak.z); ak.w = fmaf(S[i].w, k, ak.w);
-            aq.x = fmaf(S[i].x, q, aq.x); aq.y = fmaf(S[i].y, q, aq.y); aq.z = fmaf(S[i].z, q, aq.z); aq.w = fmaf(S[i].w, q, aq.w);
+            const float k = sk[n0 + i] * rk, q = sq[n0 + i] * rq;
+            float4& k4 = ak[i >> 3];
+            float4& q4 = aq[i >> 3];
+            if ((i & 7) == 0) {
+                k4 = make_float4(S[i].x * k, S[i].y * k, S[i].z * k, S[i].w * k);
+                q4 = make_float4(S[i].x * q, S[i].y * q, S[i].z * q, S[i].w * q);
+            } else {
+                k4.x = fmaf(S[i].x, k, k4.x); k4.y = fmaf(S[i].y, k, k4.y); k4.z = fmaf(S[i].z, k, k4.z); k4.w = fmaf(S[i].w, k, k4.w);
+                q4.x = fmaf(S[i].x, q, q4.x); q4.y = fmaf(S[i].y, q, q4.y); q4.z = fmaf(S[i].z, q, q4.z); q4.w = fmaf(S[i].w, q, q4.w);
+            }
         }
-        *reinterpret_cast<float4*>(&pk[warp][cl]) = ak;
-        *reinterpret_cast<float4*>(&pq[warp][cl]) = aq;
+        *reinterpret_cast<float4*>(&pk[warp][cl]) = make_float4(ak[0].x + ak[1].x, ak[0].y + ak[1].y, ak[0].z + ak[1].z, ak[0].w + ak[1].w);
+        *reinterpret_cast<float4*>(&pq[warp][cl]) = make_float4(aq[0].x + aq[1].x, aq[0].y + aq[1].y, aq[0].z + aq[1].z, aq[0].w + aq[1].w);
         __syncthreads();
         if (tid < 128 && blockIdx.x * 128 + tid < vd) {
             const int c = blockIdx.x * 128 + tid;
-            float kv = 0.f, qv = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) { kv += pk[w][tid]; qv += pq[w][tid]; }
+            const float kv = ((pk[0][tid] + pk[1][tid]) + (pk[2][tid] + pk[3][tid])) + ((pk[4][tid] + pk[5][tid]) + (pk[6][tid] + pk[7][tid]));
+            const float qv = ((pq[0][tid] + pq[1][tid]) + (pq[2][tid] + pq[3][tid])) + ((pq[4][tid] + pq[5][tid]) + (pq[6][tid] + pq[7][tid]));
             const float beta = 1.0f / (1.0f + expf(-proj[(size_t)t * proj_stride + b_col0 + h]));
-            const float u = beta * (rv_load_any(qkv, qkv_dtype, row + 2 * qk + (size_t)h * vd + c) - g * kv);
-            const float kq = (sums[2][0] + sums[2][1] + sums[2][2] + sums[2][3]) * rq * rk;
+            const float u = beta * fmaf(-g, kv, rv_load_any(qkv, qkv_dtype, row + 2 * qk + (size_t)h * vd + c));
             su[tid] = u;
-            out[((size_t)t * heads + h) * vd + c] = fmaf(g, qv, kq * u);
+            out[((size_t)t * heads + h) * vd + c] = fmaf(g, qv, x2 * rq * rk * u);
         }
         __syncthreads();
         const float4 u = *reinterpret_cast<const float4*>(&su[cl]);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float k = sk[n0 + i];
+            const float k = sk[n0 + i] * rk;
             S[i].x = fmaf(g, S[i].x, k * u.x); S[i].y = fmaf(g, S[i].y, k * u.y);
             S[i].z = fmaf(g, S[i].z, k * u.z); S[i].w = fmaf(g, S[i].w, k * u.w);
         }
-        __syncthreads();                                   // sums, sk and su are written again for the next token
+        __syncthreads();                                   // the rows of q and k and su are written again for the next token
     }
     if (live && end > start) {
 #pragma unroll
@@ -1466,41 +1475,49 @@ delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
 template <int PARTS>
 static int launch_delta_walk(cudaStream_t stream, int n_seqs, int heads, int vd, const void* qkv, int qkv_dtype, int qkv_stride, const float* proj,
                              int proj_stride, int b_col0, int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens,
-                             const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps) {
+                             const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps, int least) {
     constexpr int smem = 2 * (int)sizeof(DeltaStage<PARTS>), cols = DeltaStage<PARTS>::COLS;
     static RvPerDevice once;
     if (int st = rv_configure_smem(once, delta_rule_walk_kernel<PARTS>, smem)) return st;
     return rv_launch(delta_rule_walk_kernel<PARTS>, dim3((vd + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, qkv, qkv_dtype,
                      qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, state_stride, out, heads,
-                     qk_heads, d, vd, unit_eps);
+                     qk_heads, d, vd, unit_eps, least);
+}
+
+// Whether rows of the state are whole words of four columns.
+RV_EXPORT int rv_delta_rule_words(int vd, const float* state, long long state_stride) {
+    return vd % 4 == 0 && state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
 }
 
 // qkv rows: [q: qk_heads x d | k: qk_heads x d | v: heads x vd] (after the convolution); the logits of beta and of the
-// decay are float columns b_col0 .. and a_col0 .. of `proj`; out: float [n_tokens, heads x vd].
+// decay are float columns b_col0 .. and a_col0 .. of `proj`; out: float [tokens, heads x vd].  For keys of 33 to 128 elements and
+// values and states of whole words of four columns, `which` names the kernel: 1 the one for single tokens, 2 the walk, 3 the first
+// for sequences of up to `short_tokens` tokens and the second for the others (all give the same bits).
 RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, const float* proj, int proj_stride, int b_col0,
                             int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens, const int* state_slots,
                             float* state, long long state_stride, float* out, int n_seqs, int heads, int qk_heads, int d, int vd,
-                            float unit_eps, int n_tokens, cudaStream_t stream) {
+                            float unit_eps, int which, int short_tokens, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || qk_heads <= 0 || heads % qk_heads || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 ||
-        heads > 65535)
+        heads > 65535 || which < 1 || which > 3)
         return RV_ERR_BAD_SIZE;
-    if (qkv_stride < 2 * qk_heads * d + heads * vd || b_col0 < 0 || a_col0 < 0 || b_col0 + heads > proj_stride ||
-        a_col0 + heads > proj_stride || state_stride < (long long)heads * d * vd)
+    const int qk = qk_heads * d;
+    if (qkv_stride < 2 * qk + heads * vd || b_col0 < 0 || a_col0 < 0 || b_col0 + heads > proj_stride || a_col0 + heads > proj_stride ||
+        state_stride < (long long)heads * d * vd)
         return RV_ERR_BAD_SIZE;
     if (qkv_dtype & ~1) return RV_ERR_BAD_DTYPE;
     if (n_seqs == 0) return RV_OK;
-    const bool words = vd % 4 == 0 && state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;      // whole words of four columns
-    if (words && d <= 128 && n_tokens <= 2LL * n_seqs) {
-        RV_LAUNCH_ST = rv_launch(delta_rule_step_kernel, dim3((vd + 127) / 128, heads, n_seqs), dim3(256), 0, stream, qkv, qkv_dtype, qkv_stride, proj,
-                                 proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, (size_t)state_stride, out, heads,
-                                 qk_heads, d, vd, unit_eps);
-        return rv_launch_status();
-    }
-    if (words && d > 32 && d <= 128) {
+    if (d > 32 && d <= 128 && rv_delta_rule_words(vd, state, state_stride)) {
+        const bool one = (long long)((vd + 127) / 128) * heads * n_seqs <= rv_sm_count();
+        if (which & 1)
+            RV_LAUNCH_ST = rv_launch(one ? delta_rule_step_kernel<1> : delta_rule_step_kernel<2>, dim3((vd + 127) / 128, heads, n_seqs), dim3(256), 0, stream, qkv, qkv_dtype, qkv_stride, proj,
+                                     proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, (size_t)state_stride, out, heads,
+                                     qk_heads, d, vd, unit_eps, which == 1 ? 0x7fffffff : short_tokens);
+        if (which == 1 || ((which & 1) && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
+        const int least = which == 2 ? 0 : short_tokens + 1;
         RV_LAUNCH_ST = d > 64 ? launch_delta_walk<16>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps)
+                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least)
                               : launch_delta_walk<8>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps);
+                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least);
         return rv_launch_status();
     }
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128

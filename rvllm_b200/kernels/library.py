@@ -1028,6 +1028,19 @@ class CudaKernels:
         each, else perhaps all.  It picks among kernels that give the same bits."""
         return max_q_len if max_q_len is not None else (1 if T <= n_seqs else T)
 
+    SHORT_PORTIONS_BESIDE = 5          # more sequences than this in a step of uneven portions: the short ones get a kernel of their own
+
+    def _portion_kernels(self, T: int, n_seqs: int, max_q_len: Optional[int], short: int) -> int:
+        """Which of two kernels a recurrence's step takes, one for portions of up to `short` tokens, one for longer ones: 1 the first
+        alone, 2 the second alone, 3 both, each sequence by its own tokens.  The second serves short portions too, only slower;
+        so the first runs beside it where the sequences are many and those behind the longest bring few tokens on average (delta
+        rule, single tokens beside a portion of 64 or 1,500: 3 of them 35.2 and 557 us in two kernels, 34.2 and 542 in one; 6: 37.7
+        and 560, 42.4 and 564; 48: 82 and 605, 136 and 657)."""
+        longest = self._longest(T, n_seqs, max_q_len)
+        if longest <= short:
+            return 1
+        return 3 if n_seqs > self.SHORT_PORTIONS_BESIDE and T - longest < (n_seqs - 1) * max(16, short + 1) else 2
+
     def causal_conv_silu(self, proj, col0: int, channels: int, weight, bias, token_seq, cu_seqlens, state_slots, state,
                          conv_off: int, out_dtype, max_q_len: Optional[int] = None) -> torch.Tensor:
         """silu(causal convolution per channel) of columns col0 .. col0 + channels of `proj`, continued from and
@@ -1271,11 +1284,14 @@ class CudaKernels:
         _check("selective_scan", st)
         return out
 
+    DELTA_SHORT_TOKENS = 4             # tokens of a portion up to which the delta rule takes the kernel of single tokens (ssm.cu has both sides)
+
     def delta_rule(self, qkv, proj, b_col0: int, a_col0: int, a_log, dt_bias, cu_seqlens, state_slots, state, heads: int,
-                   qk_heads: int, head_dim: int, value_dim: int, unit_eps: float) -> torch.Tensor:
+                   qk_heads: int, head_dim: int, value_dim: int, unit_eps: float, max_q_len: Optional[int] = None) -> torch.Tensor:
         """The gated delta rule over the step's tokens, continued from and leaving behind each request's S ([heads][head_dim]
         [value_dim] at offset 0 of its row of `state`).  qkv rows: [q | k | v] after their convolution; the logits of beta and
-        of the decay are float columns b_col0 .. and a_col0 .. of `proj`.  Returns o float32 [T, heads * value_dim]."""
+        of the decay are float columns b_col0 .. and a_col0 .. of `proj`.  Returns o float32 [T, heads * value_dim].
+        `max_q_len`: the most tokens that any sequence brings (see `_longest`); the bits do not depend on it."""
         _need(qkv, "qkv", dims=2); _need(proj, "proj", torch.float32, 2); _need(state, "state", torch.float32, 2)
         _need(a_log, "a_log", torch.float32, 1); _need(dt_bias, "dt_bias", torch.float32, 1)
         T = qkv.shape[0]
@@ -1283,12 +1299,15 @@ class CudaKernels:
                 dt_bias.shape[0] != heads:
             raise KernelError("delta_rule: shapes of q | k | v, the logits and the heads' constants do not agree")
         out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=qkv.device)
+        which = self._portion_kernels(T, state_slots.shape[0], max_q_len, self.DELTA_SHORT_TOKENS)
         st = self._lib("ssm.cu").rv_delta_rule(
             _ptr(qkv), c_int(self._dt(qkv, "qkv")), c_int(qkv.shape[1]), _ptr(proj), c_int(proj.shape[1]), c_int(b_col0), c_int(a_col0),
             _ptr(a_log), _ptr(dt_bias), _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out),
             c_int(state_slots.shape[0]), c_int(heads), c_int(qk_heads), c_int(head_dim), c_int(value_dim), c_float(unit_eps),
-            c_int(T), self._stream())
+            c_int(which), c_int(self.DELTA_SHORT_TOKENS), self._stream())
         _check("delta_rule", st)
+        if which == 3 and 32 < head_dim <= 128:
+            COUNTERS['launches'] += self._lib("ssm.cu").rv_delta_rule_words(c_int(value_dim), _ptr(state), ctypes.c_longlong(state.shape[1]))
         return out
 
     # ------------------------------------------------------------------ attention whose weights are mixed across the heads

@@ -67,7 +67,7 @@ class GatedDeltaRule(Part):
         gate_col = self.channels
         o = k.delta_rule(qkv, proj, gate_col + self.v_dim, gate_col + self.v_dim + self.heads, self.a_log, self.dt_bias,
                          ctx.cu_seqlens, ctx.state_slots, cache.state, self.heads, self.qk_heads, self.head_dim, self.value_dim,
-                         self.unit_eps)
+                         self.unit_eps, max_q_len=max(ctx.q_lens))
         o = k.head_norm_gate(o, self.norm, self.eps, proj, gate_col, self.heads, self.value_dim, x.dtype)
         return self.out(o, ctx, residual=residual, out_dtype=out_dtype)
 

@@ -644,7 +644,7 @@ class EmulatedKernels:
         return out.view(T, num_heads * value_dim).to(q.dtype)
 
     def delta_rule(self, qkv, proj, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, heads, qk_heads, head_dim,
-                   value_dim, unit_eps):
+                   value_dim, unit_eps, max_q_len=None):
         T = qkv.shape[0]
         qk = qk_heads * head_dim
         x = qkv.float()

@@ -311,9 +311,41 @@ def test_delta_rule_of_portions_and_of_single_tokens(K, d, vd, heads, qk, lens):
             S[s] = S[s] + k[t][:, :, None] * un[:, None, :]
             want[t] = torch.einsum("hdv,hd->hv", S[s], q[t])
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
-    got = K.delta_rule(qkv, proj, 1, 1 + heads, a_log, bias, i32(cu), i32(list(range(len(lens)))), state, heads, qk, d, vd, 1e-6)
+    got = K.delta_rule(qkv, proj, 1, 1 + heads, a_log, bias, i32(cu), i32(list(range(len(lens)))), state, heads, qk, d, vd, 1e-6, max_q_len=max(lens))
     # float sums of d products along a chain of at most 70 tokens
     assert rel_err(got, want.view(T, -1)) < 3e-6 and rel_err(state[:, :heads * d * vd], S.view(len(lens), -1)) < 3e-6
+
+
+@pytest.mark.parametrize("d,vd,heads,qk,lens", [(128, 128, 4, 2, (1, 40, 1, 2)), (100, 36, 2, 1, (2, 1, 3)), (64, 68, 2, 2, (1,) * 20 + (17,)), (40, 4, 2, 1, (19, 2)),
+                                                (24, 8, 2, 2, (1, 5, 2)), (160, 8, 2, 1, (1, 9))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_delta_rule_bits_do_not_depend_on_the_step(K, d, vd, heads, qk, lens, dtype):
+    """A request's outputs and state are the same bits alone, beside others and with its portion cut in two, whichever kernels the
+    steps take; a padding row (slot -1) leaves no state."""
+    torch.manual_seed(d + vd)
+    T = sum(lens)
+    qkv, proj = torch.randn(T, 2 * qk * d + heads * vd, device="cuda").to(dtype), torch.randn(T, 2 * heads, device="cuda")
+    a_log, bias = torch.randn(heads, device="cuda"), torch.randn(heads, device="cuda")
+    before = torch.randn(len(lens), heads * d * vd, device="cuda")
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    slots = list(range(len(lens)))
+    slots[len(lens) // 2] = -1
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+
+    def run(a, b, cu, slots, state, longest):
+        o = K.delta_rule(qkv[a:b].contiguous(), proj[a:b].contiguous(), 0, heads, a_log, bias, i32(cu), i32(slots), state, heads, qk, d, vd, 1e-6, max_q_len=longest)
+        return [o[cu[i]:cu[i + 1]] for i in range(len(slots)) if slots[i] >= 0], state
+    whole, state = run(0, T, cu, slots, before.clone(), max(lens))
+    for longest in (2, T, None):                            # the kernel of single tokens for all, the walk for all or beside it
+        o, s = run(0, T, cu, slots, before.clone(), longest)
+        assert all(map(torch.equal, o, whole)) and torch.equal(s, state)
+    assert torch.equal(state[len(lens) // 2], before[len(lens) // 2])
+    for i, o in zip([i for i in range(len(lens)) if slots[i] >= 0], whole):
+        s = before.clone()
+        for a, b in ((cu[i], cu[i] + 1), (cu[i] + 1, cu[i + 1])):
+            if b > a:
+                assert torch.equal(run(a, b, [0, b - a], [i], s, b - a)[0][0], o[a - cu[i]:b - cu[i]])
+        assert torch.equal(s[i], state[i])
 
 
 def test_talking_attention_on_eight_and_sixteen_warps(K):
