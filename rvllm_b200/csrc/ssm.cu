@@ -617,7 +617,7 @@ selective_scan1_kernel(const void* __restrict__ u, int u_dtype, const float* __r
                        const float* __restrict__ A, const float* __restrict__ bc, int bc_stride, int b_col0, int c_col0,
                        const float* __restrict__ d_skip, const void* __restrict__ z, int z_dtype, int z_stride, int z_col0,
                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                       size_t state_stride, void* __restrict__ out, int out_dtype, int inner, int N, int parts) {
+                       size_t state_stride, void* __restrict__ out, int out_dtype, int inner, int N, int parts, int most) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     extern __shared__ float sBC[];                     // [SCAN1_CHUNK][2 N]
@@ -625,6 +625,7 @@ selective_scan1_kernel(const void* __restrict__ u, int u_dtype, const float* __r
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok > most) return;                          // (the other kernel's)
     const int per_block = blockDim.x / parts;
     float* sDt = sBC + SCAN1_CHUNK * 2 * N;            // [SCAN1_CHUNK][per_block]
     float* sU = sDt + SCAN1_CHUNK * per_block;         // [SCAN1_CHUNK][per_block]
@@ -800,7 +801,7 @@ selective_scan1_vec_kernel(const void* __restrict__ u, int u_dtype, const float*
                            const float* __restrict__ A, const float* __restrict__ bc, int bc_stride, int b_col0, int c_col0,
                            const float* __restrict__ d_skip, const void* __restrict__ z, int z_dtype, int z_stride, int z_col0,
                            const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                           size_t state_stride, void* __restrict__ out, int out_dtype, int inner) {
+                           size_t state_stride, void* __restrict__ out, int out_dtype, int inner, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     constexpr int N = 4 * PARTS, BLK = 128 / PARTS;        // states and channels of a block
@@ -812,6 +813,7 @@ selective_scan1_vec_kernel(const void* __restrict__ u, int u_dtype, const float*
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok < least) return;                             // (the other kernel's)
     const int chunks = (n_tok + SCAN1_CHUNK - 1) / SCAN1_CHUNK;
     const int c_first = blockIdx.x * BLK;
     if (threadIdx.x < 128) {                               // ---- the walk
@@ -947,24 +949,20 @@ selective_scan1_vec_kernel(const void* __restrict__ u, int u_dtype, const float*
     if (chunks > 0) write(chunks - 1, us_out, zs_out);
 }
 
+// `which` names the kernel for rows of 16 or 32 states: 1 the one with one role, 2 the one with two, 3 the first for sequences of up to
+// `short_tokens` tokens and the second for the others (both add in the same order: the same bits).  64 sequences of 1, 4, 8 and
+// 12 tokens on 8,192 channels: 53, 76, 132 and 202 us with one role, 90, 121, 140 and 158 with two.
 RV_EXPORT int rv_selective_scan1(const void* u, int u_dtype, const float* dt_raw, const float* dt_bias, const float* A,
                                  const float* bc, int bc_stride, int b_col0, int c_col0, const float* d_skip, const void* z,
                                  int z_dtype, int z_stride, int z_col0, const int* cu_seqlens, const int* state_slots, float* state,
-                                 long long state_stride, void* out, int out_dtype, int n_tokens, int n_seqs, int inner, int N, cudaStream_t stream) {
-    if (n_seqs < 0 || inner <= 0 || N <= 0 || N > 32 * 16 || n_seqs > 65535) return RV_ERR_BAD_SIZE;
+                                 long long state_stride, void* out, int out_dtype, int n_seqs, int inner, int N, int which, int short_tokens, cudaStream_t stream) {
+    if (n_seqs < 0 || inner <= 0 || N <= 0 || N > 32 * 16 || n_seqs > 65535 || which < 1 || which > 3) return RV_ERR_BAD_SIZE;
     if (b_col0 < 0 || c_col0 < 0 || b_col0 + N > bc_stride || c_col0 + N > bc_stride || z_col0 < 0 || z_col0 + inner > z_stride ||
         state_stride < (long long)inner * N)
         return RV_ERR_BAD_SIZE;
     if ((u_dtype | z_dtype | out_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (n_seqs == 0) return RV_OK;
-    // (a decode step's single tokens are left to the kernel with one role: 64 of them on 8,192 channels 52 us against 90)
-    if ((N == 16 || N == 32) && n_tokens > 4LL * n_seqs) {
-        const int blk = 128 / (N / 4);
-        RV_LAUNCH_ST = rv_launch(N == 16 ? selective_scan1_vec_kernel<4> : selective_scan1_vec_kernel<8>, dim3((inner + blk - 1) / blk, n_seqs), dim3(256), 0,
-                                 stream, u, u_dtype, dt_raw, dt_bias, A, bc, bc_stride, b_col0, c_col0, d_skip, z, z_dtype, z_stride, z_col0, cu_seqlens,
-                                 state_slots, state, (size_t)state_stride, out, out_dtype, inner);
-        return rv_launch_status();
-    }
+    const bool two_roles = N == 16 || N == 32;
     // four states per lane where a warp's lanes can hold a channel's row so (neighbouring lanes then read neighbouring
     // 16 bytes of the state, and four times as many threads walk the tokens); sixteen per lane for longer rows
     const int ns = N <= 32 * 4 ? 4 : 16;
@@ -976,9 +974,14 @@ RV_EXPORT int rv_selective_scan1(const void* u, int u_dtype, const float* dt_raw
     const bool pre = per_block <= 8 * SCAN1_PRE && 2 * N <= 8 * SCAN1_PRE_BC;
     auto kernel = ns == 4 ? (pre ? selective_scan1_kernel<4, true> : selective_scan1_kernel<4, false>)
                           : (pre ? selective_scan1_kernel<16, true> : selective_scan1_kernel<16, false>);
-    RV_LAUNCH_ST = rv_launch(kernel, dim3((inner + per_block - 1) / per_block, n_seqs), dim3(128), smem, stream, u, u_dtype, dt_raw,
-                             dt_bias, A, bc, bc_stride, b_col0, c_col0, d_skip, z, z_dtype, z_stride, z_col0, cu_seqlens, state_slots,
-                             state, (size_t)state_stride, out, out_dtype, inner, N, parts);
+    if (!two_roles || (which & 1))
+        RV_LAUNCH_ST = rv_launch(kernel, dim3((inner + per_block - 1) / per_block, n_seqs), dim3(128), smem, stream, u, u_dtype, dt_raw,
+                                 dt_bias, A, bc, bc_stride, b_col0, c_col0, d_skip, z, z_dtype, z_stride, z_col0, cu_seqlens, state_slots,
+                                 state, (size_t)state_stride, out, out_dtype, inner, N, parts, two_roles && which == 3 ? short_tokens : 0x7fffffff);
+    if (!two_roles || which == 1 || (which == 3 && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
+    RV_LAUNCH_ST = rv_launch(N == 16 ? selective_scan1_vec_kernel<4> : selective_scan1_vec_kernel<8>, dim3((inner + per_block - 1) / per_block, n_seqs), dim3(256), 0,
+                             stream, u, u_dtype, dt_raw, dt_bias, A, bc, bc_stride, b_col0, c_col0, d_skip, z, z_dtype, z_stride, z_col0, cu_seqlens,
+                             state_slots, state, (size_t)state_stride, out, out_dtype, inner, which == 2 ? 0 : short_tokens + 1);
     return rv_launch_status();
 }
 

@@ -1028,18 +1028,14 @@ class CudaKernels:
         each, else perhaps all.  It picks among kernels that give the same bits."""
         return max_q_len if max_q_len is not None else (1 if T <= n_seqs else T)
 
-    SHORT_PORTIONS_BESIDE = 5          # more sequences than this in a step of uneven portions: the short ones get a kernel of their own
-
-    def _portion_kernels(self, T: int, n_seqs: int, max_q_len: Optional[int], short: int) -> int:
+    def _portion_kernels(self, T: int, n_seqs: int, max_q_len: Optional[int], short: int, beside: int) -> int:
         """Which of two kernels a recurrence's step takes, one for portions of up to `short` tokens, one for longer ones: 1 the first
         alone, 2 the second alone, 3 both, each sequence by its own tokens.  The second serves short portions too, only slower;
-        so the first runs beside it where the sequences are many and those behind the longest bring few tokens on average (delta
-        rule, single tokens beside a portion of 64 or 1,500: 3 of them 35.2 and 557 us in two kernels, 34.2 and 542 in one; 6: 37.7
-        and 560, 42.4 and 564; 48: 82 and 605, 136 and 657)."""
+        so the first runs beside it where the sequences are more than `beside` and those behind the longest short on average."""
         longest = self._longest(T, n_seqs, max_q_len)
         if longest <= short:
             return 1
-        return 3 if n_seqs > self.SHORT_PORTIONS_BESIDE and T - longest < (n_seqs - 1) * max(16, short + 1) else 2
+        return 3 if n_seqs > beside and T - longest <= (n_seqs - 1) * max(8, short) else 2
 
     def causal_conv_silu(self, proj, col0: int, channels: int, weight, bias, token_seq, cu_seqlens, state_slots, state,
                          conv_off: int, out_dtype, max_q_len: Optional[int] = None) -> torch.Tensor:
@@ -1260,11 +1256,16 @@ class CudaKernels:
         return out
 
     # ------------------------------------------------------------------ recurrences with one state row per channel / per head
+    SCAN1_SHORT_TOKENS = 8             # tokens of a portion up to which the per-channel scan takes the kernel with one role
+    SCAN1_SHORT_BESIDE = 24            # ... beside the other one in uneven steps of more sequences than this (single tokens beside a
+                                       # portion of 64: 24 of them 55 us either way, 63 of them 100 us in one kernel, 86 in two)
+
     def selective_scan(self, u, dt_raw, dt_bias, a, bc, b_col0: int, c_col0: int, d_skip, z, z_col0: int, cu_seqlens, state_slots,
-                       state, out_dtype) -> torch.Tensor:
+                       state, out_dtype, max_q_len: Optional[int] = None) -> torch.Tensor:
         """S[c, n] <- exp(dt_c a[c, n]) S[c, n] + dt_c u_c B_n; y_c = sum_n S[c, n] C_n + D_c u_c; returns y * silu(z) in
         `out_dtype`.  dt = softplus(dt_raw + dt_bias) per channel; B and C are float columns b_col0 .. and c_col0 .. of `bc`,
-        z columns z_col0 .. of `z`; S lives as [inner][N] at offset 0 of the request's row of `state`."""
+        z columns z_col0 .. of `z`; S lives as [inner][N] at offset 0 of the request's row of `state`.  `max_q_len`: the most tokens
+        that any sequence brings (see `_longest`); the bits do not depend on it."""
         _need(u, "u", dims=2); _need(dt_raw, "dt_raw", torch.float32, 2); _need(bc, "bc", torch.float32, 2); _need(z, "z", dims=2)
         _need(a, "a", torch.float32, 2); _need(state, "state", torch.float32, 2)
         T, inner = u.shape
@@ -1276,15 +1277,20 @@ class CudaKernels:
         if a.shape[0] != inner or dt_raw.shape != (T, inner) or bc.shape[0] != T or z.shape[0] != T:
             raise KernelError("selective_scan: shapes of u, dt, a, B | C and z do not agree")
         out = torch.empty((T, inner), dtype=out_dtype, device=u.device)
+        which = self._portion_kernels(T, state_slots.shape[0], max_q_len, self.SCAN1_SHORT_TOKENS, self.SCAN1_SHORT_BESIDE)
         st = self._lib("ssm.cu").rv_selective_scan1(
             _ptr(u), c_int(self._dt(u, "u")), _ptr(dt_raw), _ptr(dt_bias), _ptr(a), _ptr(bc), c_int(bc.shape[1]), c_int(b_col0),
             c_int(c_col0), _ptr(d_skip), _ptr(z), c_int(self._dt(z, "z")), c_int(z.shape[1]), c_int(z_col0), _ptr(cu_seqlens),
             _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out), c_int(_DT[out_dtype]),
-            c_int(T), c_int(state_slots.shape[0]), c_int(inner), c_int(N), self._stream())
+            c_int(state_slots.shape[0]), c_int(inner), c_int(N), c_int(which), c_int(self.SCAN1_SHORT_TOKENS), self._stream())
         _check("selective_scan", st)
+        COUNTERS['launches'] += 1 if which == 3 and N in (16, 32) else 0
         return out
 
     DELTA_SHORT_TOKENS = 4             # tokens of a portion up to which the delta rule takes the kernel of single tokens (ssm.cu has both sides)
+    DELTA_SHORT_BESIDE = 5             # ... beside the walk in uneven steps of more sequences than this (single tokens beside a portion of
+                                       # 64 or 1,500: 3 of them 35.2 and 557 us in two kernels, 34.2 and 542 in one; 6 37.7 and 560, 42.4
+                                       # and 564; 48 82 and 605, 136 and 657)
 
     def delta_rule(self, qkv, proj, b_col0: int, a_col0: int, a_log, dt_bias, cu_seqlens, state_slots, state, heads: int,
                    qk_heads: int, head_dim: int, value_dim: int, unit_eps: float, max_q_len: Optional[int] = None) -> torch.Tensor:
@@ -1299,7 +1305,7 @@ class CudaKernels:
                 dt_bias.shape[0] != heads:
             raise KernelError("delta_rule: shapes of q | k | v, the logits and the heads' constants do not agree")
         out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=qkv.device)
-        which = self._portion_kernels(T, state_slots.shape[0], max_q_len, self.DELTA_SHORT_TOKENS)
+        which = self._portion_kernels(T, state_slots.shape[0], max_q_len, self.DELTA_SHORT_TOKENS, self.DELTA_SHORT_BESIDE)
         st = self._lib("ssm.cu").rv_delta_rule(
             _ptr(qkv), c_int(self._dt(qkv, "qkv")), c_int(qkv.shape[1]), _ptr(proj), c_int(proj.shape[1]), c_int(b_col0), c_int(a_col0),
             _ptr(a_log), _ptr(dt_bias), _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out),

@@ -64,7 +64,7 @@ class Mamba1Mixer(Part):
         d = k.column_slice(dbc, 0, self.dt_rank, x.dtype)
         dt_raw = self.dt_proj(d, ctx, out_dtype=torch.float32)
         y = k.selective_scan(u, dt_raw, self.dt_bias, self.a, dbc, self.dt_rank, self.dt_rank + self.state, self.d_skip,
-                             proj, self.inner, ctx.cu_seqlens, ctx.state_slots, cache.state, x.dtype)
+                             proj, self.inner, ctx.cu_seqlens, ctx.state_slots, cache.state, x.dtype, max_q_len=max(ctx.q_lens))
         return self.out(y, ctx, residual=residual, out_dtype=out_dtype)
 
 

@@ -562,7 +562,7 @@ class EmulatedKernels:
         a.mul_(sa).add_(b.float() * sb)
         return a
 
-    def selective_scan(self, u, dt_raw, dt_bias, a, bc, b_col0, c_col0, d_skip, z, z_col0, cu_seqlens, state_slots, state, out_dtype):
+    def selective_scan(self, u, dt_raw, dt_bias, a, bc, b_col0, c_col0, d_skip, z, z_col0, cu_seqlens, state_slots, state, out_dtype, max_q_len=None):
         T, inner = u.shape
         N = a.shape[1]
         uf = u.float()

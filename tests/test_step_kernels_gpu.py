@@ -228,8 +228,41 @@ def test_selective_scan_in_two_roles(K, inner, N, lens):
             want[t] = (S[s] * b64[t, 3 + N:]).sum(1) + D.double().cpu() * u64[t]
     want *= torch.nn.functional.silu(z[:, 4:].double().cpu())
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
-    got = K.selective_scan(u, raw, bias, A.contiguous(), bc, 3, 3 + N, D, z, 4, i32(cu), i32(list(range(len(lens)))), state, torch.float32)
+    got = K.selective_scan(u, raw, bias, A.contiguous(), bc, 3, 3 + N, D, z, 4, i32(cu), i32(list(range(len(lens)))), state, torch.float32, max_q_len=max(lens))
     assert rel_err(got, want) < 2e-6 and rel_err(state[:, :inner * N], S.view(len(lens), -1)) < 2e-6
+
+
+@pytest.mark.parametrize("inner,N,lens", [(70, 16, (1, 5, 16, 17, 35)), (33, 32, (18, 2, 1, 1, 1, 1)), (40, 8, (1, 9)), (32, 16, (1,) * 20 + (40,))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_selective_scan_bits_do_not_depend_on_the_step(K, inner, N, lens, dtype):
+    """A request's outputs and state are the same bits alone, beside others and with its portion cut in two, whichever kernels the
+    steps take; a padding row (slot -1) leaves no state."""
+    torch.manual_seed(inner + N)
+    T = sum(lens)
+    u, z = torch.randn(T, inner, device="cuda").to(dtype), torch.randn(T, inner, device="cuda").to(dtype)
+    raw, bias, A = torch.randn(T, inner, device="cuda"), torch.randn(inner, device="cuda"), (-torch.rand(inner, N, device="cuda") * 4).contiguous()
+    bc, D = torch.randn(T, 2 * N, device="cuda"), torch.randn(inner, device="cuda")
+    before = torch.randn(len(lens), inner * N, device="cuda")
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    slots = list(range(len(lens)))
+    slots[1] = -1
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+
+    def run(a, b, cu, slots, state, longest):
+        y = K.selective_scan(u[a:b].contiguous(), raw[a:b].contiguous(), bias, A, bc[a:b].contiguous(), 0, N, D, z[a:b].contiguous(), 0, i32(cu), i32(slots),
+                             state, torch.float32, max_q_len=longest)
+        return [y[cu[i]:cu[i + 1]] for i in range(len(slots)) if slots[i] >= 0], state
+    whole, state = run(0, T, cu, slots, before.clone(), max(lens))
+    for longest in (1, T, None):
+        y, s = run(0, T, cu, slots, before.clone(), longest)
+        assert all(map(torch.equal, y, whole)) and torch.equal(s, state)
+    assert torch.equal(state[1], before[1])
+    for i, y in zip([i for i in range(len(lens)) if slots[i] >= 0], whole):
+        s = before.clone()
+        for a, b in ((cu[i], cu[i] + 1), (cu[i] + 1, cu[i + 1])):
+            if b > a:
+                assert torch.equal(run(a, b, [0, b - a], [i], s, b - a)[0][0], y[a - cu[i]:b - cu[i]])
+        assert torch.equal(s[i], state[i])
 
 
 @pytest.mark.parametrize("taps,lens", [(4, (1, 1, 1)), (3, (2, 1)), (1, (1,)), (2, (1, 1)), (4, (2,))])
