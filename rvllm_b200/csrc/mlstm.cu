@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(128)
 mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_col0, const float* __restrict__ i_bias,
                   const float* __restrict__ f_bias, const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots,
                   float* __restrict__ state, size_t state_stride, float* __restrict__ raw, float* __restrict__ top, int heads, int d,
-                  int vd, int parts, float cap) {
+                  int vd, int parts, float cap, int most) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     extern __shared__ __align__(16) float ml_smem[];
@@ -38,6 +38,7 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok > most) return;                              // (the other kernel's)
     const int row_floats = parts * (NS + 4);
     float* sQ = ml_smem;                                   // [ML_CHUNK][row_floats]
     float* sK = sQ + ML_CHUNK * row_floats;
@@ -173,16 +174,25 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
             const float4* Q4 = reinterpret_cast<const float4*>(sQ + tt * row_floats + part * (NS + 4));
             const float a = sA[tt];
             const float bu = sB[tt] * sV[tt * per_block + colb];
-            float ov4[4] = {0.f, 0.f, 0.f, 0.f};                // four sums side by side: a quarter of the chain
+            // chains of eight neighbouring entries, then neighbours, then neighbouring pairs ...: the walk's order, the same bits (keys of
+            // up to 32 entries, which it does not serve: four chains of every fourth entry)
+            constexpr int CHAINS = NS == 16 ? 2 : 4;
+            float chain[CHAINS];
+#pragma unroll
+            for (int j = 0; j < CHAINS; ++j) chain[j] = 0.f;
 #pragma unroll
             for (int i = 0; i < NS / 4; ++i) {
                 const float4 k4 = K4[i], q4 = Q4[i];
-                S[4 * i] = fmaf(a, S[4 * i], k4.x * bu);         ov4[0] = fmaf(S[4 * i], q4.x, ov4[0]);
-                S[4 * i + 1] = fmaf(a, S[4 * i + 1], k4.y * bu); ov4[1] = fmaf(S[4 * i + 1], q4.y, ov4[1]);
-                S[4 * i + 2] = fmaf(a, S[4 * i + 2], k4.z * bu); ov4[2] = fmaf(S[4 * i + 2], q4.z, ov4[2]);
-                S[4 * i + 3] = fmaf(a, S[4 * i + 3], k4.w * bu); ov4[3] = fmaf(S[4 * i + 3], q4.w, ov4[3]);
+                const float k[4] = {k4.x, k4.y, k4.z, k4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float& o = chain[NS == 8 ? j % CHAINS : (i >> 1) % CHAINS];
+                    S[4 * i + j] = fmaf(a, S[4 * i + j], k[j] * bu);
+                    o = fmaf(S[4 * i + j], q[j], o);
+                }
             }
-            float ov = (ov4[0] + ov4[1]) + (ov4[2] + ov4[3]);
+            float ov = chain[0] + chain[1];
+            if (CHAINS == 4) ov += chain[2 % CHAINS] + chain[3 % CHAINS];
             for (int o = cpw; o < 32; o <<= 1) ov += __shfl_xor_sync(0xffffffffu, ov, o);
             if (part == 0 && live) raw[trow * heads * width + (size_t)h * width + col] = ov;
         };
@@ -207,7 +217,8 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
 // entries of FOUR neighbouring columns, which PARTS lanes (8 or 16) share: a token costs it four wide reads of q and k, and the
 // four sums of S^T q are met by a reduction that deals them out.  Four warps walk, four others bring the next chunk, form
 // its gates and stage it (double buffers, one barrier a chunk); a warp walks the running maximum through a chunk with the gates
-// in its lanes.  The numbers and their order along the tokens are those of the kernel above.
+// in its lanes.  The numbers and the order of every sum are those of the kernel above, so a request's bits do not depend on which
+// of the two a step takes.
 // 2,048 tokens of 8 heads, 128 x 256: 628 -> 401 us; of 16 heads 755 -> 514; four sequences of 500, 8 heads 198 -> 143.
 template <int PARTS>
 struct MlstmStage {
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(256)
 mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_col0, const float* __restrict__ i_bias,
                   const float* __restrict__ f_bias, const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots,
                   float* __restrict__ state, size_t state_stride, float* __restrict__ raw, float* __restrict__ top, int heads, int d,
-                  int vd, float cap) {
+                  int vd, float cap, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     using Stage = MlstmStage<PARTS>;
@@ -233,6 +244,7 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok < least) return;                             // (the other kernel's)
     const int chunks = (n_tok + ML_CHUNK - 1) / ML_CHUNK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int width = vd + 1;                              // columns of a head's state: the values and the constant 1
@@ -375,34 +387,28 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
 template <int PARTS>
 static int launch_mlstm_walk(cudaStream_t stream, int n_seqs, const float* proj, int stride, int i_col0, int f_col0, const float* i_bias,
                              const float* f_bias, const int* cu_seqlens, const int* state_slots, float* state, size_t state_stride, float* raw,
-                             float* top, int heads, int d, int vd, float cap) {
+                             float* top, int heads, int d, int vd, float cap, int least) {
     constexpr int smem = 2 * (int)sizeof(MlstmStage<PARTS>), cols = MlstmStage<PARTS>::COLS;
     static RvPerDevice once;
     if (int st = rv_configure_smem(once, mlstm_walk_kernel<PARTS>, smem)) return st;
     return rv_launch(mlstm_walk_kernel<PARTS>, dim3((vd + 1 + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, proj, stride, i_col0,
-                     f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, state_stride, raw, top, heads, d, vd, cap);
+                     f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, state_stride, raw, top, heads, d, vd, cap, least);
 }
 
 // proj rows: [q: heads x d | k: heads x d | v: heads x vd | ...]; the raw gate columns at i_col0 .. and f_col0 ..;
-// raw: float [n_tokens, heads x (vd + 1)], top: float [n_tokens, heads].
+// raw: float [tokens, heads x (vd + 1)], top: float [tokens, heads].  For keys of 33 to 128 elements `which` names the kernel: 1 the one
+// with one role, 2 the one with two, 3 the first for sequences of up to `short_tokens` tokens and the second for the others.
 RV_EXPORT int rv_mlstm_scan(const float* proj, int stride, int i_col0, int f_col0, const float* i_bias, const float* f_bias,
                             const int* cu_seqlens, const int* state_slots, float* state, long long state_stride, float* raw, float* top,
-                            int n_tokens, int n_seqs, int heads, int d, int vd, float cap, cudaStream_t stream) {
-    if (n_seqs < 0 || heads <= 0 || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 || heads > 65535 || !(cap > 0.f))
+                            int n_seqs, int heads, int d, int vd, float cap, int which, int short_tokens, cudaStream_t stream) {
+    if (n_seqs < 0 || heads <= 0 || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 || heads > 65535 || !(cap > 0.f) || which < 1 || which > 3)
         return RV_ERR_BAD_SIZE;
     if (stride < 2 * heads * d + heads * vd || i_col0 < 0 || f_col0 < 0 || i_col0 + heads > stride || f_col0 + heads > stride ||
         state_stride < (long long)heads * d * (vd + 1) + heads)
         return RV_ERR_BAD_SIZE;
     if (n_seqs == 0) return RV_OK;
-    // From two chunks a sequence on: 40 tokens take 36.6 us (39.3 in one role), but 17 take 84.7 (81.5; 16 sequences, 16 heads) and 6
-    // take 57.1 (49.1): the second role has nothing to run ahead of.
-    if (d > 32 && d <= 128 && n_tokens >= 2LL * ML_CHUNK * n_seqs) {
-        RV_LAUNCH_ST = d > 64 ? launch_mlstm_walk<16>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
-                                                      (size_t)state_stride, raw, top, heads, d, vd, cap)
-                              : launch_mlstm_walk<8>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
-                                                     (size_t)state_stride, raw, top, heads, d, vd, cap);
-        return rv_launch_status();
-    }
+    const bool two_roles = d > 32 && d <= 128;
+    const int most = two_roles && which == 3 ? short_tokens : 0x7fffffff, least = which == 2 ? 0 : short_tokens + 1;
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128
     int parts = 1;
     while (parts * ns < d) parts <<= 1;                // a power of two of at most 32 lanes of one warp
@@ -413,9 +419,15 @@ RV_EXPORT int rv_mlstm_scan(const float* proj, int stride, int i_col0, int f_col
     auto kernel = ns == 32 ? (pre ? mlstm_scan_kernel<32, true> : mlstm_scan_kernel<32, false>)
                 : ns == 16 ? (pre ? mlstm_scan_kernel<16, true> : mlstm_scan_kernel<16, false>)
                            : (pre ? mlstm_scan_kernel<8, true> : mlstm_scan_kernel<8, false>);
-    RV_LAUNCH_ST = rv_launch(kernel, dim3((vd + 1 + per_block - 1) / per_block, heads, n_seqs), dim3(128), smem, stream, proj, stride,
-                             i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, (size_t)state_stride, raw, top, heads, d,
-                             vd, parts, cap);
+    if (!two_roles || (which & 1))
+        RV_LAUNCH_ST = rv_launch(kernel, dim3((vd + 1 + per_block - 1) / per_block, heads, n_seqs), dim3(128), smem, stream, proj, stride,
+                                 i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, (size_t)state_stride, raw, top, heads, d,
+                                 vd, parts, cap, most);
+    if (!two_roles || which == 1 || (which == 3 && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
+    RV_LAUNCH_ST = d > 64 ? launch_mlstm_walk<16>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
+                                                  (size_t)state_stride, raw, top, heads, d, vd, cap, least)
+                          : launch_mlstm_walk<8>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
+                                                 (size_t)state_stride, raw, top, heads, d, vd, cap, least);
     return rv_launch_status();
 }
 

@@ -2025,23 +2025,33 @@ class CudaKernels:
         _check("bigram_add", st)
         return out
 
+    MLSTM_SHORT_TOKENS = 31            # tokens of a portion up to which the mLSTM scan takes the kernel with one role
+    MLSTM_SHORT_BESIDE = 24            # ... beside the other one in uneven steps of more sequences than this (single tokens beside a portion of
+                                       # 1,500: 24 of them 473 us in two kernels, 476 in one; 48 527 and 539)
+
     def mlstm_scan(self, proj, i_col0: int, f_col0: int, i_bias, f_bias, cu_seqlens, state_slots, state, heads: int, head_dim: int,
-                   value_dim: int, cap: float):
+                   value_dim: int, cap: float, max_q_len: Optional[int] = None):
         """The mLSTM recurrence over the step's tokens, per sequence from the memory its state row holds ([heads][head_dim]
         [value_dim + 1] floats; the last column of a head is the normaliser) and back into it.  proj float32 rows
         [q | k | v | ...] with the raw input- and forget-gate columns at i_col0 and f_col0.  Returns (raw float32
         [T, heads * (value_dim + 1)]: per head the numerators S^T q and, last, n . q; top float32 [T, heads]: the running
-        maximum m_t).  The m of the state row is left as it was: `mlstm_output` stores the new one."""
+        maximum m_t).  The m of the state row is left as it was: `mlstm_output` stores the new one.  `max_q_len`: the most tokens
+        that any sequence brings (see `_longest`); the bits do not depend on it."""
         _need(proj, "proj", torch.float32, 2); _need(state, "state", torch.float32, 2)
         _need(i_bias, "i_bias", torch.float32, 1); _need(f_bias, "f_bias", torch.float32, 1)
         T = proj.shape[0]
         raw = torch.empty((T, heads * (value_dim + 1)), dtype=torch.float32, device=proj.device)
         top = torch.empty((T, heads), dtype=torch.float32, device=proj.device)
+        n_seqs = cu_seqlens.shape[0] - 1
+        which = self._portion_kernels(T, n_seqs, max_q_len, self.MLSTM_SHORT_TOKENS, self.MLSTM_SHORT_BESIDE)
+        if which == 3 and self._longest(T, n_seqs, max_q_len) <= 4 * self.MLSTM_SHORT_TOKENS:
+            which = 1              # (63 single tokens beside a portion of 64: 159 us in the first kernel alone, 169 in two launches)
         st = self._lib("mlstm.cu").rv_mlstm_scan(
             _ptr(proj), c_int(proj.shape[1]), c_int(i_col0), c_int(f_col0), _ptr(i_bias), _ptr(f_bias), _ptr(cu_seqlens), _ptr(state_slots),
-            _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(raw), _ptr(top), c_int(T), c_int(cu_seqlens.shape[0] - 1), c_int(heads),
-            c_int(head_dim), c_int(value_dim), c_float(cap), self._stream())
+            _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(raw), _ptr(top), c_int(n_seqs), c_int(heads),
+            c_int(head_dim), c_int(value_dim), c_float(cap), c_int(which), c_int(self.MLSTM_SHORT_TOKENS), self._stream())
         _check("mlstm_scan", st)
+        COUNTERS['launches'] += 1 if which == 3 and 32 < head_dim <= 128 else 0
         return raw, top
 
     def mlstm_output(self, raw, top, gamma, eps: float, den_eps: float, proj, g_col0: int, heads: int, head_dim: int, value_dim: int,

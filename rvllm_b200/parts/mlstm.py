@@ -61,7 +61,7 @@ class MLstmMixer(Part):
         gate_col = 2 * self.qk_dim + self.v_dim
         raw, top = k.mlstm_scan(proj, gate_col + self.v_dim, gate_col + self.v_dim + self.heads, self.i_bias, self.f_bias,
                                 ctx.cu_seqlens, ctx.state_slots, cache.state, self.heads, self.head_dim, self.value_dim,
-                                self.gate_cap)
+                                self.gate_cap, max_q_len=max(ctx.q_lens))
         y = k.mlstm_output(raw, top, self.norm, self.eps, self.denominator_eps, proj, gate_col, self.heads, self.head_dim,
                            self.value_dim, x.dtype, ctx.token_seq, ctx.cu_seqlens, ctx.state_slots, cache.state)
         return self.out(y, ctx, residual=residual, out_dtype=out_dtype)

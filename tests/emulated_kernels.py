@@ -330,7 +330,8 @@ class EmulatedKernels:
                 state[slot, 0] = prev
         return out
 
-    def mlstm_scan(self, proj, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, heads, head_dim, value_dim, cap):
+    def mlstm_scan(self, proj, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, heads, head_dim, value_dim, cap,
+                   max_q_len=None):
         T = proj.shape[0]
         D, V = head_dim, value_dim
         x = proj.float()

@@ -232,7 +232,7 @@ def test_selective_scan_in_two_roles(K, inner, N, lens):
     assert rel_err(got, want) < 2e-6 and rel_err(state[:, :inner * N], S.view(len(lens), -1)) < 2e-6
 
 
-@pytest.mark.parametrize("inner,N,lens", [(70, 16, (1, 5, 16, 17, 35)), (33, 32, (18, 2, 1, 1, 1, 1)), (40, 8, (1, 9)), (32, 16, (1,) * 20 + (40,))])
+@pytest.mark.parametrize("inner,N,lens", [(70, 16, (1, 5, 16, 17, 35)), (33, 32, (18, 2, 1, 1, 1, 1)), (40, 8, (1, 9)), (32, 16, (1,) * 26 + (40,))])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_selective_scan_bits_do_not_depend_on_the_step(K, inner, N, lens, dtype):
     """A request's outputs and state are the same bits alone, beside others and with its portion cut in two, whichever kernels the
@@ -425,9 +425,37 @@ def test_mlstm_of_portions_in_two_roles(K, d, vd, heads, lens):
             S[s] = torch.exp(gf[t] + m[s] - new)[:, None, None] * S[s] + torch.exp(gi[t] - new)[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
             m[s], top[t], raw[t] = new, new, torch.einsum("hdv,hd->hv", S[s], q[t])
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
-    got, got_top = K.mlstm_scan(proj, g0, g0 + heads, ib, fb, i32(cu), i32(list(range(len(lens)))), state, heads, d, vd, cap)
+    got, got_top = K.mlstm_scan(proj, g0, g0 + heads, ib, fb, i32(cu), i32(list(range(len(lens)))), state, heads, d, vd, cap, max_q_len=max(lens))
     # float sums of d products; the gates' logarithms and exponentials to a few last places
     assert rel_err(got, raw.view(T, -1)) < 3e-6 and rel_err(got_top, top) < 1e-6 and rel_err(state[:, :heads * d * W], S.view(len(lens), -1)) < 3e-6
+
+
+@pytest.mark.parametrize("d,vd,heads,lens", [(128, 256, 2, (1, 40, 16, 1)), (100, 30, 2, (33, 31, 2)), (64, 63, 1, (1,) * 26 + (130,)), (40, 5, 2, (47, 1)),
+                                             (24, 6, 2, (1, 40)), (160, 6, 1, (2, 35))])
+def test_mlstm_bits_do_not_depend_on_the_step(K, d, vd, heads, lens):
+    """A request's outputs, maxima and state are the same bits alone, beside others and whichever kernels the steps take; a
+    padding row (slot -1) leaves no state."""
+    torch.manual_seed(d + vd)
+    T, W, g0 = sum(lens), vd + 1, heads * (2 * d + vd)
+    proj, ib, fb = torch.randn(T, g0 + 2 * heads, device="cuda"), torch.randn(heads, device="cuda"), torch.randn(heads, device="cuda") + 2
+    before = torch.randn(len(lens), heads * d * W + heads, device="cuda")
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    slots = list(range(len(lens)))
+    if len(lens) > 2:
+        slots[2] = -1
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
+
+    def run(a, b, cu, slots, state, longest):
+        raw, top = K.mlstm_scan(proj[a:b].contiguous(), g0, g0 + heads, ib, fb, i32(cu), i32(slots), state, heads, d, vd, 15.0, max_q_len=longest)
+        return [torch.cat([raw[cu[i]:cu[i + 1]], top[cu[i]:cu[i + 1]]], 1) for i in range(len(slots)) if slots[i] >= 0], state
+    whole, state = run(0, T, cu, slots, before.clone(), max(lens))
+    for longest in (1, T, None):
+        y, s = run(0, T, cu, slots, before.clone(), longest)
+        assert all(map(torch.equal, y, whole)) and torch.equal(s, state)
+    assert len(lens) == 2 or torch.equal(state[2], before[2])
+    for i, y in zip([i for i in range(len(lens)) if slots[i] >= 0], whole):
+        got, s = run(cu[i], cu[i + 1], [0, lens[i]], [i], before.clone(), lens[i])
+        assert torch.equal(got[0], y) and torch.equal(s[i], state[i])
 
 
 @pytest.mark.parametrize("vocab,ctas", [(1000, 1), (2048, 2), (2049, 1), (40001, 4), (128256, 8)])
