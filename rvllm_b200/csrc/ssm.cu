@@ -245,7 +245,7 @@ ssm_scan_kernel(const void* __restrict__ xbc, int x_dtype, int channels,        
                 const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots,
                 float* __restrict__ state, size_t state_stride, float* __restrict__ y,
                 int heads, int P, int N, int groups,
-                int seg_tokens, int max_segs, float* __restrict__ seg_state, float* __restrict__ seg_decay, float* __restrict__ dcum) {
+                int seg_tokens, int max_segs, float* __restrict__ seg_state, float* __restrict__ seg_decay, float* __restrict__ dcum, int most) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     constexpr int NSL = 8;                            // slices of the state dimension
@@ -269,7 +269,7 @@ ssm_scan_kernel(const void* __restrict__ xbc, int x_dtype, int channels,        
     const int h = blockIdx.y, p0 = blockIdx.x * COLS;
     const int seq_start = cu_seqlens[seq], seq_tok = cu_seqlens[seq + 1] - seq_start;
     const int n_segs = seg_tokens > 0 ? (seq_tok + seg_tokens - 1) / seg_tokens : 1;
-    if (seg >= n_segs) return;
+    if (seg >= n_segs || seq_tok > most) return;       // (longer portions: ssm_chunk.cu's)
     const int start = seq_start + seg * seg_tokens;
     const int n_tok = seg_tokens > 0 ? (seq_tok - seg * seg_tokens < seg_tokens ? seq_tok - seg * seg_tokens : seg_tokens) : seq_tok;
     const int slot = state_slots[seq];
@@ -531,7 +531,7 @@ static int launch_scan(cudaStream_t stream, const void* xbc, int x_dtype, int ch
                        int dt_stride, int dt_col0, const void* dt_bias, const void* a_log, const void* d_skip, int p_dtype,
                        const int* cu_seqlens, const int* state_slots, float* state, size_t state_stride, float* y, int n_seqs,
                        int heads, int P, int N, int groups, int seg_tokens, int max_segs, float* seg_state, float* seg_decay,
-                       float* dcum) {
+                       float* dcum, int most) {
     constexpr int COLS = NC * 16;
     const dim3 grid((P + COLS - 1) / COLS, heads, n_seqs * max_segs);
     const size_t smem = sizeof(float) * ((size_t)2 * RV_SCAN_CHUNK * 8 * (NPT + 4) + 2 * RV_SCAN_CHUNK * COLS + 2 * RV_SCAN_CHUNK);
@@ -540,7 +540,7 @@ static int launch_scan(cudaStream_t stream, const void* xbc, int x_dtype, int ch
         if (int e = rv_configure_smem(configured, ssm_scan_kernel<NPT, NC>, (int)smem)) return e;
     return rv_launch(ssm_scan_kernel<NPT, NC>, grid, dim3(128), smem, stream, xbc, x_dtype, channels, dt_in, dt_dtype, dt_stride, dt_col0,
                      dt_bias, a_log, d_skip, p_dtype, cu_seqlens, state_slots, state, state_stride, y, heads, P, N, groups,
-                     seg_tokens, max_segs, seg_state, seg_decay, dcum);
+                     seg_tokens, max_segs, seg_state, seg_decay, dcum, most);
 }
 
 // `columns`: columns per thread, 1 or 2; 0 lets the launcher choose by the size of the grid.
@@ -548,19 +548,19 @@ static int launch_scan(cudaStream_t stream, const void* xbc, int x_dtype, int ch
 // (`max_segs` = the most segments of any sequence; scratch: seg_state [n_seqs * max_segs, heads, N, P], seg_decay
 // [n_seqs * max_segs, heads], dcum [tokens, heads], all float), then two small kernels carry the state through the segments
 // and add what each segment's starting state contributes to its outputs.  The results equal the one-pass walk up to
-// float32 rounding.
+// float32 rounding.  Sequences of more than `most` tokens are left alone (not with segments).
 RV_EXPORT int rv_ssm_scan(const void* xbc, int x_dtype, int channels, const void* dt_in, int dt_dtype, int dt_stride, int dt_col0,
                           const void* dt_bias, const void* a_log, const void* d_skip, int p_dtype, const int* cu_seqlens,
                           const int* state_slots, float* state, long long state_stride, float* y, int n_seqs, int heads, int P,
                           int N, int groups, int columns, int seg_tokens, int max_segs, float* seg_state, float* seg_decay,
-                          float* dcum, cudaStream_t stream) {
+                          float* dcum, int most, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || P <= 0 || N <= 0 || groups <= 0 || heads % groups) return RV_ERR_BAD_SIZE;
     if (channels < heads * P + 2 * groups * N || dt_stride < dt_col0 + heads || dt_col0 < 0) return RV_ERR_BAD_SIZE;
     if ((x_dtype | dt_dtype | p_dtype) & ~1) return RV_ERR_BAD_DTYPE;
     if (columns < 0 || columns > 2) return RV_ERR_BAD_SIZE;
     if (N > 256 || heads > 65535 || n_seqs > 65535) return RV_ERR_UNSUPPORTED;
     if (n_seqs == 0) return RV_OK;
-    if (seg_tokens < 0 || (seg_tokens & 15)) return RV_ERR_BAD_SIZE;
+    if (seg_tokens < 0 || (seg_tokens & 15) || (seg_tokens && most != 0x7fffffff)) return RV_ERR_BAD_SIZE;
     if (seg_tokens == 0) max_segs = 1;
     else if (max_segs < 1 || !seg_state || !seg_decay || !dcum) return RV_ERR_BAD_SIZE;
     if ((long long)n_seqs * max_segs > 65535) return RV_ERR_UNSUPPORTED;
@@ -570,7 +570,7 @@ RV_EXPORT int rv_ssm_scan(const void* xbc, int x_dtype, int channels, const void
 #define RV_SCAN_LAUNCH(NPT, NC)                                                                                                  \
     RV_LAUNCH_ST = launch_scan<NPT, NC>(stream, xbc, x_dtype, channels, dt_in, dt_dtype, dt_stride, dt_col0, dt_bias, a_log,     \
                                         d_skip, p_dtype, cu_seqlens, state_slots, state, (size_t)state_stride, y, n_seqs, heads, P, N, groups, \
-                                        seg_tokens, max_segs, seg_state, seg_decay, dcum)
+                                        seg_tokens, max_segs, seg_state, seg_decay, dcum, most)
     if (narrow || N > 128) {
         if (N <= 32) RV_SCAN_LAUNCH(4, 1);
         else if (N <= 64) RV_SCAN_LAUNCH(8, 1);

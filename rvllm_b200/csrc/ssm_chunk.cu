@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(128, 2)
 ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void* __restrict__ dt_in, int dt_dtype, int dt_stride, int dt_col0,
                  const void* __restrict__ dt_bias, const void* __restrict__ a_log, const void* __restrict__ d_skip, int p_dtype,
                  const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                 size_t state_stride, float* __restrict__ y, int heads, int P, int groups) {
+                 size_t state_stride, float* __restrict__ y, int heads, int P, int groups, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     extern __shared__ __align__(16) unsigned char ch_raw[];
@@ -105,6 +105,7 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const int seq = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * 64;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
+    if (n_tok < least) return;                             // (ssm.cu's)
     const int slot = state_slots[seq];
     const int inner = heads * P, cols = min(64, P - p0);
     if (slot < 0) {                                        // a padding row: no state; its output is zero
@@ -371,19 +372,19 @@ ssm_chunk_kernel(const __nv_bfloat16* __restrict__ xbc, int channels, const void
 template <int N>
 static int launch_chunk(const void* xbc, int channels, const void* dt_in, int dt_dtype, int dt_stride, int dt_col0, const void* dt_bias,
                         const void* a_log, const void* d_skip, int p_dtype, const int* cu_seqlens, const int* state_slots, float* state,
-                        size_t state_stride, float* y, int n_seqs, int heads, int P, int groups, cudaStream_t stream) {
+                        size_t state_stride, float* y, int n_seqs, int heads, int P, int groups, int least, cudaStream_t stream) {
     static RvPerDevice once;
     if (int st = rv_configure_smem(once, ssm_chunk_kernel<N>, (int)sizeof(ChunkSmem<N>))) return st;
     return rv_launch(ssm_chunk_kernel<N>, dim3((P + 63) / 64, heads, n_seqs), dim3(128), sizeof(ChunkSmem<N>), stream, (const __nv_bfloat16*)xbc,
                      channels, dt_in, dt_dtype, dt_stride, dt_col0, dt_bias, a_log, d_skip, p_dtype, cu_seqlens, state_slots, state,
-                     state_stride, y, heads, P, groups);
+                     state_stride, y, heads, P, groups, least);
 }
 
-// Arguments as of rv_ssm_scan (ssm.cu), xbc bfloat16.  RV_ERR_UNSUPPORTED for sizes that the kernel does not serve: state sizes
+// Arguments as of rv_ssm_scan (ssm.cu), xbc bfloat16; sequences of fewer than `least` tokens are left alone.  RV_ERR_UNSUPPORTED for sizes that the kernel does not serve: state sizes
 // other than 64 and 128, rows that are not whole 16-byte words.
 RV_EXPORT int rv_ssm_chunk(const void* xbc, int channels, const void* dt_in, int dt_dtype, int dt_stride, int dt_col0, const void* dt_bias,
                            const void* a_log, const void* d_skip, int p_dtype, const int* cu_seqlens, const int* state_slots, float* state,
-                           long long state_stride, float* y, int n_seqs, int heads, int P, int N, int groups, cudaStream_t stream) {
+                           long long state_stride, float* y, int n_seqs, int heads, int P, int N, int groups, int least, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || P <= 0 || N <= 0 || groups <= 0 || heads % groups) return RV_ERR_BAD_SIZE;
     if (channels < heads * P + 2 * groups * N || dt_stride < dt_col0 + heads || dt_col0 < 0) return RV_ERR_BAD_SIZE;
     if ((dt_dtype | p_dtype) & ~1) return RV_ERR_BAD_DTYPE;
@@ -391,10 +392,10 @@ RV_EXPORT int rv_ssm_chunk(const void* xbc, int channels, const void* dt_in, int
     if (n_seqs == 0) return RV_OK;
     if (N == 128)
         RV_LAUNCH_ST = launch_chunk<128>(xbc, channels, dt_in, dt_dtype, dt_stride, dt_col0, dt_bias, a_log, d_skip, p_dtype, cu_seqlens,
-                                         state_slots, state, (size_t)state_stride, y, n_seqs, heads, P, groups, stream);
+                                         state_slots, state, (size_t)state_stride, y, n_seqs, heads, P, groups, least, stream);
     else if (N == 64)
         RV_LAUNCH_ST = launch_chunk<64>(xbc, channels, dt_in, dt_dtype, dt_stride, dt_col0, dt_bias, a_log, d_skip, p_dtype, cu_seqlens,
-                                        state_slots, state, (size_t)state_stride, y, n_seqs, heads, P, groups, stream);
+                                        state_slots, state, (size_t)state_stride, y, n_seqs, heads, P, groups, least, stream);
     else
         return RV_ERR_UNSUPPORTED;
     return rv_launch_status();

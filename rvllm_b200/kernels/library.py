@@ -1076,7 +1076,8 @@ class CudaKernels:
         sequence brings (known on the host); long portions are then cut into segments of `segment_tokens` (default
         `SCAN_SEGMENT_TOKENS`) that are scanned side by side and joined by two small kernels.  Portions of
         `SCAN_CHUNK_MIN_TOKENS` bfloat16 tokens and more take the chunked form on the tensor cores (ssm_chunk.cu) where it serves
-        the sizes; `chunked` asks for or against it."""
+        the sizes, beside shorter ones that are walked: a request's bits depend on its own portion alone.  `chunked` asks
+        for it for every sequence, or against it."""
         _need(xbc, "xbc", dims=2); _need(proj, "proj", dims=2); _need(state, "state", torch.float32, 2)
         for name, p in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
             _need(p, name, dt_bias.dtype, 1)
@@ -1085,19 +1086,26 @@ class CudaKernels:
         if state.shape[1] < heads * state_size * head_dim:
             raise KernelError("ssm_scan: the state rows are too short")
         y = torch.empty((xbc.shape[0], heads * head_dim), dtype=torch.float32, device=xbc.device)
+        n_seqs, least = state_slots.shape[0], 0
         if chunked is None:
             chunked = columns == 0 and segment_tokens is None and max_q_len is not None and max_q_len >= self.SCAN_CHUNK_MIN_TOKENS
+            if chunked and xbc.shape[0] != n_seqs * max_q_len:         # (else: all of that length)
+                least = self.SCAN_CHUNK_MIN_TOKENS
         if chunked and xbc.dtype == torch.bfloat16 and state_size in (64, 128) and head_dim % 16 == 0 and xbc.shape[1] % 8 == 0 \
                 and xbc.data_ptr() % 16 == 0:
+            if least:
+                self._ssm_walk(xbc, proj, dt_col0, dt_bias, a_log, d_skip, cu_seqlens, state_slots, state, y, heads, head_dim, state_size, groups,
+                               most=least - 1)
+                COUNTERS['launches'] += 1
             st = self._lib("ssm_chunk.cu").rv_ssm_chunk(
                 _ptr(xbc), c_int(xbc.shape[1]), _ptr(proj), c_int(self._dt(proj, "proj")), c_int(proj.shape[1]), c_int(dt_col0),
                 _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), c_int(self._dt(dt_bias, "dt_bias")), _ptr(cu_seqlens), _ptr(state_slots),
-                _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(y), c_int(state_slots.shape[0]), c_int(heads), c_int(head_dim),
-                c_int(state_size), c_int(groups), self._stream())
+                _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(y), c_int(n_seqs), c_int(heads), c_int(head_dim),
+                c_int(state_size), c_int(groups), c_int(least), self._stream())
             _check("ssm_chunk", st)
             return y
         seg = self.SCAN_SEGMENT_TOKENS if segment_tokens is None else segment_tokens
-        n_seqs, max_segs, seg_state, seg_decay, dcum = state_slots.shape[0], 1, None, None, None
+        max_segs, seg_state, seg_decay, dcum = 1, None, None, None
         few_ctas = self.SCAN_SEGMENT_ALWAYS or segment_tokens is not None or -(-head_dim // 32) * heads * n_seqs < self.num_sms
         if seg and few_ctas and max_q_len is not None and max_q_len > 2 * seg:
             max_segs = -(-max_q_len // seg)
@@ -1109,15 +1117,20 @@ class CudaKernels:
                 max_segs = 1
         if seg_state is None:
             seg = 0
+        self._ssm_walk(xbc, proj, dt_col0, dt_bias, a_log, d_skip, cu_seqlens, state_slots, state, y, heads, head_dim, state_size, groups,
+                       columns, seg, max_segs, seg_state, seg_decay, dcum)
+        COUNTERS['launches'] += 2 if seg else 0
+        return y
+
+    def _ssm_walk(self, xbc, proj, dt_col0, dt_bias, a_log, d_skip, cu_seqlens, state_slots, state, y, heads, head_dim, state_size, groups,
+                  columns=0, seg=0, max_segs=1, seg_state=None, seg_decay=None, dcum=None, most=0x7fffffff):
         st = self._lib("ssm.cu").rv_ssm_scan(
             _ptr(xbc), c_int(self._dt(xbc, "xbc")), c_int(xbc.shape[1]), _ptr(proj), c_int(self._dt(proj, "proj")),
             c_int(proj.shape[1]), c_int(dt_col0), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), c_int(self._dt(dt_bias, "dt_bias")),
             _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(y),
             c_int(state_slots.shape[0]), c_int(heads), c_int(head_dim), c_int(state_size), c_int(groups), c_int(columns),
-            c_int(seg), c_int(max_segs), _ptr(seg_state), _ptr(seg_decay), _ptr(dcum), self._stream())
+            c_int(seg), c_int(max_segs), _ptr(seg_state), _ptr(seg_decay), _ptr(dcum), c_int(most), self._stream())
         _check("ssm_scan", st)
-        COUNTERS['launches'] += 2 if seg else 0
-        return y
 
     def gated_group_rmsnorm(self, y, proj, gamma, eps: float, parts: int, out_dtype) -> torch.Tensor:
         """(y * silu(z)) RMS-normalised in `parts` equal parts of a row, times gamma; z = the leading columns of `proj`."""

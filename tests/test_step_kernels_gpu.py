@@ -160,6 +160,37 @@ def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
     assert norm(state[:, :heads * N * P], S.view(len(lens), -1)) <= norm(walked[:, :heads * N * P], S.view(len(lens), -1)) + 3.5e-8
 
 
+@pytest.mark.parametrize("N,lens", [(128, (1, 40, 5, 64, 31)), (64, (32, 1, 1)), (128, (33, 33))])
+def test_ssm_scan_bits_depend_on_the_request_alone(K, N, lens, monkeypatch):
+    """Long portions of a step go chunk by chunk and short ones beside them token by token, each with the bits that it has alone;
+    a padding row (slot -1) leaves no state and reads as zero."""
+    torch.manual_seed(N + len(lens))
+    heads, P, T = 4, 48, sum(lens)
+    xbc = torch.randn(T, heads * P + 2 * N, device="cuda").bfloat16()
+    proj, bias = torch.randn(T, heads, device="cuda"), torch.randn(heads, device="cuda") - 2
+    a_log, D = torch.linspace(-1, 2, heads, device="cuda"), torch.randn(heads, device="cuda")
+    before = torch.randn(len(lens), heads * N * P, device="cuda")
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    slots = list(range(len(lens)))
+    if len(lens) > 2:
+        slots[2] = -1
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+
+    def run(a, b, cu, slots):
+        state = before.clone()
+        return K.ssm_scan(xbc[a:b].contiguous(), proj[a:b].contiguous(), 0, bias, a_log, D, i32(cu), i32(slots), state, heads, P, N, 1,
+                          max_q_len=max(v - u for u, v in zip(cu, cu[1:]))), state
+    used, load = [], K._lib
+    monkeypatch.setattr(K, "_lib", lambda source, *a: used.append(source) or load(source, *a))
+    whole, state = run(0, T, cu, slots)
+    assert used == (["ssm_chunk.cu"] if len(set(lens)) == 1 else ["ssm.cu", "ssm_chunk.cu"])
+    for i, n in enumerate(lens):
+        y, s = run(cu[i], cu[i + 1], [0, n], [slots[i]])
+        assert used[-1] == ("ssm_chunk.cu" if n >= 32 else "ssm.cu")
+        assert torch.equal(y, whole[cu[i]:cu[i + 1]]) and torch.equal(s[i], state[i])
+        assert slots[i] >= 0 or (torch.equal(state[i], before[i]) and not y.any())
+
+
 @pytest.mark.parametrize("N,value,where", [(128, float("inf"), 5), (64, float("nan"), 77), (128, float("-inf"), 64), (64, float("inf"), 129)])
 @pytest.mark.parametrize("place", ["x", "B", "C", "dt"])
 def test_ssm_scan_in_chunks_is_causal(K, N, value, where, place):
