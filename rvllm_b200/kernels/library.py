@@ -1066,6 +1066,19 @@ class CudaKernels:
                                        # 128 CTAs, 64 heads of 64: the step's prefill 6.4 -> 5.5 ms; 256 CTAs, 128 heads: scan + carry +
                                        # correction 0.59 + 0.16 + 0.38 ms against 0.92 ms in one pass)
 
+    def _segments_are_faster(self, n_seqs: int, heads: int, head_dim: int, state_size: int, longest: int) -> bool:
+        """Whether the segmented walk beats the chunked kernel, whose time is that of the longest portion whatever the number of its
+        CTAs: 0.142 us a token.  The segments take about 400 us while they are up to four CTAs an SM, and 0.45 us for each one more
+        (one sequence of 8,192 tokens, heads of 64 x 128: 4 heads 398 against 1,148 us, 16 577 and 1,164, 32 1,088 and 1,170, 48 1,608
+        and 1,176; of 2,048 tokens 322 and 290, 373 and 294, 409 and 295, 531 and 297)."""
+        seg = self.SCAN_SEGMENT_TOKENS
+        segs = -(-longest // seg) if seg else 0
+        few_ctas = self.SCAN_SEGMENT_ALWAYS or -(-head_dim // 32) * heads * n_seqs < self.num_sms
+        if not seg or not few_ctas or longest <= 2 * seg or n_seqs * segs * heads * state_size * head_dim * 4 > self.SCAN_SEGMENT_SCRATCH \
+                or n_seqs * segs > 65535:
+            return False
+        return longest > 2816 + 3.2 * max(0, n_seqs * segs * heads * -(-head_dim // 32) - 4 * self.num_sms)
+
     def ssm_scan(self, xbc, proj, dt_col0: int, dt_bias, a_log, d_skip, cu_seqlens, state_slots, state, heads: int,
                  head_dim: int, state_size: int, groups: int, columns: int = 0, max_q_len: Optional[int] = None,
                  segment_tokens: Optional[int] = None, chunked: Optional[bool] = None) -> torch.Tensor:
@@ -1088,7 +1101,8 @@ class CudaKernels:
         y = torch.empty((xbc.shape[0], heads * head_dim), dtype=torch.float32, device=xbc.device)
         n_seqs, least = state_slots.shape[0], 0
         if chunked is None:
-            chunked = columns == 0 and segment_tokens is None and max_q_len is not None and max_q_len >= self.SCAN_CHUNK_MIN_TOKENS
+            chunked = columns == 0 and segment_tokens is None and max_q_len is not None and max_q_len >= self.SCAN_CHUNK_MIN_TOKENS \
+                and not self._segments_are_faster(n_seqs, heads, head_dim, state_size, max_q_len)
             if chunked and xbc.shape[0] != n_seqs * max_q_len:         # (else: all of that length)
                 least = self.SCAN_CHUNK_MIN_TOKENS
         if chunked and xbc.dtype == torch.bfloat16 and state_size in (64, 128) and head_dim % 16 == 0 and xbc.shape[1] % 8 == 0 \

@@ -191,6 +191,27 @@ def test_ssm_scan_bits_depend_on_the_request_alone(K, N, lens, monkeypatch):
         assert slots[i] >= 0 or (torch.equal(state[i], before[i]) and not y.any())
 
 
+@pytest.mark.parametrize("heads,T,segments", [(2, 2816, False), (2, 2817, True), (8, 5000, True), (64, 5000, False), (300, 3000, False)])
+def test_ssm_scan_of_few_heads_takes_segments(K, heads, T, segments, monkeypatch):
+    """Long portions on few CTAs go in segments side by side where the chunks' walk is longer: the same values."""
+    torch.manual_seed(heads)
+    P, N = 16, 64
+    xbc = torch.randn(T, heads * P + 2 * N, device="cuda").bfloat16()
+    proj, bias = torch.randn(T, heads, device="cuda"), torch.randn(heads, device="cuda") - 4
+    a_log, D = torch.rand(heads, device="cuda"), torch.randn(heads, device="cuda")
+    before = torch.randn(1, heads * N * P, device="cuda")
+    cu, slots = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    used, load = [], K._lib
+    monkeypatch.setattr(K, "_lib", lambda source, *a: used.append(source) or load(source, *a))
+    runs = []
+    for chunked in (None, not segments):
+        state = before.clone()
+        runs.append((K.ssm_scan(xbc, proj, 0, bias, a_log, D, cu, slots, state, heads, P, N, 1, max_q_len=T, chunked=chunked), state))
+    assert used == ["ssm.cu" if segments else "ssm_chunk.cu", "ssm_chunk.cu" if segments else "ssm.cu"]
+    # two orders of float sums along up to 5,000 tokens with decays near 1
+    assert all(rel_err(a, b.double().cpu()) < 2e-5 for a, b in zip(*runs))
+
+
 @pytest.mark.parametrize("N,value,where", [(128, float("inf"), 5), (64, float("nan"), 77), (128, float("-inf"), 64), (64, float("inf"), 129)])
 @pytest.mark.parametrize("place", ["x", "B", "C", "dt"])
 def test_ssm_scan_in_chunks_is_causal(K, N, value, where, place):
