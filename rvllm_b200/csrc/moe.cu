@@ -227,10 +227,10 @@ static int moe_launch(const void* x, const int* chosen, const float* weights, co
 //   moe_mma_gate_up   a CTA per (expert, 16 features, or 2 x 16): eight warps share k (gated: four on the gate rows, four on the up rows),
 //                     their sums meet in shared memory
 //   moe_mma_down      a CTA per 16 columns of the result: its warps share the (expert, quarter of k) items, and the sums of a
-//                     token's slots are added in the slots' order
+//                     token's slots are added in the slots' order; a launch per block of tokens whose sums fit the shared memory
 // 32 experts (4096 x 2048, gated), 4 of them for each of 8 / 64 tokens, both products: 290 / 1,411 us with the kernels above, 179 /
 // 291 us (5.6 TB/s) with these.  The cuts of k depend on the sizes alone, so a row's result does not depend on the rest of
-// the batch.
+// the batch, as far as these kernels serve it (the caller takes grouped products from 128 tokens on).
 __device__ __forceinline__ void moe_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -496,6 +496,13 @@ static size_t moe_mma_down_smem(int pairs, int experts) {
     return (size_t)MM_QUARTERS * pairs * 16 * 4 + (size_t)(2 * experts + (pairs < experts ? pairs : experts) + pairs) * 4;
 }
 #define MM_SMEM_MAX (160 * 1024)
+// The launches of moe_mma_down for `tokens` tokens (0: the sums of one token do not fit).  A second reads the matrices again, but the
+// kernels above read them once per pair.
+RV_EXPORT int rv_moe_down_blocks(int tokens, int top, int experts) {
+    int fit = tokens;
+    while (fit > 0 && moe_mma_down_smem(fit * top, experts) > MM_SMEM_MAX) --fit;
+    return fit > 0 ? (tokens + fit - 1) / fit : 0;
+}
 
 static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float* weights, const __nv_bfloat16* gate_up,
                           const __nv_bfloat16* down, __nv_bfloat16* act, const float* add, const float* add_scale, void* out, int out_f32,
@@ -507,7 +514,7 @@ static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float
     // blocks: 15.1 us so, 16.5 with two.
     const int used = pairs < experts ? pairs : experts, blocks = (ff + 15) / 16;
     const dim3 grid(used, (long long)used * blocks > 2LL * rv_sm_count() ? (blocks + 1) / 2 : blocks);
-    const size_t smem_a = moe_mma_gate_up_smem(pairs, experts), smem_b = moe_mma_down_smem(pairs, experts);
+    const size_t smem_a = moe_mma_gate_up_smem(pairs, experts);
     // The first kernel waits for its predecessors at the launch: its loads go through L1, and CTAs that came in early, beside a product
     // whose stages fill the SM's shared memory, kept the SM in that division, with no room for what they ask for (8 tokens
     // of 4 experts, 2048 x 4096, behind the shared expert's products: 312 us for both kernels, 171 us launched so).
@@ -521,15 +528,21 @@ static int moe_mma_launch(const __nv_bfloat16* x, const int* chosen, const float
     }
     if (st != RV_OK) return st;
     const dim3 grid_b((width + 15) / 16);
-    const __nv_bfloat16* own = identity ? x : nullptr;
-    if (out_f32) {
-        if ((st = rv_configure_smem(once[2], moe_mma_down_kernel<float>, MM_SMEM_MAX)) != RV_OK) return st;
-        st = rv_launch(moe_mma_down_kernel<float>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act, chosen, down, add, (float*)out, tokens, top,
-                       experts, ff, width, weight, weights, add_scale, own);
-    } else {
-        if ((st = rv_configure_smem(once[3], moe_mma_down_kernel<__nv_bfloat16>, MM_SMEM_MAX)) != RV_OK) return st;
-        st = rv_launch(moe_mma_down_kernel<__nv_bfloat16>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act, chosen, down, add, (__nv_bfloat16*)out,
-                       tokens, top, experts, ff, width, weight, weights, add_scale, own);
+    const int blocks_b = rv_moe_down_blocks(tokens, top, experts), per = (tokens + blocks_b - 1) / blocks_b;
+    st = out_f32 ? rv_configure_smem(once[2], moe_mma_down_kernel<float>, MM_SMEM_MAX) : rv_configure_smem(once[3], moe_mma_down_kernel<__nv_bfloat16>, MM_SMEM_MAX);
+    for (int t0 = 0; t0 < tokens && st == RV_OK; t0 += per) {
+        const int n = tokens - t0 < per ? tokens - t0 : per;
+        const size_t first = (size_t)t0 * top, at = (size_t)t0 * width, smem_b = moe_mma_down_smem(n * top, experts);
+        const float* w = weights ? weights + first : nullptr;
+        const float* a = add ? add + at : nullptr;
+        const float* scale = add_scale ? add_scale + t0 : nullptr;
+        const __nv_bfloat16* own = identity ? x + at : nullptr;
+        if (out_f32)
+            st = rv_launch(moe_mma_down_kernel<float>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act + first * ff, chosen + first, down, a, (float*)out + at,
+                           n, top, experts, ff, width, weight, w, scale, own);
+        else
+            st = rv_launch(moe_mma_down_kernel<__nv_bfloat16>, grid_b, dim3(MM_WARPS * 32), smem_b, stream, act + first * ff, chosen + first, down, a,
+                           (__nv_bfloat16*)out + at, n, top, experts, ff, width, weight, w, scale, own);
     }
     RV_LAUNCH_ST = st;
     return rv_launch_status();
@@ -550,7 +563,7 @@ RV_EXPORT int rv_moe_experts_ex(const void* x, const int* chosen, const float* w
                                  stream);
     if (dtype == RV_DTYPE_BF16 && width % 32 == 0 && ff % 32 == 0 && (long long)tokens * top <= 4096 && experts <= 4096 && (ff + 15) / 16 <= 65535 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(act)) & 15) == 0 &&
-        moe_mma_gate_up_smem(tokens * top, experts) <= MM_SMEM_MAX && moe_mma_down_smem(tokens * top, experts) <= MM_SMEM_MAX)
+        moe_mma_gate_up_smem(tokens * top, experts) <= MM_SMEM_MAX && rv_moe_down_blocks(tokens, top, experts) > 0)
         return moe_mma_launch((const __nv_bfloat16*)x, chosen, weights, (const __nv_bfloat16*)gate_up, (const __nv_bfloat16*)down, (__nv_bfloat16*)act,
                               add, add_scale, out, out_f32, tokens, top, experts, ff, width, weight, gated, identity, stream);
     if (dtype == RV_DTYPE_BF16)

@@ -1681,7 +1681,8 @@ class CudaKernels:
             _ptr(out), c_int(1 if out_dtype == torch.float32 else 0), c_int(T), c_int(top), c_int(E), c_int(ff), c_int(width), c_float(weight),
             c_int(1 if gated else 0), c_int(1 if identity else 0), c_int(self._dt(x, "x")), self._stream())
         _check("moe_experts", st)
-        COUNTERS['launches'] += 1
+        blocks = self._lib("moe.cu").rv_moe_down_blocks(c_int(T), c_int(top), c_int(E)) if x.dtype == torch.bfloat16 and not (width | ff) % 32 else 1
+        COUNTERS['launches'] += max(1, blocks)
         return out
 
     MOE_GROUPED_MIN_TOKENS = 128      # tokens of a step from which the experts' products run grouped on the tcgen05 GEMM ...

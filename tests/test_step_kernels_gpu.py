@@ -56,10 +56,12 @@ def test_stream_norms_in_words_of_four(K, rows, cols, y_dtype):
 
 
 @pytest.mark.parametrize("T,E,top,ff,width,gated,identity", [(1, 8, 2, 32, 64, True, False), (7, 5, 3, 96, 160, False, True), (33, 40, 4, 160, 96, True, False),
-                                                             (100, 3, 2, 64, 96, True, False), (9, 70, 4, 1408, 2048, False, False)])
+                                                             (100, 3, 2, 64, 96, True, False), (9, 70, 4, 1408, 2048, False, False),
+                                                             (100, 12, 8, 64, 96, True, True), (127, 9, 16, 32, 64, False, False)])
 def test_moe_of_few_tokens_on_the_tensor_cores(K, T, E, top, ff, width, gated, identity):
     """Every expert's pairs as the columns of one product: lists of one to many pairs (several passes), numbers that name
-    nobody (-1) or the token itself, rows of 16 that end inside the matrix; and a token's bits do not depend on the others."""
+    nobody (-1) or the token itself, rows of 16 that end inside the matrix, sums of more pairs than shared memory holds at a
+    time (from about 620 on); and a token's bits do not depend on the others."""
     torch.manual_seed(T * E)
     gu = (torch.randn(E, (2 if gated else 1) * ff, width, device="cuda") * 0.1).bfloat16()
     dn = (torch.randn(E, width, ff, device="cuda") * 0.1).bfloat16()
