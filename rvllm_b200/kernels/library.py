@@ -573,7 +573,8 @@ class CudaKernels:
                 and (residual is None or (residual.dtype == torch.bfloat16 and out_dtype == torch.bfloat16)):
             return self.linear_decode(x, weight, bias, residual, out_dtype)
         if self._tcgen05_fills(M, weight.shape[0]) and K % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32) \
-                and (residual is None or (residual.dtype == torch.bfloat16 and out_dtype == torch.bfloat16)):
+                and (residual is None or (residual.dtype == torch.bfloat16 and out_dtype == torch.bfloat16)) \
+                and self._epilogue_takes(x, weight, bias, residual):
             return self.linear_tcgen05(x, weight, residual, out_dtype, bias=bias)
         if out_dtype == torch.float32:
             out = torch.mm(x, weight.t(), out_dtype=torch.float32)
@@ -591,6 +592,16 @@ class CudaKernels:
             out += residual.float()
             return out.to(out_dtype)
         return torch.nn.functional.linear(x, weight, bias.to(x.dtype) if bias is not None else None)
+
+    @staticmethod
+    def _epilogue_takes(x, weight, bias, residual=None) -> bool:
+        """Whether the tcgen05 GEMM can take this bias in its epilogue: one packed value of float32 or bfloat16 per feature, a residual
+        of the result's own shape, rows on 16-byte boundaries.  Other types, strides and shapes that broadcast go to the library."""
+        if bias is None:
+            return True
+        M, N = x.shape[0], weight.shape[0]
+        return (bias.dtype in _DT and tuple(bias.shape) == (N,) and bias.is_contiguous() and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+                and (residual is None or (tuple(residual.shape) == (M, N) and residual.is_contiguous() and residual.data_ptr() % 16 == 0)))
 
     def _tcgen05_fills(self, M: int, N: int, gated: bool = False) -> bool:
         """Whether this project's tcgen05 GEMM is the one to use for M rows and N weight rows: from
@@ -655,10 +666,14 @@ class CudaKernels:
         _need(x, "x", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
         M, K = x.shape
         N = weight.shape[0]
+        if weight.shape[1] != K:
+            raise KernelError(f"linear: x has {K} columns, weight has {weight.shape[1]}")
         out_dtype = out_dtype or torch.bfloat16
         out = torch.empty((M, N // 2 if gated else N), dtype=out_dtype, device=x.device)
         if residual is not None:
             _need(residual, "residual", torch.bfloat16, 2)
+            if residual.shape != out.shape:
+                raise KernelError(f"linear: a residual of {tuple(residual.shape)} for a result of {tuple(out.shape)}")
         if bias is not None:
             _need(bias, "bias", dims=1)
             if bias.shape[0] != N:
@@ -908,7 +923,10 @@ class CudaKernels:
         290 MB for the activation, 230 us of a layer)."""
         M, K = x.shape
         N = weight.shape[0]
-        if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and N % 2 == 0 and K % 8 == 0 and limit > 0:
+        if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and N % 2 == 0 and K % 8 == 0 and limit > 0 \
+                and self._epilogue_takes(x, weight, bias):
+            if weight.shape[1] != K:
+                raise KernelError(f"gate_up_clamp: x has {K} columns, weight has {weight.shape[1]}")
             options = dict(bias=bias, gated=True, activation="swiglu_clamp", limit=limit, alpha=alpha)
             if self._use_decode_gemm(M, N, K, True):
                 return self.linear_decode(x, weight, **options)

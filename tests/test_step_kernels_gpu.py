@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from rvllm_b200.errors import KernelError
 from rvllm_b200.kernels import get_library
 
 pytestmark = pytest.mark.gpu
@@ -120,6 +121,40 @@ def test_bias_and_clamped_gate_in_the_products_epilogues(K, M, N, Kd, bias_dtype
     gate, up = ref[:, :half].clamp(max=2.0), ref[:, half:].clamp(-2.0, 2.0)
     want = gate * torch.sigmoid(1.7 * gate) * (up + 1)
     assert rel_err(K.gate_up_clamp(x, w, b, 2.0, 1.7), want) < 5e-3
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("form", ["float64", "strided", "one value", "strided residual", "one residual row", "odd address", "odd residual", "no multiple of 8"])
+def test_biases_and_residuals_that_no_epilogue_takes(K, form, out_dtype):
+    """Types, strides, addresses and shapes that broadcast: what the library's product takes beside a bias, and a clamped gate too."""
+    torch.manual_seed(4)
+    M, N, Kd = 300, 130 if form == "no multiple of 8" else 96, 128
+    x, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") * 0.1).bfloat16()
+    b, r = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda").bfloat16()
+    if form == "float64":
+        b = b.double()
+    elif form == "strided":
+        b = torch.randn(2 * N, device="cuda")[::2]
+    elif form == "one value":
+        b = b[:1]
+    elif form == "strided residual":
+        r = torch.randn(M, 2 * N, device="cuda").bfloat16()[:, ::2]
+    elif form == "one residual row":
+        r = r[:1]
+    elif form == "odd address":
+        x = torch.randn(M * Kd + 1, device="cuda").bfloat16()[1:].view(M, Kd)
+    elif form == "odd residual":
+        r = torch.randn(M * N + 1, device="cuda").bfloat16()[1:].view(M, N)
+    ref = x.double().cpu() @ w.double().cpu().t() + b.double().cpu()
+    tol = 2e-5 if out_dtype == torch.float32 else 1e-2      # float sums; two roundings to bfloat16 where the bias is one
+    assert rel_err(K.linear(x, w, b, None, out_dtype), ref) < tol
+    if out_dtype == torch.bfloat16:
+        assert rel_err(K.linear(x, w, b, r, out_dtype), ref + r.double().cpu()) < tol
+    gate, up = ref[:, :N // 2].clamp(max=2.0), ref[:, N // 2:].clamp(-2.0, 2.0)
+    assert rel_err(K.gate_up_clamp(x, w, b, 2.0, 1.7), gate * torch.sigmoid(1.7 * gate) * (up + 1)) < 5e-3
+    for m in (4, M):                                        # a weight of fewer columns is refused, whatever the path
+        with pytest.raises(KernelError):
+            K.gate_up_clamp(x[:m].clone(), w[:, :64].contiguous(), torch.randn(N, device="cuda"), 2.0, 1.7)
 
 
 @pytest.mark.parametrize("heads,P,N,groups,lens", [(4, 64, 128, 2, (33, 1, 64, 65)), (6, 48, 64, 3, (130, 2)), (2, 80, 128, 1, (40,)), (2, 16, 64, 1, (200,))])
