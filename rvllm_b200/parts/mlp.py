@@ -4,8 +4,6 @@ residual added in the last product's epilogue.  gate and up are one stacked prod
 of the reference)."""
 from __future__ import annotations
 
-import torch
-
 from .base import FEED_FORWARDS, Part
 from .linear import Linear
 
@@ -65,12 +63,7 @@ class ClampedGluMLP(Part):
         self.down.bind(get)
 
     def __call__(self, x, ctx, residual=None, out_dtype=None):
-        fused = getattr(ctx.kernels, "gate_up_clamp", None)
-        if fused is not None:
-            h = fused(x, self.gate_up.weight, self.gate_up.bias, self.limit, self.alpha)
-        else:
-            gu = self.gate_up(x, ctx, out_dtype=torch.float32)
-            h = ctx.kernels.act_mul(gu, "swiglu_clamp", x.dtype, limit=self.limit, alpha=self.alpha)
+        h = ctx.kernels.gate_up_clamp(x, self.gate_up.weight, self.gate_up.bias, self.limit, self.alpha)
         return self.down(h, ctx, residual=residual, out_dtype=out_dtype)
 
 

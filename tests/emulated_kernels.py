@@ -383,6 +383,9 @@ class EmulatedKernels:
             a = 0.5 * g * (1.0 + torch.tanh(math.sqrt(2.0 / math.pi) * (g + 0.044715 * g ** 3)))
         return (a * u).to(out_dtype or gate_up.dtype)
 
+    def gate_up_clamp(self, x, weight, bias, limit, alpha):
+        return self.act_mul(self.linear(x, weight, bias, None, torch.float32), "swiglu_clamp", x.dtype, limit=limit, alpha=alpha)
+
     def gate_up_act(self, x, weight, activation="silu", norm=None):
         return self.act_mul(self.linear(x, weight, out_dtype=torch.float32, norm=norm), activation, x.dtype)
 
