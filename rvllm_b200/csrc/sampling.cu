@@ -568,7 +568,7 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
     return true;
 }
 
-__device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two)
+__device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two), 2: rows that need it get -1
 
 __global__ void __launch_bounds__(SAMPLE_THREADS, 1)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
@@ -610,6 +610,10 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
             return;
         have_max = true;
         sc_sync();                                       // (the first CTA's shared memory is no longer written from outside)
+        if (g_sample_short_way == 2) {
+            if (rank == 0 && tid == 0) out[r] = -1;
+            return;
+        }
     }
     if (!have_max) {
     // ---- arg-max of the row
@@ -815,9 +819,10 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 static int g_sample_cluster = 0;
 // CTAs per row: 0 chosen by the number of rows, else 1, 2, 4 or 8 (for tests: the result is the same).
 RV_EXPORT void rv_sample_set_cluster(int ctas_per_row) { g_sample_cluster = ctas_per_row; }
-// 1 (default): top-k / top-p rows try the short way first; 0: always the general search.
-RV_EXPORT int rv_sample_set_short_way(int on) {
-    const int v = on ? 1 : 0;
+// 1 (default): top-k / top-p rows try the short way first; 0: always the general search; 2: the short way alone, rows that it
+// does not serve get the id -1 (for tests).
+RV_EXPORT int rv_sample_set_short_way(int mode) {
+    const int v = mode == 2 ? 2 : (mode ? 1 : 0);
     return (int)cudaMemcpyToSymbol(g_sample_short_way, &v, sizeof(int));
 }
 

@@ -106,10 +106,12 @@ def test_moe_sums_of_whole_activations(K, T, E, top, ff, width):
     assert float((out.double() - ref).norm() / ref.norm()) < 5e-8
 
 
-@pytest.mark.parametrize("M,N,Kd", [(130, 264, 72), (300, 96, 128), (512, 512, 4096), (5, 200, 136), (64, 1024, 264), (200, 130, 72)])
+@pytest.mark.parametrize("M,N,Kd", [(130, 264, 72), (300, 96, 128), (512, 512, 4096), (5, 200, 136), (64, 1024, 264), (200, 130, 72), (5, 1024, 4096)])
 @pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16])
 def test_bias_and_clamped_gate_in_the_products_epilogues(K, M, N, Kd, bias_dtype):
-    """Plain, residual and clamp-gated products with a bias: both GEMMs, one CTA, pairs and K split over a cluster."""
+    """Plain, residual and clamp-gated products with a bias: both GEMMs, one CTA, pairs, K split over a cluster and (few gated rows of
+    a long K) over CTAs that meet in scratch memory."""
+    assert (M, Kd) != (5, 4096) or K.gemm_splits((N // 2 + 63) // 64, Kd) > 1
     torch.manual_seed(M + N)
     x, w = torch.randn(M, Kd, device="cuda").bfloat16(), (torch.randn(N, Kd, device="cuda") * 0.1).bfloat16()
     b, r = torch.randn(N, device="cuda").to(bias_dtype), torch.randn(M, N, device="cuda").bfloat16()
@@ -158,7 +160,7 @@ def test_biases_and_residuals_that_no_epilogue_takes(K, form, out_dtype):
 
 
 @pytest.mark.parametrize("heads,P,N,groups,lens", [(4, 64, 128, 2, (33, 1, 64, 65)), (6, 48, 64, 3, (130, 2)), (2, 80, 128, 1, (40,)), (2, 16, 64, 1, (200,))])
-def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
+def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens, monkeypatch):
     """The chunked form against the recurrence in float64: portions that end inside a chunk, single tokens, a padding row, column
     blocks that are not full, a state to continue from, decays from weak to total."""
     torch.manual_seed(P)
@@ -187,7 +189,10 @@ def test_ssm_scan_in_chunks(K, heads, P, N, groups, lens):
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
     walked = state.clone()
     run = lambda st, chunked: K.ssm_scan(xbc, proj, 3, bias, a_log, D, i32(cu), i32(slots), st, heads, P, N, groups, max_q_len=max(lens), chunked=chunked)      # noqa: E731
+    used, load = [], K._lib
+    monkeypatch.setattr(K, "_lib", lambda source, *a: used.append(source) or load(source, *a))
     got, walk = run(state, True), run(walked, False)
+    assert used == ["ssm_chunk.cu", "ssm.cu"]
     # three bfloat16 terms hold a float: the error is that of float sums over N and 64 products
     assert rel_err(got, want.view(T, -1)) < 2e-6
     assert rel_err(state[:, :heads * N * P], S.view(len(lens), -1)) < 2e-6
@@ -471,7 +476,8 @@ def test_delta_rule_bits_do_not_depend_on_the_step(K, d, vd, heads, qk, lens, dt
 
 
 def test_talking_attention_on_eight_and_sixteen_warps(K):
-    """The same tiles for twice the tokens a CTA: the same bits."""
+    """The same tiles for twice the tokens a CTA: the same bits, and those of the attention's formula in float64."""
+    import plain_tibepel as P
     from rvllm_b200.kernels.library import AttentionMeta
     torch.manual_seed(3)
     nh, nkv, hd, ps, T = 8, 4, 64, 16, 75
@@ -488,6 +494,11 @@ def test_talking_attention_on_eight_and_sixteen_warps(K):
     finally:
         del K.TALKING_WARPS
     assert torch.equal(*out)
+    rows = cache[[3, 1, 0, 4, 2]].double().cpu().view(5, 2, nkv, ps, hd).permute(1, 0, 3, 2, 4).reshape(2, 5 * ps, nkv, hd)[:, :T]
+    f64 = lambda v: v.double().cpu()      # noqa: E731
+    want = P.mixed_head_attention(f64(q).view(T, nh, hd), rows[0], rows[1], hd ** -0.5, f64(r), f64(r), f64(talk), 10 ** 9)
+    # the mixed weights and the result are rounded to bfloat16 (2^-9 each)
+    assert rel_err(out[0], want.reshape(T, -1)) < 1e-2
 
 
 @pytest.mark.parametrize("d,vd,heads,lens", [(128, 256, 2, (5, 15, 16, 50, 80)), (100, 30, 2, (33,)), (64, 63, 1, (48, 17)), (40, 5, 2, (47,))])
@@ -566,9 +577,16 @@ def test_top_p_rows_by_their_candidates(K, vocab, ctas):
         general = K.sample(*args).tolist()
         assert lib.rv_sample_set_short_way(c_int(1)) == 0
         short = K.sample(*args).tolist()
+        assert lib.rv_sample_set_short_way(c_int(2)) == 0
+        served = K.sample(*args).tolist()                    # -1 where the short way hands the row on
     finally:
         lib.rv_sample_set_cluster(c_int(0)), lib.rv_sample_set_short_way(c_int(1))
     assert short[5] == vocab - 2
     # masses are added in different orders: a draw within rounding (2^-24 log2(vocab)) of a step may differ, one row in thousands
     rows = [r for r in range(24) if r != 5]
     assert sum(short[r] != general[r] for r in rows) <= 1
+    # peaked rows go the short way (all but a thousandth of a wide row's mass may need more tokens than it holds); a flat row whose
+    # tokens are more than it holds does not
+    assert all(served[r] == short[r] for r in rows if spread[r] >= 4 and (r % 3 != 1 or vocab <= 2048))
+    assert all(served[r] in (-1, short[r]) for r in rows)
+    assert all((served[r] == -1) == (vocab > 2048) for r in (0, 8, 16))
