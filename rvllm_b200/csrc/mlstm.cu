@@ -219,7 +219,7 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
 // its gates and stage it (double buffers, one barrier a chunk); a warp walks the running maximum through a chunk with the gates
 // in its lanes.  The numbers and the order of every sum are those of the kernel above, so a request's bits do not depend on which
 // of the two a step takes.
-// 2,048 tokens of 8 heads, 128 x 256: 628 -> 401 us; of 16 heads 755 -> 514; four sequences of 500, 8 heads 198 -> 143.
+// 2,048 tokens of 8 heads, 128 x 256: 648 -> 416 us; of 16 heads 759 -> 531; four sequences of 500, 8 heads 198 -> 143.
 template <int PARTS>
 struct MlstmStage {
     static constexpr int ROW = PARTS * 12;                 // 8 entries a lane, 12 floats apart: a lane's reads fall on banks of their own

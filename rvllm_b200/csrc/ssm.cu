@@ -793,8 +793,8 @@ selective_scan1_kernel(const void* __restrict__ u, int u_dtype, const float* __r
 // two roles: four warps walk a chunk while four others bring, turn and stage the next one (softplus, input times step
 // size, silu of the gate) and write out the one before; every buffer is double, with one barrier a chunk.  The walk itself is
 // bound by instructions, seven of them an expf per state and token: B and C of a lane are one 16-byte read each, step size
-// and input one 8-byte read, and nothing is tested per state.  8,192 / 4,096 channels of 16 states, 2,048 tokens: 732 / 595 us
-// with one role and a read and test per state, 391 / 262 us with these.
+// and input one 8-byte read, and nothing is tested per state.  8,192 / 4,096 channels of 16 states, 2,048 tokens: 765 / 608 us
+// with one role and a read and test per state, 394 / 304 us with these.
 template <int PARTS>
 __global__ void __launch_bounds__(256)
 selective_scan1_vec_kernel(const void* __restrict__ u, int u_dtype, const float* __restrict__ dt_raw, const float* __restrict__ dt_bias,
@@ -1207,7 +1207,7 @@ delta_rule_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, c
 // then form that column's u.  S^T q is formed of the state before the token, beside S^T k, and the result is
 // g S^T q + (k . q) u: the chain from token to token is one sum over the lanes, not two.  Four warps walk, four others
 // bring the next chunk, turn q and k into unit vectors and stage them (double buffers, one barrier a chunk).  2,048 tokens of
-// 32 / 16 heads of 128 x 128: 1,051 / 923 us before, 694 / 536 us; portions of 1,024 twice: 569 / 524 and 378 / 350 us.  (The
+// 32 / 16 heads of 128 x 128: 1,087 / 932 us before, 711 / 561 us; portions of 1,024 twice: 569 / 524 and 378 / 350 us.  (The
 // kernel above with more lanes a column - 16 or 8 entries each - is slower: 1,078 and 1,109 us.)
 template <int PARTS>
 struct DeltaStage {
