@@ -7,7 +7,7 @@
 // multiple of 32), each segment is one chain of FMAs in ascending k from zero, four consecutive
 // segments are added in order, and the four groups as (g0 + g1) + (g2 + g3).  Then bias, then residual.
 //
-//   gemm_f32_stream_kernel   up to 32 rows: bound by the stream of weights.  A CTA takes 16 rows of W whole;
+//   gemm_f32_stream_kernel   up to 32 rows (more in blocks of 32 where the product is small): bound by the stream of weights.  A CTA takes 16 rows of W whole;
 //                            each half warp walks one segment, a lane one row of W, against all rows of x,
 //                            from a ring of warp-private stages that cp.async fills (no CTA barrier in the loop;
 //                            the first weights are asked for before griddepcontrol.wait).
@@ -52,6 +52,13 @@ gemm_f32_stream_kernel(const float* __restrict__ x, const float* __restrict__ w,
                        int bias_dtype, const float* __restrict__ residual, float* __restrict__ out,
                        int M, int N, int K) {
     extern __shared__ __align__(128) float smem[];
+    if (blockIdx.y) {                                       // (rows beyond the first MB)
+        const size_t m0 = (size_t)blockIdx.y * MB;
+        x += m0 * K;
+        out += m0 * N;
+        if (residual) residual += m0 * N;
+        M -= (int)m0;
+    }
     constexpr int WROWS = 16;
     constexpr int STAGE = (WROWS + MB) * ST_K;              // floats of a half warp's stage
     const int tid = threadIdx.x, half = tid >> 4, l16 = tid & 15;
@@ -150,7 +157,7 @@ static int launch_stream(const float* x, const float* w, const void* bias, int b
     static_assert(ring >= MAX_SEGMENTS * MB * 16 * 4, "the sums fit the ring");
     static RvPerDevice configured;
     if (int st = rv_configure_smem(configured, gemm_f32_stream_kernel<MB, STAGES>, ring)) return st;
-    return rv_launch(gemm_f32_stream_kernel<MB, STAGES>, dim3((N + 15) / 16), dim3(ST_WARPS * 32), ring, stream,
+    return rv_launch(gemm_f32_stream_kernel<MB, STAGES>, dim3((N + 15) / 16, (M + MB - 1) / MB), dim3(ST_WARPS * 32), ring, stream,
                      x, w, bias, bias_dtype, residual, out, M, N, K);
 }
 
@@ -388,8 +395,10 @@ RV_EXPORT int rv_gemm_f32(const float* x, const float* w, const void* bias, int 
     if (M == 0) return RV_OK;
     const bool vec = (K & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
     // Up to 32 rows the weights' stream is the longer side (8 rows) or level with the FMAs (32); beyond, W would be
-    // read once per 32 rows.  The ring needs rows of whole 16-byte words.
-    if (vec && M <= 32) {
+    // read once per 32 rows.  The ring needs rows of whole 16-byte words.  Products of up to 512 k (one step of the ring) whose
+    // blocks of 32 rows are one CTA an SM at most are all latency, of which a tile has more (64 rows of 64 x 64: 9.0 us).
+    const bool small = K <= ST_K * MAX_SEGMENTS && (long long)((N + 15) / 16) * ((M + 31) / 32) <= rv_sm_count();
+    if (vec && (M <= 32 || small)) {
         int st;
         if (M == 1) st = launch_stream<1, 3>(x, w, bias, bias_dtype, residual, out, M, N, K, stream);
         else if (M == 2) st = launch_stream<2, 3>(x, w, bias, bias_dtype, residual, out, M, N, K, stream);
