@@ -600,12 +600,13 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     const int k_row = top_k ? top_k[r] : 0;
     const float p_row = top_p ? top_p[r] : 1.0f;
     const bool uk_row = k_row > 0 && k_row < V, up_row = p_row < 1.0f;
+    const float inv_t = fminf(1.0f / T, 3.402823466e38f);      // (a temperature below 2.9e-39 would make the maximum's own mass 0 x infinity)
     float m = -INFINITY;
     int best = 0x7fffffff;
     bool have_max = false;
     if (T > 0.f && (uk_row || up_row) && g_sample_short_way) {
         // maximum, counts and candidates in two passes; too many candidates: the maximum is kept, the search below goes on
-        if (sample_short_way(row, V, 1.0f / T, k_row, p_row, uk_row, up_row, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan,
+        if (sample_short_way(row, V, inv_t, k_row, p_row, uk_row, up_row, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan,
                                s_val, s_idx, &fast_shared, m, best))
             return;
         have_max = true;
@@ -636,7 +637,6 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         if (rank == 0 && tid == 0) out[r] = best;
         return;
     }
-    const float inv_t = 1.0f / T;
 
     // ---- mass of everything, where a top-p is measured by it
     float total = 0.f;

@@ -593,6 +593,19 @@ def test_top_p_rows_by_their_candidates(K, vocab, ctas):
     assert all((served[r] == -1) == (vocab > 2048) for r in (0, 16))
 
 
+@pytest.mark.parametrize("temperature", [1e-30, 1e-39, 1e-42])
+@pytest.mark.parametrize("k,p", [(0, 0.9), (50, 1.0), (50, 0.5), (0, 1.0)])
+def test_temperatures_whose_reciprocal_overflows(K, temperature, k, p):
+    """Ever lower temperatures draw the maximum, also where 1 / T is beyond the largest float; one of them where it is there twice."""
+    torch.manual_seed(2)
+    x = torch.randn(4, 5000, device="cuda")
+    x[3, 7] = x[3, 9] = x[3].max() + 1
+    full = lambda v, dtype: torch.full((4,), v, dtype=dtype, device="cuda")      # noqa: E731
+    got = K.sample(x, full(temperature, torch.float32), full(k, torch.int32) if k else None, full(p, torch.float32) if p < 1 else None,
+                   torch.arange(4, device="cuda"), torch.arange(4, device="cuda")).tolist()
+    assert got[:3] == x[:3].argmax(1).tolist() and got[3] in (7, 9)
+
+
 @pytest.mark.parametrize("T,nh,nkv,hd,dtype", [(3, 4, 2, 64, torch.bfloat16), (300, 6, 3, 20, torch.float32), (17, 32, 8, 128, torch.bfloat16), (1, 1, 1, 4, torch.float32)])
 def test_row_kernels_in_words_of_four(K, T, nh, nkv, hd, dtype):
     """Rows on 16-byte boundaries are read in words of four elements by several blocks, rows at odd addresses one by one: the same
