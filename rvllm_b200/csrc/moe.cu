@@ -497,7 +497,8 @@ static size_t moe_mma_down_smem(int pairs, int experts) {
 }
 #define MM_SMEM_MAX (160 * 1024)
 // The launches of moe_mma_down for `tokens` tokens (0: the sums of one token do not fit).  A second reads the matrices again, but the
-// kernels above read them once per pair.
+// kernels above read them once per pair: 80 tokens of 8 of 64 experts of 2048 x 1408, 640 pairs, 455 us so and 1,324 with those; 127
+// tokens of 8 of 32 of 4096 x 2048 742 and 5,146.
 RV_EXPORT int rv_moe_down_blocks(int tokens, int top, int experts) {
     int fit = tokens;
     while (fit > 0 && moe_mma_down_smem(fit * top, experts) > MM_SMEM_MAX) --fit;
