@@ -80,6 +80,10 @@ class CudaKernels:
     PAIR_GEMM = True                   # the tcgen05 GEMM runs on pairs of CTAs (cta_group::2) where the rows fill its 256-row tiles
     TALKING_MMA = True                 # attention with mixed head weights: bfloat16 prompt portions go to the tensor-core kernel when it fits
     TALKING_WARPS = 0                  # ... whose CTAs have up to 8 or 16 warps (0: by the number of CTAs)
+    TALKING_WIDE = True                # ... where its sizes allow, to the tcgen05 kernel, which mixes behind the sum over the keys
+    TALKING_WIDE_MIN_TOKENS = 16       # ... from this many tokens in the longest portion of the step (80 tokens of 16 heads on 4: 20 us against 32;
+                                       # steps of up to TALKING_SPLIT_MAX_TOKENS behind more keys do not come here)
+    TALKING_WIDE_MAX_SCRATCH = 256 << 20   # ... in windows of tokens whose sums over the keys fit this many bytes
     TALKING_SPLIT = True               # attention with mixed head weights: few tokens behind many keys go to the split-key kernels
     TALKING_SPLIT_MAX_TOKENS = 64      # ... up to this many tokens in the step
     TALKING_SPLIT_MIN_KEYS = 64        # ... behind more than this many keys
@@ -1434,6 +1438,23 @@ class CudaKernels:
                 c_int(self._dt(q, "q")), self._stream())
             _check("talking_attention_split", st)
             return out
+        if self.TALKING_MMA and self.TALKING_WIDE and not self.TALKING_WARPS and q.dtype == torch.bfloat16 and talk is not None \
+                and scale > 0 and meta.max_q_len >= self.TALKING_WIDE_MIN_TOKENS:
+            lib = self._lib("talking_attention_tcgen05.cu")
+            if lib.rv_talking_wide_fits(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim), c_int(ps)):
+                per_token = num_kv_heads * num_heads * value_dim
+                window = max(1, min(T, self.TALKING_WIDE_MAX_SCRATCH // (4 * per_token)))
+                u = torch.empty((window * per_token,), dtype=torch.float32, device=q.device)
+                for lo in range(0, T, window):
+                    st = lib.rv_talking_wide(
+                        _ptr(q), _ptr(cache_layer), ctypes.c_longlong(cache_layer.shape[0]), _ptr(meta.block_tables), _ptr(meta.cu_seqlens),
+                        _ptr(meta.ctx_lens), _ptr(out), _ptr(u), c_int(T), c_int(lo), c_int(min(T, lo + window)), c_int(meta.num_seqs),
+                        c_int(meta.max_q_len), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim), c_int(ps),
+                        c_int(meta.max_blocks), c_float(scale), _ptr(r1), _ptr(r2), _ptr(talk), c_int(chunk or 0), _ptr(self._status),
+                        self._stream())
+                    _check("talking_attention_wide", st)
+                    COUNTERS['launches'] += 1
+                return out
         if self.TALKING_MMA and q.dtype == torch.bfloat16 and T > 0:
             lib = self._lib("talking_attention_mma.cu")
             if lib.rv_talking_attention_mma_fits(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim)):

@@ -311,6 +311,45 @@ def test_every_build_of_the_mixed_head_attention_gives_the_plain_result(K, H, G,
         K.TALKING_MMA, K.TALKING_SPLIT = old
 
 
+@pytest.mark.parametrize("H,G,d,vd,chunk,page", [(16, 4, 128, 128, None, 16), (8, 8, 64, 128, 97, 8), (16, 1, 128, 64, 150, 64), (4, 2, 64, 64, 40, 128),
+                                                 (14, 7, 64, 64, 64, 16), (32, 4, 64, 128, None, 32)])
+def test_mixing_behind_the_sum_over_the_keys(K, H, G, d, vd, chunk, page):
+    """The tcgen05 build: one to several blocks of value heads, portions that start and end inside tiles, chunks and pages, single
+    tokens among them; whatever lies in slots that nobody wrote - here NaN - stays outside; windows of tokens give the bits of the
+    whole step."""
+    from rvllm_b200.kernels.library import COUNTERS
+    dtype = torch.bfloat16
+    ctx, q_lens = (230, 171, 1, 260, 64), (150, 37, 1, 70, 2)
+    ks = [rnd(c, G, d, seed=180 + i).to(dtype).double() for i, c in enumerate(ctx)]
+    vs = [rnd(c, G, vd, seed=190 + i).to(dtype).double() for i, c in enumerate(ctx)]
+    qs = [rnd(n, H, d, seed=200 + i).to(dtype).double() for i, n in enumerate(q_lens)]
+    r1, r2 = torch.rand(H, generator=torch.Generator().manual_seed(1), dtype=F64) * 1.5, torch.rand(H, generator=torch.Generator().manual_seed(2), dtype=F64) + 0.1
+    talk = torch.eye(H, dtype=F64) + 0.4 * rnd(H, H, seed=3)
+    cache, meta, positions = flat_pages(ks, vs, q_lens, page, dtype, chunk)
+    unwritten = flat_pages([k * 0 for k in ks], [v * 0 for v in vs], q_lens, page, dtype, chunk)[0] != 0
+    cache[unwritten] = float("nan")
+    q = torch.cat(qs).reshape(sum(q_lens), H * d).to(dtype).cuda()
+    for use_bias in (True, False):
+        r = (r1.float().cuda(), r2.float().cuda()) if use_bias else (None, None)
+        before = COUNTERS["launches"]
+        got = K.talking_attention(q, cache, meta, positions, H, G, d, vd, 0.3, *r, talk.float().cuda(), chunk)
+        assert COUNTERS["launches"] == before + 2          # the sums over the keys and the mixing
+        at = 0
+        for i, n in enumerate(q_lens):
+            full_q = torch.zeros(ctx[i], H, d, dtype=F64)
+            full_q[ctx[i] - n:] = qs[i]
+            want = P.mixed_head_attention(full_q, ks[i], vs[i], 0.3, r1 if use_bias else torch.zeros(H, dtype=F64), r2, talk, chunk or 10 ** 9)[ctx[i] - n:]
+            assert rel_err(got[at:at + n], want.reshape(n, -1)) < TOL[dtype], (i, use_bias)
+            at += n
+        old = K.TALKING_WIDE_MAX_SCRATCH
+        try:
+            K.TALKING_WIDE_MAX_SCRATCH = 4 * H * G * vd * 101
+            assert torch.equal(K.talking_attention(q, cache, meta, positions, H, G, d, vd, 0.3, *r, talk.float().cuda(), chunk), got)
+        finally:
+            K.TALKING_WIDE_MAX_SCRATCH = old
+    K.raise_on_abort()
+
+
 def test_a_large_batch_of_single_tokens_takes_the_split_keys(K):
     """Seventy sequences of unequal lengths, one token each: more tokens than the tensor-core build is preferred from, yet
     all of them single, so the keys are split (into fewer ranges than for a small batch); against the slow implementation."""
