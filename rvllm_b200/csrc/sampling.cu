@@ -20,6 +20,7 @@
 // passes of four bits over the row.  All sums that decide anything are integers or are added in a fixed
 // order, so a token depends neither on the run nor on how many CTAs share the row.
 #include "common.cuh"
+#include <string.h>
 
 #define SAMPLE_THREADS 1024
 
@@ -570,11 +571,37 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
 
 __device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two), 2: rows that need it get -1
 
+// Where a row's parameters are: in arrays on the device (null: greedy, or off), or, for up to SAMPLE_VALUE_ROWS rows whose
+// parameters the host has, in the launch itself: no buffer on the device, no copy of 1.8 KB that the host prepares and the kernel waits
+// for (64 rows: 76 us of the host's time with them, 23 without).
+#define SAMPLE_VALUE_ROWS 128               // 28 bytes each: with the other arguments below the 4 KB that every launch may carry
+struct SampleArrays {
+    const float* temperature;
+    const int* top_k;
+    const float* top_p;
+    const unsigned long long* seeds;
+    const long long* draw_index;
+    __device__ __forceinline__ float t(int r) const { return temperature ? temperature[r] : 0.f; }
+    __device__ __forceinline__ int k(int r) const { return top_k ? top_k[r] : 0; }
+    __device__ __forceinline__ float p(int r) const { return top_p ? top_p[r] : 1.0f; }
+    __device__ __forceinline__ unsigned long long seed(int r) const { return seeds[r]; }
+    __device__ __forceinline__ long long draw(int r) const { return draw_index[r]; }
+};
+struct SampleValues {
+    unsigned long long seeds[SAMPLE_VALUE_ROWS];
+    long long draw_index[SAMPLE_VALUE_ROWS];
+    float temperature[SAMPLE_VALUE_ROWS], top_p[SAMPLE_VALUE_ROWS];
+    int top_k[SAMPLE_VALUE_ROWS];
+    __device__ __forceinline__ float t(int r) const { return temperature[r]; }
+    __device__ __forceinline__ int k(int r) const { return top_k[r]; }
+    __device__ __forceinline__ float p(int r) const { return top_p[r]; }
+    __device__ __forceinline__ unsigned long long seed(int r) const { return seeds[r]; }
+    __device__ __forceinline__ long long draw(int r) const { return draw_index[r]; }
+};
+
+template <typename Rows>
 __global__ void __launch_bounds__(SAMPLE_THREADS, 1)
-sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const unsigned long long* __restrict__ seeds, const long long* __restrict__ draw_index,
-              int* __restrict__ out, int V) {
+sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows rows, int* __restrict__ out, int V) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     __shared__ float s_val[33];
@@ -593,12 +620,12 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     const int r = blockIdx.y;
     const float* row = logits + (size_t)r * V;
     const int S = (((V + SAMPLE_SLICES - 1) / SAMPLE_SLICES) + 3) & ~3;     // slices of an aligned row start on 16-byte boundaries
-    const float T = temperature ? temperature[r] : 0.f;
+    const float T = rows.t(r);
     int turn = 0;                                        // which copy of the exchange buffers is written next
     sc_sync();                                           // every CTA of the cluster runs before its memory is written
 
-    const int k_row = top_k ? top_k[r] : 0;
-    const float p_row = top_p ? top_p[r] : 1.0f;
+    const int k_row = rows.k(r);
+    const float p_row = rows.p(r);
     const bool uk_row = k_row > 0 && k_row < V, up_row = p_row < 1.0f;
     const float inv_t = fminf(1.0f / T, 3.402823466e38f);      // (a temperature below 2.9e-39 would make the maximum's own mass 0 x infinity)
     float m = -INFINITY;
@@ -606,7 +633,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     bool have_max = false;
     if (T > 0.f && (uk_row || up_row) && g_sample_short_way) {
         // maximum, counts and candidates in two passes; too many candidates: the maximum is kept, the search below goes on
-        if (sample_short_way(row, V, inv_t, k_row, p_row, uk_row, up_row, seeds[r], draw_index[r], out + r, s_dyn_fast, s_scan,
+        if (sample_short_way(row, V, inv_t, k_row, p_row, uk_row, up_row, rows.seed(r), rows.draw(r), out + r, s_dyn_fast, s_scan,
                                s_val, s_idx, &fast_shared, m, best))
             return;
         have_max = true;
@@ -661,8 +688,8 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     // sums are added in slice order, and the largest digit that still satisfies the condition is
     // taken.  No atomics: the same result in every run.  NaN is never kept.
     uint32_t tau = 0;
-    const int k = top_k ? top_k[r] : 0;
-    const float pp = top_p ? top_p[r] : 1.0f;
+    const int k = k_row;
+    const float pp = p_row;
     bool use_k = k > 0 && k < V;
     bool use_p = pp < 1.0f;
     if (use_k || use_p) {
@@ -768,8 +795,9 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     for (int sl = 0; sl < SAMPLE_SLICES; ++sl) kept_total += xch[turn].val[sl];
 
     // ---- the draw: the first token, in vocabulary order, whose cumulated kept mass exceeds u * (kept mass)
-    uint32_t c4[4] = {(uint32_t)(draw_index[r] & 0xffffffffll), (uint32_t)((unsigned long long)draw_index[r] >> 32), 0u, 0u};
-    philox4x32_10(c4, (uint32_t)(seeds[r] & 0xffffffffull), (uint32_t)(seeds[r] >> 32));
+    const unsigned long long seed = rows.seed(r), draw = (unsigned long long)rows.draw(r);
+    uint32_t c4[4] = {(uint32_t)draw, (uint32_t)(draw >> 32), 0u, 0u};
+    philox4x32_10(c4, (uint32_t)seed, (uint32_t)(seed >> 32));
     const float u = (float)(c4[0] >> 8) * (1.0f / 16777216.0f);
     const float target = u * kept_total;
     // the slice the target falls into (the same arithmetic in every CTA); if rounding put the target at
@@ -826,6 +854,23 @@ RV_EXPORT int rv_sample_set_short_way(int mode) {
     return (int)cudaMemcpyToSymbol(g_sample_short_way, &v, sizeof(int));
 }
 
+// `filtered`: some row has a top-k or a top-p.
+template <typename Rows>
+static int launch_sample(const float* logits, const Rows& rows, int* out, int n_rows, int vocab, bool filtered, cudaStream_t stream) {
+    // the threshold search of top-k / top-p keeps 16 counters and 16 sums per thread in shared memory
+    const size_t smem = filtered ? (size_t)2 * 16 * SAMPLE_THREADS * 4 : 0;
+    static RvPerDevice configured;
+    if (smem) {
+        if (int e = rv_configure_smem(configured, sample_kernel<Rows>, (int)(2 * 16 * SAMPLE_THREADS * 4))) return e;
+    }
+    // CTAs per row: as many (8, 4, 2 or 1) as keep rows x CTAs within the SMs; the result is the same for each
+    const int sms = rv_sm_count();
+    int cl = g_sample_cluster > 0 ? g_sample_cluster : (n_rows * 8 <= sms ? 8 : (n_rows * 4 <= sms ? 4 : (n_rows * 2 <= sms ? 2 : 1)));
+    if (cl != 1 && cl != 2 && cl != 4 && cl != 8) return RV_ERR_BAD_SIZE;
+    RV_LAUNCH_ST = rv_launch_cluster(sample_kernel<Rows>, dim3(cl, n_rows), dim3(SAMPLE_THREADS), smem, stream, (unsigned)cl, logits, rows, out, vocab);
+    return rv_launch_status();
+}
+
 // temperature, top_k, top_p may be null (greedy / disabled).  seeds and draw_index are read
 // only for rows with temperature > 0.
 RV_EXPORT int rv_sample(const float* logits, const float* temperature, const int* top_k, const float* top_p,
@@ -834,18 +879,26 @@ RV_EXPORT int rv_sample(const float* logits, const float* temperature, const int
     if (n_rows < 0 || vocab <= 0) return RV_ERR_BAD_SIZE;
     if (n_rows == 0) return RV_OK;
     if (temperature && (!seeds || !draw_index)) return RV_ERR_BAD_SIZE;
-    // the threshold search of top-k / top-p keeps 16 counters and 16 sums per thread in shared memory
-    const size_t smem = (temperature && (top_k || top_p)) ? (size_t)2 * 16 * SAMPLE_THREADS * 4 : 0;
-    static RvPerDevice configured;
-    if (smem) {
-        if (int e = rv_configure_smem(configured, sample_kernel, (int)(2 * 16 * SAMPLE_THREADS * 4))) return e;
-    }
     if (n_rows > 65535) return RV_ERR_BAD_SIZE;
-    // CTAs per row: as many (8, 4, 2 or 1) as keep rows x CTAs within the SMs; the result is the same for each
-    const int sms = rv_sm_count();
-    int cl = g_sample_cluster > 0 ? g_sample_cluster : (n_rows * 8 <= sms ? 8 : (n_rows * 4 <= sms ? 4 : (n_rows * 2 <= sms ? 2 : 1)));
-    if (cl != 1 && cl != 2 && cl != 4 && cl != 8) return RV_ERR_BAD_SIZE;
-    RV_LAUNCH_ST = rv_launch_cluster(sample_kernel, dim3(cl, n_rows), dim3(SAMPLE_THREADS), smem, stream, (unsigned)cl,
-                                     logits, temperature, top_k, top_p, seeds, draw_index, out, vocab);
-    return rv_launch_status();
+    return launch_sample(logits, SampleArrays{temperature, top_k, top_p, seeds, draw_index}, out, n_rows, vocab,
+                         temperature && (top_k || top_p), stream);
+}
+
+RV_EXPORT int rv_sample_value_rows() { return SAMPLE_VALUE_ROWS; }
+
+// The same for up to SAMPLE_VALUE_ROWS rows whose parameters lie packed on the HOST: seeds (64 bits) of all rows, draw indices (64
+// bits), temperatures, top-p, top-k (32 bits each).  They are read before the call returns.
+RV_EXPORT int rv_sample_rows(const float* logits, const unsigned char* packed, int* out, int n_rows, int vocab, cudaStream_t stream) {
+    if (n_rows < 0 || n_rows > SAMPLE_VALUE_ROWS || vocab <= 0 || !packed) return RV_ERR_BAD_SIZE;
+    if (n_rows == 0) return RV_OK;
+    SampleValues v;
+    const size_t n = (size_t)n_rows;
+    memcpy(v.seeds, packed, 8 * n);
+    memcpy(v.draw_index, packed + 8 * n, 8 * n);
+    memcpy(v.temperature, packed + 16 * n, 4 * n);
+    memcpy(v.top_p, packed + 20 * n, 4 * n);
+    memcpy(v.top_k, packed + 24 * n, 4 * n);
+    bool filtered = false;
+    for (int r = 0; r < n_rows; ++r) filtered = filtered || v.top_k[r] > 0 || v.top_p[r] < 1.0f;
+    return launch_sample(logits, v, out, n_rows, vocab, filtered, stream);
 }

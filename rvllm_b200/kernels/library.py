@@ -2157,3 +2157,17 @@ class CudaKernels:
                                                 self._stream())
         _check("sample", st)
         return out
+
+    def sample_rows(self, logits, packed: bytes) -> Optional[torch.Tensor]:
+        """`sample` for rows whose parameters the host has: `packed` holds the seeds and draw indices (64 bits) and the temperatures,
+        top-p and top-k (32 bits) of all rows, which travel with the launch.  None: more rows than a launch can carry."""
+        _need(logits, "logits", torch.float32, 2)
+        R, V = logits.shape
+        lib = self._lib("sampling.cu")
+        if R > lib.rv_sample_value_rows():
+            return None
+        if len(packed) != 28 * R:
+            raise KernelError(f"sample_rows: {len(packed)} bytes of parameters for {R} rows")
+        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        _check("sample", lib.rv_sample_rows(_ptr(logits), packed, _ptr(out), c_int(R), c_int(V), self._stream()))
+        return out

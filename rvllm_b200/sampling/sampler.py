@@ -6,6 +6,7 @@ kernel and returns the token ids; only these ids leave the GPU
 """
 from __future__ import annotations
 
+import struct
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -41,14 +42,22 @@ class Sampler:
                                 f"{len(draw_index)} draw indices")
         if all(p.is_greedy for p in params):
             return self.kernels.sample(logits)
-        # one buffer and one copy: seeds and draw indices (64 bits), then temperatures, top-p and top-k (32 bits); the
-        # parameters' tensors are views of it on the device
+        top_ps, top_ks = [p.top_p for p in params], [p.top_k for p in params]
+        temperatures = [p.temperature for p in params]
+        try:      # with the launch itself: seeds and draw indices (64 bits), then temperatures, top-p and top-k (32 bits)
+            packed = struct.pack(f"={2 * R}q{2 * R}f{R}i", *seeds, *draw_index, *temperatures, *top_ps, *top_ks)
+        except (struct.error, OverflowError, TypeError):
+            packed = None
+        if packed is not None and hasattr(self.kernels, "sample_rows"):
+            ids = self.kernels.sample_rows(logits, packed)
+            if ids is not None:
+                return ids
+        # more rows than a launch carries: one buffer and one copy; the parameters' tensors are views of it on the device
         host = np.empty((7 * R,), dtype=np.int32)
         wide, real = host[:4 * R].view(np.int64), host[4 * R:6 * R].view(np.float32)
         wide[:R] = seeds
         wide[R:] = draw_index
-        top_ps, top_ks = [p.top_p for p in params], [p.top_k for p in params]
-        real[:R] = [p.temperature for p in params]
+        real[:R] = temperatures
         real[R:] = top_ps
         host[6 * R:] = top_ks
         flat = torch.from_numpy(host).to(logits.device, non_blocking=True)

@@ -165,3 +165,20 @@ def test_the_short_way_and_the_general_search_draw_the_same_tokens(K, vocab, spr
         assert margin < 1e-4, f"row {r}: short way {short[r]}, general search {general[r]}, margin {margin:.2e}"
     assert len(differ) <= 3
     assert all(0 <= t < vocab for t in short + short_k)
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129])
+def test_parameters_that_travel_with_the_launch(K, rows):
+    """Up to 128 rows carry their parameters in the launch, more in arrays on the device: the same tokens, whatever is mixed."""
+    from rvllm_b200 import Sampler, SamplingParams
+    kinds = [SamplingParams(temperature=0.8, top_k=5, top_p=0.9), SamplingParams(), SamplingParams(temperature=1.5), SamplingParams(temperature=0.6, top_p=0.7),
+             SamplingParams(temperature=2.0, top_k=3)]
+    params = [kinds[(i + 3) % 5] for i in range(rows)]
+    seeds, draws = [(2 ** 63 - 1 - 977 * i) for i in range(rows)], [i * 2 ** 31 for i in range(rows)]
+    logits = torch.randn(rows, 1003, generator=torch.Generator().manual_seed(rows)).cuda() * 3
+    f = lambda v, t: torch.tensor(v, dtype=t).cuda()      # noqa: E731
+    want = K.sample(logits, f([p.temperature for p in params], torch.float32), f([p.top_k for p in params], torch.int32),
+                    f([p.top_p for p in params], torch.float32), f(seeds, torch.int64), f(draws, torch.int64))
+    assert torch.equal(Sampler(K).sample(logits, params, seeds, draws), want)
+    with pytest.raises(OverflowError):
+        Sampler(K).sample(logits, [kinds[0]] * rows, [2 ** 63] * rows, draws)
