@@ -161,7 +161,8 @@ class CudaKernels:
 
     @staticmethod
     def _stream():
-        return c_void_p(torch.cuda.current_stream().cuda_stream)
+        # (the pointer alone: `torch.cuda.current_stream()` makes a stream object of it, a quarter of what a launch cost the host)
+        return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
     @staticmethod
     def _dt(t: torch.Tensor, name: str) -> int:
@@ -771,7 +772,7 @@ class CudaKernels:
         splits = max(1, min(splits, (K + 63) // 64))
         splits, cluster = self._cluster_policy(M, gated, splits, cluster, tiles, K, chosen)
         scratch = None
-        if splits > 1 and not (cluster and M > self.DECODE_MAX_ROWS):
+        if splits > 1 and not (cluster and (M > self.DECODE_MAX_ROWS or (splits <= 8 and not gated))):     # (a cluster adds up in its shared memory)
             if self._decode_counters is None or self._decode_counters.numel() < tiles:
                 self._decode_counters = torch.zeros((max(tiles, 4096),), dtype=torch.int32, device=x.device)
             mb = lib.rv_gemm_decode_padded_rows(c_int(M))
@@ -878,7 +879,7 @@ class CudaKernels:
         splits = max(1, min(splits, (K + 63) // 64))
         splits, cluster = self._cluster_policy(M, False, splits, cluster, tiles, K, chosen)
         scratch = None
-        if splits > 1 and not (cluster and M > self.DECODE_MAX_ROWS):
+        if splits > 1 and not (cluster and (M > self.DECODE_MAX_ROWS or (splits <= 8 and head_dim >= 8))):
             if self._decode_counters is None or self._decode_counters.numel() < tiles:
                 self._decode_counters = torch.zeros((max(tiles, 4096),), dtype=torch.int32, device=x.device)
             mb = lib.rv_gemm_decode_padded_rows(c_int(M))
