@@ -229,20 +229,10 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
             }
         }
     };
-    auto store = [&](int t) {
-        float* xs = smem + (t & 1) * 2 * TK * TPITCH;
-        float* ws = xs + TK * TPITCH;
-        const float4* from = mail + (t & 1) * 4 * 256 + tid;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float4 xa = from[h * 256], wa = from[(2 + h) * 256];
-            const float a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {wa.x, wa.y, wa.z, wa.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                xs[(ld_k + j) * TPITCH + ld_row + h * 64] = a[j];
-                ws[(ld_k + j) * TPITCH + ld_row + h * 64] = b[j];
-            }
-        }
+    auto store = [&](int t, int i) {                         // one of the thread's four words of tile t: x for i < 2, w for the others
+        float* to = smem + ((t & 1) * 2 + (i >> 1)) * TK * TPITCH + ld_k * TPITCH + ld_row + (i & 1) * 64;
+        const float4 v = mail[(t & 1) * 4 * 256 + tid + i * 256];
+        to[0] = v.x; to[TPITCH] = v.y; to[2 * TPITCH] = v.z; to[3 * TPITCH] = v.w;
     };
 
     // acc: the running segment; group: the running group of four; total: the groups of this part (all packed column pairs)
@@ -258,7 +248,7 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (n_tiles > 1) fetch(1);
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
-    if (n_tiles) store(0);
+    if (n_tiles) { store(0, 0); store(0, 1); store(0, 2); store(0, 3); }
     __syncthreads();
     int in_seg = 0, seg_i = 0;
     // the sums of a tile: groups of four segments; the first group's sum waits in shared memory behind the stages while the
@@ -267,12 +257,11 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
     for (int t = 0; t < n_tiles; ++t) {
         const int buf = t & 1;
         if (t + 2 < n_tiles) fetch(t + 2);                  // (its places were read, by this thread, before the last barrier)
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
         const float* xs = smem + buf * 2 * TK * TPITCH;
         const float* ws = xs + TK * TPITCH;
-        if (active)
-#pragma unroll
-        for (int k = 0; k < TK; ++k) {
+        const bool more = t + 1 < n_tiles;
+        auto products = [&](int k) {
             const float4 a0 = *reinterpret_cast<const float4*>(xs + k * TPITCH + am);
             const float4 a1 = *reinterpret_cast<const float4*>(xs + k * TPITCH + am + 16);
             const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(ws + k * TPITCH + bn);
@@ -285,6 +274,20 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
 #pragma unroll
                 for (int j = 0; j < 4; ++j) fma2(acc[i][j], aa, b[j]);
             }
+        };
+        // the next tile's words go to their columns between the products (the other stage has not been read since the last barrier);
+        // behind them, with every warp at it and the multiply-adds idle, they took 4 to 5 % of the time
+        if (active && more) {
+#pragma unroll
+            for (int k = 0; k < TK; ++k) {
+                products(k);
+                if ((k & 3) == 3) store(t + 1, k >> 2);
+            }
+        } else if (active) {
+#pragma unroll
+            for (int k = 0; k < TK; ++k) products(k);
+        } else if (more) {
+            store(t + 1, 0); store(t + 1, 1); store(t + 1, 2); store(t + 1, 3);
         }
         if (++in_seg == seg_tiles || t + 1 == n_tiles) {    // a segment is done
             in_seg = 0;
@@ -327,8 +330,6 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, c
                 }
             }
         }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        if (t + 1 < n_tiles) store(t + 1);
         __syncthreads();
     }
 
