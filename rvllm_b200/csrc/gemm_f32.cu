@@ -17,7 +17,7 @@
 //
 // Measured against one 64 x 64 tile kernel for every M (4 x 4 outputs a thread), which this replaced: 3 rows of 3584 x 18944
 // 2,120 -> 72 us (3.8 TB/s), of 37888 x 3584 836 -> 105 us (5.2 TB/s), of 152064 x 3584 3,235 -> 349 us (6.2 TB/s); 433 rows of
-// 37888 x 3584 5,381 -> 2,835 us (41.5 TFLOP/s); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
+// 37888 x 3584 5,381 -> 2,803 us (42 TFLOP/s; the loop over shared memory with nothing brought there reaches 61); error against float64 1.1e-6 -> 2.7e-7 (2-norms, K = 3,584).
 //
 // Shapes of the layer's five products: v3/crates/rvllm-runtime/src/layer_exec.rs:240-266,
 // 433-444, 478-488, 511-522 of the reference (which calls cuBLASLt there); bias as a row

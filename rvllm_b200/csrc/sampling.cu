@@ -34,70 +34,6 @@ __device__ __forceinline__ void argmax_combine(float& v, int& i, float ov, int o
     if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
 
-__device__ int block_argmax(const float* row, int V, float* s_val, int* s_idx) {
-    float best = -INFINITY;
-    int idx = 0x7fffffff;
-    if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-        // 16-byte loads, two independent chains; indices rise within a chain, so a strict
-        // comparison keeps the lowest index of equal values
-        float b1 = -INFINITY;
-        int i1 = 0x7fffffff;
-        const float4* r4 = reinterpret_cast<const float4*>(row);
-        const int n4 = V >> 2;
-        int i = threadIdx.x;
-        for (; i + (int)blockDim.x < n4; i += 2 * blockDim.x) {
-            const float4 a = r4[i], b = r4[i + blockDim.x];
-            const int ia = i * 4, ib = (i + blockDim.x) * 4;
-            if (a.x > best) { best = a.x; idx = ia; }
-            if (a.y > best) { best = a.y; idx = ia + 1; }
-            if (a.z > best) { best = a.z; idx = ia + 2; }
-            if (a.w > best) { best = a.w; idx = ia + 3; }
-            if (b.x > b1) { b1 = b.x; i1 = ib; }
-            if (b.y > b1) { b1 = b.y; i1 = ib + 1; }
-            if (b.z > b1) { b1 = b.z; i1 = ib + 2; }
-            if (b.w > b1) { b1 = b.w; i1 = ib + 3; }
-        }
-        if (i < n4) {
-            const float4 a = r4[i];
-            const int ia = i * 4;
-            if (a.x > best || (a.x == best && ia < idx)) { best = a.x; idx = ia; }
-            if (a.y > best || (a.y == best && ia + 1 < idx)) { best = a.y; idx = ia + 1; }
-            if (a.z > best || (a.z == best && ia + 2 < idx)) { best = a.z; idx = ia + 2; }
-            if (a.w > best || (a.w == best && ia + 3 < idx)) { best = a.w; idx = ia + 3; }
-        }
-        argmax_combine(best, idx, b1, i1);
-    } else {
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            const float v = row[i];
-            if (v > best || (v == best && i < idx)) { best = v; idx = i; }   // NaN compares false
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        argmax_combine(best, idx, ov, oi);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) { s_val[warp] = best; s_idx[warp] = idx; }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        best = lane < nw ? s_val[lane] : -INFINITY;
-        idx = lane < nw ? s_idx[lane] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            argmax_combine(best, idx, ov, oi);
-        }
-        if (lane == 0) { s_val[0] = best; s_idx[0] = idx == 0x7fffffff ? 0 : idx; }
-    }
-    __syncthreads();
-    return s_idx[0];
-}
-
 // ---------------------------------------------------------------------------------------------
 // One to eight CTAs per row.  A row is always cut into SAMPLE_SLICES contiguous slices of the
 // vocabulary; every reduction over the row (arg-max, mass, the 16 + 16 sums of a pass of the
@@ -136,58 +72,74 @@ struct SampleExchange {
     float mass[SAMPLE_SLICES][16];           // ... and their mass
 };
 
-// Kept mass of a slice in vocabulary order: thread t owns the contiguous chunk [lo, hi) of the slice;
-// on return excl / upto are the kept mass before and up to the end of its chunk, s_incl[last] the
-// slice's kept mass and *s_last its last kept token (-1: none).
-__device__ __forceinline__ void slice_scan(const float* row, int lo_s, int hi_s, uint32_t tau, float m, float inv_t, float* s_scan,
-                           float* s_incl, int* s_last, int& lo, int& hi, int& last_kept, float& excl, float& upto) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// The chunk of slice [lo_s, hi_s) that thread `tid` owns.
+__device__ __forceinline__ void slice_chunk(int lo_s, int hi_s, int tid, int& lo, int& hi) {
     const int C = (hi_s - lo_s + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
     lo = min(hi_s, lo_s + tid * C);
     hi = min(hi_s, lo + C);
-    float local = 0.f;
-    last_kept = -1;
-    auto take = [&](float v, int i) {
-        if (order_key(v) >= tau && !(v != v)) { local += expf((v - m) * inv_t); last_kept = i; }
-    };
-    if (((lo | hi) & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-#pragma unroll 4
-        for (int i = lo; i < hi; i += 4) {
-            const float4 q = *reinterpret_cast<const float4*>(row + i);
-            take(q.x, i); take(q.y, i + 1); take(q.z, i + 2); take(q.w, i + 3);
-        }
-    } else {
-        for (int i = lo; i < hi; ++i) take(row[i], i);
-    }
-    float incl = local;
+}
+
+// Kept mass of the `per` slices from `first` on, in vocabulary order: thread t owns a contiguous chunk of each.  On return
+// s_incl[sl][t] is slice first + sl's kept mass up to the end of thread t's chunk, s_last[sl] its last kept token (-1: none).  (The
+// slices side by side: one after the other, each with its own barriers, four of 16,032 tokens took 12 us.)
+__device__ void slices_scan(const float* row, int V, int S, int first, int per, uint32_t tau, float m, float inv_t, float (*s_scan)[SAMPLE_THREADS / 32],
+                            float (*s_incl)[SAMPLE_THREADS], int* s_last) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float incl[SAMPLE_SLICES];
+    int last_kept[SAMPLE_SLICES];
+    __syncthreads();                                       // the previous use of the shared arrays is over
+    if (tid < per) s_last[tid] = -1;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float n = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += n;
+    for (int sl = 0; sl < SAMPLE_SLICES; ++sl) {
+        if (sl >= per) break;
+        const int lo_s = min(V, (first + sl) * S), hi_s = min(V, lo_s + S);
+        int lo, hi, last = -1;
+        slice_chunk(lo_s, hi_s, tid, lo, hi);
+        float local = 0.f;
+        auto take = [&](float v, int i) {
+            if (order_key(v) >= tau && !(v != v)) { local += expf((v - m) * inv_t); last = i; }
+        };
+        if (((lo | hi) & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+#pragma unroll 4
+            for (int i = lo; i < hi; i += 4) {
+                const float4 q = *reinterpret_cast<const float4*>(row + i);
+                take(q.x, i); take(q.y, i + 1); take(q.z, i + 2); take(q.w, i + 3);
+            }
+        } else {
+            for (int i = lo; i < hi; ++i) take(row[i], i);
+        }
+        float in = local;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float n = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o) in += n;
+        }
+        if (lane == 31) s_scan[sl][warp] = in;
+        incl[sl] = in;
+        last_kept[sl] = last;
     }
-    __syncthreads();                                   // the previous use of the shared arrays is over
-    if (tid == 0) *s_last = -1;
-    if (lane == 31) s_scan[warp] = incl;
     __syncthreads();
-    if (last_kept >= 0) atomicMax(s_last, last_kept);
-    if (warp == 0) {
-        const int nw = SAMPLE_THREADS >> 5;
-        float w = lane < nw ? s_scan[lane] : 0.f;
+#pragma unroll
+    for (int sl = 0; sl < SAMPLE_SLICES; ++sl)
+        if (sl < per && last_kept[sl] >= 0) atomicMax(&s_last[sl], last_kept[sl]);
+    if (warp < per) {
+        static_assert(SAMPLE_THREADS / 32 == 32, "a warp adds up the warps of a slice");
+        const float w = s_scan[warp][lane];
         float wi = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float n = __shfl_up_sync(0xffffffffu, wi, o);
             if (lane >= o) wi += n;
         }
-        if (lane < nw) s_scan[lane] = wi - w;          // exclusive prefix of the warp
+        s_scan[warp][lane] = wi - w;                       // exclusive prefix of the warps
     }
     __syncthreads();
     // inclusive prefixes in shared memory, so that neighbouring chunks tile [0, kept mass)
     // without gaps or overlaps whatever the rounding
-    s_incl[tid] = s_scan[warp] + incl;
+#pragma unroll
+    for (int sl = 0; sl < SAMPLE_SLICES; ++sl)
+        if (sl < per) s_incl[sl][tid] = s_scan[sl][warp] + incl[sl];
     __syncthreads();
-    excl = tid > 0 ? s_incl[tid - 1] : 0.f;
-    upto = s_incl[tid];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -209,28 +161,75 @@ __device__ __forceinline__ void slice_scan(const float* row, int lo_s, int hi_s,
 
 __device__ __forceinline__ void sc_red_add(uint32_t addr, unsigned int v) { asm volatile("red.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void sc_red_add(uint32_t addr, unsigned long long v) { asm volatile("red.shared::cluster.add.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
-__device__ __forceinline__ unsigned int sc_atom_add(uint32_t addr, unsigned int v) {
-    unsigned int old;
-    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
-    return old;
-}
 __device__ __forceinline__ void sc_store(uint32_t addr, unsigned long long v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
 __device__ __forceinline__ float key_value(uint32_t key) {
     return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
 }
 
-// Bitonic sort of n_pad (a power of two, <= 2 * SAMPLE_THREADS) 64-bit keys in shared memory, descending.
+__device__ __forceinline__ unsigned long long sort_keep(unsigned long long x, unsigned long long y, bool larger) { return (x > y) == larger ? x : y; }
+
+// Bitonic sort of n_pad (a power of two, SORT_LEAST ... FAST_CANDIDATES) 64-bit keys in shared memory, descending: eight neighbouring
+// keys a thread, so that most pairs meet in a thread's registers or by shuffles, and only those 256 and more apart through
+// shared memory, behind a barrier of the few warps that take part.  (A key a thread, every pair through shared memory behind a barrier of
+// 1,024 threads: 64 keys 3.5 us, 1,024 keys 11; with shuffles within a warp 1,024 still 8.5.)
+#define SORT_LEAST 256
 __device__ void sort_desc(unsigned long long* a, int n_pad) {
-    for (int k = 2; k <= n_pad; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int t = threadIdx.x; t < n_pad / 2; t += SAMPLE_THREADS) {
-                const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i | j;          // the pair (i, i + j)
-                const bool desc = (i & k) == 0;
-                const unsigned long long x = a[i], y = a[l];
-                if ((x < y) == desc) { a[i] = y; a[l] = x; }
+    const int t = threadIdx.x, threads = n_pad / 8;
+    if (t < threads) {                                     // (whole warps)
+        unsigned long long x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = a[8 * t + e];
+        auto in_thread = [&](int j, auto&& down) {          // pairs j < 8 apart
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if ((e & j) == 0 && (x[e] < x[e | j]) == down(e)) { const unsigned long long s = x[e]; x[e] = x[e | j]; x[e | j] = s; }
+        };
+        in_thread(1, [](int e) { return (e & 2) == 0; });
+        in_thread(2, [](int e) { return (e & 4) == 0; });
+        in_thread(1, [](int e) { return (e & 4) == 0; });
+        for (int k = 8; k <= n_pad; k <<= 1) {
+            const bool is_down = ((8 * t) & k) == 0;
+            auto down = [&](int) { return is_down; };
+            int j = k >> 1;
+            for (; j >= 256; j >>= 1) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) a[8 * t + e] = x[e];
+                asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory");
+                const int other = 8 * (t ^ (j >> 3));
+                const bool larger = ((8 * t & j) == 0) == is_down;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = sort_keep(x[e], a[other + e], larger);
+                asm volatile("bar.sync 1, %0;" :: "r"(threads) : "memory");
             }
-            __syncthreads();
+            for (; j >= 8; j >>= 1) {
+                const bool larger = ((8 * t & j) == 0) == is_down;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = sort_keep(x[e], __shfl_xor_sync(0xffffffffu, x[e], j >> 3), larger);
+            }
+            in_thread(4, down);
+            in_thread(2, down);
+            in_thread(1, down);
         }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[8 * t + e] = x[e];
+    }
+    __syncthreads();
+}
+
+// The same for 64 keys of one warp: keys l and l + 32 of lane l.
+__device__ __forceinline__ void sort_desc_64(unsigned long long& x, unsigned long long& y) {
+    const int l = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 64; k <<= 1) {
+        const bool up_x = (l & k) == 0, up_y = ((l + 32) & k) == 0;
+        if (k == 64 && x < y) { const unsigned long long s = x; x = y; y = s; }
+#pragma unroll
+        for (int j = k == 64 ? 16 : k >> 1; j > 0; j >>= 1) {
+            const bool first = (l & j) == 0;
+            x = sort_keep(x, __shfl_xor_sync(0xffffffffu, x, j), first == up_x);
+            y = sort_keep(y, __shfl_xor_sync(0xffffffffu, y, j), first == up_y);
+        }
+    }
 }
 
 // Inclusive sums of n (<= 2 * SAMPLE_THREADS) floats in shared memory, in place, in index order: thread t owns
@@ -271,11 +270,89 @@ struct FastShared {
     unsigned long long z_q;     // the row's whole mass, fixed point
 };
 
+// `scan_inclusive` of 64 floats by one warp, in the same order: lane l owns elements 2l (x0) and 2l + 1 (x1).
+__device__ __forceinline__ void scan_inclusive_64(float& x0, float& x1) {
+    const int lane = threadIdx.x & 31;
+    const float pair = x0 + x1;
+    float incl = pair;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const float all = __shfl_sync(0xffffffffu, incl, 31);
+    const float before = (all - all) + incl - pair;
+    x1 = before + x0 + x1;
+    x0 = before + x0;
+}
+
+// `short_way_finish` for at most 64 candidates: one warp, nothing to wait for (the same sums in the same order).
+__device__ void short_way_finish_64(unsigned long long* cand, int n, float m, float inv_t, int k, float pp, bool use_k, bool use_p,
+                                    unsigned long long seed, long long draw, int* out_token, unsigned long long z_q) {
+    const int lane = threadIdx.x & 31;
+    auto relay = [&](unsigned long long& x, unsigned long long& y) {     // from keys l and l + 32 to keys 2l and 2l + 1
+        cand[lane] = x; cand[lane + 32] = y;
+        __syncwarp();
+        x = cand[2 * lane]; y = cand[2 * lane + 1];
+        __syncwarp();
+    };
+    unsigned long long x = lane < n ? cand[lane] : 0ull, y = lane + 32 < n ? cand[lane + 32] : 0ull;
+    __syncwarp();
+    sort_desc_64(x, y);
+    relay(x, y);
+    auto mass = [&](unsigned long long c) { return expf((key_value((uint32_t)(c >> 32)) - m) * inv_t); };
+    const bool hx = 2 * lane < n, hy = 2 * lane + 1 < n;
+    const float mx = hx ? mass(x) : 0.f, my = hy ? mass(y) : 0.f;
+    float sx = mx, sy = my;
+    scan_inclusive_64(sx, sy);
+    uint32_t tau = 0u;
+    if (use_k) {
+        const int at = min(k, n) - 1;
+        const uint32_t kx = __shfl_sync(0xffffffffu, (uint32_t)(x >> 32), at >> 1), ky = __shfl_sync(0xffffffffu, (uint32_t)(y >> 32), at >> 1);
+        tau = at & 1 ? ky : kx;
+    }
+    if (use_p) {
+        const float target = pp * (float)((double)z_q * (1.0 / (double)FAST_SCALE));
+        const float before = __shfl_up_sync(0xffffffffu, sy, 1);
+        const unsigned int ox = __ballot_sync(0xffffffffu, hx && sx >= target && (lane == 0 || before < target));
+        const unsigned int oy = __ballot_sync(0xffffffffu, hy && sy >= target && sx < target);
+        const int lx = ox ? __ffs(ox) - 1 : 32, ly = oy ? __ffs(oy) - 1 : 32;
+        const uint32_t kx = __shfl_sync(0xffffffffu, (uint32_t)(x >> 32), lx & 31), ky = __shfl_sync(0xffffffffu, (uint32_t)(y >> 32), ly & 31);
+        if (lx < 32 && lx <= ly) tau = max(tau, kx);
+        else if (ly < 32) tau = max(tau, ky);
+    }
+    // kept: the candidates whose value is at least the threshold - a prefix of the sorted list; back into vocabulary order
+    const bool kept_x = hx && (uint32_t)(x >> 32) >= tau, kept_y = hy && (uint32_t)(y >> 32) >= tau;
+    const int L = __popc(__ballot_sync(0xffffffffu, kept_x)) + __popc(__ballot_sync(0xffffffffu, kept_y));
+    x = kept_x ? ((unsigned long long)(uint32_t)x << 32) | (unsigned long long)__float_as_uint(mx) : 0ull;
+    y = kept_y ? ((unsigned long long)(uint32_t)y << 32) | (unsigned long long)__float_as_uint(my) : 0ull;
+    sort_desc_64(x, y);
+    relay(x, y);
+    sx = 2 * lane < L ? __uint_as_float((uint32_t)x) : 0.f;
+    sy = 2 * lane + 1 < L ? __uint_as_float((uint32_t)y) : 0.f;
+    scan_inclusive_64(sx, sy);
+    uint32_t c4[4] = {(uint32_t)(draw & 0xffffffffll), (uint32_t)((unsigned long long)draw >> 32), 0u, 0u};
+    philox4x32_10(c4, (uint32_t)(seed & 0xffffffffull), (uint32_t)(seed >> 32));
+    const float u = (float)(c4[0] >> 8) * (1.0f / 16777216.0f);
+    const float all_x = __shfl_sync(0xffffffffu, sx, (L - 1) >> 1), all_y = __shfl_sync(0xffffffffu, sy, (L - 1) >> 1);
+    const float t_draw = u * ((L - 1) & 1 ? all_y : all_x);
+    const float before = __shfl_up_sync(0xffffffffu, sy, 1);
+    const unsigned int ox = __ballot_sync(0xffffffffu, 2 * lane < L && sx > t_draw && (lane == 0 || before <= t_draw));
+    const unsigned int oy = __ballot_sync(0xffffffffu, 2 * lane + 1 < L && sy > t_draw && sx <= t_draw);
+    int pick = L - 1;                                     // rounding put the target at the kept mass: the last kept token
+    if (ox || oy) {
+        const int px = ox ? 2 * (__ffs(ox) - 1) : 64, py = oy ? 2 * (__ffs(oy) - 1) + 1 : 64;
+        pick = min(px, py);
+    }
+    const uint32_t ix = __shfl_sync(0xffffffffu, (uint32_t)(x >> 32), pick >> 1), iy = __shfl_sync(0xffffffffu, (uint32_t)(y >> 32), pick >> 1);
+    if (lane == 0) *out_token = (int)(0xffffffffu - (pick & 1 ? iy : ix));
+}
+
 // The first CTA's end of the short way: sort the gathered candidates, cut by count and by mass, draw.
 __device__ void short_way_finish(unsigned long long* cand, float* cmass, int n, float m, float inv_t, int k, float pp, bool use_k,
                                  bool use_p, unsigned long long seed, long long draw, int* out_token, float* s_scan, FastShared* fs) {
     const int tid = threadIdx.x;
-    int n_pad = 2;
+    int n_pad = SORT_LEAST;
     while (n_pad < n) n_pad <<= 1;
     for (int i = n + tid; i < n_pad; i += SAMPLE_THREADS) cand[i] = 0ull;       // sorts behind every candidate
     __syncthreads();
@@ -304,7 +381,7 @@ __device__ void short_way_finish(unsigned long long* cand, float* cmass, int n, 
     __syncthreads();
     const int L = fs->kept;
     // back into vocabulary order: (index, mass bits), ascending = descending of the complement
-    int l_pad = 2;
+    int l_pad = SORT_LEAST;
     while (l_pad < L) l_pad <<= 1;
     for (int i = tid; i < l_pad; i += SAMPLE_THREADS) {
         unsigned long long w = 0ull;
@@ -480,8 +557,9 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
     if (!fs->go) return false;
     // ---- pass B: candidates to the first CTA; the whole mass, if a top-p cut wants it
     {
+        // (gathered in the CTA's own memory: a count in another CTA's kept the warp waiting most of a microsecond for every
+        // word with a candidate in it)
         const uint32_t bin = (uint32_t)fs->bin;
-        const uint32_t cnt_addr = sc_map(&fs->n_cand, 0), cand_addr = sc_map(cand, 0);
         unsigned long long z = 0ull;
         sample_walk(row, lo, hi, [&](float v, int i) {
             if (v != v) return;
@@ -490,9 +568,9 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
             if ((key >> 20) >= bin) {
                 const unsigned int now = __activemask(), first = __ffs(now) - 1;       // one add for the lanes that are here together
                 unsigned int pos = 0u;
-                if (lane == (int)first) pos = sc_atom_add(cnt_addr, __popc(now));
+                if (lane == (int)first) pos = atomicAdd(&fs->n_cand, __popc(now));
                 pos = __shfl_sync(now, pos, first) + __popc(now & ((1u << lane) - 1u));
-                if (pos < FAST_CANDIDATES) sc_store(cand_addr + pos * 8u, ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i));
+                if (pos < FAST_CANDIDATES) cand[pos] = ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i);
             }
         });
         if (use_p) {
@@ -501,9 +579,24 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
             if (lane == 0) sc_red_add(sc_map(&fs->z_q, 0), z);
         }
     }
-    sc_sync();
     int n = 0;
-    if (rank == 0) n = (int)min(fs->n_cand, (unsigned int)FAST_CANDIDATES);
+    if (CL > 1) {                                         // the CTAs' candidates side by side in the first CTA's memory
+        __shared__ unsigned int x_cnt[8];
+        __syncthreads();
+        if (tid < CL) sc_store(sc_map(&x_cnt[rank], tid), (int)fs->n_cand);
+        sc_sync();
+        unsigned int base = 0u, all = 0u;
+        for (int c = 0; c < CL; ++c) { if (c < rank) base += x_cnt[c]; all += x_cnt[c]; }
+        if (rank != 0) {
+            const uint32_t to = sc_map(cand, 0);
+            for (unsigned int i = tid; i < x_cnt[rank] && base + i < FAST_CANDIDATES; i += SAMPLE_THREADS) sc_store(to + (base + i) * 8u, cand[i]);
+        }
+        if (rank == 0) n = (int)min(all, (unsigned int)FAST_CANDIDATES);
+        sc_sync();
+    } else {
+        __syncthreads();
+        n = (int)min(fs->n_cand, (unsigned int)FAST_CANDIDATES);
+    }
     if (!use_k) {
         // ---- the bin in which the candidates' masses, from the top down, reach top_p x the whole mass
         if (rank == 0) {
@@ -546,7 +639,6 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
             if (tid == 0 && m == INFINITY) s_bp = fs->z_q ? (int)(order_key(INFINITY) >> 20) : -1;
             __syncthreads();
             // candidates below that bin are none: the others close ranks (what is sorted is what a cut can keep)
-            static_assert(FAST_CANDIDATES <= 2 * SAMPLE_THREADS, "a thread holds two candidates");
             unsigned long long own[2] = {tid < n ? cand[tid] : 0ull, tid + SAMPLE_THREADS < n ? cand[tid + SAMPLE_THREADS] : 0ull};
             __syncthreads();
 #pragma unroll
@@ -565,6 +657,10 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
         if (!fs->go) return false;                         // (not reached, or rounding keeps the mass below the target)
     }
     if (rank != 0) return true;                           // the first CTA finishes the row; nobody's shared memory is touched from outside any more
+    if (n <= 64) {
+        if (warp == 0) short_way_finish_64(cand, n, m, inv_t, k, pp, use_k, use_p, seed, draw, out_token, fs->z_q);
+        return true;
+    }
     short_way_finish(cand, cmass, n, m, inv_t, k, pp, use_k, use_p, seed, draw, out_token, s_scan, fs);
     return true;
 }
@@ -607,8 +703,8 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     __shared__ float s_val[33];
     __shared__ int s_idx[33];
     __shared__ float s_scan[SAMPLE_THREADS / 32 + 1];
-    __shared__ int s_result, s_last;
-    __shared__ float s_incl[SAMPLE_THREADS];
+    __shared__ int s_result, s_last[SAMPLE_SLICES];
+    __shared__ float s_incl[SAMPLE_SLICES][SAMPLE_THREADS], s_warps[SAMPLE_SLICES][SAMPLE_THREADS / 32];
     __shared__ int s_cnt[2][16];
     __shared__ float s_mass[2][16];
     __shared__ SampleExchange xch[2];
@@ -644,19 +740,32 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
         }
     }
     if (!have_max) {
-    // ---- arg-max of the row
-    for (int sl = first; sl < first + per; ++sl) {
-        const int lo_s = min(V, sl * S), n_s = min(V, lo_s + S) - lo_s;
-        int bi = lo_s;
-        float bv = -INFINITY;
-        if (n_s > 0) { bi = lo_s + block_argmax(row + lo_s, n_s, s_val, s_idx); bv = s_val[0]; }
-        if (tid < CL) {
-            sc_store(sc_map(&xch[turn].val[sl], tid), bv);
-            sc_store(sc_map(&xch[turn].idx[sl], tid), bi);
+    // ---- arg-max of the row: this CTA's slices lie side by side
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+    sample_walk(row, min(V, first * S), min(V, (first + per) * S), [&](float v, int i) {
+        if (v > bv) { bv = v; bi = i; }                   // indices rise within a thread; NaN compares false
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        argmax_combine(bv, bi, ov, oi);
+    }
+    if (lane == 0) { s_val[warp] = bv; s_idx[warp] = bi; }
+    __syncthreads();
+    if (warp == 0) {
+        bv = s_val[lane]; bi = s_idx[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            argmax_combine(bv, bi, ov, oi);
         }
+        if (lane < CL) { sc_store(sc_map(&xch[turn].val[rank], lane), bv); sc_store(sc_map(&xch[turn].idx[rank], lane), bi); }
     }
     sc_sync();
-    for (int sl = 0; sl < SAMPLE_SLICES; ++sl) argmax_combine(m, best, xch[turn].val[sl], xch[turn].idx[sl]);   // larger value, then lower index
+    for (int c = 0; c < CL; ++c) argmax_combine(m, best, xch[turn].val[c], xch[turn].idx[c]);   // larger value, then lower index
     if (best == 0x7fffffff) best = 0;
     turn ^= 1;
     }
@@ -780,15 +889,11 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     }
 
     // ---- kept mass and last kept token of every slice, to every CTA
-    int lo, hi, last_kept;
-    float excl, upto;
-    for (int sl = first; sl < first + per; ++sl) {
-        const int lo_s = min(V, sl * S), hi_s = min(V, lo_s + S);
-        slice_scan(row, lo_s, hi_s, tau, m, inv_t, s_scan, s_incl, &s_last, lo, hi, last_kept, excl, upto);
-        if (tid < CL) {
-            sc_store(sc_map(&xch[turn].val[sl], tid), s_incl[SAMPLE_THREADS - 1]);
-            sc_store(sc_map(&xch[turn].idx[sl], tid), s_last);
-        }
+    slices_scan(row, V, S, first, per, tau, m, inv_t, s_warps, s_incl, s_last);
+    for (int i = tid; i < per * CL; i += SAMPLE_THREADS) {
+        const int sl = i % per, to = i / per;
+        sc_store(sc_map(&xch[turn].val[first + sl], to), s_incl[sl][SAMPLE_THREADS - 1]);
+        sc_store(sc_map(&xch[turn].idx[first + sl], to), s_last[sl]);
     }
     sc_sync();
     float kept_total = 0.f;
@@ -821,26 +926,33 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     }
     if (resp / per != rank) return;                       // (nothing of another CTA is touched after the barrier above)
     {
-        const int lo_s = min(V, resp * S), hi_s = min(V, lo_s + S);
-        slice_scan(row, lo_s, hi_s, tau, m, inv_t, s_scan, s_incl, &s_last, lo, hi, last_kept, excl, upto);
+        const int own = resp - first, lo_s = min(V, resp * S), hi_s = min(V, lo_s + S);
         if (tid == 0) s_result = -1;
         __syncthreads();
-        const float t_loc = target - resp_off;
+        const float t_loc = target - resp_off, excl = tid > 0 ? s_incl[own][tid - 1] : 0.f, upto = s_incl[own][tid];
         if (!beyond && upto > excl && excl <= t_loc && t_loc < upto) {
+            int lo, hi;
+            slice_chunk(lo_s, hi_s, tid, lo, hi);
             float run = excl;
-            int pick = last_kept;
-            for (int i = lo; i < hi; ++i) {
-                const float v = row[i];
-                if (order_key(v) >= tau && !(v != v)) {
-                    run += expf((v - m) * inv_t);
-                    if (run > t_loc) { pick = i; break; }
+            int pick = -1;
+            bool found = false;
+            for (int i0 = lo; i0 < hi && !found; i0 += 16) {             // sixteen values in flight: one thread does this, the others wait
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = i0 + j < hi ? row[i0 + j] : __int_as_float(0x7fc00000);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (found || order_key(v[j]) < tau || v[j] != v[j]) continue;
+                    run += expf((v[j] - m) * inv_t);
+                    pick = i0 + j;                        // (none passes it, by rounding: the chunk's last kept token)
+                    found = run > t_loc;
                 }
             }
             atomicMax(&s_result, pick);   // at most one thread matches; max is only a tie guard
         }
         __syncthreads();
         // no chunk took it (rounding): the last kept token of the slice
-        if (tid == 0) out[r] = s_result >= 0 ? s_result : (s_last >= 0 ? s_last : best);
+        if (tid == 0) out[r] = s_result >= 0 ? s_result : (s_last[own] >= 0 ? s_last[own] : best);
     }
 }
 

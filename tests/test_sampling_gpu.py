@@ -182,3 +182,24 @@ def test_parameters_that_travel_with_the_launch(K, rows):
     assert torch.equal(Sampler(K).sample(logits, params, seeds, draws), want)
     with pytest.raises(OverflowError):
         Sampler(K).sample(logits, [kinds[0]] * rows, [2 ** 63] * rows, draws)
+
+
+@pytest.mark.parametrize("top_k", [1, 2, 31, 32, 33, 63, 64, 65, 128, 1023, 1024, 1025, 2047, 2048])
+@pytest.mark.parametrize("top_p", [1.0, 0.6])
+def test_numbers_of_candidates(K, top_k, top_p):
+    """As many candidates as a warp, a block or two a thread sort, and one fewer or more (all values differ, a bin's own tokens
+    come along): what the general search draws."""
+    from ctypes import c_int
+    V, R = 9001, 40
+    x = (torch.randperm(V * R, generator=torch.Generator().manual_seed(top_k)).view(R, V).double() / (V * R) * 9 - 4.5).float().cuda()
+    args = (x, torch.full((R,), 1.3).cuda(), torch.full((R,), top_k, dtype=torch.int32).cuda(), torch.full((R,), top_p).cuda() if top_p < 1 else None,
+            torch.arange(R).cuda(), torch.arange(R).cuda() * 11)
+    lib = K._lib("sampling.cu")
+    got = K.sample(*args)
+    try:
+        assert lib.rv_sample_set_short_way(c_int(0)) == 0
+        want = K.sample(*args)
+    finally:
+        assert lib.rv_sample_set_short_way(c_int(1)) == 0
+    # the masses are added in another order: a draw within a few 2^-24 of a token's edge may take its neighbour
+    assert int((got != want).sum()) <= 1
