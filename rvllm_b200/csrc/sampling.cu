@@ -433,6 +433,35 @@ __device__ __forceinline__ void sample_walk(const float* __restrict__ row, int l
     for (int i = lo + threadIdx.x; i < hi; i += SAMPLE_THREADS) f(row[i], i);
 }
 
+// The CTAs' candidates (n_cand of them in `cand`, at most FAST_CANDIDATES in all) side by side in the first CTA's memory; it gets their number,
+// the others 0.
+__device__ __forceinline__ int gather_in_first(unsigned long long* cand, const unsigned int* n_cand, int CL, int rank) {
+    __shared__ unsigned int x_cnt[8];
+    const int tid = threadIdx.x;
+    __syncthreads();
+    if (CL == 1) return (int)min(*n_cand, (unsigned int)FAST_CANDIDATES);
+    if (tid < CL) sc_store(sc_map(&x_cnt[rank], tid), (int)*n_cand);
+    sc_sync();
+    unsigned int base = 0u, all = 0u;
+    for (int c = 0; c < CL; ++c) { if (c < rank) base += x_cnt[c]; all += x_cnt[c]; }
+    if (rank != 0) {
+        const uint32_t to = sc_map(cand, 0);
+        for (unsigned int i = tid; i < x_cnt[rank] && base + i < FAST_CANDIDATES; i += SAMPLE_THREADS) sc_store(to + (base + i) * 8u, cand[i]);
+    }
+    sc_sync();
+    return rank == 0 ? (int)min(all, (unsigned int)FAST_CANDIDATES) : 0;
+}
+
+// A token among the candidates of this CTA.  (Gathered in the CTA's own memory: a count in another CTA's kept the warp waiting.)
+__device__ __forceinline__ void gather_one(unsigned long long* cand, unsigned int* n_cand, uint32_t key, int i) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int now = __activemask(), first = __ffs(now) - 1;           // one add for the lanes that are here together
+    unsigned int pos = 0u;
+    if (lane == (int)first) pos = atomicAdd(n_cand, __popc(now));
+    pos = __shfl_sync(now, pos, first) + __popc(now & ((1u << lane) - 1u));
+    if (pos < FAST_CANDIDATES) cand[pos] = ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i);
+}
+
 // The short way: TWO passes over the row.  Pass A finds the row's maximum (larger value, then lower index - the same whatever
 // the order) and counts the tokens per bin; no exponential, no mass.  With a top-k the bin of the k-th token follows from the
 // counts alone; with a top-p alone, pass B takes the tokens of as many bins from the top as hold at most FAST_CANDIDATES.
@@ -557,21 +586,13 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
     if (!fs->go) return false;
     // ---- pass B: candidates to the first CTA; the whole mass, if a top-p cut wants it
     {
-        // (gathered in the CTA's own memory: a count in another CTA's kept the warp waiting most of a microsecond for every
-        // word with a candidate in it)
         const uint32_t bin = (uint32_t)fs->bin;
         unsigned long long z = 0ull;
         sample_walk(row, lo, hi, [&](float v, int i) {
             if (v != v) return;
             const uint32_t key = order_key(v);
             if (use_p) z += __float2ull_rz(expf((v - m) * inv_t) * FAST_SCALE);
-            if ((key >> 20) >= bin) {
-                const unsigned int now = __activemask(), first = __ffs(now) - 1;       // one add for the lanes that are here together
-                unsigned int pos = 0u;
-                if (lane == (int)first) pos = atomicAdd(&fs->n_cand, __popc(now));
-                pos = __shfl_sync(now, pos, first) + __popc(now & ((1u << lane) - 1u));
-                if (pos < FAST_CANDIDATES) cand[pos] = ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)i);
-            }
+            if ((key >> 20) >= bin) gather_one(cand, &fs->n_cand, key, i);
         });
         if (use_p) {
 #pragma unroll
@@ -579,24 +600,7 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
             if (lane == 0) sc_red_add(sc_map(&fs->z_q, 0), z);
         }
     }
-    int n = 0;
-    if (CL > 1) {                                         // the CTAs' candidates side by side in the first CTA's memory
-        __shared__ unsigned int x_cnt[8];
-        __syncthreads();
-        if (tid < CL) sc_store(sc_map(&x_cnt[rank], tid), (int)fs->n_cand);
-        sc_sync();
-        unsigned int base = 0u, all = 0u;
-        for (int c = 0; c < CL; ++c) { if (c < rank) base += x_cnt[c]; all += x_cnt[c]; }
-        if (rank != 0) {
-            const uint32_t to = sc_map(cand, 0);
-            for (unsigned int i = tid; i < x_cnt[rank] && base + i < FAST_CANDIDATES; i += SAMPLE_THREADS) sc_store(to + (base + i) * 8u, cand[i]);
-        }
-        if (rank == 0) n = (int)min(all, (unsigned int)FAST_CANDIDATES);
-        sc_sync();
-    } else {
-        __syncthreads();
-        n = (int)min(fs->n_cand, (unsigned int)FAST_CANDIDATES);
-    }
+    int n = gather_in_first(cand, &fs->n_cand, CL, rank);
     if (!use_k) {
         // ---- the bin in which the candidates' masses, from the top down, reach top_p x the whole mass
         if (rank == 0) {
@@ -665,6 +669,170 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
     return true;
 }
 
+// The threshold of a top-p alone whose cut lies below FAST_CANDIDATES tokens (a flat row): the key tau with
+// mass(key >= tau) >= top_p x (the whole mass) > mass(key > tau), masses as 40-bit fixed-point integers.  One pass adds up the masses (and
+// counts) of 16 groups of neighbouring bins, each about a sixteenth of the tokens by the histogram that the short way left in the
+// first CTA; a group of more than FAST_CANDIDATES tokens is divided again, by key; the tokens of the last group are gathered, sorted and
+// cut.  Every thread adds in places of its own (16 sums of 64 bits, the count above the mass), so nothing is atomic and the sums
+// are exact.  Three passes over the row in place of the search's eight: a step of 64 rows
+// of 128,256 tokens with one such row 212 -> 117 us, 36 without.
+#define MASS_GROUPS 16
+#define MASS_BITS 52                       // of a thread's sum: 4,096 masses of 2^40; the count above
+struct MassShared {
+    unsigned long long mass[2][MASS_GROUPS];               // of the row's groups; two copies, used in turn
+    unsigned int count[2][MASS_GROUPS];
+    unsigned int group_of[FAST_BINS / 4];                  // per bin, a byte each (255: no token)
+    uint32_t lo, hi, tau;
+};
+
+__device__ bool sample_mass_way(const float* __restrict__ row, int V, float inv_t, float pp, float m, unsigned char* s_dyn, float* s_scan,
+                                FastShared* fs, MassShared* ms, uint32_t& tau) {
+    const int CL = gridDim.x, rank = (int)sc_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int per = (((V + CL - 1) / CL) + 3) & ~3;
+    const int lo_v = min(V, rank * per), hi_v = min(V, lo_v + per);
+    if (per > (SAMPLE_THREADS << 11) || !(fabsf(m) < INFINITY)) return false;  // (every CTA alike)
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(s_dyn);  // [MASS_GROUPS][SAMPLE_THREADS]
+    unsigned long long* cand = slots;                                           // later
+    if (tid < 2 * MASS_GROUPS) { ms->mass[tid / MASS_GROUPS][tid % MASS_GROUPS] = 0ull; ms->count[tid / MASS_GROUPS][tid % MASS_GROUPS] = 0u; }
+    if (tid == 0) { ms->lo = 0xffffffffu; ms->hi = 0u; fs->n_cand = 0u; }
+    __syncthreads();
+    sc_sync();                                             // (every CTA's places are zero)
+    if (rank == 0) {
+        // the group of a bin, by the tokens above it: thread t owns the bins 4095 - 4t ... 4092 - 4t
+        const unsigned int* h_cnt = reinterpret_cast<const unsigned int*>(s_dyn);
+        unsigned int* w_cnt = reinterpret_cast<unsigned int*>(s_scan);
+        unsigned int own = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) own += h_cnt[FAST_BINS - 1 - 4 * tid - j];
+        unsigned int inc = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const unsigned int v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
+        if (lane == 31) w_cnt[warp] = inc;
+        __syncthreads();
+        unsigned int run = inc - own, all = 0u;
+        for (int w = 0; w < SAMPLE_THREADS / 32; ++w) { if (w < warp) run += w_cnt[w]; all += w_cnt[w]; }
+        unsigned int word = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned int g = (unsigned int)(((unsigned long long)run * MASS_GROUPS) / max(all, 1u));
+            const unsigned int c = h_cnt[FAST_BINS - 1 - 4 * tid - j];
+            word |= (c ? min(g, MASS_GROUPS - 1u) : 0xffu) << (8 * (3 - j));          // (empty bins are nobody's: a group's keys are those of its tokens)
+            run += c;
+        }
+        for (int c = 0; c < CL; ++c) sc_store(sc_map(&ms->group_of[FAST_BINS / 4 - 1 - tid], c), (int)word);
+    }
+    sc_sync();                                             // the groups are known; the histogram is read
+    const unsigned char* group_of = reinterpret_cast<const unsigned char*>(ms->group_of);
+    auto clear = [&]() {
+#pragma unroll
+        for (int g = 0; g < MASS_GROUPS; ++g) slots[g * SAMPLE_THREADS + tid] = 0ull;
+    };
+    auto add = [&](int g, float v) {
+        slots[g * SAMPLE_THREADS + tid] += __float2ull_rz(expf((v - m) * inv_t) * FAST_SCALE) + (1ull << MASS_BITS);
+    };
+    auto meet = [&](int turn) {                            // a warp adds up a group and tells every CTA
+        __syncthreads();
+        if (warp < MASS_GROUPS) {
+            unsigned long long mass = 0ull;
+            unsigned int count = 0u;
+            for (int i = lane; i < SAMPLE_THREADS; i += 32) {
+                const unsigned long long v = slots[warp * SAMPLE_THREADS + i];
+                mass += v & ((1ull << MASS_BITS) - 1);
+                count += (unsigned int)(v >> MASS_BITS);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                mass += __shfl_xor_sync(0xffffffffu, mass, o);
+                count += __shfl_xor_sync(0xffffffffu, count, o);
+            }
+            if (lane < CL) { sc_red_add(sc_map(&ms->mass[turn][warp], lane), mass); sc_red_add(sc_map(&ms->count[turn][warp], lane), count); }
+        }
+        sc_sync();
+    };
+    clear();
+    sample_walk(row, lo_v, hi_v, [&](float v, int) {
+        if (v == v) add(group_of[order_key(v) >> 20], v);
+    });
+    meet(0);
+    unsigned long long z = 0ull, above = 0ull;
+    for (int g = 0; g < MASS_GROUPS; ++g) z += ms->mass[0][g];
+    const unsigned long long target = (unsigned long long)((double)pp * (double)z);
+    if (target == 0ull) return false;
+    int g = 0;
+    while (g < MASS_GROUPS - 1 && above + ms->mass[0][g] < target) above += ms->mass[0][g++];
+    unsigned int count = ms->count[0][g];
+    // the group's keys
+    for (int b = tid; b < FAST_BINS; b += SAMPLE_THREADS)
+        if (group_of[b] == g) { atomicMin(&ms->lo, (uint32_t)b << 20); atomicMax(&ms->hi, ((uint32_t)b << 20) | 0xfffffu); }
+    __syncthreads();
+    uint32_t lo = ms->lo, hi = ms->hi;
+    int turn = 0;
+    while (count > FAST_CANDIDATES && hi > lo) {           // (every CTA decides alike)
+        const int shift = max(0, 28 - __clz(hi - lo));     // sixteen parts at most, counted from the top
+        clear();
+        turn ^= 1;
+        if (tid < MASS_GROUPS && turn == 0) { ms->mass[0][tid] = 0ull; ms->count[0][tid] = 0u; }
+        if (turn == 0) sc_sync();                          // (read by everyone, and zero again)
+        sample_walk(row, lo_v, hi_v, [&](float v, int) {
+            if (v != v) return;
+            const uint32_t key = order_key(v);
+            if (key >= lo && key <= hi) add((int)((hi - key) >> shift), v);
+        });
+        meet(turn);
+        g = 0;
+        while (g < MASS_GROUPS - 1 && above + ms->mass[turn][g] < target) above += ms->mass[turn][g++];
+        count = ms->count[turn][g];
+        const uint32_t top = hi - ((uint32_t)g << shift);
+        lo = max(lo, top - min(top, (1u << shift) - 1u));
+        hi = top;
+        if (turn == 1) {                                   // the next turn's places
+            sc_sync();
+            if (tid < MASS_GROUPS) { ms->mass[1][tid] = 0ull; ms->count[1][tid] = 0u; }
+        }
+    }
+    if (count > FAST_CANDIDATES) { tau = hi; return true; }                     // many tokens of one value
+    __syncthreads();
+    sample_walk(row, lo_v, hi_v, [&](float v, int i) {
+        if (v != v) return;
+        const uint32_t key = order_key(v);
+        if (key >= lo && key <= hi) gather_one(cand, &fs->n_cand, key, i);
+    });
+    const int n = gather_in_first(cand, &fs->n_cand, CL, rank);
+    if (rank == 0) {
+        int n_pad = SORT_LEAST;
+        while (n_pad < n) n_pad <<= 1;
+        for (int i = n + tid; i < n_pad; i += SAMPLE_THREADS) cand[i] = 0ull;
+        if (tid == 0) ms->tau = 0u;
+        __syncthreads();
+        sort_desc(cand, n_pad);
+        // the first whose running mass, behind what lies above, reaches the target: thread t owns keys 2t and 2t + 1
+        unsigned long long* w_mass = cand + FAST_CANDIDATES;
+        unsigned long long q[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            q[j] = 2 * tid + j < n ? __float2ull_rz(expf((key_value((uint32_t)(cand[2 * tid + j] >> 32)) - m) * inv_t) * FAST_SCALE) : 0ull;
+        unsigned long long inc = q[0] + q[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
+        if (lane == 31) w_mass[warp] = inc;
+        __syncthreads();
+        unsigned long long run = above + inc - q[0] - q[1];
+        for (int w = 0; w < warp; ++w) run += w_mass[w];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {                      // (exactly one finds it)
+            if (2 * tid + j < n && run < target && run + q[j] >= target) ms->tau = (uint32_t)(cand[2 * tid + j] >> 32);
+            run += q[j];
+        }
+        __syncthreads();
+        const uint32_t found = ms->tau;
+        __syncthreads();
+        if (tid < CL) sc_store(sc_map(&ms->tau, tid), (int)found);
+    }
+    sc_sync();
+    tau = ms->tau;
+    return tau != 0u;
+}
+
 __device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two), 2: rows that need it get -1
 
 // Where a row's parameters are: in arrays on the device (null: greedy, or off), or, for up to SAMPLE_VALUE_ROWS rows whose
@@ -709,6 +877,7 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     __shared__ float s_mass[2][16];
     __shared__ SampleExchange xch[2];
     __shared__ FastShared fast_shared;
+    __shared__ MassShared mass_shared;
     extern __shared__ __align__(16) unsigned char s_dyn_fast[];      // the dynamic shared memory, as the short way lays it out
     // gridDim.x CTAs (1, 2, 4 or 8: the cluster) share row blockIdx.y; this one owns the slices [first, first + per)
     const int CL = gridDim.x, rank = (int)sc_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -726,7 +895,8 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     const float inv_t = fminf(1.0f / T, 3.402823466e38f);      // (a temperature below 2.9e-39 would make the maximum's own mass 0 x infinity)
     float m = -INFINITY;
     int best = 0x7fffffff;
-    bool have_max = false;
+    bool have_max = false, have_tau = false;
+    uint32_t tau = 0;
     if (T > 0.f && (uk_row || up_row) && g_sample_short_way) {
         // maximum, counts and candidates in two passes; too many candidates: the maximum is kept, the search below goes on
         if (sample_short_way(row, V, inv_t, k_row, p_row, uk_row, up_row, rows.seed(r), rows.draw(r), out + r, s_dyn_fast, s_scan,
@@ -738,6 +908,7 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
             if (rank == 0 && tid == 0) out[r] = -1;
             return;
         }
+        if (!uk_row) have_tau = sample_mass_way(row, V, inv_t, p_row, m, s_dyn_fast, s_scan, &fast_shared, &mass_shared, tau);
     }
     if (!have_max) {
     // ---- arg-max of the row: this CTA's slices lie side by side
@@ -776,7 +947,7 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
 
     // ---- mass of everything, where a top-p is measured by it
     float total = 0.f;
-    if (up_row) {
+    if (up_row && !have_tau) {
     for (int sl = first; sl < first + per; ++sl) {
         const int lo_s = min(V, sl * S), hi_s = min(V, lo_s + S);
         float part = 0.f;
@@ -796,12 +967,11 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     // agree with the bits decided so far; the block adds the slots up in a fixed order, the slices'
     // sums are added in slice order, and the largest digit that still satisfies the condition is
     // taken.  No atomics: the same result in every run.  NaN is never kept.
-    uint32_t tau = 0;
     const int k = k_row;
     const float pp = p_row;
     bool use_k = k > 0 && k < V;
     bool use_p = pp < 1.0f;
-    if (use_k || use_p) {
+    if (!have_tau && (use_k || use_p)) {
         extern __shared__ __align__(16) unsigned char s_dyn[];
         int* h_cnt = reinterpret_cast<int*>(s_dyn);                                   // [16][SAMPLE_THREADS]
         float* h_mass = reinterpret_cast<float*>(s_dyn) + 16 * SAMPLE_THREADS;       // [16][SAMPLE_THREADS]

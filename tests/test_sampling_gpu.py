@@ -203,3 +203,35 @@ def test_numbers_of_candidates(K, top_k, top_p):
         assert lib.rv_sample_set_short_way(c_int(1)) == 0
     # the masses are added in another order: a draw within a few 2^-24 of a token's edge may take its neighbour
     assert int((got != want).sum()) <= 1
+
+
+@pytest.mark.parametrize("vocab", [5001, 128256])
+@pytest.mark.parametrize("ctas", [1, 2, 8])
+def test_flat_rows_under_top_p_alone(K, vocab, ctas):
+    """Cuts below the 2,048 most likely tokens: groups of bins, a bin divided by key once and twice, thousands of equal values at the
+    cut, values apart by one bit; what the general search draws."""
+    from ctypes import c_int
+    torch.manual_seed(vocab)
+    kinds = [torch.randn(vocab), torch.randn(vocab) * 0.01 + 5, torch.full((vocab,), -2.5), torch.where(torch.arange(vocab) % 3 == 0, 1.0, 1.25),
+             torch.rand(vocab) * 20, torch.randn(vocab) * 1e-6 + 1, torch.randn(vocab) * 2]
+    kinds[6][::2] = float("nan")
+    kinds[4][5:vocab:7] = float("-inf")
+    x = torch.stack([k for k in kinds for _ in range(4)])
+    R = len(x)
+    ps = torch.tensor([0.6, 0.9, 0.99, 0.9999] * 7)
+    args = (x.cuda(), torch.full((R,), 0.9).cuda(), None, ps.cuda(), torch.arange(R).cuda() + 5, torch.arange(R).cuda())
+    lib = K._lib("sampling.cu")
+    try:
+        lib.rv_sample_set_cluster(c_int(ctas))
+        got = K.sample(*args).tolist()
+        assert lib.rv_sample_set_short_way(c_int(0)) == 0
+        want = K.sample(*args).tolist()
+    finally:
+        assert lib.rv_sample_set_short_way(c_int(1)) == 0
+        lib.rv_sample_set_cluster(c_int(0))
+    # the search adds floats and may cut a token early or late where the mass there is the target's within their rounding; the
+    # token of float64 is then the right one
+    for r in range(R):
+        if got[r] != want[r]:
+            token, margin = P.sample(x[r].nan_to_num(float("-inf")), 0.9, r + 5, r, 0, float(ps[r]))
+            assert got[r] == token or margin < 1e-4, (r, got[r], want[r], token, margin)
