@@ -1223,7 +1223,7 @@ __global__ void __launch_bounds__(256)
 delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
                        int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                        const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ state,
-                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps, int least, int most) {
+                       size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
     using Stage = DeltaStage<PARTS>;
@@ -1233,7 +1233,7 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     const int slot = state_slots[seq];
     if (slot < 0) return;
     const int start = cu_seqlens[seq], n_tok = cu_seqlens[seq + 1] - start;
-    if (n_tok < least || n_tok > most) return;             // (another kernel's)
+    if (n_tok < least) return;                             // (the other kernel's)
     const int chunks = (n_tok + DR_CHUNK - 1) / DR_CHUNK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < 4) {                                        // ---- the walk
@@ -1478,13 +1478,13 @@ delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
 template <int PARTS>
 static int launch_delta_walk(cudaStream_t stream, int n_seqs, int heads, int vd, const void* qkv, int qkv_dtype, int qkv_stride, const float* proj,
                              int proj_stride, int b_col0, int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens,
-                             const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps, int least, int most) {
+                             const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps, int least) {
     constexpr int smem = 2 * (int)sizeof(DeltaStage<PARTS>), cols = DeltaStage<PARTS>::COLS;
     static RvPerDevice once;
     if (int st = rv_configure_smem(once, delta_rule_walk_kernel<PARTS>, smem)) return st;
     return rv_launch(delta_rule_walk_kernel<PARTS>, dim3((vd + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, qkv, qkv_dtype,
                      qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, state_stride, out, heads,
-                     qk_heads, d, vd, unit_eps, least, most);
+                     qk_heads, d, vd, unit_eps, least);
 }
 
 // Whether rows of the state are whole words of four columns.
@@ -1495,14 +1495,13 @@ RV_EXPORT int rv_delta_rule_words(int vd, const float* state, long long state_st
 // qkv rows: [q: qk_heads x d | k: qk_heads x d | v: heads x vd] (after the convolution); the logits of beta and of the
 // decay are float columns b_col0 .. and a_col0 .. of `proj`; out: float [tokens, heads x vd].  For keys of 33 to 128 elements and
 // values and states of whole words of four columns, `which` names the kernel: 1 the one for single tokens, 2 the walk, 3 the first
-// for sequences of up to `short_tokens` tokens and the second for the others (all give the same bits); sequences of more than `most` tokens
-// are left alone (delta_chunk.cu's).
+// for sequences of up to `short_tokens` tokens and the second for the others (all give the same bits).
 RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, const float* proj, int proj_stride, int b_col0,
                             int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens, const int* state_slots,
                             float* state, long long state_stride, float* out, int n_seqs, int heads, int qk_heads, int d, int vd,
-                            float unit_eps, int which, int short_tokens, int most, cudaStream_t stream) {
+                            float unit_eps, int which, int short_tokens, cudaStream_t stream) {
     if (n_seqs < 0 || heads <= 0 || qk_heads <= 0 || heads % qk_heads || d <= 0 || d > 32 * 32 || vd <= 0 || n_seqs > 65535 ||
-        heads > 65535 || which < 1 || which > 3 || most < 0)
+        heads > 65535 || which < 1 || which > 3)
         return RV_ERR_BAD_SIZE;
     const int qk = qk_heads * d;
     if (qkv_stride < 2 * qk + heads * vd || b_col0 < 0 || a_col0 < 0 || b_col0 + heads > proj_stride || a_col0 + heads > proj_stride ||
@@ -1515,16 +1514,15 @@ RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, cons
         if (which & 1)
             RV_LAUNCH_ST = rv_launch(one ? delta_rule_step_kernel<1> : delta_rule_step_kernel<2>, dim3((vd + 127) / 128, heads, n_seqs), dim3(256), 0, stream, qkv, qkv_dtype, qkv_stride, proj,
                                      proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, (size_t)state_stride, out, heads,
-                                     qk_heads, d, vd, unit_eps, which == 1 ? most : min(most, short_tokens));
+                                     qk_heads, d, vd, unit_eps, which == 1 ? 0x7fffffff : short_tokens);
         if (which == 1 || ((which & 1) && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
         const int least = which == 2 ? 0 : short_tokens + 1;
         RV_LAUNCH_ST = d > 64 ? launch_delta_walk<16>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least, most)
+                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least)
                               : launch_delta_walk<8>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least, most);
+                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least);
         return rv_launch_status();
     }
-    if (most != 0x7fffffff) return RV_ERR_UNSUPPORTED;   // (this kernel serves every sequence)
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128
     int parts = 1;
     while (parts * ns < d) parts <<= 1;                // a power of two of at most 32 lanes of one warp

@@ -1337,7 +1337,6 @@ class CudaKernels:
         COUNTERS['launches'] += 1 if which == 3 and N in (16, 32) else 0
         return out
 
-    DELTA_CHUNK_TOKENS = 1 << 30       # tokens of a portion from which the delta rule goes chunk by chunk (delta_chunk.cu)
     DELTA_SHORT_TOKENS = 4             # tokens of a portion up to which the delta rule takes the kernel of single tokens (ssm.cu has both sides)
     DELTA_SHORT_BESIDE = 5             # ... beside the walk in uneven steps of more sequences than this (single tokens beside a portion of
                                        # 64 or 1,500: 3 of them 35.2 and 557 us in two kernels, 34.2 and 542 in one; 6 37.7 and 560, 42.4
@@ -1348,8 +1347,7 @@ class CudaKernels:
         """The gated delta rule over the step's tokens, continued from and leaving behind each request's S ([heads][head_dim]
         [value_dim] at offset 0 of its row of `state`).  qkv rows: [q | k | v] after their convolution; the logits of beta and
         of the decay are float columns b_col0 .. and a_col0 .. of `proj`.  Returns o float32 [T, heads * value_dim].
-        `max_q_len`: the most tokens that any sequence brings (see `_longest`).  bfloat16 portions of `DELTA_CHUNK_TOKENS` tokens and
-        more go chunk by chunk where the sizes allow, each by its own tokens: a request's bits depend on its portions alone."""
+        `max_q_len`: the most tokens that any sequence brings (see `_longest`); the bits do not depend on it."""
         _need(qkv, "qkv", dims=2); _need(proj, "proj", torch.float32, 2); _need(state, "state", torch.float32, 2)
         _need(a_log, "a_log", torch.float32, 1); _need(dt_bias, "dt_bias", torch.float32, 1)
         T = qkv.shape[0]
@@ -1357,23 +1355,12 @@ class CudaKernels:
                 dt_bias.shape[0] != heads:
             raise KernelError("delta_rule: shapes of q | k | v, the logits and the heads' constants do not agree")
         out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=qkv.device)
-        n_seqs, most = state_slots.shape[0], 0x7fffffff
-        if qkv.dtype == torch.bfloat16 and self._longest(T, n_seqs, max_q_len) >= self.DELTA_CHUNK_TOKENS:
-            st = self._lib("delta_chunk.cu").rv_delta_chunk(
-                _ptr(qkv), c_int(qkv.shape[1]), _ptr(proj), c_int(proj.shape[1]), c_int(b_col0), c_int(a_col0), _ptr(a_log), _ptr(dt_bias),
-                _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out), c_int(n_seqs), c_int(heads),
-                c_int(qk_heads), c_int(head_dim), c_int(value_dim), c_float(unit_eps), c_int(self.DELTA_CHUNK_TOKENS), self._stream())
-            if st != -4:                   # (-4: sizes that this kernel does not serve)
-                _check("delta_chunk", st)
-                most = self.DELTA_CHUNK_TOKENS - 1
-                if n_seqs == 1 and T > most:
-                    return out
-        which = self._portion_kernels(T, n_seqs, max_q_len, self.DELTA_SHORT_TOKENS, self.DELTA_SHORT_BESIDE)
+        which = self._portion_kernels(T, state_slots.shape[0], max_q_len, self.DELTA_SHORT_TOKENS, self.DELTA_SHORT_BESIDE)
         st = self._lib("ssm.cu").rv_delta_rule(
             _ptr(qkv), c_int(self._dt(qkv, "qkv")), c_int(qkv.shape[1]), _ptr(proj), c_int(proj.shape[1]), c_int(b_col0), c_int(a_col0),
             _ptr(a_log), _ptr(dt_bias), _ptr(cu_seqlens), _ptr(state_slots), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(out),
-            c_int(n_seqs), c_int(heads), c_int(qk_heads), c_int(head_dim), c_int(value_dim), c_float(unit_eps),
-            c_int(which), c_int(self.DELTA_SHORT_TOKENS), c_int(most), self._stream())
+            c_int(state_slots.shape[0]), c_int(heads), c_int(qk_heads), c_int(head_dim), c_int(value_dim), c_float(unit_eps),
+            c_int(which), c_int(self.DELTA_SHORT_TOKENS), self._stream())
         _check("delta_rule", st)
         if which == 3 and 32 < head_dim <= 128:
             COUNTERS['launches'] += self._lib("ssm.cu").rv_delta_rule_words(c_int(value_dim), _ptr(state), ctypes.c_longlong(state.shape[1]))
