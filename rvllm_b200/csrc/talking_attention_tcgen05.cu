@@ -13,8 +13,8 @@
 //                         384 columns).  U is O over the row's sum of weights, float32.
 //   talking_mix_kernel    out[t, h] = sum_g talk[h, g] U[t][kv(h)][g], float32 sums in the order of g, rounded once.
 //
-// Against the kernel that mixes inside the walk (talking_attention_mma.cu; heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 473 -> 134 us,
-// 80 tokens 32 -> 20, 100 tokens behind 3,990 keys 959 -> 134; 32 heads on 8, 2,048 tokens 974 -> 406, 100 behind 3,990 1,328 -> 138.
+// Against the kernel that mixes inside the walk (talking_attention_mma.cu; heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 473 -> 118 us,
+// 80 tokens 32 -> 20, 100 tokens behind 3,990 keys 959 -> 97; 32 heads on 8, 2,048 tokens 974 -> 392, 100 behind 3,990 1,328 -> 114.
 // Error against float64 2.3e-3 -> 1.9e-3 to 2.3e-3 (2-norms; 1.7e-3 is the rounding of the result).  The walk is bound by the
 // softmax warps, one a scheduler; the products are 1,024 of a tile's cycles at three value heads of 128.
 //
@@ -78,7 +78,9 @@ __device__ __forceinline__ float fast_log2(float x) {
     return y;
 }
 
-template <int HD, int VD>
+// G: heads on one key/value head (a constant, so that the reads of the biases have constant offsets: 64 registers of addresses less; 134
+// -> 118 and 406 -> 392 us)
+template <int HD, int VD, int G>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const WideParams p) {
@@ -103,12 +105,11 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // the row tile is the slowest index, counted down: the tiles with the most keys start first (attention_tcgen05.cu)
     const int kvh = blockIdx.x / p.blocks, c0 = (blockIdx.x % p.blocks) * p.per_block, nv = min(p.per_block, p.nkv - c0);
     const int seq = blockIdx.y, tile_m = gridDim.z - 1 - blockIdx.z;
-    const int G = p.nh / p.nkv;
     rv_pdl_wait();
     const int ctx = p.ctx_lens[seq];
     const int q_start = p.cu_seqlens[seq];
     const int q_len = p.cu_seqlens[seq + 1] - q_start;
-    const int tile_tokens = ROWS / G;
+    constexpr int tile_tokens = ROWS / G;
     const int tok0 = tile_m * tile_tokens, n_tok = min(tile_tokens, q_len - tok0);      // this CTA's tokens of the portion
     if (n_tok <= 0 || q_start + tok0 >= p.tok_hi || q_start + tok0 + n_tok <= p.tok_lo) return;
     if (ctx <= 0) {                                          // padding: its result is zero
@@ -275,12 +276,13 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int lo = p.chunk > 0 && in_range ? (pos / p.chunk) * p.chunk : 0;
         const uint32_t t_lane = tmem_base + ((uint32_t)(warp * 32) << 16);
         // the warp's tokens and their biases of a tile: entry (distance - nearest) * G + head; the rows of a token read neighbours
-        const int w_tok0 = warp * 32 / G, w_toks = 32 / G;   // (G divides 32)
+        const int w_tok0 = warp * 32 / G;
+        constexpr int w_toks = 32 / G, b_step = 32 / G;
         const int w_pos0 = pos_first + w_tok0;               // (also of rows beyond the portion: their scores are masked)
         float* bias = bias_s + warp * BIAS_FLOATS;
         const bool biased = p.r1 != nullptr;
         // distances of a tile at key0: w_pos0 - key0 - 63 ... w_pos0 - key0 + w_toks - 1
-        const int b_head = lane % G, b_step = 32 / G;        // a lane forms the biases of one head
+        const int b_head = lane % G;                         // a lane forms the biases of one head
         const float b_r1 = biased ? -p.r1[kvh * G + b_head] : 0.f, b_r2 = biased ? p.r2[kvh * G + b_head] : 0.f;
         const float* my_bias = bias + (KV_TILE - 1 + tok_i - w_tok0) * G + (row_l - tok_i * G);      // of the tile's first key; a key on is G back
         float m_ref = -INFINITY, l_run = 0.f;
@@ -292,8 +294,11 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (biased) {
                 const int d0 = w_pos0 - key0 - (KV_TILE - 1);
                 __syncwarp();                                // (the tile before has been read)
-                for (int e = lane / G; e < KV_TILE - 1 + w_toks; e += b_step)
-                    bias[e * G + b_head] = b_r1 * fast_log2(fmaf(b_r2, (float)max(d0 + e, 0), 1.0f));
+#pragma unroll
+                for (int e0 = 0; e0 < KV_TILE - 1 + w_toks; e0 += b_step) {
+                    const int e = e0 + lane / G;
+                    if (e < KV_TILE - 1 + w_toks) bias[e * G + b_head] = b_r1 * fast_log2(fmaf(b_r2, (float)max(d0 + e, 0), 1.0f));
+                }
                 __syncwarp();
             }
             if (!mbar_wait(bar_s_full0 + 8 * sb, (it >> 1) & 1, &abort_flag, 9)) { ok = false; break; }
@@ -485,11 +490,22 @@ static int make_query_map(CUtensorMap* map, const void* q, int n_tokens, int nh,
     return r == CUDA_SUCCESS ? RV_OK : RV_ERR_BAD_SIZE;
 }
 
+template <int HD, int VD, int G>
+static int launch_wide_group(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const WideParams& p, dim3 grid, cudaStream_t stream) {
+    static RvPerDevice once;
+    if (int st = rv_configure_smem(once, talking_wide_kernel<HD, VD, G>, WideSizes<HD, VD>::SMEM)) return st;
+    return rv_launch(talking_wide_kernel<HD, VD, G>, grid, dim3(NUM_THREADS), WideSizes<HD, VD>::SMEM, stream, mq, mk, mv, p);
+}
+
 template <int HD, int VD>
 static int launch_wide(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const WideParams& p, dim3 grid, cudaStream_t stream) {
-    static RvPerDevice once;
-    if (int st = rv_configure_smem(once, talking_wide_kernel<HD, VD>, WideSizes<HD, VD>::SMEM)) return st;
-    return rv_launch(talking_wide_kernel<HD, VD>, grid, dim3(NUM_THREADS), WideSizes<HD, VD>::SMEM, stream, mq, mk, mv, p);
+    switch (p.nh / p.nkv) {
+        case 1: return launch_wide_group<HD, VD, 1>(mq, mk, mv, p, grid, stream);
+        case 2: return launch_wide_group<HD, VD, 2>(mq, mk, mv, p, grid, stream);
+        case 4: return launch_wide_group<HD, VD, 4>(mq, mk, mv, p, grid, stream);
+        case 8: return launch_wide_group<HD, VD, 8>(mq, mk, mv, p, grid, stream);
+        default: return launch_wide_group<HD, VD, 16>(mq, mk, mv, p, grid, stream);
+    }
 }
 
 template <int VD>
