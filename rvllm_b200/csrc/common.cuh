@@ -195,6 +195,18 @@ __device__ __forceinline__ float rv_sum4_dealt(const float (&v)[4], int part) {
     return r;
 }
 
+// The same of four or of two sums; a lane gets sum number part & 3, or part & 1.
+template <int PARTS>
+__device__ __forceinline__ float rv_sum_dealt(const float (&v)[4], int part) { return rv_sum4_dealt<PARTS>(v, part); }
+template <int PARTS>
+__device__ __forceinline__ float rv_sum_dealt(const float (&v)[2], int part) {
+    const bool odd = part & 1;
+    float r = (odd ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 1);
+#pragma unroll
+    for (int o = 2; o < PARTS; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
 __device__ __forceinline__ float rv_warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -214,22 +214,22 @@ mlstm_scan_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
 
 // The same for keys of 33 to 128 elements and portions of tokens, in two roles and with another cut of the columns.  What bound the
 // kernel above is shared memory: every warp reads the whole of q and k for the eight columns it holds.  Here a lane holds 8
-// entries of FOUR neighbouring columns, which PARTS lanes (8 or 16) share: a token costs it four wide reads of q and k, and the
+// entries of CW = four (or two) neighbouring columns, which PARTS lanes (8 or 16) share: with four a token costs it four wide reads of q and k, and the
 // four sums of S^T q are met by a reduction that deals them out.  Four warps walk, four others bring the next chunk, form
 // its gates and stage it (double buffers, one barrier a chunk); a warp walks the running maximum through a chunk with the gates
 // in its lanes.  The numbers and the order of every sum are those of the kernel above, so a request's bits do not depend on which
 // of the two a step takes.
 // 2,048 tokens of 8 heads, 128 x 256: 648 -> 416 us; of 16 heads 759 -> 531; four sequences of 500, 8 heads 198 -> 143.
-template <int PARTS>
+template <int PARTS, int CW>
 struct MlstmStage {
     static constexpr int ROW = PARTS * 12;                 // 8 entries a lane, 12 floats apart: a lane's reads fall on banks of their own
-    static constexpr int COLS = 4 * (32 / PARTS) * 4;      // columns of a block
+    static constexpr int COLS = CW * (32 / PARTS) * 4;     // columns of a block
     float q[ML_CHUNK][ROW], k[ML_CHUNK][ROW];
     float v[ML_CHUNK][COLS];
     float a[ML_CHUNK], b[ML_CHUNK];
 };
 
-template <int PARTS>
+template <int PARTS, int CW>
 __global__ void __launch_bounds__(256)
 mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_col0, const float* __restrict__ i_bias,
                   const float* __restrict__ f_bias, const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots,
@@ -237,7 +237,7 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
                   int vd, float cap, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
-    using Stage = MlstmStage<PARTS>;
+    using Stage = MlstmStage<PARTS, CW>;
     extern __shared__ __align__(16) unsigned char mw_raw[];
     Stage* stages = reinterpret_cast<Stage*>(mw_raw);      // [2]
     const int seq = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * Stage::COLS;
@@ -250,14 +250,14 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     const int width = vd + 1;                              // columns of a head's state: the values and the constant 1
     if (warp < 4) {                                        // ---- the walk
         const int part = lane % PARTS, group = lane / PARTS;
-        const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;
-        const int n0 = part * 8, mine = part & 3;          // this lane's column after the reduction
-        float S[8][4];
+        const int cb = (warp * (32 / PARTS) + group) * CW, col = col0 + cb;
+        const int n0 = part * 8, mine = part & (CW - 1);   // this lane's column after the reduction
+        float S[8][CW];
         float* srow = state + (size_t)slot * state_stride + (size_t)h * d * width + col;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) S[i][j] = (col + j < width && n0 + i < d) ? srow[(size_t)(n0 + i) * width + j] : 0.f;
+            for (int j = 0; j < CW; ++j) S[i][j] = (col + j < width && n0 + i < d) ? srow[(size_t)(n0 + i) * width + j] : 0.f;
         __syncthreads();                                   // the first chunk is staged
         for (int c = 0; c < chunks; ++c) {
             const Stage& st = stages[c & 1];
@@ -269,19 +269,21 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
                 *reinterpret_cast<float4*>(kr + 4) = *reinterpret_cast<const float4*>(&st.k[tt][part * 12 + 4]);
                 *reinterpret_cast<float4*>(qr) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12]);
                 *reinterpret_cast<float4*>(qr + 4) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12 + 4]);
-                const float4 v = *reinterpret_cast<const float4*>(&st.v[tt][cb]);
                 const float a = st.a[tt], b = st.b[tt];
-                const float bu[4] = {b * v.x, b * v.y, b * v.z, b * v.w};
-                float aq[4] = {0.f, 0.f, 0.f, 0.f};
+                float bu[CW], aq[CW];
+                if constexpr (CW == 4) { const float4 v = *reinterpret_cast<const float4*>(&st.v[tt][cb]); bu[0] = v.x; bu[1] = v.y; bu[2] = v.z; bu[3] = v.w; }
+                else { const float2 v = *reinterpret_cast<const float2*>(&st.v[tt][cb]); bu[0] = v.x; bu[1] = v.y; }
+#pragma unroll
+                for (int j = 0; j < CW; ++j) { bu[j] *= b; aq[j] = 0.f; }
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < CW; ++j) {
                         S[i][j] = fmaf(a, S[i][j], kr[i] * bu[j]);
                         aq[j] = fmaf(S[i][j], qr[i], aq[j]);
                     }
-                const float ov = rv_sum4_dealt<PARTS>(aq, part);
-                if (part < 4 && col + mine < width) raw[((size_t)(start + t0 + tt) * heads + h) * width + col + mine] = ov;
+                const float ov = rv_sum_dealt<PARTS>(aq, part);
+                if (part < CW && col + mine < width) raw[((size_t)(start + t0 + tt) * heads + h) * width + col + mine] = ov;
             };
             if (nt == ML_CHUNK) {
 #pragma unroll 4
@@ -294,7 +296,7 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < CW; ++j)
                 if (col + j < width && n0 + i < d) srow[(size_t)(n0 + i) * width + j] = S[i][j];
         return;
     }
@@ -384,14 +386,14 @@ mlstm_walk_kernel(const float* __restrict__ proj, int stride, int i_col0, int f_
     // all of them, stores the sequence's last m)
 }
 
-template <int PARTS>
+template <int PARTS, int CW>
 static int launch_mlstm_walk(cudaStream_t stream, int n_seqs, const float* proj, int stride, int i_col0, int f_col0, const float* i_bias,
                              const float* f_bias, const int* cu_seqlens, const int* state_slots, float* state, size_t state_stride, float* raw,
                              float* top, int heads, int d, int vd, float cap, int least) {
-    constexpr int smem = 2 * (int)sizeof(MlstmStage<PARTS>), cols = MlstmStage<PARTS>::COLS;
+    constexpr int smem = 2 * (int)sizeof(MlstmStage<PARTS, CW>), cols = MlstmStage<PARTS, CW>::COLS;
     static RvPerDevice once;
-    if (int st = rv_configure_smem(once, mlstm_walk_kernel<PARTS>, smem)) return st;
-    return rv_launch(mlstm_walk_kernel<PARTS>, dim3((vd + 1 + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, proj, stride, i_col0,
+    if (int st = rv_configure_smem(once, mlstm_walk_kernel<PARTS, CW>, smem)) return st;
+    return rv_launch(mlstm_walk_kernel<PARTS, CW>, dim3((vd + 1 + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, proj, stride, i_col0,
                      f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, state_stride, raw, top, heads, d, vd, cap, least);
 }
 
@@ -424,10 +426,13 @@ RV_EXPORT int rv_mlstm_scan(const float* proj, int stride, int i_col0, int f_col
                                  i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, (size_t)state_stride, raw, top, heads, d,
                                  vd, parts, cap, most);
     if (!two_roles || which == 1 || (which == 3 && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
-    RV_LAUNCH_ST = d > 64 ? launch_mlstm_walk<16>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
-                                                  (size_t)state_stride, raw, top, heads, d, vd, cap, least)
-                          : launch_mlstm_walk<8>(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state,
-                                                 (size_t)state_stride, raw, top, heads, d, vd, cap, least);
+    // Two columns a lane where the blocks then have an SM each, as in the delta rule (ssm.cu): 2,048 tokens of 8 heads of 128 x 256 (136
+    // blocks, or 72) 414 -> 324 us; of 16 heads 414 and 415.
+    const int wide = d > 64 ? MlstmStage<16, 2>::COLS : MlstmStage<8, 2>::COLS;
+    const bool two = (long long)((vd + wide) / wide) * heads * n_seqs <= rv_sm_count();
+    auto walk = d > 64 ? (two ? launch_mlstm_walk<16, 2> : launch_mlstm_walk<16, 4>) : (two ? launch_mlstm_walk<8, 2> : launch_mlstm_walk<8, 4>);
+    RV_LAUNCH_ST = walk(stream, n_seqs, proj, stride, i_col0, f_col0, i_bias, f_bias, cu_seqlens, state_slots, state, (size_t)state_stride, raw, top,
+                        heads, d, vd, cap, least);
     return rv_launch_status();
 }
 

@@ -1209,16 +1209,16 @@ delta_rule_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, c
 // bring the next chunk, turn q and k into unit vectors and stage them (double buffers, one barrier a chunk).  2,048 tokens of
 // 32 / 16 heads of 128 x 128: 1,087 / 932 us before, 711 / 561 us; portions of 1,024 twice: 569 / 524 and 378 / 350 us.  (The
 // kernel above with more lanes a column - 16 or 8 entries each - is slower: 1,078 and 1,109 us.)
-template <int PARTS>
+template <int PARTS, int CW>
 struct DeltaStage {
     static constexpr int ROW = PARTS * 12;                 // 8 entries a lane, 12 floats apart: a lane's reads fall on banks of their own
-    static constexpr int COLS = 4 * (32 / PARTS) * 4;      // columns of a block
+    static constexpr int COLS = CW * (32 / PARTS) * 4;     // columns of a block
     float q[DR_CHUNK][ROW], k[DR_CHUNK][ROW];
     float v[DR_CHUNK][COLS];
     float g[DR_CHUNK], beta[DR_CHUNK], kq[DR_CHUNK];
 };
 
-template <int PARTS>
+template <int PARTS, int CW>
 __global__ void __launch_bounds__(256)
 delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, const float* __restrict__ proj, int proj_stride,
                        int b_col0, int a_col0, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -1226,7 +1226,7 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
                        size_t state_stride, float* __restrict__ out, int heads, int qk_heads, int d, int vd, float unit_eps, int least) {
     rv_pdl_launch_dependents();
     rv_pdl_wait();
-    using Stage = DeltaStage<PARTS>;
+    using Stage = DeltaStage<PARTS, CW>;
     extern __shared__ __align__(16) unsigned char dw_raw[];
     Stage* stages = reinterpret_cast<Stage*>(dw_raw);      // [2]
     const int seq = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * Stage::COLS;
@@ -1238,16 +1238,20 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < 4) {                                        // ---- the walk
         const int part = lane % PARTS, group = lane / PARTS;
-        const int cb = (warp * (32 / PARTS) + group) * 4, col = col0 + cb;      // (vd is a multiple of 4: a group's columns are all there or none)
+        const int cb = (warp * (32 / PARTS) + group) * CW, col = col0 + cb;     // (vd is a multiple of 4: a group's columns are all there or none)
         const bool live = col < vd;
-        const int n0 = part * 8, mine = part & 3;          // this lane's column after the reduction
-        float S[8][4];
+        const int n0 = part * 8, mine = part & (CW - 1);   // this lane's column after the reduction
+        float S[8][CW];
         float* srow = state + (size_t)slot * state_stride + (size_t)h * d * vd + col;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live && n0 + i < d) v = *reinterpret_cast<const float4*>(srow + (size_t)(n0 + i) * vd);
-            S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
+#pragma unroll
+            for (int j = 0; j < CW; ++j) S[i][j] = 0.f;
+            if (live && n0 + i < d) {
+                const float* p = srow + (size_t)(n0 + i) * vd;
+                if constexpr (CW == 4) { const float4 v = *reinterpret_cast<const float4*>(p); S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w; }
+                else { const float2 v = *reinterpret_cast<const float2*>(p); S[i][0] = v.x; S[i][1] = v.y; }
+            }
         }
         __syncthreads();                                   // the first chunk is staged
         for (int c = 0; c < chunks; ++c) {
@@ -1261,24 +1265,24 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
                 *reinterpret_cast<float4*>(qr) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12]);
                 *reinterpret_cast<float4*>(qr + 4) = *reinterpret_cast<const float4*>(&st.q[tt][part * 12 + 4]);
                 const float g = st.g[tt], vv = st.v[tt][cb + mine];
-                float ak[4], aq[4];
+                float ak[CW], aq[CW];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { ak[j] = S[0][j] * kr[0]; aq[j] = S[0][j] * qr[0]; }
+                for (int j = 0; j < CW; ++j) { ak[j] = S[0][j] * kr[0]; aq[j] = S[0][j] * qr[0]; }
 #pragma unroll
                 for (int i = 1; i < 8; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) { ak[j] = fmaf(S[i][j], kr[i], ak[j]); aq[j] = fmaf(S[i][j], qr[i], aq[j]); }
-                const float acc = rv_sum4_dealt<PARTS>(ak, part);
+                    for (int j = 0; j < CW; ++j) { ak[j] = fmaf(S[i][j], kr[i], ak[j]); aq[j] = fmaf(S[i][j], qr[i], aq[j]); }
+                const float acc = rv_sum_dealt<PARTS>(ak, part);
                 const float u = st.beta[tt] * fmaf(-g, acc, vv);
-                float uj[4];
+                float uj[CW];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) uj[j] = __shfl_sync(0xffffffffu, u, group * PARTS + j);
+                for (int j = 0; j < CW; ++j) uj[j] = __shfl_sync(0xffffffffu, u, group * PARTS + j);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) S[i][j] = fmaf(g, S[i][j], kr[i] * uj[j]);
-                const float ov = rv_sum4_dealt<PARTS>(aq, part);
-                if (part < 4 && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
+                    for (int j = 0; j < CW; ++j) S[i][j] = fmaf(g, S[i][j], kr[i] * uj[j]);
+                const float ov = rv_sum_dealt<PARTS>(aq, part);
+                if (part < CW && live) out[((size_t)(start + t0 + tt) * heads + h) * vd + col + mine] = fmaf(g, ov, st.kq[tt] * u);
             };
             if (nt == DR_CHUNK) {                          // a whole chunk: neighbouring tokens may run into one another
 #pragma unroll 4
@@ -1291,7 +1295,11 @@ delta_rule_walk_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
         if (live) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                if (n0 + i < d) *reinterpret_cast<float4*>(srow + (size_t)(n0 + i) * vd) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+                if (n0 + i < d) {
+                    float* p = srow + (size_t)(n0 + i) * vd;
+                    if constexpr (CW == 4) *reinterpret_cast<float4*>(p) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+                    else *reinterpret_cast<float2*>(p) = make_float2(S[i][0], S[i][1]);
+                }
         }
         return;
     }
@@ -1475,14 +1483,14 @@ delta_rule_step_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stri
     }
 }
 
-template <int PARTS>
+template <int PARTS, int CW>
 static int launch_delta_walk(cudaStream_t stream, int n_seqs, int heads, int vd, const void* qkv, int qkv_dtype, int qkv_stride, const float* proj,
                              int proj_stride, int b_col0, int a_col0, const float* a_log, const float* dt_bias, const int* cu_seqlens,
                              const int* state_slots, float* state, size_t state_stride, float* out, int qk_heads, int d, float unit_eps, int least) {
-    constexpr int smem = 2 * (int)sizeof(DeltaStage<PARTS>), cols = DeltaStage<PARTS>::COLS;
+    constexpr int smem = 2 * (int)sizeof(DeltaStage<PARTS, CW>), cols = DeltaStage<PARTS, CW>::COLS;
     static RvPerDevice once;
-    if (int st = rv_configure_smem(once, delta_rule_walk_kernel<PARTS>, smem)) return st;
-    return rv_launch(delta_rule_walk_kernel<PARTS>, dim3((vd + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, qkv, qkv_dtype,
+    if (int st = rv_configure_smem(once, delta_rule_walk_kernel<PARTS, CW>, smem)) return st;
+    return rv_launch(delta_rule_walk_kernel<PARTS, CW>, dim3((vd + cols - 1) / cols, heads, n_seqs), dim3(256), smem, stream, qkv, qkv_dtype,
                      qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens, state_slots, state, state_stride, out, heads,
                      qk_heads, d, vd, unit_eps, least);
 }
@@ -1517,10 +1525,14 @@ RV_EXPORT int rv_delta_rule(const void* qkv, int qkv_dtype, int qkv_stride, cons
                                      qk_heads, d, vd, unit_eps, which == 1 ? 0x7fffffff : short_tokens);
         if (which == 1 || ((which & 1) && RV_LAUNCH_ST != RV_OK)) return rv_launch_status();
         const int least = which == 2 ? 0 : short_tokens + 1;
-        RV_LAUNCH_ST = d > 64 ? launch_delta_walk<16>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                      cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least)
-                              : launch_delta_walk<8>(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias,
-                                                     cu_seqlens, state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least);
+        // Two columns a lane make a token's chain shorter, four read q and k half as often: two where the blocks then have an SM each.
+        // One prompt of 2,048 tokens, 16 heads of 128 x 128 (128 blocks, or 64): 550 -> 410 us, of 953 263 -> 198; 32 heads (256 blocks) 551
+        // and 541, portions of 1,228 and 820 421 and 421.
+        const int wide = d > 64 ? DeltaStage<16, 2>::COLS : DeltaStage<8, 2>::COLS;
+        const bool two = (long long)((vd + wide - 1) / wide) * heads * n_seqs <= rv_sm_count();
+        auto walk = d > 64 ? (two ? launch_delta_walk<16, 2> : launch_delta_walk<16, 4>) : (two ? launch_delta_walk<8, 2> : launch_delta_walk<8, 4>);
+        RV_LAUNCH_ST = walk(stream, n_seqs, heads, vd, qkv, qkv_dtype, qkv_stride, proj, proj_stride, b_col0, a_col0, a_log, dt_bias, cu_seqlens,
+                            state_slots, state, (size_t)state_stride, out, qk_heads, d, unit_eps, least);
         return rv_launch_status();
     }
     const int ns = d > 64 ? 32 : (d > 32 ? 16 : 8);    // four lanes per column up to a key size of 128

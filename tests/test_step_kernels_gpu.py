@@ -475,6 +475,35 @@ def test_delta_rule_bits_do_not_depend_on_the_step(K, d, vd, heads, qk, lens, dt
                 assert torch.equal(run(a, b, [0, b - a], [i], s, b - a)[0][0], o[a - cu[i]:b - cu[i]])
         assert torch.equal(s[i], state[i])
 
+@pytest.mark.parametrize("d,vd,lens", [(128, 128, (33, 16, 20)), (64, 132, (17, 40, 8, 9)), (100, 36, (47,) * 12)])
+def test_walks_of_two_and_of_four_columns_a_lane(K, d, vd, lens):
+    """Steps whose blocks of two columns a lane are more than the SMs take four: the bits of each request alone, which takes two."""
+    heads = 16
+    torch.manual_seed(d + vd)
+    T, N, W = sum(lens), len(lens), vd + 1
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert -(-vd // (16 if d > 64 else 32)) * heads * N > sms >= -(-W // (16 if d > 64 else 32)) * heads
+    cu = torch.tensor((0,) + lens).cumsum(0).tolist()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")      # noqa: E731
+    qkv, gates = torch.randn(T, (2 * d + vd) * heads, device="cuda").bfloat16(), torch.randn(T, 2 * heads, device="cuda")
+    proj = torch.cat([qkv.float(), gates], dim=1)
+    a, b = torch.randn(heads, device="cuda"), torch.randn(heads, device="cuda")
+    first = torch.randn(N, heads * d * vd, device="cuda")
+    memory = torch.randn(N, heads * d * W + heads, device="cuda")
+
+    def delta(i, j, cu, slots, s):
+        return K.delta_rule(qkv[i:j].contiguous(), gates[i:j].contiguous(), 0, heads, a, b, i32(cu), i32(slots), s, heads, heads, d, vd, 1e-6, max_q_len=max(lens))
+
+    def matrix(i, j, cu, slots, s):
+        g0 = (2 * d + vd) * heads
+        return torch.cat(K.mlstm_scan(proj[i:j].contiguous(), g0, g0 + heads, a, b + 2, i32(cu), i32(slots), s, heads, d, vd, 15.0, max_q_len=max(lens)), dim=1)
+    for run, start in ((delta, first), (matrix, memory)):
+        state = start.clone()
+        whole = run(0, T, cu, list(range(N)), state)
+        for n, (i, j) in enumerate(zip(cu, cu[1:])):
+            own = start.clone()
+            assert torch.equal(run(i, j, [0, j - i], [n], own), whole[i:j]) and torch.equal(own[n], state[n])
+
 
 def test_talking_attention_on_eight_and_sixteen_warps(K):
     """The same tiles for twice the tokens a CTA: the same bits, and those of the attention's formula in float64."""
