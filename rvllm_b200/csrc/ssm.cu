@@ -1202,8 +1202,8 @@ delta_rule_kernel(const void* __restrict__ qkv, int qkv_dtype, int qkv_stride, c
 
 // The same for keys of 33 to 128 elements and values in multiples of four columns.  What bound the kernel above is shared
 // memory: every warp reads the whole of q and k for the eight columns it holds, 16 wide reads a lane and token.  Here a lane
-// holds 8 entries of FOUR columns: PARTS lanes (8 or 16) share four neighbouring columns, a token costs a lane four wide reads,
-// and the four sums of S^T k are met by a reduction that also deals them out, one column to every PARTS / 4 lanes, which
+// holds 8 entries of CW = four columns (two: see the launch): PARTS lanes (8 or 16) share them, a token costs a lane four wide reads,
+// and the sums of S^T k are met by a reduction that also deals them out, one column to every PARTS / CW lanes, which
 // then form that column's u.  S^T q is formed of the state before the token, beside S^T k, and the result is
 // g S^T q + (k . q) u: the chain from token to token is one sum over the lanes, not two.  Four warps walk, four others
 // bring the next chunk, turn q and k into unit vectors and stage them (double buffers, one barrier a chunk).  2,048 tokens of
