@@ -16,7 +16,7 @@
 // Against the kernel that mixes inside the walk (talking_attention_mma.cu; heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 473 -> 118 us,
 // 80 tokens 32 -> 20, 100 tokens behind 3,990 keys 959 -> 97; 32 heads on 8, 2,048 tokens 974 -> 392, 100 behind 3,990 1,328 -> 114.
 // Error against float64 2.3e-3 -> 1.9e-3 to 2.3e-3 (2-norms; 1.7e-3 is the rounding of the result).  The walk is bound by the
-// softmax warps, one a scheduler; the products are 1,024 of a tile's cycles at three value heads of 128.
+// softmax warps, one a scheduler: 2,070 cycles a tile with two value heads, 310 of them the biases; with three 2,650, of which the products are 1,024.
 //
 // The distance bias r1 ln(1 + r2 d) takes a logarithm per (head, distance), not per score: a warp's 32 rows are few tokens, so
 // a tile of 64 keys meets only 63 + tokens distances, whose biases the warp forms in shared memory a tile ahead.
