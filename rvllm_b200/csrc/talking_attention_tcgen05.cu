@@ -13,10 +13,17 @@
 //                         384 columns).  U is O over the row's sum of weights, float32.
 //   talking_mix_kernel    out[t, h] = sum_g talk[h, g] U[t][kv(h)][g], float32 sums in the order of g, rounded once.
 //
-// Against the kernel that mixes inside the walk (talking_attention_mma.cu; heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 473 -> 118 us,
-// 80 tokens 32 -> 20, 100 tokens behind 3,990 keys 959 -> 97; 32 heads on 8, 2,048 tokens 974 -> 392, 100 behind 3,990 1,328 -> 114.
-// Error against float64 2.3e-3 -> 1.9e-3 to 2.3e-3 (2-norms; 1.7e-3 is the rounding of the result).  The walk is bound by the
-// softmax warps, one a scheduler: 2,070 cycles a tile with two value heads, 310 of them the biases; with three 2,650, of which the products are 1,024.
+// A weight goes into the products as TWO bfloat16 numbers, its rounding and what the rounding left (16 bits and more of the float32
+// weight).  The mixing may take heads that attend alike from one another: then the weights cancel and what they were rounded by does
+// not.  Error against float64 (2-norms; 16 heads on 4, 32 on 8, 8 on 8; contexts of 150 to 4,000), mixing by the identity, at random,
+// and by differences of heads whose scores are 0.3 to 0.005 of themselves apart: 1.6e-3 to 1.8e-3, where the rounding of the result
+// alone is 1.6e-3 and the kernel that mixes inside the walk (talking_attention_mma.cu: mixed weights rounded once) has 2.3e-3 to
+// 2.4e-3.  With one bfloat16 number a weight it was 2.0e-3 to 2.4e-3 for the first two, 6e-3 to 3.5e-1 for the differences.
+//
+// Against the kernel that mixes inside the walk (heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 475 -> 155 us,
+// 80 tokens 31 -> 19, 100 tokens behind 3,990 keys 960 -> 106; 32 heads on 8, 2,048 tokens 975 -> 475, 100 behind 3,990 1,329 -> 185.  (One
+// number a weight: 118, 19, 97; 392, 114.  The softmax warps, one a scheduler, bind the walk: forming the low parts and storing them cost
+// more than the second products.)
 //
 // The distance bias r1 ln(1 + r2 d) takes a logarithm per (head, distance), not per score: a warp's 32 rows are few tokens, so
 // a tile of 64 keys meets only 63 + tokens distances, whose biases the warp forms in shared memory a tile ahead.
@@ -32,7 +39,7 @@
 #define PV_WARP (SOFTMAX_WARPS + 3)            // issues O += P V
 #define NUM_THREADS (32 * (SOFTMAX_WARPS + 4))
 #define TMEM_COLS 512
-#define S_COL 0                                // two S buffers of 64 columns; P (bf16 pairs) reuses the first 32 columns of each
+#define S_COL 0                                // two S buffers of 64 columns; P (two bf16 numbers a weight) reuses them
 #define O_COL 128
 #define O_COLS (TMEM_COLS - O_COL)
 #define MAX_GROUP 16                           // heads on one key/value head
@@ -78,8 +85,8 @@ __device__ __forceinline__ float fast_log2(float x) {
     return y;
 }
 
-// G: heads on one key/value head (a constant, so that the reads of the biases have constant offsets: 64 registers of addresses less; 134
-// -> 118 and 406 -> 392 us)
+// G: heads on one key/value head (a constant, so that the reads of the biases have constant offsets: 64 registers of addresses less; 2,048
+// tokens, with one number a weight, 134 -> 118 and 406 -> 392 us)
 template <int HD, int VD, int G>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -239,12 +246,14 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int b = it & 1, v_stage = it % NV;
             if (!(ok = mbar_wait(bar_p_full0 + 8 * b, (it >> 1) & 1, &abort_flag, 8))) return;
             tcgen05_fence_after();
-            const uint32_t tp = tmem_base + S_COL + b * KV_TILE;         // P(it): bf16 pairs in the first half of S buffer b
+            const uint32_t tp = tmem_base + S_COL + b * KV_TILE;         // P(it) over S buffer b: of 32 keys 16 columns of roundings and 16 of rests
             for (int c = 0; c < nv; ++c) {
                 const uint64_t dv = umma_desc_mn(smem_u32(v_s) + v_stage * Z::V_BYTES + c * (Z::V_HALVES * KV_TILE * 128), KV_TILE * 128);
 #pragma unroll
-                for (int j = 0; j < 4; ++j)              // 16 keys per MMA: 8 columns along P's rows, 2048 bytes down V
-                    tcgen05_mma_bf16_ts(tmem_base + O_COL + c * VD, tp + 8 * j, dv + (uint64_t)(128 * j), idesc_o, (it | j) != 0);
+                for (int j = 0; j < 8; ++j) {            // 16 keys per MMA: 8 columns along P's rows, 2048 bytes down V
+                    const int keys = 2 * (j >> 2) + (j & 1);
+                    tcgen05_mma_bf16_ts(tmem_base + O_COL + c * VD, tp + 8 * j, dv + (uint64_t)(128 * keys), idesc_o, (it | j) != 0);
+                }
             }
             tcgen05_commit(bar_vfree0 + 8 * v_stage);
             tcgen05_commit(bar_o_full0 + 8 * b);
@@ -358,20 +367,24 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
             float l_tile = 0.f, l_tile2 = 0.f;
-            uint32_t pk[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {                   // keys 2j and 2j + 1 of the tile: one column of P
-                const int e = 2 * j;
-                float a0, a1;
-                fma2(a0, a1, __uint_as_float(e < 32 ? s0[e] : s1[e - 32]), __uint_as_float(e + 1 < 32 ? s0[e + 1] : s1[e + 1 - 32]),
-                     eff_scale, neg_m);
-                const float x0 = fast_exp2(a0), x1 = fast_exp2(a1);
-                add2(l_tile, l_tile2, x0, x1);
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(x0, x1);
-                pk[j] = *reinterpret_cast<uint32_t*>(&h2);
+            for (int half = 0; half < 2; ++half) {           // 32 keys: 16 columns of their roundings, 16 of the rests (a store of each
+                const uint32_t* s = half ? s1 : s0;          // half as it is done: 100 tokens behind 3,990 keys 159 -> 106 us)
+                uint32_t pk[32];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {               // keys 2j and 2j + 1
+                    float a0, a1;
+                    fma2(a0, a1, __uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1]), eff_scale, neg_m);
+                    const float x0 = fast_exp2(a0), x1 = fast_exp2(a1);
+                    add2(l_tile, l_tile2, x0, x1);
+                    __nv_bfloat162 h2 = __floats2bfloat162_rn(x0, x1);
+                    pk[j] = *reinterpret_cast<uint32_t*>(&h2);
+                    h2 = __floats2bfloat162_rn(x0 - __uint_as_float(pk[j] << 16), x1 - __uint_as_float(pk[j] & 0xffff0000u));
+                    pk[16 + j] = *reinterpret_cast<uint32_t*>(&h2);
+                }
+                tmem_st_32x32(t_lane + S_COL + sb * KV_TILE + 32 * half, pk);
             }
             l_run += l_tile + l_tile2;
-            tmem_st_32x32(t_lane + S_COL + sb * KV_TILE, pk);
             tmem_st_wait();
             tcgen05_fence_before();
             __syncwarp();

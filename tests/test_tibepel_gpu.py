@@ -350,6 +350,34 @@ def test_mixing_behind_the_sum_over_the_keys(K, H, G, d, vd, chunk, page):
     K.raise_on_abort()
 
 
+@pytest.mark.parametrize("H,G,d,vd,q_len,ctx", [(16, 4, 128, 128, 100, 700), (8, 8, 64, 64, 150, 150), (32, 8, 128, 128, 70, 330)])
+@pytest.mark.parametrize("apart", [0.3, 0.05])
+def test_mixing_that_takes_agreeing_heads_from_one_another(K, H, G, d, vd, q_len, ctx, apart):
+    """Neighbouring heads attend almost alike (the scores of one are 1 + `apart` times the other's) and a row of the mixing is their
+    difference: most of the weights cancels, what a weight was rounded by does not.  2-norms: a rounding to bfloat16 is at most 2^-9 of
+    a number, the result's is one, a mixed weight's (the build that mixes inside the walk) another; float32 weights add some 2^-22 over
+    `apart`.  Each head's own weight rounded to bfloat16 would be 2^-9 over `apart` away, 1e-2 and more."""
+    dtype = torch.bfloat16
+    k, v, q = (rnd(n, h, w, seed=i).to(dtype).double() for i, (n, h, w) in enumerate(((ctx, G, d), (ctx, G, vd), (q_len, H, d))))
+    q[:, 1::2] = (q[:, 0::2] * (1 + apart)).to(dtype).double()
+    if G == H:
+        k[:, 1::2] = k[:, 0::2]
+    r1, r2 = (torch.rand(H // 2, generator=torch.Generator().manual_seed(i)).double().repeat_interleave(2) for i in (1, 2))
+    talk = torch.eye(H, dtype=F64) - torch.eye(H, dtype=F64).view(H // 2, 2, H).flip(1).reshape(H, H)
+    cache, meta, positions = flat_pages([k], [v], [q_len], 16, dtype)
+    full_q = torch.zeros(ctx, H, d, dtype=F64)
+    full_q[ctx - q_len:] = q
+    want = P.mixed_head_attention(full_q, k, v, d ** -0.5, r1, r2, talk, 10 ** 9)[ctx - q_len:].reshape(q_len, -1)
+    old = K.TALKING_WIDE
+    try:
+        for K.TALKING_WIDE in (True, False):
+            got = K.talking_attention(q.reshape(q_len, H * d).to(dtype).cuda(), cache, meta, positions, H, G, d, vd, d ** -0.5, r1.float().cuda(),
+                                      r2.float().cuda(), talk.float().cuda(), None).double().cpu()
+            assert float((got - want).norm() / want.norm()) < 2 * 2 ** -9, K.TALKING_WIDE
+    finally:
+        K.TALKING_WIDE = old
+
+
 def test_a_large_batch_of_single_tokens_takes_the_split_keys(K):
     """Seventy sequences of unequal lengths, one token each: more tokens than the tensor-core build is preferred from, yet
     all of them single, so the keys are split (into fewer ranges than for a small batch); against the slow implementation."""
