@@ -378,6 +378,41 @@ def test_mixing_that_takes_agreeing_heads_from_one_another(K, H, G, d, vd, q_len
         K.TALKING_WIDE = old
 
 
+@pytest.mark.parametrize("H,G,d,vd,chunk,page", [(16, 4, 128, 128, None, 16), (8, 8, 64, 64, 150, 32), (4, 4, 64, 128, 40, 8), (16, 1, 128, 64, 230, 64)])
+def test_a_value_that_is_not_finite_stays_with_the_tokens_that_see_it(K, H, G, d, vd, chunk, page):
+    """Infinities and NaN among the values of single keys: the portion's first, one in its middle, the last of the chunk before and one
+    that a whole tile behind it sees.  The results of the tokens that see such a key, on its key/value head and in its
+    elements, are not finite; all others, also of tokens before it in the same tile, have the bits they have without it.  The same for a key:
+    whatever it holds, tokens that do not see it keep their bits."""
+    dtype, ctx, q_len = torch.bfloat16, 330, 200
+    k, v, q = (rnd(n, h, w, seed=i).to(dtype).double() for i, (n, h, w) in enumerate(((ctx, G, d), (ctx, G, vd), (q_len, H, d))))
+    talk = (torch.eye(H) + 0.4 * rnd(H, H, seed=3).float()).cuda()
+    pos = torch.arange(ctx - q_len, ctx)
+    first = (pos // chunk) * chunk if chunk else pos * 0
+
+    def run(k, v):
+        cache, meta, positions = flat_pages([k], [v], [q_len], page, dtype, chunk)
+        return K.talking_attention(q.reshape(q_len, H * d).to(dtype).cuda(), cache, meta, positions, H, G, d, vd, d ** -0.5, None, None, talk, chunk).cpu().view(q_len, H, vd)
+
+    clean = run(k, v)
+    assert bool(clean.isfinite().all())
+    keys = [ctx - q_len, 230, 262, int(first[-1]) + 2] + ([int(first[-1]) - 1] if chunk else [])
+    for n, key in enumerate(keys):
+        sees = (pos >= key) & (first <= key)
+        for bad in ((float("inf"), float("-inf"), float("nan")), (float("nan"),) * 3):
+            w, c, at = v.clone(), n % G, torch.tensor([1, 17, vd - 1])
+            w[key, c, at] = torch.tensor(bad, dtype=F64)
+            got = run(k, w)
+            hit = torch.zeros(q_len, H, vd, dtype=torch.bool)
+            hit[:, c * (H // G):(c + 1) * (H // G), at] = sees[:, None, None]
+            assert torch.equal(~got.isfinite(), hit) and torch.equal(got[~hit], clean[~hit]), (key, bad)
+        w = k.clone()
+        w[key, n % G, 5] = float("nan")
+        got = run(w, v)
+        assert torch.equal(got[~sees], clean[~sees]) and bool(got[sees].isnan().all()), key
+    K.raise_on_abort()
+
+
 def test_a_large_batch_of_single_tokens_takes_the_split_keys(K):
     """Seventy sequences of unequal lengths, one token each: more tokens than the tensor-core build is preferred from, yet
     all of them single, so the keys are split (into fewer ranges than for a small batch); against the slow implementation."""
