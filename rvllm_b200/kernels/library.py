@@ -81,8 +81,16 @@ class CudaKernels:
     TALKING_MMA = True                 # attention with mixed head weights: bfloat16 prompt portions go to the tensor-core kernel when it fits
     TALKING_WARPS = 0                  # ... whose CTAs have up to 8 or 16 warps (0: by the number of CTAs)
     TALKING_WIDE = True                # ... where its sizes allow, to the tcgen05 kernel, which mixes behind the sum over the keys
-    TALKING_WIDE_MIN_TOKENS = 16       # ... from this many tokens in the longest portion of the step (80 tokens of 16 heads on 4: 20 us against 32;
-                                       # steps of up to TALKING_SPLIT_MAX_TOKENS behind more keys do not come here)
+    TALKING_WIDE_MIN_TOKENS = 16       # ... from this many tokens in the longest portion of the step, behind more than
+    TALKING_WIDE_MIN_KEYS = 32         # ... this many keys (portions of 16 to 32 tokens behind nothing: 18 to 22 us inside the walk, 17 to 25 in two
+                                       # launches; of 48, 25 and 20, 31 and 26; five of 16 behind 1,000 keys 241 and 50, 338 and 62), and
+    TALKING_WIDE_MAX_SHORT = 6         # ... while its walks for sequences of few tokens are at most this many CTAs an SM: a sequence takes
+    TALKING_WIDE_SHORT = 48            # kv_heads x blocks CTAs of 128 rows however few tokens it brings, one CTA of the other kernel's up to 8.
+                                       # 32 heads on 8, 80 tokens beside 32, 63 and 127 single ones behind 1,000 keys 504, 508 and 522 us inside the
+                                       # walk, 286, 509 and 982 here, 2,000 tokens beside them 1,345, 1,401 and 1,594, 964, 1,940 and 3,370; 16 on 4
+                                       # beside 63, 127 and 255 368, 371 and 729, 181, 314 and 587, but 16 tokens beside 127 250 and 302
+    TALKING_WIDE_MAX_SHORT_PLAIN = 24  # ... where the kernel that mixes inside the walk does not fit (16 heads on 16, 80 tokens beside 32 single ones, 21
+                                       # CTAs an SM: 1,039 us the plain kernel, 947 here; beside 63, 41 an SM, 1,040 and 1,840)
     TALKING_WIDE_MAX_SCRATCH = 256 << 20   # ... in windows of tokens whose sums over the keys fit this many bytes
     TALKING_SPLIT = True               # attention with mixed head weights: few tokens behind many keys go to the split-key kernels
     TALKING_SPLIT_MAX_TOKENS = 64      # ... up to this many tokens in the step
@@ -1400,6 +1408,18 @@ class CudaKernels:
         _check("kv_prepare", st)
         return q
 
+    def _talking_wide_pays(self, T: int, meta: AttentionMeta, visible: int, num_heads: int, num_kv_heads: int, value_dim: int) -> bool:
+        """Whether the tcgen05 kernel of `talking_attention` is the faster one for a step's portions (the constants have the measurements)."""
+        tile_tokens = max(1, 128 * num_kv_heads // num_heads)          # of a CTA's 128 rows
+        if meta.max_q_len < self.TALKING_WIDE_MIN_TOKENS or visible <= self.TALKING_WIDE_MIN_KEYS \
+                or -(-meta.max_q_len // tile_tokens) > 65535:           # (the grid's limit; the others have none there)
+            return False
+        portions = meta.num_seqs - meta.num_decode
+        short = meta.num_decode + (portions if T - meta.num_decode < self.TALKING_WIDE_SHORT * portions else 0)
+        blocks = -(-num_kv_heads // max(1, 384 // value_dim))          # of value heads that a CTA's columns hold
+        most = self.TALKING_WIDE_MAX_SHORT if num_kv_heads <= 8 else self.TALKING_WIDE_MAX_SHORT_PLAIN
+        return short * num_kv_heads * blocks <= most * self.num_sms
+
     def talking_attention(self, q, cache_layer, meta: AttentionMeta, positions, num_heads: int, num_kv_heads: int, head_dim: int,
                           value_dim: int, scale: float, r1, r2, talk, chunk: Optional[int]) -> torch.Tensor:
         """softmax attention over the paged cache whose weights are mixed across the heads (`talk` [heads, heads], float32)
@@ -1440,7 +1460,7 @@ class CudaKernels:
             _check("talking_attention_split", st)
             return out
         if self.TALKING_MMA and self.TALKING_WIDE and not self.TALKING_WARPS and q.dtype == torch.bfloat16 and talk is not None \
-                and scale > 0 and meta.max_q_len >= self.TALKING_WIDE_MIN_TOKENS:
+                and scale > 0 and self._talking_wide_pays(T, meta, visible, num_heads, num_kv_heads, value_dim):
             lib = self._lib("talking_attention_tcgen05.cu")
             if lib.rv_talking_wide_fits(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim), c_int(ps)):
                 per_token = num_kv_heads * num_heads * value_dim

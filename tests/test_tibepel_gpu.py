@@ -413,6 +413,35 @@ def test_a_value_that_is_not_finite_stays_with_the_tokens_that_see_it(K, H, G, d
     K.raise_on_abort()
 
 
+@pytest.mark.parametrize("q_lens,ctx,wide", [((15,) * 5, 60, False), ((16,) * 5, 60, True), ((16,) * 5, 32, False), ((16,) * 5, 33, True),
+                                             ((16,) + (1,) * 54, 60, True), ((16,) + (1,) * 55, 60, False), ((48,) + (1,) * 55, 60, True),
+                                             ((48,) + (1,) * 56, 60, False), ((16,) + (9,) * 55, 60, False), ((49,) * 60, 60, True)])
+def test_which_steps_mix_behind_the_sum_over_the_keys(K, q_lens, ctx, wide):
+    """At the edges of the rule - the longest portion, the visible keys, sequences of few tokens - the kernel that it names runs
+    and gives the plain result."""
+    from rvllm_b200.kernels.library import COUNTERS
+    H, G, d, vd, dtype, n = 32, 8, 64, 64, torch.bfloat16, len(q_lens)
+    ks, vs = ([rnd(ctx, G, w, seed=s + i % 3).to(dtype).double() for i in range(n)] for w, s in ((d, 1), (vd, 11)))
+    qs = [rnd(m, H, d, seed=21 + i % 3).to(dtype).double() for i, m in enumerate(q_lens)]
+    talk = torch.eye(H, dtype=F64) + 0.4 * rnd(H, H, seed=3)
+    cache, meta, positions = flat_pages(ks, vs, q_lens, 16, dtype)
+    sms, before = K.num_sms, COUNTERS["launches"]
+    try:
+        K.num_sms = 148                                    # (the rule counts CTAs an SM)
+        got = K.talking_attention(torch.cat(qs).reshape(sum(q_lens), H * d).to(dtype).cuda(), cache, meta, positions, H, G, d, vd, 0.125, None, None,
+                                  talk.float().cuda(), None)
+    finally:
+        K.num_sms = sms
+    assert COUNTERS["launches"] == before + (2 if wide else 1)
+    zero = torch.zeros(H, dtype=F64)
+    for i in (0, n - 1):
+        full_q = torch.zeros(ctx, H, d, dtype=F64)
+        full_q[ctx - q_lens[i]:] = qs[i]
+        want = P.mixed_head_attention(full_q, ks[i], vs[i], 0.125, zero, zero, talk, 10 ** 9)[ctx - q_lens[i]:].reshape(q_lens[i], -1)
+        at = sum(q_lens[:i])
+        assert rel_err(got[at:at + q_lens[i]], want) < TOL[dtype], i
+
+
 def test_a_large_batch_of_single_tokens_takes_the_split_keys(K):
     """Seventy sequences of unequal lengths, one token each: more tokens than the tensor-core build is preferred from, yet
     all of them single, so the keys are split (into fewer ranges than for a small batch); against the slow implementation."""
