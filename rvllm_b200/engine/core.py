@@ -98,6 +98,7 @@ class Engine:
         # a step keeps a handful of [tokens, hidden] buffers and two of the widest projection
         act = ec.max_num_batched_tokens * self.spec.hidden_size * el * 24
         act += ec.max_num_seqs * self.spec.vocab_size * 4 * 3
+        act += self.model.scratch_bytes(self.kernels, ec.max_num_batched_tokens)
         usable = free - (1.0 - ec.gpu_memory_utilization) * total - act - (1 << 30)
         pages = int(usable // per_page)
         if pages < 1:

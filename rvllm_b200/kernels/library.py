@@ -1408,6 +1408,11 @@ class CudaKernels:
         _check("kv_prepare", st)
         return q
 
+    def talking_scratch_bytes(self, tokens: int, num_heads: int, num_kv_heads: int, value_dim: int) -> int:
+        """The sums over the keys of `talking_attention`, at most, for a step of so many tokens (the engine leaves room for them)."""
+        per_token = 4 * num_kv_heads * num_heads * value_dim
+        return per_token * max(1, min(tokens, self.TALKING_WIDE_MAX_SCRATCH // per_token))
+
     def _talking_wide_pays(self, T: int, meta: AttentionMeta, visible: int, num_heads: int, num_kv_heads: int, value_dim: int) -> bool:
         """Whether the tcgen05 kernel of `talking_attention` is the faster one for a step's portions (the constants have the measurements)."""
         tile_tokens = max(1, 128 * num_kv_heads // num_heads)          # of a CTA's 128 rows
@@ -1464,8 +1469,8 @@ class CudaKernels:
             lib = self._lib("talking_attention_tcgen05.cu")
             if lib.rv_talking_wide_fits(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim), c_int(ps)):
                 per_token = num_kv_heads * num_heads * value_dim
-                window = max(1, min(T, self.TALKING_WIDE_MAX_SCRATCH // (4 * per_token)))
-                u = torch.empty((window * per_token,), dtype=torch.float32, device=q.device)
+                u = torch.empty((self.talking_scratch_bytes(T, num_heads, num_kv_heads, value_dim) // 4,), dtype=torch.float32, device=q.device)
+                window = u.numel() // per_token
                 for lo in range(0, T, window):
                     st = lib.rv_talking_wide(
                         _ptr(q), _ptr(cache_layer), ctypes.c_longlong(cache_layer.shape[0]), _ptr(meta.block_tables), _ptr(meta.cu_seqlens),

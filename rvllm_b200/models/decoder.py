@@ -145,6 +145,10 @@ class DecoderModel:
             needs[slot] = self.embedding_hooks[i].cache_need()
         return needs
 
+    def scratch_bytes(self, kernels, tokens: int) -> int:
+        """What the parts of a step of so many tokens take at most, one after the other, beside the step's tensors."""
+        return max((part.scratch_bytes(kernels, tokens, self.dtype) for _, part in self.named_parts() if hasattr(part, "scratch_bytes")), default=0)
+
     # ---- the forward pass of one step ----------------------------------------------------------
     def forward(self, ctx, caches) -> torch.Tensor:
         x = ctx.kernels.gather_rows(self.embedding, ctx.token_ids)

@@ -94,6 +94,10 @@ class Part:
     def bind(self, get: Callable[[str], torch.Tensor]) -> None:
         """`get(name)` returns the device tensor stored under the part's prefix + name."""
 
+    def scratch_bytes(self, kernels, tokens: int, dtype: torch.dtype) -> int:
+        """What a step of so many tokens takes, at most, beside the tensors a part is given and returns (0: nothing worth counting)."""
+        return 0
+
 
 class Registry:
     def __init__(self, what: str):

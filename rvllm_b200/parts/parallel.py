@@ -43,6 +43,9 @@ class ParallelMixers(Part):
     def cache_need(self):
         return CompositeNeed(tuple(m.cache_need() for m in self.members))
 
+    def scratch_bytes(self, kernels, tokens, dtype):
+        return max((m.scratch_bytes(kernels, tokens, dtype) for m in self.members if hasattr(m, "scratch_bytes")), default=0)
+
     def terms(self, x, ctx, cache, write_cache=True):
         """[(float32 result, factor), ...], one per member, in their order."""
         return [(m(x, ctx, view, residual=None, write_cache=write_cache, out_dtype=torch.float32), scale)

@@ -68,6 +68,11 @@ class TalkingHeadsAttention(Part):
     def cache_need(self):
         return KvCacheNeed(self.num_kv_heads, self.head_dim, None, 2, self.value_dim, self.chunk)
 
+    def scratch_bytes(self, kernels, tokens, dtype):
+        if not self.has_talk or dtype != torch.bfloat16:
+            return 0
+        return kernels.talking_scratch_bytes(tokens, self.num_heads, self.num_kv_heads, self.value_dim)
+
     def __call__(self, x, ctx, cache, residual=None, write_cache=True, out_dtype=None):
         k = ctx.kernels
         meta = ctx.attention[cache.group]

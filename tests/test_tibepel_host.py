@@ -246,6 +246,32 @@ def test_chunk_pages_come_back_while_a_request_runs(emulated):
     assert all(n == 12 for n in engine.cache.num_free_pages())
 
 
+def test_the_cache_leaves_room_for_the_sums_over_the_keys(emulated, tmp_path, monkeypatch):
+    """Attention with mixed head weights keeps a float per token, head, key/value head and value column beside the step's tensors, up to
+    a bound: the number of pages that the engine derives from the free memory is smaller by that much."""
+    from types import SimpleNamespace
+    from rvllm_b200.engine.core import Engine
+    from rvllm_b200.kernels.library import CudaKernels
+    kernels = CudaKernels.__new__(CudaKernels)
+    model = DecoderModel(config_from_dict(X.small_a()).to_spec())
+    model.dtype = torch.bfloat16
+    mixers = [m for layer in model.layers for m in getattr(layer.mixer, "members", [layer.mixer]) if getattr(m, "has_talk", False)]
+    want = max(4 * 512 * m.num_heads * m.num_kv_heads * m.value_dim for m in mixers)
+    assert want > 0 and model.scratch_bytes(kernels, 512) == want
+    assert kernels.talking_scratch_bytes(10 ** 6, 32, 8, 128) == 256 << 20 and kernels.talking_scratch_bytes(1, 64, 64, 128) == 4 * 64 * 64 * 128
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (100 << 30, 100 << 30))
+    ec = SimpleNamespace(block_size=16, max_num_seqs=10 ** 6, max_model_len=1 << 20, max_num_batched_tokens=512, gpu_memory_utilization=1.0)
+    needs = model.cache_needs()
+    engine = SimpleNamespace(device=torch.device("cuda"), dtype=torch.bfloat16, spec=model.spec, model=model, kernels=kernels)
+    pages = Engine._pages_from_memory(engine, needs, ec)
+    model.dtype = torch.float32                            # (the float32 engine takes other kernels)
+    assert model.scratch_bytes(kernels, 512) == 0
+    more = Engine._pages_from_memory(engine, needs, ec)
+    from rvllm_b200.cache.manager import CacheManager
+    per_page = CacheManager.bytes_per_page(needs, 16, torch.bfloat16)
+    assert abs((more - pages) * per_page - want) <= per_page
+
+
 def test_state_rows_start_at_zero_for_a_new_request(emulated):
     """Five requests through two slots: a slot's recurrent state and convolution inputs are those of the new request."""
     folder, vocab, reqs, ref = _reference("b")
