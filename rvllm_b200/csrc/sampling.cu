@@ -487,13 +487,14 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
     const int per = (((V + CL - 1) / CL) + 3) & ~3;
     const int lo = min(V, rank * per), hi = min(V, lo + per);
     // ---- pass A: maximum and counts
-    float bv = -INFINITY;
+    float bv = __int_as_float(0x7fc00000);                // (the first token that is not NaN is larger than nothing, also -inf)
     int bi = 0x7fffffff;
     sample_walk(row, lo, hi, [&](float v, int i) {
         if (v != v) return;
-        if (v > bv) { bv = v; bi = i; }                   // indices rise within a thread: a strict comparison keeps the lowest
+        if (!(v <= bv)) { bv = v; bi = i; }               // indices rise within a thread: equal values keep the lowest
         atomicAdd(&h_cnt[order_key(v) >> 20], 1u);
     });
+    if (bi == 0x7fffffff) bv = -INFINITY;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -912,11 +913,12 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     }
     if (!have_max) {
     // ---- arg-max of the row: this CTA's slices lie side by side
-    float bv = -INFINITY;
+    float bv = __int_as_float(0x7fc00000);                // (as in the short way)
     int bi = 0x7fffffff;
     sample_walk(row, min(V, first * S), min(V, (first + per) * S), [&](float v, int i) {
-        if (v > bv) { bv = v; bi = i; }                   // indices rise within a thread; NaN compares false
+        if (v == v && !(v <= bv)) { bv = v; bi = i; }
     });
+    if (bi == 0x7fffffff) bv = -INFINITY;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);

@@ -28,6 +28,24 @@ def test_greedy_ties_and_nan(K):
     assert K.sample(big.cuda()).tolist() == [P.argmax_lowest(r) for r in big]
 
 
+@pytest.mark.parametrize("vocab", [5, 1003, 128256])
+@pytest.mark.parametrize("ctas", [1, 2, 8])
+def test_a_greedy_row_with_nothing_above_minus_infinity(K, vocab, ctas):
+    """NaN never wins, not even against -inf: the lowest index that is not NaN, wherever it lies; 0 where all are NaN."""
+    from ctypes import c_int
+    firsts = [0, 1, 2, 3, vocab // 2, vocab - 2, vocab - 1]
+    x = torch.full((len(firsts) + 1, vocab), float("nan"))
+    for r, at in enumerate(firsts):
+        x[r, at:] = float("-inf")
+        x[r, at + 1::3] = float("nan")
+    lib = K._lib("sampling.cu")
+    try:
+        lib.rv_sample_set_cluster(c_int(ctas))
+        assert K.sample(x.cuda()).tolist() == firsts + [0]
+    finally:
+        lib.rv_sample_set_cluster(c_int(0))
+
+
 @pytest.mark.parametrize("vocab", [383, 5000, 128256])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (20, 1.0), (0, 0.8), (50, 0.9)])
 def test_draws_match_the_plain_sampler(K, vocab, top_k, top_p):
