@@ -953,7 +953,10 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
     for (int sl = first; sl < first + per; ++sl) {
         const int lo_s = min(V, sl * S), hi_s = min(V, lo_s + S);
         float part = 0.f;
-        for (int i = lo_s + tid; i < hi_s; i += SAMPLE_THREADS) part += expf((row[i] - m) * inv_t);
+        for (int i = lo_s + tid; i < hi_s; i += SAMPLE_THREADS) {
+            const float v = row[i];
+            if (v == v) part += expf((v - m) * inv_t);   // (with a NaN among them the target was none, and everything was kept)
+        }
         part = rv_block_sum(part, s_val);
         if (tid < CL) sc_store(sc_map(&xch[turn].val[sl], tid), part);
     }

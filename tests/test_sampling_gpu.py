@@ -223,6 +223,20 @@ def test_numbers_of_candidates(K, top_k, top_p):
     assert int((got != want).sum()) <= 1
 
 
+def test_a_top_p_measured_by_the_general_search_leaves_nan_out(K):
+    """Rows whose k-th token does not exist, or lies behind more candidates than the short way sorts: the top-p is still a share of the mass
+    of the tokens that are numbers."""
+    V, R = 5001, 24
+    x = torch.randn(R, V, generator=torch.Generator().manual_seed(3)) * 1.5
+    x[:, ::2] = float("nan")
+    tk = torch.tensor([2400, 4000] * (R // 2), dtype=torch.int32)
+    got = K.sample(x.cuda(), torch.ones(R).cuda(), tk.cuda(), torch.full((R,), 0.5).cuda(), torch.arange(R).cuda(), torch.arange(R).cuda()).tolist()
+    for r in range(R):
+        z = torch.softmax(x[r].nan_to_num(float("-inf")).double(), 0)
+        z = torch.where(x[r].isnan(), 0.0, z)
+        assert float(z[got[r]]) > 0 and float(z[z > z[got[r]]].sum()) < 0.5 + 1e-6, r
+
+
 @pytest.mark.parametrize("vocab", [5001, 128256])
 @pytest.mark.parametrize("ctas", [1, 2, 8])
 def test_flat_rows_under_top_p_alone(K, vocab, ctas):
