@@ -834,7 +834,7 @@ __device__ bool sample_mass_way(const float* __restrict__ row, int V, float inv_
     return tau != 0u;
 }
 
-__device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two), 2: rows that need it get -1
+__device__ int g_sample_short_way = 1;      // 0: always the general search (tests compare the two), 2: rows the short way leaves get -1, 3: rows left to the search do
 
 // Where a row's parameters are: in arrays on the device (null: greedy, or off), or, for up to SAMPLE_VALUE_ROWS rows whose
 // parameters the host has, in the launch itself: no buffer on the device, no copy of 1.8 KB that the host prepares and the kernel waits
@@ -910,6 +910,10 @@ sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows row
             return;
         }
         if (!uk_row) have_tau = sample_mass_way(row, V, inv_t, p_row, m, s_dyn_fast, s_scan, &fast_shared, &mass_shared, tau);
+        if (g_sample_short_way == 3 && !have_tau) {
+            if (rank == 0 && tid == 0) out[r] = -1;
+            return;
+        }
     }
     if (!have_max) {
     // ---- arg-max of the row: this CTA's slices lie side by side
@@ -1135,9 +1139,9 @@ static int g_sample_cluster = 0;
 // CTAs per row: 0 chosen by the number of rows, else 1, 2, 4 or 8 (for tests: the result is the same).
 RV_EXPORT void rv_sample_set_cluster(int ctas_per_row) { g_sample_cluster = ctas_per_row; }
 // 1 (default): top-k / top-p rows try the short way first; 0: always the general search; 2: the short way alone, rows that it
-// does not serve get the id -1 (for tests).
+// does not serve get the id -1; 3: rows left to the general search get -1 (for tests).
 RV_EXPORT int rv_sample_set_short_way(int mode) {
-    const int v = mode == 2 ? 2 : (mode ? 1 : 0);
+    const int v = mode == 2 || mode == 3 ? mode : (mode ? 1 : 0);
     return (int)cudaMemcpyToSymbol(g_sample_short_way, &v, sizeof(int));
 }
 
