@@ -281,7 +281,7 @@ def test_mixed_head_attention_over_pages(K, dtype, H, G, d, vd, chunk, page):
                                                  (8, 8, 48, 96, 97, 16), (2, 1, 128, 128, 31, 8), (12, 6, 64, 32, 70, 16)])
 @pytest.mark.parametrize("path", ["tensor", "split", "plain"])
 def test_every_build_of_the_mixed_head_attention_gives_the_plain_result(K, H, G, d, vd, chunk, page, path):
-    """The tensor-core build (many tokens), the split-key build (few tokens behind many keys) and the plain kernel against
+    """The mma.sync build (many tokens), the split-key build (few tokens behind many keys) and the plain kernel against
     the slow implementation: portions that start and end inside tiles, chunks and pages, single tokens among them, head
     groups of 1 to 16, key and value widths that differ."""
     dtype = torch.bfloat16
@@ -293,8 +293,8 @@ def test_every_build_of_the_mixed_head_attention_gives_the_plain_result(K, H, G,
     talk = torch.eye(H, dtype=F64) + 0.4 * rnd(H, H, seed=3)
     cache, meta, positions = flat_pages(ks, vs, q_lens, page, dtype, chunk)
     q = torch.cat(qs).reshape(sum(q_lens), H * d).to(dtype).cuda()
-    old = K.TALKING_MMA, K.TALKING_SPLIT
-    K.TALKING_MMA, K.TALKING_SPLIT = path == "tensor", path == "split"
+    old = K.TALKING_MMA, K.TALKING_SPLIT, K.TALKING_WIDE
+    K.TALKING_MMA, K.TALKING_SPLIT, K.TALKING_WIDE = path == "tensor", path == "split", False
     try:
         for use_bias, use_talk in ((True, True), (False, False)):
             got = K.talking_attention(q, cache, meta, positions, H, G, d, vd, 0.3, r1.float().cuda() if use_bias else None,
@@ -308,7 +308,7 @@ def test_every_build_of_the_mixed_head_attention_gives_the_plain_result(K, H, G,
                 assert rel_err(got[at:at + n], want.reshape(n, -1)) < TOL[dtype], (i, use_bias, use_talk)
                 at += n
     finally:
-        K.TALKING_MMA, K.TALKING_SPLIT = old
+        K.TALKING_MMA, K.TALKING_SPLIT, K.TALKING_WIDE = old
 
 
 @pytest.mark.parametrize("H,G,d,vd,chunk,page", [(16, 4, 128, 128, None, 16), (8, 8, 64, 128, 97, 8), (16, 1, 128, 64, 150, 64), (4, 2, 64, 64, 40, 128),
@@ -410,6 +410,30 @@ def test_a_value_that_is_not_finite_stays_with_the_tokens_that_see_it(K, H, G, d
         w[key, n % G, 5] = float("nan")
         got = run(w, v)
         assert torch.equal(got[~sees], clean[~sees]) and bool(got[sees].isnan().all()), key
+    K.raise_on_abort()
+
+
+@pytest.mark.parametrize("H,G,d,vd,chunk", [(16, 4, 128, 128, None), (8, 8, 64, 64, 1500), (32, 8, 128, 128, None)])
+def test_mixing_behind_the_sum_over_thousands_of_keys(K, H, G, d, vd, chunk):
+    """The tcgen05 build over some forty tiles: its rings of keys and values many times around, the running maximum raised on the way (a key
+    late in the context outweighs those before it), against float64."""
+    dtype, ctx, q_len = torch.bfloat16, 2600, 70
+    k, v, q = (rnd(n, h, w, seed=i).to(dtype).double() for i, (n, h, w) in enumerate(((ctx, G, d), (ctx, G, vd), (q_len, H, d))))
+    for key, size in ((900, 0.5), (1700, 0.7), (2400, 0.9)):       # along every query of the group's first head
+        k[key] = (q[35].view(G, H // G, d)[:, 0] * size).to(dtype).double()
+    r1, r2 = (torch.rand(H, generator=torch.Generator().manual_seed(i)).double() for i in (1, 2))
+    talk = torch.eye(H, dtype=F64) + 0.4 * rnd(H, H, seed=3)
+    cache, meta, positions = flat_pages([k], [v], [q_len], 16, dtype, chunk)
+    got = K.talking_attention(q.reshape(q_len, H * d).to(dtype).cuda(), cache, meta, positions, H, G, d, vd, 0.25, r1.float().cuda(), r2.float().cuda(),
+                              talk.float().cuda(), chunk)
+    # (the same as the slow implementation, for the portion's queries alone)
+    at = torch.arange(ctx - q_len, ctx, dtype=F64)
+    dist = at[:, None] - torch.arange(ctx, dtype=F64)[None]
+    hidden = (dist < 0) | (torch.arange(ctx)[None] < ((at // chunk) * chunk)[:, None] if chunk else dist < 0)
+    s = torch.einsum("thd,jhd->htj", q, k.repeat_interleave(H // G, 1)) * 0.25 - r1[:, None, None] * torch.log1p(r2[:, None, None] * dist.clamp(min=0))
+    w = torch.einsum("hg,gtj->htj", talk, torch.softmax(s.masked_fill(hidden[None], float("-inf")), -1))
+    want = torch.einsum("htj,jhd->thd", w, v.repeat_interleave(H // G, 1)).reshape(q_len, -1)
+    assert rel_err(got, want) < TOL[dtype]
     K.raise_on_abort()
 
 
