@@ -81,6 +81,9 @@ struct WideSizes {
     static constexpr int SMEM = Q_BYTES + NK * K_BYTES + NV * V_BYTES + 256 + SOFTMAX_WARPS * BIAS_FLOATS * 4;
 };
 
+template <int W> struct WideVec { using type = float4; };
+template <> struct WideVec<2> { using type = float2; };
+
 __device__ __forceinline__ float fast_log2(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -467,16 +470,50 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         __syncthreads();
     }
-    if (left_out != 0 && abort_flag == 0 && warp < SOFTMAX_WARPS) {      // (a thread has its row of the walk)
-        const int row_l = warp * 32 + lane, tok_i = row_l / G, pos = pos_first + tok_i, t = q_start + tok0 + tok_i;
-        if (tok_i < n_tok && t >= p.tok_lo && t < p.tok_hi) {
-            float* dst = p.u + (((size_t)(t - p.tok_lo) * p.nkv + c0) * p.nh + kvh * G + row_l - tok_i * G) * VD;
-            for (int j = p.chunk > 0 ? (pos / p.chunk) * p.chunk : 0; j <= pos; ++j) {
-                if (!partly_seen(j / KV_TILE)) continue;
-                const __nv_bfloat16* v = p.values + (size_t)table[j >> p.page_shift] * p.page_elems + ((size_t)c0 * p.page_size + (j & (p.page_size - 1))) * VD;
-                for (int e = 0; e < nv * VD; ++e) {
-                    const float x = __bfloat162float(v[(size_t)(e / VD) * p.page_size * VD + e % VD]);
-                    if (!(fabsf(x) < INFINITY)) dst[(size_t)(e / VD) * p.nh * VD + e % VD] += x;
+    if (left_out != 0 && abort_flag == 0 && warp < SOFTMAX_WARPS) {
+        // A warp has the tokens of its rows, a lane some columns of each head: one walk over the keys of those tiles, whose sum up to a
+        // token's own key is what its rows are due.
+        constexpr int W = VD / 32;
+        using Vec = typename WideVec<W>::type;
+        const int first = pos_first + warp * 32 / G, last = pos_first + min(n_tok, (warp + 1) * 32 / G) - 1;
+        const int skip_lo = (lo_last + KV_TILE - 1) / KV_TILE * KV_TILE, skip_hi = (pos_first + 1) / KV_TILE * KV_TILE;      // between: seen by all
+        for (int c = 0; c < nv; ++c) {
+            float sum[W] = {};
+            int j = p.chunk > 0 ? (first / p.chunk) * p.chunk : 0;
+            auto take = [&](int end) {
+#pragma unroll 8
+                for (; j < end; ++j) {
+                    const __nv_bfloat16* v = p.values + (size_t)__ldg(table + (j >> p.page_shift)) * p.page_elems +
+                                             ((size_t)(c0 + c) * p.page_size + (j & (p.page_size - 1))) * VD + lane * W;
+#pragma unroll
+                    for (int w = 0; w < W; w += 2) {
+                        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(v + w));
+                        if (!(fabsf(x.x) < INFINITY)) sum[w] += x.x;
+                        if (!(fabsf(x.y) < INFINITY)) sum[w + 1] += x.y;
+                    }
+                }
+            };
+            for (int pos = first; pos <= last; ++pos) {
+                if (p.chunk > 0 && pos % p.chunk == 0) {     // a chunk begins here
+#pragma unroll
+                    for (int w = 0; w < W; ++w) sum[w] = 0.f;
+                    j = pos;
+                }
+                take(min(pos + 1, skip_lo));
+                if (j >= skip_lo) j = max(j, skip_hi);
+                take(pos + 1);
+                const int t = q_start + tok0 + pos - pos_first;
+                bool due = false;
+#pragma unroll
+                for (int w = 0; w < W; ++w) due |= sum[w] != 0.f;                // (also where it is no number)
+                if (!due || t < p.tok_lo || t >= p.tok_hi) continue;
+                float* dst = p.u + (((size_t)(t - p.tok_lo) * p.nkv + c0 + c) * p.nh + kvh * G) * VD + lane * W;
+#pragma unroll
+                for (int h = 0; h < G; ++h) {
+                    Vec x = *reinterpret_cast<const Vec*>(dst + h * VD);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) reinterpret_cast<float*>(&x)[w] += sum[w];
+                    *reinterpret_cast<Vec*>(dst + h * VD) = x;
                 }
             }
         }
