@@ -15,10 +15,12 @@
 //
 // Rows with a top-k or a top-p take two passes over the row (maximum + counts per bin of the top 12 bits of
 // the ordered bit pattern, then the tokens from a bin upwards and the whole mass); the at most
-// 2,048 candidates are sorted and cut exactly in the first CTA's shared memory.  Rows whose candidates
-// do not fit (a flat distribution under top-p alone, a k beyond 2,048) take the general search: eight
-// passes of four bits over the row.  All sums that decide anything are integers or are added in a fixed
-// order, so a token depends neither on the run nor on how many CTAs share the row.
+// 2,048 candidates are sorted and cut exactly in the first CTA's shared memory.  Rows under a top-p alone whose cut
+// lies below their 2,048 most likely tokens take three passes over the masses (`sample_mass_way`).  The general search, eight
+// passes of four bits over the row, is left with: rows under a top-k with fewer than k tokens that are numbers, or
+// more than 2,048 tokens down to the end of the k-th one's bin (k beyond 2,048, or a flat row); under a top-p alone, rows whose maximum is
+// infinite, a share above 2 M tokens a CTA, a top-p that no fixed-point mass is small enough for.  All sums that decide anything are integers or
+// are added in a fixed order, so a token depends neither on the run nor on how many CTAs share the row.
 #include "common.cuh"
 #include <string.h>
 
@@ -153,8 +155,8 @@ __device__ void slices_scan(const float* row, int V, int S, int first, int per, 
 // candidate.  If there are at most FAST_CANDIDATES of them (a peaked distribution, or a small k), they are gathered
 // - ordered bit pattern and index, in any order - in the first CTA's shared memory, where they are sorted (bitonic, by
 // value then index: a total order, so the result is the same whatever order they arrived in), cut exactly by count and by
-// cumulated mass, sorted back into vocabulary order and drawn from.  Otherwise (a flat distribution under
-// top-p alone, a huge k) the kernel goes on with the general search below.
+// cumulated mass, sorted back into vocabulary order and drawn from.  Otherwise the kernel goes on below: a flat row under
+// top-p alone by its masses, any other by the general search.
 #define FAST_BINS 4096
 #define FAST_CANDIDATES 2048
 #define FAST_SCALE 1099511627776.0f      // 2^40
@@ -676,7 +678,7 @@ __device__ bool sample_short_way(const float* __restrict__ row, int V, float inv
 // first CTA; a group of more than FAST_CANDIDATES tokens is divided again, by key; the tokens of the last group are gathered, sorted and
 // cut.  Every thread adds in places of its own (16 sums of 64 bits, the count above the mass), so nothing is atomic and the sums
 // are exact.  Three passes over the row in place of the search's eight: a step of 64 rows
-// of 128,256 tokens with one such row 212 -> 117 us, 36 without.
+// of 128,256 tokens with one such row 212 -> 101 us, 36 without.
 #define MASS_GROUPS 16
 #define MASS_BITS 52                       // of a thread's sum: 4,096 masses of 2^40; the count above
 struct MassShared {

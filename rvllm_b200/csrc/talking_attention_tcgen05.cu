@@ -20,13 +20,13 @@
 // alone is 1.6e-3 and the kernel that mixes inside the walk (talking_attention_mma.cu: mixed weights rounded once) has 2.3e-3 to
 // 2.4e-3.  With one bfloat16 number a weight it was 2.0e-3 to 2.4e-3 for the first two, 6e-3 to 3.5e-1 for the differences.
 //
-// Against the kernel that mixes inside the walk (heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 475 -> 155 us,
-// 80 tokens 31 -> 19, 100 tokens behind 3,990 keys 960 -> 106; 32 heads on 8, 2,048 tokens 975 -> 475, 100 behind 3,990 1,329 -> 185.  (One
-// number a weight: 118, 19, 97; 392, 114.  The softmax warps, one a scheduler, bind the walk: forming the low parts and storing them cost
-// more than the second products.)
+// Against the kernel that mixes inside the walk (heads of 128, L2 flushed): 16 heads on 4, 2,048 tokens 475 -> 160 us,
+// 80 tokens 31 -> 21, 100 tokens behind 3,990 keys 960 -> 110 to 160; 32 heads on 8, 2,048 tokens 975 -> 490, 100 behind 3,990 1,329 -> 185.  (One
+// number a weight and no look at the values: 118, 19, 97; 392, 114.  The softmax warps, one a scheduler, bind the walk: forming the rests and
+// storing them takes 25 us of 2,048 tokens of 16 heads, the second products 12, the look at the values 5.)
 //
 // The distance bias r1 ln(1 + r2 d) takes a logarithm per (head, distance), not per score: a warp's 32 rows are few tokens, so
-// a tile of 64 keys meets only 63 + tokens distances, whose biases the warp forms in shared memory a tile ahead.
+// a tile of 64 keys meets only 63 + tokens distances, whose biases the warp forms in shared memory while the tile's Q K^T runs.
 #include "common.cuh"
 #include "tcgen05_attention.cuh"
 
@@ -406,7 +406,7 @@ talking_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             float l_tile = 0.f, l_tile2 = 0.f;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {           // 32 keys: 16 columns of their roundings, 16 of the rests (a store of each
-                const uint32_t* s = half ? s1 : s0;          // half as it is done: 100 tokens behind 3,990 keys 159 -> 106 us)
+                const uint32_t* s = half ? s1 : s0;          // half as it is done: 2,048 tokens of 16 heads on 4 163 -> 153 us, of 32 on 8 490 -> 472)
                 uint32_t pk[32];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {               // keys 2j and 2j + 1
